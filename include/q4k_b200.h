@@ -72,6 +72,7 @@ typedef struct q4k_q8_input {
 #define Q4K_KERNEL_TCGEN05 3   /* m >= 32: tcgen05 kind::i8, TMEM accumulators */
 #define Q4K_KERNEL_GEMV_MMA 4  /* m <= 16: warp-level int8 mma, split-K inside a block cluster */
 #define Q4K_KERNEL_GEMV_TMA 5  /* m <= 16: weights streamed by TMA, activations held in registers */
+#define Q4K_KERNEL_F16 6       /* any m  : tcgen05 kind::f16 on SM pairs, activations as two fp16 planes; no partials */
 
 typedef struct q4k_project_options {
   uint32_t kernel;       /* Q4K_KERNEL_* */

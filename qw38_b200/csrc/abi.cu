@@ -20,6 +20,7 @@
 
 #include "../../include/q4k_b200.h"
 #include "launch.h"
+#include "stream_scratch.h"
 
 namespace {
 
@@ -220,6 +221,18 @@ int caller_scratch(const q4k_project_options* opt, uint64_t partial_bytes, uint6
 
 constexpr uint32_t kFlagTrustedSpans = 1u, kFlagInputSettled = 2u;
 
+// The fp16-plane kernel with scratch of its own (stream_scratch.cu).
+int project_f16(const q4k_weight& w, const q4k_q8_input& x, const q4k::TcOutput& out, cudaStream_t stream) {
+  int* const status = q4k::kernel_status_word();
+  if (!status) return Q4K_ERR_STATUS;
+  q4k::F16Plan const plan = q4k::plan_f16(x.m, w.n, w.padded_k / 256);
+  q4k::StreamScratch scratch;
+  Q4K_CUDA(scratch.acquire(stream, q4k::f16_scratch_bytes(x.m, w.padded_k / 256, plan)), "scratch.acquire");
+  Q4K_CUDA(q4k::launch_mmq_f16(view(w), view(x), out, plan, scratch.p(), status, stream), "q4k_q8.mmq_f16");
+  Q4K_CUDA(scratch.release(), "scratch.release");
+  return Q4K_OK;
+}
+
 int project_impl(const q4k_weight* weight, const q4k_q8_input& x, float* output, uint64_t output_len,
                  const float* residual, uint64_t residual_len, const q4k_project_options* opt,
                  cudaStream_t stream, bool residual_in_place = false, char const* role = "projection") {
@@ -257,6 +270,7 @@ int project_impl(const q4k_weight* weight, const q4k_q8_input& x, float* output,
     if (tma_ok && (x.m >= 2 || q4k::launch_overlap())) kernel = Q4K_KERNEL_GEMV_TMA;
     else if (x.m <= 2 || (x.m <= q4k::kGemvDp4aMaxTokens && w.padded_n >= 32768)) kernel = Q4K_KERNEL_GEMV_DP4A;
     else if (x.m <= 16) kernel = Q4K_KERNEL_GEMV_MMA;
+    else if (!partials && !(opt && opt->split_k) && q4k::f16_supported(view(w), view(x))) kernel = Q4K_KERNEL_F16;
     else kernel = q4k::tcgen05_supported(view(w), view(x)) ? Q4K_KERNEL_TCGEN05 : Q4K_KERNEL_MMA;
   }
   const float* res = residual_len ? residual : nullptr;
@@ -295,6 +309,11 @@ int project_impl(const q4k_weight* weight, const q4k_q8_input& x, float* output,
                                   status, stream),
              "q4k_q8.gemv_tma");
     return Q4K_OK;
+  }
+  if (kernel == Q4K_KERNEL_F16) {
+    if (!q4k::f16_supported(view(w), view(x)) || partials)
+      return fail(Q4K_ERR_INVALID_ARGUMENT, "q8.project: the fp16 kernel needs aligned operands and has no partial dots");
+    return project_f16(w, x, q4k::tc_output(output, res), stream);
   }
   if (kernel == Q4K_KERNEL_TCGEN05) {
     if (!q4k::tcgen05_supported(view(w), view(x)))

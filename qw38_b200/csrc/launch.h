@@ -87,6 +87,21 @@ TcPlan plan_tcgen05(uint32_t m, uint32_t n, uint32_t tiles_k, uint32_t split_k_r
 cudaError_t launch_mmq_tcgen05(const WeightView& w, const Q8View& x, const TcOutput& out, int32_t* partials,
                                const TcPlan& plan, void* partial_tiles, uint32_t* tickets, int* status, cudaStream_t stream);
 
+// mmq_f16.cu : tcgen05 kind::f16 on SM pairs, weights expanded into TMEM, activations as two fp16 planes.  scratch holds
+// f16_scratch_bytes (256-byte aligned) and is used until the launch ends.
+struct F16Plan {
+  uint32_t nt;             // tokens per tile: 16, 32, 64 or 128
+  uint32_t chunk;          // tokens per pass
+  uint32_t workers;        // clusters of two SMs
+  uint32_t unit_step;      // granularity of a cluster's run of super-blocks: 1, or tiles_k = whole tiles
+  uint32_t slot_clusters;  // clusters for whose partial tiles the scratch has room
+};
+bool f16_supported(const WeightView& w, const Q8View& x);
+F16Plan plan_f16(uint32_t m, uint32_t n, uint32_t tiles_k);
+uint64_t f16_scratch_bytes(uint32_t m, uint32_t tiles_k, const F16Plan& plan);
+cudaError_t launch_mmq_f16(const WeightView& w, const Q8View& x, const TcOutput& out, const F16Plan& plan, void* scratch, int* status,
+                           cudaStream_t stream);
+
 // gemv_tma.cu : m <= 16.  Weights streamed by TMA into a shared-memory ring, activations held in
 // registers by warps that each own one super-block column of the block's K slice; K slices of
 // different blocks are added in slice order through `slices` ([split_k][m][n] floats) by the last

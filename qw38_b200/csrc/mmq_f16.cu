@@ -1,0 +1,877 @@
+// Q4_K x Q8 matmul for more than sixteen tokens: tcgen05.mma kind::f16 on pairs of SMs, weights expanded straight
+// into tensor memory, accumulators drained once per super-block of 256 columns.
+//
+// The equation is  out[t][n] = sum_kb ( d[n,kb] * sum_{k in kb} (sc*q)[n,k] * (a*z)[t,k]
+//                                       - dmin[n,kb] * sum_{g in kb} m[n,g] * (a*s)[t,g] ).
+// Scaling one partial per 32 columns on the CUDA cores (what the int8 kernel in mmq_tcgen05.cu does) costs two FMAs and
+// one TMEM word per 32 multiply-adds and bounds that kernel far below the tensor pipe.  Here both group factors go into
+// the operands, where they are exact or as good as fp32, and only the super-block scale is left for the epilogue:
+//   * weight side: sc*q is an integer <= 63 * 15 = 945, exact in fp16 (11 bits).  A nibble becomes fp16 by or-ing it under
+//     the exponent of 1024; one HFMA2 turns (1024 + q) into sc * q exactly (-1024 * sc is the addend).
+//   * token side: a*z is written by a small kernel in front as two fp16 planes, hi = fp16(x), lo = fp16(x - hi), which
+//     carry 23 bits -- what an fp32 product of a and z carries, less at most one bit.  A power of two per token (and one of
+//     its own for a super-block far below the token's largest scale), applied exactly in the epilogue, keeps |x| < 65504
+//     whatever the scales are.
+//   * the products (at most 21 bits) are exact and the tensor core accumulates them in fp32; per accumulator only the 16
+//     steps of one super-block are added before it is drained and folded into fp32 registers.
+//   * min term: m is exact in fp16, a*s is split into two fp16 terms like x, and one more MMA of K = 16 (eight groups, hi
+//     and lo) per super-block adds their products into an accumulator of its own.
+// Error against the equation in double precision: 1.8e-7 to 2.2e-7 of the result's norm at K = 256 .. 17408 (the int8 kernel:
+// 0.7e-7 to 2.3e-7).
+//
+// Rates that the design rests on (measured, clk per SM): tcgen05.mma with A in TMEM takes max(17, N/2) + 4 per K16 step
+// (45 at N = 16 when A comes from shared memory), the paired form the same; tcgen05.st 32x32b of 32 lanes x 16 words 17 with
+// four warps storing, a pair of tcgen05.ld of that shape 48 with eight warps reading.  So a super-block of 128 rows x 64
+// tokens costs 32 * 39 clk of tensor time, of 128 tokens 32 * 71; the expansion (1800 warp instructions) and the epilogue
+// (~100 per warp) run beside it.  Two SMs share a tile (cta_group::2: 256 rows, each SM holds the operand rows of half of
+// N), because one SM alone would have to take in 60 bytes per clock of activation planes next to the weights, and L2
+// delivers about 10 TB/s to all of them.
+//
+// Measured on 17408 x 5120: 2048 tokens 0.59 ms (620 TOP/s; the int8 kernel 1.20 ms), tensor pipe 72 % active with the
+// clock at the power limit; 64 tokens x 34816 rows 49 us (95 us), of which about 10 us are launch, prologue and tile end.
+// Bound: at prefill sizes tensor pipe and power, below 64 tokens the hand-offs between the roles (barrier to barrier a
+// super-block takes ~1.4x its tensor time).  Tried and slower: a back-off in the waits (nanosleep 16 .. 128: 1.5 - 2x), a
+// suspend hint, a four-instruction retry loop (1.5x: the retries queue up in front of the arrivals), one polling lane or
+// one polling warp per role, arrivals with cluster-scope release (a memory barrier each: 1.4x), the min term on mma.sync
+// (queues behind the tcgen05 MMAs: 1.16x).
+//
+// Work is a list of (row pair, token tile, super-block) units in that order.  Each cluster takes one contiguous run of
+// units; tiles cut by a run's ends go through fp32 scratch and are added in run order by whoever arrives last.  When
+// whole tiles per cluster are about as quick, runs are cut at tile boundaries instead (plan_f16).
+//
+// Warps: 0 raw weights (TMA), 1 activation planes (TMA), 2 MMA issue (leader CTA), 3 TMEM allocation and launch overlap,
+// then expanders, then epilogue.  Every wait is bounded; a wait that gives up sets the abort flag and the status word, and
+// every role leaves its loop.
+#include <cuda.h>
+#include <cuda_fp16.h>
+
+#include "common.cuh"
+#include "launch.h"
+#include "tma.cuh"
+#include "umma.cuh"
+
+namespace q4k {
+namespace {
+
+constexpr int kRows = 128;  // weight rows per CTA; a pair covers 256
+constexpr int kExpanders = 8, kFirstExpander = 4;  // expander warps that share a super-block; the first of them
+
+template <int NT> struct F16Cfg {
+  // Up to 32 tokens the hi and lo planes lie side by side along N (an MMA of N = 32 costs nearly as much as one of 64);
+  // from 64 on they share the accumulator, all lo products of a super-block before the hi ones: the tensor core truncates
+  // when it accumulates, and so only the sixteen hi steps do so at full magnitude.
+  static constexpr bool kStack = NT <= 32;
+  static constexpr int kN = kStack ? 2 * NT : NT;       // MMA width = accumulator columns
+  static constexpr int kN2 = NT < 32 ? 32 : NT;         // min-term accumulator columns
+  static constexpr int kColSplit = NT >= 128 ? 4 : (NT >= 32 ? 2 : 1);
+  static constexpr int kCols = NT / kColSplit;          // tokens per epilogue warp (lane = row)
+  static constexpr int kEpilogueWarps = 4 * kColSplit;
+  // Up to 64 tokens two groups of expanders take alternate super-blocks: one group needs ~1200 clk for one, a
+  // super-block of 64 tokens 1112 clk of tensor time and 790 clk of HBM time.
+  static constexpr int kGroups = NT >= 128 ? 1 : 2;
+  static constexpr int kFirstEpilogue = kFirstExpander + kGroups * kExpanders;
+  static constexpr int kWarps = kFirstEpilogue + kEpilogueWarps, kThreads = kWarps * 32;
+  // The block starts with kLaunchRegs registers per thread; control, expander and epilogue warps redistribute them.
+  static constexpr int kLaunchRegs = 65536 / kThreads / 8 * 8;
+  static constexpr int kRegsControl = 40, kRegsExpander = 56;
+  static constexpr int kRegsLeft = (kWarps * kLaunchRegs - 4 * kRegsControl - kGroups * kExpanders * kRegsExpander) / kEpilogueWarps / 8 * 8;
+  static constexpr int kRegsEpilogue = kRegsLeft > 160 ? 160 : kRegsLeft;
+  // TMEM: two accumulators, one min-term accumulator, weight stages.  A group of expanders always uses the same kQ stages
+  // (one super-block), so that a warp sees every phase of the barriers it waits on.
+  static constexpr int kQ = kStack ? 2 : 4, kACols = 128 / kQ, kAStages = kGroups * kQ;
+  static constexpr int kD2Col = 2 * kN, kACol = kD2Col + kN2;
+  static_assert(kACol + kAStages * kACols <= 512, "TMEM columns");
+  // operand stage: plane boxes, then a*s of kTRows tokens as a K-major operand without swizzle ([hi | lo][row][16 bytes])
+  static constexpr int kBRows = kStack ? NT : NT / 2;   // plane rows per box and CTA
+  static constexpr int kBBox = 4 * kBRows * 128;        // 256 columns
+  static constexpr int kPlanes = kStack ? kBBox : 2 * kBBox;  // NT = 128: lo box, then hi box
+  static constexpr int kTRows = kN2 / 2;
+  static constexpr int kBTx = kPlanes + kTRows * 32, kB = (kBTx + 1023) / 1024 * 1024;
+  static constexpr int kRaw = 16 * 1024 + 16 * 128;
+  static constexpr int kBStages = NT >= 128 ? 2 : (NT >= 64 ? 3 : 4);  // any number: one producer, one consumer
+  static constexpr int kRawStages = NT >= 128 ? 3 : 6, kSclStages = NT >= 128 ? 3 : 4;
+  static_assert(kRawStages % kGroups == 0 && kSclStages % kGroups == 0, "a stage belongs to one group of expanders");
+  static constexpr int kMins = kRows * 16;              // six-bit mins as fp16, one buffer per group
+  static constexpr int oE = kRows * 8, kScl = oE + NT * 4;  // scale stage: {d, -32 dmin} [row] | 2^e [token]
+  static constexpr int oB = 0, oRaw = oB + kBStages * kB, oMins = oRaw + kRawStages * kRaw, oScl = oMins + kGroups * kMins,
+                       oCtrl = oScl + kSclStages * kScl;
+  static constexpr int kBars = 2 * kRawStages + 2 * kBStages + 2 * kAStages + 4 + 2 * kSclStages;
+  static constexpr int kSmem = oCtrl + kBars * 8 + 32 + 1024;
+  static_assert(kSmem <= 227 * 1024, "shared memory budget");
+  static_assert(kRaw % 1024 == 0 && kScl % 64 == 0, "swizzled tiles need 1024-byte alignment");
+};
+
+struct F16Params {
+  const float* residual;
+  float* out[8];
+  uint16_t* out_bf16;
+  uint32_t* peer_flag[8];
+  uint32_t* done;
+  uint32_t* unsignalled;
+  uint32_t ndst, rank, out_stride, out_row0;
+  const float* exps;       // power of two of (super-block, token) relative to the token's: [kb][m_pad], 1 but for outliers
+  const float* tokens;     // power of two of the token [m_pad]
+  float* slots;            // partial tiles: [cluster][2][CTA][epilogue warp][value / 4][lane] float4
+  uint32_t* tickets;       // [cluster][CTA][epilogue warp]
+  int* status;
+  uint32_t n, m, m_pad, tiles_k, tok_tiles;
+  // Cluster w takes units [first(w), first(w + 1)): run_each steps of unit_step units, the first run_rest clusters one more.
+  uint32_t run_each, run_rest, unit_step;
+};
+
+// Accumulator columns of a token tile: its tokens rounded up to what one MMA takes (N is a multiple of 32), so that a last
+// tile of few tokens does not pay for a full one.
+template <int NT> __device__ __forceinline__ uint32_t tile_cols(const F16Params& p, uint32_t tok) {
+  uint32_t const left = p.m - tok * NT;
+  constexpr uint32_t unit = F16Cfg<NT>::kStack ? 16 : 32;
+  return left >= NT ? NT : (left + unit - 1) / unit * unit;
+}
+
+__device__ __forceinline__ uint32_t first_unit(const F16Params& p, uint32_t w) {
+  return (w * p.run_each + min(w, p.run_rest)) * p.unit_step;
+}
+
+// Position in a cluster's run of units, and in a ring of N stages (phase = parity of the stage's current use; a producer
+// waits for the opposite parity, which a fresh barrier satisfies).
+struct Cursor {
+  uint32_t row_pair, tok, kb;
+  __device__ __forceinline__ Cursor(const F16Params& p, uint32_t u) {
+    uint32_t const tile = u / p.tiles_k;
+    kb = u - tile * p.tiles_k;
+    row_pair = tile / p.tok_tiles;
+    tok = tile - row_pair * p.tok_tiles;
+  }
+  __device__ __forceinline__ void next(const F16Params& p) {
+    if (++kb == p.tiles_k) {
+      kb = 0;
+      if (++tok == p.tok_tiles) { tok = 0; ++row_pair; }
+    }
+  }
+};
+template <int N> struct Ring {
+  uint32_t s = 0, phase = 0;
+  __device__ __forceinline__ void next() {
+    if (++s == N) { s = 0; phase ^= 1; }
+  }
+};
+
+// ---- PTX of the paired form ------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ uint32_t map_to(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void arrive_cluster(uint32_t cluster_addr) {
+  // Relaxed: what it announces are TMEM accesses, ordered by tcgen05.fence; a release at cluster scope costs a memory
+  // barrier of several hundred clocks per arrival.
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Execution only: no wait for the block's outstanding stores.
+__device__ __forceinline__ void cluster_meet() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
+}
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{ .reg .pred q; elect.sync _|q, 0xffffffff; selp.u32 %0, 1, 0, q; }" : "=r"(p));
+  return p != 0;
+}
+// Box of the activation planes into this CTA's shared memory; the bytes are counted on a barrier of the leader.
+__device__ __forceinline__ void tma_3d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t leader_bar) {
+  asm volatile("cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+               ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(leader_bar) : "memory");
+}
+__device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+// D (256 rows x n, 128 per CTA) = A (TMEM of both CTAs) * B (shared memory of both) (+ D).
+template <bool Acc> __device__ __forceinline__ void mma_pair(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc) {
+  if constexpr (Acc)
+    asm volatile("{ .reg .pred p; setp.eq.b32 p, 0, 0;\n tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p; }"
+                 ::"r"(d), "r"(a), "l"(b), "r"(idesc) : "memory");
+  else
+    asm volatile("{ .reg .pred p; setp.ne.b32 p, 0, 0;\n tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p; }"
+                 ::"r"(d), "r"(a), "l"(b), "r"(idesc) : "memory");
+}
+// The same with A in shared memory; overwrites D.
+__device__ __forceinline__ void mma_pair_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc) {
+  asm volatile("{ .reg .pred p; setp.ne.b32 p, 0, 0;\n tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p; }"
+               ::"r"(d), "l"(a), "l"(b), "r"(idesc) : "memory");
+}
+// One arrival on the barrier at this offset of both CTAs when every MMA issued so far has completed.
+__device__ __forceinline__ void commit_pair(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(bar), "h"(uint16_t(3)) : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t t, const uint32_t (&r)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+               ::"r"(t), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+                 "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+__device__ __forceinline__ float lds32f(uint32_t a) { return __uint_as_float(lds32(a)); }
+__device__ __forceinline__ float ldg_here(const float* a) {  // not to be hoisted (sixty-four of them would spill)
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(a));
+  return v;
+}
+__device__ __forceinline__ uint32_t round32(uint32_t v) { return (v + 31) / 32 * 32; }
+__device__ __forceinline__ uint32_t f16_idesc(uint32_t n) { return (1u << 4) | ((n >> 3) << 17) | (uint32_t(256 >> 4) << 24); }  // f16 -> f32, M = 256
+__device__ __forceinline__ float2 as_float2(const uint32_t* r) { return make_float2(__uint_as_float(r[0]), __uint_as_float(r[1])); }
+// (w & mask) | magic in one instruction: only one operand of LOP3 may be a constant, so the caller keeps both in registers.
+__device__ __forceinline__ uint32_t and_or(uint32_t w, uint32_t mask, uint32_t magic) {
+  uint32_t r;
+  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(w), "r"(mask), "r"(magic));
+  return r;
+}
+__device__ __forceinline__ uint32_t opaque(uint32_t v) {  // a constant that stays in its register
+  asm volatile("mov.u32 %0, %0;" : "+r"(v));
+  return v;
+}
+__device__ __forceinline__ uint32_t h2u(__half2 v) { return *reinterpret_cast<uint32_t*>(&v); }
+__device__ __forceinline__ __half2 u2h(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
+// ---- activation planes -----------------------------------------------------------------------------
+// Column order inside eight columns as the expanders' nibble words produce them: pairs (0,4) (1,5) (2,6) (3,7).
+// A block takes eight super-blocks of one token, a warp one of them, lane l columns 8l..8l+7.  Rows m..m_pad are zeros.
+//
+// Powers of two: the token's own, T = 2^E with its largest scale a / T in [256, 512), goes into tokens[] and is applied
+// once at the end of a tile.  A super-block whose largest scale is more than 2^12 below the token's would start to lose
+// bits in fp16 and takes its own power; exps[] holds the quotient of the two, 1 for all others.
+__device__ __forceinline__ int scale_exponent(float top) {  // clamped so that 2^E and 2^-E are normal numbers
+  return min(max(int((__float_as_uint(top) >> 23) & 255u) - 127 - 8, -118), 118);
+}
+__device__ __forceinline__ float power_of_two(int e) { return __uint_as_float(uint32_t(127 + e) << 23); }
+
+__global__ void __launch_bounds__(256) planes_kernel(const int8_t* __restrict__ codes, const float* __restrict__ scales,
+                                                     const int32_t* __restrict__ sums, uint32_t m, uint32_t m_pad, uint32_t tiles_k,
+                                                     __half* __restrict__ planes, __half* __restrict__ sums16, float* __restrict__ exps,
+                                                     float* __restrict__ tokens, uint32_t* __restrict__ tickets, uint32_t ticket_count) {
+  __shared__ float warp_top[8];
+  pdl_wait();
+  pdl_launch_dependents();
+  if (blockIdx.x == 0)
+    for (uint32_t i = threadIdx.x; i < ticket_count; i += 256) tickets[i] = 0u;
+  uint32_t const warp = threadIdx.x >> 5, lane = threadIdx.x & 31, pk = tiles_k * 256, G = tiles_k * 8;
+  uint32_t const chunks = (tiles_k + 7) / 8, tok = blockIdx.x / chunks, kb = blockIdx.x % chunks * 8 + warp;
+  bool const real = tok < m, live = kb < tiles_k;
+  // this lane's share of the conversion is requested before the block meets
+  float a = 0.f;
+  int sum = 0;
+  uint2 z = make_uint2(0u, 0u);
+  if (real && live) {
+    z = *reinterpret_cast<const uint2*>(codes + uint64_t(tok) * pk + kb * 256 + lane * 8);
+    uint64_t const g = uint64_t(tok) * G + kb * 8 + (lane >> 2);
+    a = scales[g];
+    sum = sums[g];
+  }
+  float row = 0.f;
+  if (real)
+    for (uint32_t i = threadIdx.x; i < G; i += 256) row = fmaxf(row, fabsf(scales[uint64_t(tok) * G + i]));
+#pragma unroll
+  for (int off = 16; off; off >>= 1) row = fmaxf(row, __shfl_xor_sync(0xffffffffu, row, off));
+  if (lane == 0) warp_top[warp] = row;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) row = fmaxf(row, warp_top[i]);
+  if (!live) return;
+  float top = fabsf(a);
+#pragma unroll
+  for (int off = 4; off < 32; off <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
+  int const e_row = scale_exponent(row), e_own = scale_exponent(top);
+  int const e = top == 0.f || e_own >= e_row - 12 ? e_row : e_own;
+  a *= power_of_two(-e);
+  float const as = a * float(sum) * 0.03125f;  // |sum| <= 32 * 127
+  uint32_t hi[4], lo[4];
+  uint32_t const zw[2] = {z.x, z.y};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {  // columns i and i + 4
+    float const x0 = a * float(int(zw[0] << (24 - 8 * i)) >> 24), x1 = a * float(int(zw[1] << (24 - 8 * i)) >> 24);
+    __half2 const h = __floats2half2_rn(x0, x1);
+    hi[i] = h2u(h);
+    lo[i] = h2u(__floats2half2_rn(x0 - __low2float(h), x1 - __high2float(h)));
+  }
+  __half* const dst = planes + uint64_t(tok) * pk + kb * 256 + lane * 8;
+  *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+  *reinterpret_cast<uint4*>(dst + uint64_t(m_pad) * pk) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+  if ((lane & 3) == 0) {  // a * s: [kb][hi | lo][token][group]
+    __half const h = __float2half_rn(as);
+    __half* const t = sums16 + ((uint64_t(kb) * 2) * m_pad + tok) * 8 + (lane >> 2);
+    t[0] = h;
+    t[uint64_t(m_pad) * 8] = __float2half_rn(as - __half2float(h));
+  }
+  if (lane == 0) {
+    exps[uint64_t(kb) * m_pad + tok] = e == e_row || e - e_row < -126 ? (e == e_row ? 1.f : 0.f) : power_of_two(e - e_row);
+    if (kb == 0) tokens[tok] = power_of_two(e_row);
+  }
+}
+
+// ---- the matmul ------------------------------------------------------------------------------------
+template <int NT>
+__global__ void __launch_bounds__(F16Cfg<NT>::kThreads, 1)
+mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_constant__ CUtensorMap tm_meta,
+               const __grid_constant__ CUtensorMap tm_planes, const __grid_constant__ CUtensorMap tm_sums, const F16Params p) {
+  using C = F16Cfg<NT>;
+  extern __shared__ uint8_t smem_raw[];
+  uint32_t const smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* const smem_g = smem_raw + (smem - smem_u32(smem_raw));
+  uint32_t const warp = threadIdx.x >> 5, lane = threadIdx.x & 31, cta = cluster_rank();
+  uint32_t const bar0 = smem + C::oCtrl;
+  auto raw_full = [&](uint32_t i) { return bar0 + 8 * i; };
+  auto raw_free = [&](uint32_t i) { return bar0 + 8 * (C::kRawStages + i); };
+  constexpr int oBb = 2 * C::kRawStages;
+  auto b_full = [&](uint32_t i) { return bar0 + 8 * (oBb + i); };                 // leader's is used
+  auto b_free = [&](uint32_t i) { return bar0 + 8 * (oBb + C::kBStages + i); };
+  constexpr int oAb = oBb + 2 * C::kBStages;
+  auto a_full = [&](uint32_t i) { return bar0 + 8 * (oAb + i); };                 // leader's is used
+  auto a_free = [&](uint32_t i) { return bar0 + 8 * (oAb + C::kAStages + i); };
+  constexpr int oDb = oAb + 2 * C::kAStages;
+  auto d_full = [&](uint32_t i) { return bar0 + 8 * (oDb + i); };
+  auto d_free = [&](uint32_t i) { return bar0 + 8 * (oDb + 2 + i); };             // leader's is used
+  constexpr int oSb = oDb + 4;
+  auto s_full = [&](uint32_t i) { return bar0 + 8 * (oSb + i); };
+  auto s_free = [&](uint32_t i) { return bar0 + 8 * (oSb + C::kSclStages + i); };
+  uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(smem_g + C::oCtrl + C::kBars * 8);
+  volatile int* const abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  uint32_t const worker = blockIdx.x >> 1;
+  uint32_t const u0 = first_unit(p, worker), u1 = first_unit(p, worker + 1);
+  uint32_t const KB = p.tiles_k;
+
+  // Raw weights are never written by an earlier launch, so they stream before any wait; the first ring of them even
+  // before the block has met.
+  auto load_raw = [&](const Cursor& c, uint32_t stage) {
+    int const rg = int((c.row_pair * 2 + cta) * (kRows / 8));
+    uint32_t const dst = smem + C::oRaw + stage * C::kRaw;
+    mbar_expect_tx(raw_full(stage), C::kRaw);
+    tma_3d(dst, &tm_codes, 0, int(c.kb * 8), rg, raw_full(stage));
+    tma_3d(dst + 16 * 1024, &tm_meta, 0, int(c.kb), rg, raw_full(stage));
+  };
+  if (warp == 0) {
+    for (uint32_t i = lane; i < uint32_t(C::kBars); i += 32) {  // in the order of the offsets above
+      uint32_t count = 1;
+      if (i >= C::kRawStages && i < oBb) count = kExpanders;                                      // raw_free
+      else if (i >= oAb && i < oAb + C::kAStages) count = 2 * 4;                                  // a_full: four warps of both CTAs
+      else if (i >= oDb + 2 && i < oSb) count = 2 * C::kEpilogueWarps;                            // d_free
+      else if (i >= oSb) count = i < oSb + C::kSclStages ? kExpanders / 2 + 1 : C::kEpilogueWarps;  // s_full | s_free
+      mbar_init(bar0 + 8 * i, count);
+    }
+    if (lane == 0) *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (lane == 0) {
+      Cursor c(p, u0);
+      for (uint32_t i = 0; i < C::kRawStages && u0 + i < u1; ++i, c.next(p)) load_raw(c, i);
+    }
+  }
+  if (warp == 3) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_slot)) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();  // the peer's barriers exist before anything is signalled across
+  tc_fence_after();
+  uint32_t const tmem = *tmem_slot;
+
+  if (warp < kFirstExpander) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kRegsControl));
+    if (warp == 0) {
+      // ---- raw weights beyond the first ring
+      if (lane == 0 && u1 - u0 > C::kRawStages) {
+        Cursor c(p, u0 + C::kRawStages);
+        Ring<C::kRawStages> r;
+        r.phase = 1;
+        for (uint32_t u = u0 + C::kRawStages; u < u1; ++u, c.next(p), r.next()) {
+          if (!mbar_wait_inline(raw_free(r.s), r.phase ^ 1, abort_flag, p.status, 0x801)) break;
+          load_raw(c, r.s);
+        }
+      }
+    } else if (warp == 1) {
+      // ---- activation planes and a*s (both CTAs' halves are counted on the leader's barrier), 2^e of the tile
+      if (lane == 0) {
+        pdl_wait();
+        Cursor c(p, u0);
+        Ring<C::kBStages> b;
+        Ring<C::kSclStages> t;
+        uint32_t const b_full0 = map_to(b_full(0), 0);
+        for (uint32_t u = u0; u < u1; ++u, c.next(p), b.next(), t.next()) {
+          if (!mbar_wait_inline(b_free(b.s), b.phase ^ 1, abort_flag, p.status, 0x802)) break;
+          uint32_t const dst = smem + C::oB + b.s * C::kB, bar = b_full0 + 8 * b.s, cols = tile_cols<NT>(p, c.tok);
+          if (cta == 0) mbar_expect_tx(b_full(b.s), 2 * C::kBTx);
+          if constexpr (C::kStack) {  // leader: hi rows, peer: lo rows
+            tma_3d_pair(dst, &tm_planes, 0, int(cta * p.m_pad + c.tok * NT), int(c.kb * 4), bar);
+          } else {                    // lo box first: small terms are accumulated before the large ones
+            uint32_t const row = c.tok * NT + cta * (cols / 2);
+            tma_3d_pair(dst, &tm_planes, 0, int(p.m_pad + row), int(c.kb * 4), bar);
+            tma_3d_pair(dst + C::kBBox, &tm_planes, 0, int(row), int(c.kb * 4), bar);
+          }
+          tma_3d_pair(dst + C::kPlanes, &tm_sums, 0, int(c.tok * NT + cta * (round32(cols) / 2)), int(c.kb * 2), bar);
+          if (!mbar_wait_inline(s_free(t.s), t.phase ^ 1, abort_flag, p.status, 0x803)) break;
+          mbar_expect_tx(s_full(t.s), NT * 4);
+          bulk_copy(smem + C::oScl + t.s * C::kScl + C::oE, p.exps + uint64_t(c.kb) * p.m_pad + c.tok * NT, NT * 4, s_full(t.s));
+        }
+      }
+    } else if (warp == 2) {
+      // ---- MMA issue
+      if (cta == 0 && elect_one()) {
+        Cursor c(p, u0);
+        Ring<C::kBStages> b_;
+        Ring<C::kGroups> g_;
+        Ring<2> d_, before;
+        for (uint32_t u = u0; u < u1; ++u, c.next(p), b_.next(), g_.next(), before = d_, d_.next()) {
+          uint32_t const cols = tile_cols<NT>(p, c.tok);
+          uint32_t const idesc = f16_idesc(cols * (C::kStack ? 2 : 1)), idesc2 = f16_idesc(round32(cols));
+          uint32_t const dt = tmem + d_.s * C::kN, stage = smem + C::oB + b_.s * C::kB, a0 = g_.s * C::kQ;
+          uint64_t const b0 = umma_desc_sw128(stage);
+          bool ok = mbar_wait_inline(d_free(d_.s), d_.phase ^ 1, abort_flag, p.status, 0x804) &&
+                    mbar_wait_inline(b_full(b_.s), b_.phase, abort_flag, p.status, 0x805);
+#pragma unroll
+          for (int pass = 0; pass < (C::kStack ? 1 : 2); ++pass) {
+#pragma unroll
+            for (int q = 0; q < C::kQ; ++q) {
+              bool const last = C::kStack || pass == 1;  // the stage's last use
+              if (pass == 0) ok = ok && mbar_wait_inline(a_full(a0 + q), g_.phase, abort_flag, p.status, 0x806);
+              if (last && q == C::kQ - 1 && u > u0) ok = ok && mbar_wait_inline(d_free(before.s), before.phase, abort_flag, p.status, 0x807);
+              if (!ok) break;
+              tc_fence_after();
+              uint32_t const at = tmem + C::kACol + (a0 + q) * C::kACols;
+              constexpr int kSteps = 16 / C::kQ;
+#pragma unroll
+              for (int i = 0; i < kSteps; ++i) {
+                int const k = q * kSteps + i;
+                uint64_t const b = b0 + uint64_t((pass * C::kBBox + (k >> 2) * (C::kBRows * 128) + (k & 3) * 32) / 16);
+                if (pass == 0 && k == 0) mma_pair<false>(dt, at, b, idesc);
+                else mma_pair<true>(dt, at + i * 8, b, idesc);
+              }
+              if (last && q == C::kQ - 1)  // m * (a*s): sixteen K columns = eight groups, hi and lo; the mins serve both (K stride 0)
+                mma_pair_ss(tmem + C::kD2Col, umma_desc_plain(smem + C::oMins + g_.s * C::kMins, 0, 128),
+                            umma_desc_plain(stage + C::kPlanes, C::kTRows * 16, 128), idesc2);
+              if (last) commit_pair(a_free(a0 + q));
+            }
+            if (!ok) break;
+          }
+          if (!ok) break;
+          commit_pair(b_free(b_.s));
+          commit_pair(d_full(d_.s));
+        }
+      }
+    } else {
+      pdl_wait();
+      pdl_launch_dependents();
+      if (p.done != nullptr && blockIdx.x == 0 && lane == 0) announce_deliveries(p.unsignalled, p.peer_flag, p.ndst, p.rank);
+    }
+  } else if (warp < C::kFirstEpilogue) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kRegsExpander));
+    // ---- expanders: warp (quarter, half) turns its 32 rows' groups 4 half .. 4 half + 3 into fp16 in TMEM.  Lane = row.
+    uint32_t const quarter = warp & 3, half = ((warp - kFirstExpander) >> 2) & 1, group = (warp - kFirstExpander) / kExpanders;
+    uint32_t const row = quarter * 32 + lane;
+    uint32_t const a_full0 = map_to(a_full(0), 0);
+    Ring<C::kRawStages> r_;
+    Ring<C::kSclStages> t_;
+    if (group == 1) { r_.next(); t_.next(); }
+    uint32_t const low = opaque(0x000f000fu), high = opaque(0x00f000f0u), magic = opaque(0x64006400u);
+    uint32_t phase = 0;
+    bool ok = true;
+    for (uint32_t u = u0 + group; ok && u < u1; u += C::kGroups, phase ^= 1) {
+      uint32_t const r = r_.s, sc = t_.s;
+      if (!mbar_wait_inline(raw_full(r), r_.phase, abort_flag, p.status, 0x808)) break;
+      uint32_t const raw = smem + C::oRaw + r * C::kRaw;
+      uint4 const cm = lds128(raw + 16 * 1024 + row * 16);
+      uint4 w[4];
+#pragma unroll
+      for (int g = 0; g < 4; ++g) w[g] = lds128(raw + row * 128 + (((half * 4 + g) ^ (row & 7)) << 4));
+      if (half == 0) {
+        if (!mbar_wait_inline(s_free(sc), t_.phase ^ 1, abort_flag, p.status, 0x809)) break;
+        // The tensor core truncates when it accumulates, which shortens a super-block's sum by 2^-22 on average (measured
+        // on normal data, sixteen steps): the row scale takes the mean of that out.
+        sts64f(smem + C::oScl + sc * C::kScl + row * 8, fp16_bits_to_f32(cm.x & 0xffffu) * (1.f + 0x1p-22f), -32.f * fp16_bits_to_f32(cm.x >> 16));
+      }
+      uint32_t const scw = half == 0 ? (cm.y & 0x3f3f3f3fu) : ((cm.w & 0x0f0f0f0fu) | ((cm.y >> 2) & 0x30303030u));
+      constexpr int kMine = C::kQ / 2, kGroupsPer = 4 / kMine;  // stages of this warp, K32 groups per stage
+#pragma unroll
+      for (int i = 0; i < kMine; ++i) {
+        uint32_t const sa = group * C::kQ + half * kMine + i;
+        if (!mbar_wait_inline(a_free(sa), phase ^ 1, abort_flag, p.status, 0x80a)) { ok = false; break; }
+        tc_fence_after();
+        if (half == 1 && i == kMine - 1) {
+          ScaleMinWords const sm = decode_scale_min(cm.y, cm.z, cm.w);
+          uint32_t mh[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            uint32_t const mw = j < 2 ? sm.mn_lo : sm.mn_hi;
+            // two bytes under the exponent of 1024, minus 1024: exact
+            mh[j] = h2u(__hsub2(u2h(__byte_perm(mw, 0x64646464u, (j & 1) ? 0x4342 : 0x4140)), u2h(0x64006400u)));
+          }
+          sts128(smem + C::oMins + group * C::kMins + row * 16, mh[0], mh[1], mh[2], mh[3]);
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // read by the MMA
+        }
+#pragma unroll
+        for (int gg = 0; gg < kGroupsPer; ++gg) {
+          int const g = i * kGroupsPer + gg;
+          __half2 const S = __hsub2(u2h(__byte_perm(scw, 0x64646464u, 0x4040 | (g * 0x0101))), u2h(0x64006400u));
+          // low nibbles: (1024 + q) * sc - 1024 sc; high nibbles, four bits up: (1024 + 16 q) * (sc / 16) - 64 sc
+          __half2 const S16 = __hmul2(S, u2h(0x2c002c00u)), B = __hmul2(S, u2h(0xe400e400u)), B16 = __hmul2(S, u2h(0xd400d400u));
+          uint32_t const ww[4] = {w[g].x, w[g].y, w[g].z, w[g].w};
+          uint32_t v[16];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            uint32_t const t = ww[j] >> 8;
+            v[4 * j + 0] = h2u(__hfma2(u2h(and_or(ww[j], low, magic)), S, B));
+            v[4 * j + 1] = h2u(__hfma2(u2h(and_or(ww[j], high, magic)), S16, B16));
+            v[4 * j + 2] = h2u(__hfma2(u2h(and_or(t, low, magic)), S, B));
+            v[4 * j + 3] = h2u(__hfma2(u2h(and_or(t, high, magic)), S16, B16));
+          }
+          tmem_st16(tmem + ((quarter * 32u) << 16) + C::kACol + sa * C::kACols + gg * 16, v);
+        }
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) arrive_cluster(a_full0 + 8 * sa);
+      }
+      if (lane == 0) {
+        if (half == 0) mbar_arrive(s_full(sc));
+        mbar_arrive(raw_free(r));
+      }
+#pragma unroll
+      for (int i = 0; i < C::kGroups; ++i) { r_.next(); t_.next(); }
+    }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::kRegsEpilogue));
+    // ---- epilogue: warp (quarter, column part) owns 32 rows x kCols tokens; lane = row, as the TMEM lanes are.
+    uint32_t const ep = warp - C::kFirstEpilogue, quarter = warp & 3, col0 = (ep >> 2) * C::kCols;
+    uint32_t const row = quarter * 32 + lane, lane_base = tmem + ((quarter * 32u) << 16) + col0;
+    uint32_t const d_free0 = map_to(d_free(0), 0);
+    constexpr int W = NT >= 128 ? 8 : 16;  // tokens per TMEM read: what 88 registers (sixteen epilogue warps) hold without spilling
+    pdl_wait();
+    float2 acc[C::kCols / 2];
+#pragma unroll
+    for (int j = 0; j < C::kCols / 2; ++j) acc[j] = make_float2(0.f, 0.f);
+    Cursor c(p, u0);
+    Ring<C::kSclStages> t_;
+    Ring<2> d_;
+    for (uint32_t u = u0; u < u1; ++u, c.next(p), t_.next(), d_.next()) {
+      uint32_t const sc = t_.s, d = d_.s, cols = tile_cols<NT>(p, c.tok);
+      if (!mbar_wait_inline(s_full(sc), t_.phase, abort_flag, p.status, 0x80b)) break;
+      uint32_t const scl = smem + C::oScl + sc * C::kScl, et = scl + C::oE + col0 * 4;
+      float2 const dm = lds64f(scl + row * 8);
+      float2 const dd = make_float2(dm.x, dm.x), nm = make_float2(dm.y, dm.y);
+      // Does any of the warp's tokens have a power of its own in this super-block?
+      bool plain = true;
+#pragma unroll
+      for (int c0 = 0; c0 < C::kCols; c0 += 32) plain = plain && lds32f(et + (c0 + (C::kCols < 32 ? lane & 15 : lane)) * 4) == 1.f;
+      plain = __all_sync(0xffffffffu, plain);
+      if (!mbar_wait_inline(d_full(d), d_.phase, abort_flag, p.status, 0x80c)) break;
+      tc_fence_after();
+#pragma unroll
+      for (int c0 = 0; c0 < C::kCols; c0 += W) {
+        uint32_t P[W], L[C::kStack ? W : 1], M[W];
+        // Columns beyond a short tile's hold stale words: they are read and folded like the others and never stored.
+        tmem_ld<W>(lane_base + d * C::kN + c0, P);
+        if constexpr (C::kStack) tmem_ld<W>(lane_base + d * C::kN + cols + c0, L);
+        tmem_ld<W>(lane_base + C::kD2Col + c0, M);
+        tmem_wait_ld();
+        if (c0 + W == C::kCols) {  // everything of this super-block is in registers
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) arrive_cluster(d_free0 + 8 * d);
+        }
+        if (!plain) {
+#pragma unroll
+          for (int j = 0; j < W; ++j) {
+            float const e = lds32f(et + (c0 + j) * 4);
+            P[j] = __float_as_uint(__uint_as_float(P[j]) * e);
+            if constexpr (C::kStack) L[j] = __float_as_uint(__uint_as_float(L[j]) * e);
+            M[j] = __float_as_uint(__uint_as_float(M[j]) * e);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < W; j += 2) {
+          float2 v = as_float2(P + j);
+          float2 const mt = as_float2(M + j);
+          if constexpr (C::kStack) v = __fadd2_rn(v, as_float2(L + j));
+          float2& a = acc[(c0 + j) / 2];
+          a = __ffma2_rn(nm, mt, __ffma2_rn(dd, v, a));
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(s_free(sc));
+      if (u + 1 < u1 && c.kb + 1 != KB) continue;
+
+      // ---- end of this cluster's part of the tile
+      uint32_t const tile = c.row_pair * p.tok_tiles + c.tok;
+      bool write = true;
+      if (max(u0, tile * KB) != tile * KB || u + 1 != (tile + 1) * KB) {
+        // Partial: [cluster][first or later tile of its run][CTA][warp][token / 4][lane].
+        auto slot = [&](uint32_t w) {
+          uint32_t const later = first_unit(p, w) < tile * KB || first_unit(p, w) >= (tile + 1) * KB;
+          return reinterpret_cast<float4*>(p.slots) +
+                 ((uint64_t(w * 2 + later) * 2 + cta) * C::kEpilogueWarps + ep) * (C::kCols * 8) + lane;
+        };
+        float4* const mine = slot(worker);
+#pragma unroll
+        for (int j = 0; j < C::kCols / 4; ++j) __stcg(mine + j * 32, make_float4(acc[2 * j].x, acc[2 * j].y, acc[2 * j + 1].x, acc[2 * j + 1].y));
+        __threadfence();
+        __syncwarp();
+        // Clusters that share the tile: from the one whose run holds its first unit to the one that holds its last.
+        uint32_t w0 = worker, w1 = worker;
+        while (first_unit(p, w0) > tile * KB) --w0;
+        while (first_unit(p, w1 + 1) < (tile + 1) * KB) ++w1;
+        uint32_t old = 0;
+        uint32_t* const ticket = p.tickets + (w0 * 2 + cta) * C::kEpilogueWarps + ep;
+        if (lane == 0) old = atomicAdd(ticket, 1u);
+        old = __shfl_sync(0xffffffffu, old, 0);
+        write = old == w1 - w0;
+        if (write) {
+          __threadfence();
+#pragma unroll
+          for (int j = 0; j < C::kCols / 2; ++j) acc[j] = make_float2(0.f, 0.f);
+          for (uint32_t w = w0; w <= w1; ++w) {  // in run order, whoever arrives last
+            const float4* const src = slot(w);
+#pragma unroll
+            for (int j0 = 0; j0 < C::kCols / 4; j0 += 4) {
+              float4 x[4];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) x[j] = __ldcg(src + (j0 + j) * 32);
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                float2 &lo = acc[2 * (j0 + j)], &hi = acc[2 * (j0 + j) + 1];
+                lo = __fadd2_rn(lo, make_float2(x[j].x, x[j].y));
+                hi = __fadd2_rn(hi, make_float2(x[j].z, x[j].w));
+              }
+            }
+          }
+        }
+      }
+      // A lane's values are one row of consecutive tokens: every store of a warp is 32 neighbouring rows of one token.
+      uint32_t const n_row = (c.row_pair * 2 + cta) * kRows + row, tok0 = c.tok * NT + col0;
+      if (write && n_row < p.n && tok0 < p.m) {
+        uint32_t const live = min(p.m - tok0, uint32_t(C::kCols));
+        uint64_t o = uint64_t(tok0) * p.out_stride + p.out_row0 + n_row;
+#pragma unroll
+        for (int j0 = 0; j0 < C::kCols; j0 += 8) {  // eight tokens at a time: eight residual loads in flight, few registers
+          if (j0 >= live) break;
+          float v[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[j] = ((j & 1) ? acc[(j0 + j) / 2].y : acc[(j0 + j) / 2].x) * ldg_here(p.tokens + tok0 + j0 + j);
+          if (p.residual) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              if (j0 + j < live) v[j] += p.residual[o + j * uint64_t(p.out_stride)];
+          }
+          if (p.out_bf16) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              if (j0 + j < live) p.out_bf16[o + j * uint64_t(p.out_stride)] = f32_to_bf16_rne(v[j]);
+          } else {
+            for (uint32_t g = 0; g < p.ndst; ++g) {
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                if (j0 + j < live) p.out[g][o + j * uint64_t(p.out_stride)] = v[j];
+            }
+          }
+          o += 8 * uint64_t(p.out_stride);
+          asm volatile("" ::: "memory");
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < C::kCols / 2; ++j) acc[j] = make_float2(0.f, 0.f);
+    }
+  }
+
+  // ---- teardown
+  __syncwarp();
+  if (*abort_flag) {  // copies still in flight land before shared memory goes away
+    long long const t0 = clock64();
+    while (clock64() - t0 < 4000000LL) {}
+  }
+  if (warp >= C::kFirstEpilogue) tmem_wait_ld();
+  tc_fence_before();
+  __syncthreads();
+  cluster_meet();  // neither CTA leaves while the other may still signal it or read its operands
+  tc_fence_after();
+  if (warp == 3) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+  if (p.done != nullptr && threadIdx.x == 0) {
+    __threadfence();
+    uint32_t const old = atomicAdd(p.done, 1u);
+    if (old == gridDim.x - 1) {
+      *p.done = 0;
+      if (*reinterpret_cast<volatile int*>(p.status) == 0) atomicAdd(p.unsignalled, 1u);
+    }
+  }
+}
+
+// ------------------------------------------------------------------------------------------
+constexpr uint32_t kMaxClusters = 128;  // clusters of two SMs on the device at most (tickets)
+constexpr uint64_t kTicketBytes = uint64_t(kMaxClusters) * 2 * 16 * 4;
+
+uint64_t align1k(uint64_t v) { return (v + 1023) / 1024 * 1024; }
+
+struct Carve {
+  uint64_t slots, sums, exps, tokens, planes, total;
+};
+Carve carve(uint32_t m, uint32_t tiles_k, const F16Plan& plan) {
+  uint64_t const m_pad = uint64_t((m + plan.nt - 1) / plan.nt) * plan.nt;
+  Carve c;
+  c.slots = align1k(kTicketBytes);
+  c.sums = c.slots + align1k(uint64_t(plan.slot_clusters) * 4 * kRows * plan.nt * 4);
+  c.exps = c.sums + align1k(m_pad * tiles_k * 32);
+  c.tokens = c.exps + align1k(m_pad * tiles_k * 4);
+  c.planes = c.tokens + align1k(m_pad * 4);
+  c.total = c.planes + m_pad * tiles_k * 256 * 4;
+  return c;
+}
+
+template <int NT>
+cudaError_t launch_f16(const WeightView& w, const Q8View& x, const TcOutput& o, const F16Plan& plan, uint8_t* scratch, int* status,
+                       cudaStream_t stream) {
+  using C = F16Cfg<NT>;
+  Carve const c = carve(x.m, w.tiles_k, plan);
+  uint32_t const m_pad = (x.m + NT - 1) / NT * NT, pk = w.tiles_k * 256;
+  uint32_t const grid = m_pad * ((w.tiles_k + 7) / 8);
+  cudaError_t st = launch_kernel(planes_kernel, grid, 256, 0, stream, launch_overlap(), x.codes, x.scales, x.sums, x.m, m_pad, w.tiles_k,
+                                 reinterpret_cast<__half*>(scratch + c.planes), reinterpret_cast<__half*>(scratch + c.sums),
+                                 reinterpret_cast<float*>(scratch + c.exps), reinterpret_cast<float*>(scratch + c.tokens),
+                                 reinterpret_cast<uint32_t*>(scratch), plan.unit_step == 1 ? uint32_t(kTicketBytes / 4) : 0u);
+  if (st != cudaSuccess) return st;
+  CUtensorMap tm_codes, tm_meta, tm_planes, tm_sums;
+  uint64_t const rgs = w.padded_n / 8;
+  {
+    uint64_t dims[3] = {128, uint64_t(w.tiles_k) * 8, rgs}, strides[2] = {128, uint64_t(w.tiles_k) * 1024};
+    uint32_t box[3] = {128, 8, 16};
+    if (!make_map(&tm_codes, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, w.codes, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B))
+      return cudaErrorInvalidValue;
+  }
+  {
+    uint64_t dims[3] = {128, w.tiles_k, rgs}, strides[2] = {128, uint64_t(w.tiles_k) * 128};
+    uint32_t box[3] = {128, 1, 16};
+    if (!make_map(&tm_meta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, w.meta, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE))
+      return cudaErrorInvalidValue;
+  }
+  {
+    uint64_t dims[3] = {64, 2 * uint64_t(m_pad), pk / 64}, strides[2] = {uint64_t(pk) * 2, 128};
+    uint32_t box[3] = {64, uint32_t(C::kBRows), 4};
+    if (!make_map(&tm_planes, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, scratch + c.planes, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B))
+      return cudaErrorInvalidValue;
+  }
+  {
+    uint64_t dims[3] = {8, m_pad, 2 * uint64_t(w.tiles_k)}, strides[2] = {16, uint64_t(m_pad) * 16};
+    uint32_t box[3] = {8, uint32_t(C::kTRows), 2};
+    if (!make_map(&tm_sums, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, scratch + c.sums, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE))
+      return cudaErrorInvalidValue;
+  }
+  F16Params p{};
+  p.residual = o.residual;
+  for (uint32_t g = 0; g < o.ndst; ++g) { p.out[g] = o.out[g]; p.peer_flag[g] = o.flags[g]; }
+  p.out_bf16 = o.out_bf16; p.done = o.done; p.unsignalled = o.unsignalled; p.ndst = o.ndst; p.rank = o.rank;
+  p.out_stride = o.stride ? o.stride : w.n; p.out_row0 = o.row0;
+  p.exps = reinterpret_cast<const float*>(scratch + c.exps); p.tokens = reinterpret_cast<const float*>(scratch + c.tokens); p.slots = reinterpret_cast<float*>(scratch + c.slots); p.tickets = reinterpret_cast<uint32_t*>(scratch);
+  p.status = status; p.n = w.n; p.m = x.m; p.m_pad = m_pad; p.tiles_k = w.tiles_k; p.tok_tiles = m_pad / NT;
+  uint32_t const steps = (w.padded_n + 2 * kRows - 1) / (2 * kRows) * p.tok_tiles * w.tiles_k / plan.unit_step;
+  p.run_each = steps / plan.workers; p.run_rest = steps % plan.workers; p.unit_step = plan.unit_step;
+  static bool configured[64] = {};
+  int device = 0;
+  if ((st = cudaGetDevice(&device)) != cudaSuccess) return st;
+  if (device < 0 || device >= 64 || !configured[device]) {
+    if ((st = cudaFuncSetAttribute(mmq_f16_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem)) != cudaSuccess) return st;
+    if (device >= 0 && device < 64) configured[device] = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = 2 * plan.workers;
+  cfg.blockDim = C::kThreads;
+  cfg.dynamicSmemBytes = C::kSmem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  // Always allowed to start beside the kernel that writes the planes: that one starts (or, with launch overlap, waits
+  // until) everything before it has completed, so the weights are final by then.
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, mmq_f16_kernel<NT>, tm_codes, tm_meta, tm_planes, tm_sums, p);
+}
+
+}  // namespace
+
+bool f16_supported(const WeightView& w, const Q8View& x) {
+  return encode_fn() != nullptr && reinterpret_cast<uintptr_t>(w.codes) % 16 == 0 && reinterpret_cast<uintptr_t>(w.meta) % 16 == 0 &&
+         reinterpret_cast<uintptr_t>(x.codes) % 8 == 0;
+}
+
+F16Plan plan_f16(uint32_t m, uint32_t n, uint32_t tiles_k) {
+  F16Plan p;
+  // Tokens per pass: the planes of one pass (four bytes per element) stay below 64 MB, half of L2.
+  uint64_t const most = (64ull << 20) / (uint64_t(tiles_k) * 1024) / 128 * 128;
+  uint32_t const passes = uint32_t((m + most - 1) / most);
+  p.chunk = passes <= 1 ? m : ((m + passes - 1) / passes + 127) & ~127u;
+  uint32_t const mc = p.chunk < m ? p.chunk : m;
+  p.nt = mc <= 16 ? 16 : (mc <= 32 ? 32 : (mc <= 64 ? 64 : 128));
+  uint32_t const clusters = uint32_t(sm_count()) / 2;
+  uint64_t const tiles = uint64_t((n + 2 * kRows - 1) / (2 * kRows)) * ((mc + p.nt - 1) / p.nt), units = tiles * tiles_k;
+  // Whole tiles per cluster, or equal runs of super-blocks (at least four) whose cut tiles are added through scratch?
+  // In units of one super-block; the cut costs about as much as kCut of them.
+  double const kCut = p.nt >= 128 ? 2.0 : (p.nt >= 64 ? 3.0 : 5.0);
+  uint64_t const run_workers = units / 4 < 1 ? 1 : (units / 4 < clusters ? units / 4 : clusters);
+  double const whole = double((tiles + clusters - 1) / clusters * tiles_k);
+  double const run = double((units + run_workers - 1) / run_workers) + kCut;
+  if (whole <= run) {
+    p.unit_step = tiles_k;
+    p.workers = uint32_t(tiles < clusters ? tiles : clusters);
+  } else {
+    p.unit_step = 1;
+    p.workers = uint32_t(run_workers);
+  }
+  p.slot_clusters = p.chunk < m ? clusters : (p.unit_step == 1 ? p.workers : 0);
+  return p;
+}
+
+uint64_t f16_scratch_bytes(uint32_t m, uint32_t tiles_k, const F16Plan& plan) {
+  return carve(m < plan.chunk ? m : plan.chunk, tiles_k, plan).total;
+}
+
+cudaError_t launch_mmq_f16(const WeightView& w, const Q8View& x, const TcOutput& out, const F16Plan& plan, void* scratch, int* status,
+                           cudaStream_t stream) {
+  if (out.ndst < 1 || out.ndst > 8 || (out.out_bf16 ? out.ndst != 1 : out.out[0] == nullptr) || plan.workers < 1 ||
+      plan.workers > kMaxClusters)
+    return cudaErrorInvalidValue;
+  uint64_t const stride = out.stride ? out.stride : w.n;
+  for (uint32_t t0 = 0; t0 < x.m; t0 += plan.chunk) {
+    Q8View xc = x;
+    uint64_t const G = x.padded_k / 32;
+    xc.m = x.m - t0 < plan.chunk ? x.m - t0 : plan.chunk;
+    xc.codes += uint64_t(t0) * x.padded_k; xc.scales += t0 * G; xc.sums += t0 * G;
+    TcOutput oc = out;
+    for (uint32_t g = 0; g < out.ndst; ++g) if (oc.out[g]) oc.out[g] += t0 * stride;
+    if (oc.out_bf16) oc.out_bf16 += t0 * stride;
+    if (oc.residual) oc.residual += t0 * stride;
+    if (t0 + plan.chunk < x.m) oc.done = nullptr;  // row-sharded use: the projection counts once, with its last pass
+    F16Plan pc = plan;
+    if (xc.m < plan.chunk) {  // a shorter last pass: fewer token tiles of the same width
+      F16Plan const last = plan_f16(xc.m, w.n, w.tiles_k);
+      if (last.nt == plan.nt) { pc.workers = last.workers; pc.unit_step = last.unit_step; }
+      else {
+        uint64_t const tiles = uint64_t((w.n + 2 * kRows - 1) / (2 * kRows)) * ((xc.m + plan.nt - 1) / plan.nt);
+        pc.unit_step = w.tiles_k;
+        pc.workers = uint32_t(tiles < uint64_t(plan.workers) ? tiles : uint64_t(plan.workers));
+      }
+    }
+    uint8_t* const s = static_cast<uint8_t*>(scratch);
+    cudaError_t st;
+    switch (plan.nt) {
+      case 16: st = launch_f16<16>(w, xc, oc, pc, s, status, stream); break;
+      case 32: st = launch_f16<32>(w, xc, oc, pc, s, status, stream); break;
+      case 64: st = launch_f16<64>(w, xc, oc, pc, s, status, stream); break;
+      case 128: st = launch_f16<128>(w, xc, oc, pc, s, status, stream); break;
+      default: return cudaErrorInvalidValue;
+    }
+    if (st != cudaSuccess) return st;
+  }
+  return cudaSuccess;
+}
+
+}  // namespace q4k

@@ -1,0 +1,26 @@
+// Scratch that one call needs from its first kernel to its last (stream_scratch.cu).
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace q4k {
+
+// acquire() before the call's first kernel, release() after its last launch: in between p() is the call's own memory,
+// whatever other streams, threads and graphs do.  Nothing about its contents may be assumed.
+class StreamScratch {
+ public:
+  cudaError_t acquire(cudaStream_t stream, uint64_t bytes);
+  cudaError_t release();
+  void* p() const { return p_; }
+  ~StreamScratch() { (void)release(); }
+  StreamScratch() = default;
+  StreamScratch(StreamScratch const&) = delete;
+  StreamScratch& operator=(StreamScratch const&) = delete;
+
+ private:
+  void* p_ = nullptr;
+  cudaStream_t stream_ = nullptr;
+  bool owned_ = false;  // to be freed in stream order
+};
+
+}  // namespace q4k

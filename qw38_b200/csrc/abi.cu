@@ -68,16 +68,16 @@ class ScopedRange {
   bool active_;
 };
 
-using MemGetAddressRange = CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr);
-MemGetAddressRange address_range_fn() {
-  static MemGetAddressRange fn = [] {
+using PointerGetAttributes = CUresult (*)(unsigned int, CUpointer_attribute*, void**, CUdeviceptr);
+PointerGetAttributes pointer_attributes_fn() {
+  static PointerGetAttributes fn = [] {
     void* p = nullptr;
     cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &p, cudaEnableDefault, &q) != cudaSuccess ||
+    if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &p, cudaEnableDefault, &q) != cudaSuccess ||
         q != cudaDriverEntryPointSuccess)
       p = nullptr;
     (void)cudaGetLastError();
-    return reinterpret_cast<MemGetAddressRange>(p);
+    return reinterpret_cast<PointerGetAttributes>(p);
   }();
   return fn;
 }
@@ -96,21 +96,25 @@ int check_span(const Region& r, int device) {
     return fail(Q4K_ERR_OVERFLOW, "%s: address overflow", r.name);
   if (r.alignment == 0 || begin % r.alignment != 0)
     return fail(Q4K_ERR_INVALID_ARGUMENT, "%s: misaligned pointer", r.name);
-  cudaPointerAttributes attr{};
-  if (cudaPointerGetAttributes(&attr, r.p) != cudaSuccess) {
-    (void)cudaGetLastError();
+  // Memory type, device and allocation of the pointer in one driver call (the checks run on every operand of every call:
+  // two runtime calls per operand were most of a decode call's host time).  A pointer the driver does not know leaves the
+  // outputs zero.
+  auto const fn = pointer_attributes_fn();
+  if (!fn) return fail(Q4K_ERR_STATUS, "%s: cuPointerGetAttributes is not available", r.name);
+  unsigned int type = 0;
+  int ordinal = -1;
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  CUpointer_attribute what[4] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,
+                                 CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  void* to[4] = {&type, &ordinal, &base, &size};
+  if (fn(4, what, to, static_cast<CUdeviceptr>(begin)) != CUDA_SUCCESS)
     return fail(Q4K_ERR_INVALID_ARGUMENT, "%s: pointer is not device memory", r.name);
-  }
-  if (attr.type != cudaMemoryTypeDevice || attr.device != device)
+  if (type != CU_MEMORYTYPE_DEVICE || ordinal != device)
     return fail(Q4K_ERR_INVALID_ARGUMENT, "%s: not device memory of the current device", r.name);
-  if (auto fn = address_range_fn()) {
-    CUdeviceptr base = 0;
-    size_t size = 0;
-    if (fn(&base, &size, static_cast<CUdeviceptr>(begin)) != CUDA_SUCCESS)
-      return fail(Q4K_ERR_INVALID_ARGUMENT, "%s: unknown device allocation", r.name);
-    if (begin < base || begin + r.bytes > base + size)
-      return fail(Q4K_ERR_INVALID_ARGUMENT, "%s: operand exceeds its allocation", r.name);
-  }
+  if (base == 0) return fail(Q4K_ERR_INVALID_ARGUMENT, "%s: unknown device allocation", r.name);
+  if (begin < base || begin + r.bytes > base + size)
+    return fail(Q4K_ERR_INVALID_ARGUMENT, "%s: operand exceeds its allocation", r.name);
   return Q4K_OK;
 }
 
@@ -643,21 +647,35 @@ int decode_one(const q4k_decode_desc& d, const q4k_q8_input& q8, float* rows, cu
   }
 }
 
+int decode_pack(const q4k_decode_desc& d, const q4k_q8_input& q8, int* failure, cudaStream_t stream) {
+  if (d.activation_policy == Q4K_ACTIVATION_BF16) return Q4K_OK;  // that policy multiplies the bf16 input as it is
+  if (!failure) return fail(Q4K_ERR_INVALID_ARGUMENT, "decode_mmv: null failure flag");
+  return pack_impl(d.input, false, d.input_len, q8, failure, stream);
+}
+
 // One launch for up to three descriptors that share the (already quantised) input: every weight's rows, its bf16 /
 // fp32 store or residual add, or -- swiglu -- bf16(SiLU(a) * b) of a gate / up pair, all inside the TMA decode kernel
 // (the reference applies these epilogues inside its decode kernels too, cuda/decode_mmv.cu:182-250,619-677).
 // *fused = false when the operands do not qualify (more than 16 rows, unaligned weights, another activation policy);
 // the caller then composes separate launches.
-int decode_fused(const q4k_decode_desc* const* descs, uint32_t count, bool swiglu, const q4k_q8_input& q8, cudaStream_t stream,
+// Up to kDecodeRawTokens rows the launch also quantises: each block its own K slice, which at one to four tokens takes
+// less than the pack launch it saves (at eight, five warps per scheduler spend as long on it as that launch takes).
+constexpr uint32_t kDecodeRawTokens = 4;
+int decode_fused(const q4k_decode_desc* const* descs, uint32_t count, bool swiglu, const q4k_q8_input& q8, int* failure, cudaStream_t stream,
                  bool* fused) {
   *fused = false;
+  bool const raw = q8.m <= kDecodeRawTokens;
   q4k::WeightView ws[3];
   q4k::GemvTmaOutput outs[3] = {};
   Region regions[16];
   int nreg = 0;
-  regions[nreg++] = {q8.codes, q8.codes_len, 4, "input.codes"};
-  regions[nreg++] = {q8.scales, q8.scales_len * 4, 4, "input.scales"};
-  regions[nreg++] = {q8.sums, q8.sums_len * 4, 4, "input.sums"};
+  // the pack of the workspace is one run of memory: codes, scales, sums
+  regions[nreg++] = {q8.codes, uint64_t(reinterpret_cast<uint8_t*>(q8.sums + q8.sums_len) - reinterpret_cast<uint8_t*>(q8.codes)), 4, "workspace"};
+  if (raw) {
+    if (!failure) return fail(Q4K_ERR_INVALID_ARGUMENT, "decode_mmv: null failure flag");
+    regions[nreg++] = {descs[0]->input, descs[0]->input_len * 2, 2, "input"};
+    regions[nreg++] = {failure, 4, 4, "failure"};
+  }
   uint64_t n_total = 0, tiles = 0;
   for (uint32_t i = 0; i < count; ++i) {
     const q4k_decode_desc& d = *descs[i];
@@ -696,6 +714,9 @@ int decode_fused(const q4k_decode_desc* const* descs, uint32_t count, bool swigl
     tiles += (d.weight.padded_n + 15) / 16;
   }
   if (int st = check_distinct(regions, nreg, false)) return st;
+  if (!raw)
+    if (int st = decode_pack(*descs[0], q8, failure, stream)) return st;
+  q4k::GemvTmaRaw const rows{descs[0]->input, descs[0]->weight.k, failure};
   q4k::GemvTmaPlan plan = q4k::plan_gemv_tma_tiles(q8.m, uint32_t(tiles), ws[0].tiles_k, 0, 0, swiglu);
   uint64_t const partial_bytes = plan.split_k > 1 ? uint64_t(plan.split_k) * q8.m * n_total * 4 : 0;
   void* scratch = nullptr;
@@ -704,16 +725,10 @@ int decode_fused(const q4k_decode_desc* const* descs, uint32_t count, bool swigl
   if (!status) return Q4K_ERR_STATUS;
   uint8_t* const base = static_cast<uint8_t*>(scratch);
   Q4K_CUDA(q4k::launch_gemv_tma_multi(ws, outs, count, swiglu, view(q8), plan, base + kTicketRegion, reinterpret_cast<uint32_t*>(base),
-                                      status, stream),
+                                      status, stream, raw ? &rows : nullptr),
            "decode_mmv.fused");
   *fused = true;
   return Q4K_OK;
-}
-
-int decode_pack(const q4k_decode_desc& d, const DecodeScratch& s, int* failure, cudaStream_t stream) {
-  if (d.activation_policy == Q4K_ACTIVATION_BF16) return Q4K_OK;  // that policy multiplies the bf16 input as it is
-  if (!failure) return fail(Q4K_ERR_INVALID_ARGUMENT, "decode_mmv: null failure flag");
-  return pack_impl(d.input, false, d.input_len, s.q8, failure, stream);
 }
 }  // namespace
 
@@ -724,10 +739,10 @@ int q4k_decode_mmv(const q4k_decode_desc* desc, void* workspace, uint64_t worksp
   if (int st = valid_decode_desc(desc, false, "desc")) return st;
   DecodeScratch s{};
   if (int st = carve_decode_scratch(workspace, workspace_bytes, desc->m, desc->weight.n, desc->weight.k, &s)) return st;
-  if (int st = decode_pack(*desc, s, failure, stream)) return st;
   bool fused = false;
-  if (int st = decode_fused(&desc, 1, false, s.q8, stream, &fused)) return st;
+  if (int st = decode_fused(&desc, 1, false, s.q8, failure, stream, &fused)) return st;
   if (fused) return Q4K_OK;
+  if (int st = decode_pack(*desc, s.q8, failure, stream)) return st;
   return decode_one(*desc, s.q8, s.rows, stream);
 }
 
@@ -751,14 +766,14 @@ int q4k_decode_mmv_paired(const q4k_decode_desc* a, const q4k_decode_desc* b, vo
     return fail(Q4K_ERR_INVALID_ARGUMENT, "decode_mmv_paired: paired B must match A shape, layout, input, and epilogue contract");
   DecodeScratch s{};
   if (int st = carve_decode_scratch(workspace, workspace_bytes, a->m, a->weight.n, a->weight.k, &s)) return st;
-  if (int st = decode_pack(*a, s, failure, stream)) return st;
   uint64_t const cells = uint64_t(a->m) * a->weight.n;
   {
     const q4k_decode_desc* pair[2] = {a, &bv};
     bool fused = false;
-    if (int st = decode_fused(pair, 2, swiglu, s.q8, stream, &fused)) return st;
+    if (int st = decode_fused(pair, 2, swiglu, s.q8, failure, stream, &fused)) return st;
     if (fused) return Q4K_OK;
   }
+  if (int st = decode_pack(*a, s.q8, failure, stream)) return st;
   if (!swiglu) {
     if (int st = decode_one(*a, s.q8, s.rows, stream)) return st;
     return decode_one(*b, s.q8, s.rows + cells, stream);
@@ -779,7 +794,7 @@ int q4k_prefill_project(const q4k_decode_desc* projection, void* workspace, uint
   DecodeScratch s{};
   if (int st = carve_decode_scratch(workspace, workspace_bytes, projection->m, projection->weight.n, projection->weight.k, &s))
     return st;
-  if (int st = decode_pack(*projection, s, failure, stream)) return st;
+  if (int st = decode_pack(*projection, s.q8, failure, stream)) return st;
   return decode_one(*projection, s.q8, s.rows, stream);
 }
 
@@ -798,7 +813,7 @@ int q4k_prefill_paired_swiglu(const q4k_weight* gate, const q4k_weight* up, cons
     return fail(Q4K_ERR_INVALID_ARGUMENT, "paired_swiglu: gate and up must have the same shape and layout");
   DecodeScratch s{};
   if (int st = carve_decode_scratch(workspace, workspace_bytes, valid_tokens, gate->n, gate->k, &s)) return st;
-  if (int st = decode_pack(a, s, failure, stream)) return st;
+  if (int st = decode_pack(a, s.q8, failure, stream)) return st;
   uint64_t const cells = uint64_t(valid_tokens) * gate->n;
   if (int st = project_impl(gate, s.q8, s.rows, cells, nullptr, 0, nullptr, stream)) return st;
   if (int st = project_impl(up, s.q8, s.rows + cells, cells, nullptr, 0, nullptr, stream)) return st;
@@ -822,13 +837,13 @@ int q4k_decode_mmv_ranges(const q4k_decode_desc* ranges, uint32_t count, void* w
   }
   DecodeScratch s{};
   if (int st = carve_decode_scratch(workspace, workspace_bytes, ranges[0].m, n_total, ranges[0].weight.k, &s)) return st;
-  if (int st = decode_pack(ranges[0], s, failure, stream)) return st;
   {
     const q4k_decode_desc* list[3] = {&ranges[0], &ranges[1], count > 2 ? &ranges[2] : nullptr};
     bool fused = false;
-    if (int st = decode_fused(list, count, false, s.q8, stream, &fused)) return st;
+    if (int st = decode_fused(list, count, false, s.q8, failure, stream, &fused)) return st;
     if (fused) return Q4K_OK;
   }
+  if (int st = decode_pack(ranges[0], s.q8, failure, stream)) return st;
   uint64_t off = 0;
   for (uint32_t i = 0; i < count; ++i) {
     if (int st = decode_one(ranges[i], s.q8, s.rows + off, stream)) return st;

@@ -74,7 +74,7 @@ cudaError_t launch_m(const WeightView& w, const uint16_t* x, uint32_t k, uint32_
   size_t const smem = size_t(M) * padded_k * 4;
   auto kernel = gemv_bf16w_kernel<M>;
   if (smem > 48 * 1024) {
-    cudaError_t st = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    cudaError_t st = allow_smem(reinterpret_cast<const void*>(kernel), int(smem));
     if (st != cudaSuccess) return st;
   }
   return launch_kernel(kernel, (w.n + 7) / 8, kThreads, smem, stream, launch_overlap(), w, x, k, padded_k, out, residual);

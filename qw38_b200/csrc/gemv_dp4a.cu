@@ -218,7 +218,7 @@ cudaError_t launch_m(const WeightView& w, const Q8View& x, float* out, const flo
   bool const wide = (reinterpret_cast<uintptr_t>(w.codes) % 16 == 0) && (reinterpret_cast<uintptr_t>(w.meta) % 16 == 0);
   auto kernel = partials ? gemv_dp4a_kernel<M, true> : gemv_dp4a_kernel<M, false>;
   if (smem > 48 * 1024) {
-    cudaError_t st = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    cudaError_t st = allow_smem(reinterpret_cast<const void*>(kernel), int(smem));
     if (st != cudaSuccess) return st;
   }
   return launch_kernel(kernel, grid, kThreads, smem, stream, launch_overlap(), w, x, out, residual, partials, rgc, wide);

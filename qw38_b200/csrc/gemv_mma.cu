@@ -349,7 +349,7 @@ cudaError_t launch_cfg(const WeightView& w, const Q8View& x, float* out, const f
   if (partials) kernel = wide ? gemv_mma_kernel<Upper, true, true, Warps> : gemv_mma_kernel<Upper, true, false, Warps>;
   else kernel = wide ? gemv_mma_kernel<Upper, false, true, Warps> : gemv_mma_kernel<Upper, false, false, Warps>;
   constexpr int smem = Smem<Warps, Upper ? 16 : 8>::kTotal;
-  cudaError_t st = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaError_t st = allow_smem(reinterpret_cast<const void*>(kernel), int(smem));
   if (st != cudaSuccess) return st;
   uint32_t const row_tiles = (w.padded_n / 8 + Warps - 1) / Warps;
   cudaLaunchConfig_t cfg{};

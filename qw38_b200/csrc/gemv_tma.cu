@@ -42,6 +42,7 @@
 
 #include "common.cuh"
 #include "launch.h"
+#include "q8_pack.cuh"
 #include "tma.cuh"
 
 namespace q4k {
@@ -97,6 +98,10 @@ struct GtParams {
   int32_t* q8_sums;
   int* q8_failure;
   uint32_t q8_pk;                // row stride of the codes = padded row count of the pair
+  // Raw kernels: the activations are bf16 rows [m][k] and the consumers quantise their own super-block (xvec: 16-byte loads)
+  const uint16_t* xraw;
+  uint32_t xk, xvec;
+  int* pack_failure;
 };
 
 __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
@@ -144,8 +149,9 @@ __device__ __forceinline__ void locate_tile(const GtParams& p, uint32_t T, uint3
   }
 }
 
-// NT = token octets (1: m <= 8, 2: m <= 16).  MAXW bounds the block size for register allocation.
-template <int NT, int MAXW, bool Dump>
+// NT = token octets (1: m <= 8, 2: m <= 16).  MAXW bounds the block size for register allocation.  Raw: the activations
+// are bf16 rows that the consumers quantise (a kernel of its own: the extra path costs the others registers).
+template <int NT, int MAXW, bool Dump, bool Raw>
 __global__ void __launch_bounds__(MAXW * 32, 1)
 gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_constant__ CUtensorMap tm_meta,
                 const __grid_constant__ CUtensorMap tm_codes1, const __grid_constant__ CUtensorMap tm_meta1,
@@ -408,6 +414,72 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
     uint32_t const rd_ap = tab + kTabBytes + q * 16;
     uint32_t bfrag[NT][8][2];  // int8 activations of token nt*8 + r: even / odd columns of 8q..8q+7 in group g
     uint32_t asplit[NT][3][2]; // tf32 terms of a*sum for token nt*8 + r, groups q and q+4
+    auto split = [&](int nt, int h, float as) {  // a * sum as three tf32 terms that add up to it exactly
+      uint32_t const hi = to_tf32(as);
+      float const r1 = as - __uint_as_float(hi);
+      uint32_t const mid = to_tf32(r1);
+      asplit[nt][0][h] = hi;
+      asplit[nt][1][h] = mid;
+      asplit[nt][2][h] = to_tf32(r1 - __uint_as_float(mid));
+    };
+    if constexpr (Raw) {
+      // bf16 rows: the warp quantises the 256 columns of its super-block, a token at a time with all lanes, four tokens per
+      // pass through its (still unused) decode table: codes [4][256], scales [4][8], sums [4][8].
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+#pragma unroll
+        for (int g = 0; g < 8; ++g) bfrag[nt][g][0] = bfrag[nt][g][1] = 0u;
+        split(nt, 0, 0.f);
+        split(nt, 1, 0.f);
+      }
+      for (uint32_t i = lane; i < NT * 64; i += 32) sts32f(tab + kTabBytes + i * 4, 0.f);
+      for (uint32_t t0 = 0; t0 < p.m; t0 += 4) {
+        __syncwarp();
+        for (uint32_t j = 0; j < 4 && t0 + j < p.m; ++j) {
+          const uint16_t* const src = p.xraw + size_t(t0 + j) * p.xk;
+          uint32_t const col = sb * 256 + lane * 8;
+          float x[8];
+          if (p.xvec && col + 8 <= p.xk) {
+            uint4 const v = *reinterpret_cast<const uint4*>(src + col);
+            uint32_t const vw[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { x[2 * i] = __uint_as_float(vw[i] << 16); x[2 * i + 1] = __uint_as_float(vw[i] & 0xffff0000u); }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) x[i] = col + i < p.xk ? bf16_bits_to_f32(src[col + i]) : 0.f;
+          }
+          Packed8 const z = quantize8(x);
+          asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(tab + j * 256 + lane * 8), "r"(z.w0), "r"(z.w1) : "memory");
+          if ((lane & 3) == 0) {
+            sts32f(tab + 1024 + (j * 8 + (lane >> 2)) * 4, z.a);
+            sts32f(tab + 1152 + (j * 8 + (lane >> 2)) * 4, float(z.sum));
+            if (!z.valid) atomicExch(p.pack_failure, 1);
+          }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+          uint32_t const j = nt * 8 + r - t0;  // this lane's fragment token in the pass
+          if (j < 4 && nt * 8 + r < p.m) {
+#pragma unroll
+            for (int g = 0; g < 8; ++g) {
+              uint32_t const at = tab + j * 256 + g * 32 + q * 8, z0 = lds32(at), z1 = lds32(at + 4);
+              bfrag[nt][g][0] = even_bytes(z0, z1);
+              bfrag[nt][g][1] = odd_bytes(z0, z1);
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              uint32_t const at = tab + 1024 + (j * 8 + q + 4 * h) * 4;
+              split(nt, h, __uint_as_float(lds32(at)) * __uint_as_float(lds32(at + 128)));
+            }
+          }
+        }
+        uint32_t const tok = t0 + (lane >> 3), g = lane & 7;
+        if (tok < p.m)
+          sts32f(tab + kTabBytes + ((tok & 7) >> 1) * 16 + ((tok >> 3) * 4 + g / 2) * 64 + (g % 2) * 8 + (tok & 1) * 4,
+                 __uint_as_float(lds32(tab + 1024 + ((lane >> 3) * 8 + g) * 4)));
+      }
+    } else {
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
       uint32_t const tokb = nt * 8 + r, tokc = nt * 8 + 2 * q;
@@ -430,14 +502,9 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
           size_t const i = size_t(tokb) * p.G + sb * 8 + q + 4 * h;
           as = p.xscales[i] * float(p.xsums[i]);
         }
-        uint32_t const hi = to_tf32(as);
-        float const r1 = as - __uint_as_float(hi);
-        uint32_t const mid = to_tf32(r1);
-        float const r2 = r1 - __uint_as_float(mid);
-        asplit[nt][0][h] = hi;
-        asplit[nt][1][h] = mid;
-        asplit[nt][2][h] = to_tf32(r2);
+        split(nt, h, as);
       }
+    }
     }
     __syncwarp();
     float2 const nmagic2 = make_float2(-kMagicF, -kMagicF);
@@ -651,8 +718,11 @@ struct Maps {
 
 template <int NT, int MAXW>
 cudaError_t launch_cfg(const Maps& t, const GtParams& p, bool dump, uint32_t grid, uint32_t smem, cudaStream_t stream) {
-  auto kernel = dump ? gemv_tma_kernel<NT, MAXW, true> : gemv_tma_kernel<NT, MAXW, false>;
-  cudaError_t st = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  auto kernel = dump ? gemv_tma_kernel<NT, MAXW, true, false> : gemv_tma_kernel<NT, MAXW, false, false>;
+  if constexpr (NT == 1) {
+    if (p.xraw != nullptr) kernel = gemv_tma_kernel<NT, MAXW, false, true>;
+  }
+  cudaError_t st = allow_smem(reinterpret_cast<const void*>(kernel), int(smem));
   if (st != cudaSuccess) return st;
   return launch_kernel(kernel, grid, (p.cw + kFirstReducer + NT) * 32, smem, stream, launch_overlap(), t.codes[0], t.meta[0],
                        t.codes[1], t.meta[1], t.codes[2], t.meta[2], p);
@@ -763,13 +833,14 @@ cudaError_t launch_gemv_tma(const WeightView& w, const Q8View& x, float* out, co
 }
 
 cudaError_t launch_gemv_tma_multi(const WeightView* ws, const GemvTmaOutput* outs, uint32_t count, bool swiglu_pair, const Q8View& x,
-                                  const GemvTmaPlan& plan, void* slices, uint32_t* tickets, int* status, cudaStream_t stream) {
+                                  const GemvTmaPlan& plan, void* slices, uint32_t* tickets, int* status, cudaStream_t stream,
+                                  const GemvTmaRaw* raw) {
   uint32_t const nt = x.m <= 8 ? 1 : 2;
   uint32_t const cw = plan.warps;
   if (count < 1 || count > 3 || (swiglu_pair && count != 2) || x.m == 0 || x.m > kGemvTmaMaxTokens || cw < 1 ||
       cw > (nt == 1 ? kGemvTmaMaxWarpsNarrow : kGemvTmaMaxWarpsWide) || plan.stages < 2 || plan.stages > uint32_t(kMaxStages) ||
       (plan.red_slots != 1 && plan.red_slots != 2) || smem_bytes(cw, nt, plan.stages, plan.red_slots) > kSmemBudget ||
-      (plan.split_k > 1 && (!slices || !tickets)) || (swiglu_pair && (plan.tiles_per_range & 1u)))
+      (plan.split_k > 1 && (!slices || !tickets)) || (swiglu_pair && (plan.tiles_per_range & 1u)) || (raw && nt != 1))
     return cudaErrorInvalidValue;
   Maps t{};
   GtParams p{};
@@ -791,6 +862,10 @@ cudaError_t launch_gemv_tma_multi(const WeightView* ws, const GemvTmaOutput* out
   p.tiles_per_range = plan.tiles_per_range; p.stages = plan.stages; p.red_slots = plan.red_slots;
   p.input_settled = plan.input_settled;
   p.nseg = count; p.pair = swiglu_pair ? 1u : 0u; p.n_total = total_rows;
+  if (raw) {
+    p.xraw = raw->x; p.xk = raw->k; p.pack_failure = raw->failure;
+    p.xvec = raw->k % 8 == 0 && reinterpret_cast<uintptr_t>(raw->x) % 16 == 0;
+  }
   uint32_t const grid = plan.ranges * plan.split_k, smem = smem_bytes(cw, nt, plan.stages, plan.red_slots);
   return launch_by_shape(nt, cw, t, p, false, grid, smem, stream);
 }

@@ -3,6 +3,10 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <map>
+#include <mutex>
+#include <utility>
+
 #include "common.cuh"
 
 namespace q4k {
@@ -141,8 +145,16 @@ struct GemvTmaOutput {
   uint16_t* out_bf16;
   const float* residual;
 };
+// raw, if given: the activations are still bf16 rows [m][k]; every block quantises its K slice itself (x then only says m
+// and padded_k), and a non-finite group raises *failure, as the pack kernel does.
+struct GemvTmaRaw {
+  const uint16_t* x;
+  uint32_t k;
+  int* failure;
+};
 cudaError_t launch_gemv_tma_multi(const WeightView* ws, const GemvTmaOutput* outs, uint32_t count, bool swiglu_pair, const Q8View& x,
-                                  const GemvTmaPlan& plan, void* slices, uint32_t* tickets, int* status, cudaStream_t stream);
+                                  const GemvTmaPlan& plan, void* slices, uint32_t* tickets, int* status, cudaStream_t stream,
+                                  const GemvTmaRaw* raw = nullptr);
 // The gate / up pair of an MLP in one launch whose reducer writes the Q8 activation of the down projection directly
 // (codes, scales, sums of bf16(silu(gate) * up), non-finite values raise `failure`): the reference's gate, up and
 // swiglu_pack launches in one.  The plan function says whether the shape qualifies (whole K in one block, rows a
@@ -172,6 +184,29 @@ cudaError_t launch_gemv_bf16w(const WeightView& w, const uint16_t* x, uint32_t m
 // (pack, dp4a, TMA gemv) are launched with programmatic stream serialization: they may start,
 // and the TMA kernel may prefetch weights, while the preceding kernel of the stream drains.
 bool launch_overlap();
+
+// cudaFuncSetAttribute(MaxDynamicSharedMemorySize), skipped where this thread has already asked for as much on the current
+// device (the runtime call costs a quarter of a microsecond on every launch).  The limit of a kernel is only ever raised,
+// so that what one thread remembers stays true whatever the others ask for.
+inline cudaError_t allow_smem(const void* kernel, int bytes) {
+  struct Seen { const void* kernel; int device, bytes; };
+  static thread_local Seen seen[64];
+  static std::mutex mutex;
+  static std::map<std::pair<const void*, int>, int> limits;
+  int device = 0;
+  cudaError_t st = cudaGetDevice(&device);
+  if (st != cudaSuccess) return st;
+  Seen& slot = seen[(reinterpret_cast<uintptr_t>(kernel) >> 4) % 64];
+  if (slot.kernel == kernel && slot.device == device && slot.bytes >= bytes) return cudaSuccess;
+  std::lock_guard<std::mutex> lock(mutex);
+  int& limit = limits[{kernel, device}];
+  if (limit < bytes) {
+    if ((st = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)) != cudaSuccess) return st;
+    limit = bytes;
+  }
+  slot = Seen{kernel, device, limit};
+  return cudaSuccess;
+}
 
 // Launch with or without the programmatic-stream-serialization attribute.
 template <typename... KArgs, typename... Args>

@@ -772,13 +772,7 @@ cudaError_t launch_f16(const WeightView& w, const Q8View& x, const TcOutput& o, 
   p.status = status; p.n = w.n; p.m = x.m; p.m_pad = m_pad; p.tiles_k = w.tiles_k; p.tok_tiles = m_pad / NT;
   uint32_t const steps = (w.padded_n + 2 * kRows - 1) / (2 * kRows) * p.tok_tiles * w.tiles_k / plan.unit_step;
   p.run_each = steps / plan.workers; p.run_rest = steps % plan.workers; p.unit_step = plan.unit_step;
-  static bool configured[64] = {};
-  int device = 0;
-  if ((st = cudaGetDevice(&device)) != cudaSuccess) return st;
-  if (device < 0 || device >= 64 || !configured[device]) {
-    if ((st = cudaFuncSetAttribute(mmq_f16_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem)) != cudaSuccess) return st;
-    if (device >= 0 && device < 64) configured[device] = true;
-  }
+  if ((st = allow_smem(reinterpret_cast<const void*>(mmq_f16_kernel<NT>), C::kSmem)) != cudaSuccess) return st;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = 2 * plan.workers;
   cfg.blockDim = C::kThreads;

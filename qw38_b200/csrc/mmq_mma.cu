@@ -291,7 +291,7 @@ cudaError_t launch_tt(const WeightView& w, const Q8View& x, float* out, const fl
   if (partials) kernel = wide ? mmq_mma_kernel<TT, true, true> : mmq_mma_kernel<TT, true, false>;
   else kernel = wide ? mmq_mma_kernel<TT, false, true> : mmq_mma_kernel<TT, false, false>;
   size_t const smem = smem_bytes(16 * TT, plan.kbs_per_step);
-  cudaError_t st = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  cudaError_t st = allow_smem(reinterpret_cast<const void*>(kernel), int(smem));
   if (st != cudaSuccess) return st;
   uint32_t const row_tiles = (w.padded_n / 8 + kWarps - 1) / kWarps;
   uint32_t const token_tiles = (x.m + 16 * TT - 1) / (16 * TT);

@@ -849,7 +849,7 @@ cudaError_t launch_ntok(const WeightView& w, const Q8View& x, const TcOutput& o,
       return cudaErrorInvalidValue;
   }
   auto kernel = partials ? mmq_tcgen05_kernel<NTOK, NCOL, true> : mmq_tcgen05_kernel<NTOK, NCOL, false>;
-  cudaError_t st = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
+  cudaError_t st = allow_smem(reinterpret_cast<const void*>(kernel), C::kSmem);
   if (st != cudaSuccess) return st;
   uint32_t const row_tiles = (w.padded_n + kRows - 1) / kRows, tok_tiles = (x.m + NTOK - 1) / NTOK;
   TcParams p{};

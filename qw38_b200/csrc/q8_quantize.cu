@@ -1,18 +1,13 @@
 // Activation producers: bf16/fp32 rows -> Q8 (int8 codes, fp32 scale, int32 sum per 32),
 // the fused RMS-norm and SwiGLU producers, and the 36-byte record export.
 //
-// Arithmetic contract (reference: q8_pack_warp, cuda/q8_device.cuh:5-25):
-//   peak = max |x| over the 32 values (columns >= k count as 0),
-//   a    = peak == 0 ? 1 : peak / 127      (IEEE fp32 division),
-//   z    = clamp(rint(x / a), -127, 127)   (round to nearest even),
-//   sum  = sum z.
-// A group with a non-finite value (or a scale that is not positive and finite)
-// stores zero codes, a NaN scale, sum 0 and raises the failure flag.
+// The arithmetic of a group is in q8_pack.cuh; columns >= k count as 0.  An invalid group raises the failure flag.
 //
 // Mapping: four lanes own one K32 group, eight values per lane, so a warp covers
 // 256 consecutive columns with 16-byte loads and 8-byte stores.
 #include "common.cuh"
 #include "launch.h"
+#include "q8_pack.cuh"
 
 namespace q4k {
 namespace {
@@ -22,41 +17,14 @@ constexpr int kThreads = 256;
 // Quantise the eight values of this lane; lanes (4j..4j+3) share a group.
 __device__ __forceinline__ void pack8(const float (&x)[8], int8_t* codes, float* scales,
                                       int32_t* sums, uint64_t group, uint32_t sub, int* failure) {
-  bool finite = true;
-  float peak = 0.f;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    bool f = isfinite(x[i]);
-    finite = finite && f;
-    peak = fmaxf(peak, f ? fabsf(x[i]) : 0.f);
-  }
-  peak = fmaxf(peak, __shfl_xor_sync(0xffffffffu, peak, 1));
-  peak = fmaxf(peak, __shfl_xor_sync(0xffffffffu, peak, 2));
-  int fin = finite ? 1 : 0;
-  fin &= __shfl_xor_sync(0xffffffffu, fin, 1);
-  fin &= __shfl_xor_sync(0xffffffffu, fin, 2);
-  float const a = peak == 0.f ? 1.f : __fdiv_rn(peak, 127.f);
-  bool const valid = fin && isfinite(a) && a > 0.f;
-  int z[8];
-  int sum = 0;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    z[i] = valid ? max(-127, min(127, __float2int_rn(__fdiv_rn(x[i], a)))) : 0;
-    sum += z[i];
-  }
-  sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-  sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-  uint32_t w0 = (uint32_t(z[0]) & 255u) | ((uint32_t(z[1]) & 255u) << 8) |
-                ((uint32_t(z[2]) & 255u) << 16) | ((uint32_t(z[3]) & 255u) << 24);
-  uint32_t w1 = (uint32_t(z[4]) & 255u) | ((uint32_t(z[5]) & 255u) << 8) |
-                ((uint32_t(z[6]) & 255u) << 16) | ((uint32_t(z[7]) & 255u) << 24);
+  Packed8 const r = quantize8(x);
   uint32_t* dst = reinterpret_cast<uint32_t*>(codes + group * 32 + sub * 8);
-  dst[0] = w0;
-  dst[1] = w1;
+  dst[0] = r.w0;
+  dst[1] = r.w1;
   if (sub == 0) {
-    scales[group] = valid ? a : __int_as_float(0x7fc00000);
-    sums[group] = sum;
-    if (!valid) atomicExch(failure, 1);
+    scales[group] = r.a;
+    sums[group] = r.sum;
+    if (!r.valid) atomicExch(failure, 1);
   }
 }
 
@@ -237,7 +205,7 @@ cudaError_t launch_hidden_rms_q8(const float* residual, const uint16_t* gamma, f
                                  uint32_t hidden, Q8Out out, int* failure, cudaStream_t stream) {
   size_t const smem = size_t(hidden) * 2;
   if (smem > 48 * 1024) {
-    cudaError_t st = cudaFuncSetAttribute(hidden_rms_q8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    cudaError_t st = allow_smem(reinterpret_cast<const void*>(hidden_rms_q8_kernel), int(smem));
     if (st != cudaSuccess) return st;
   }
   hidden_rms_q8_kernel<<<out.m, kThreads, smem, stream>>>(residual, gamma, eps, hidden, out.codes, out.scales, out.sums, failure);

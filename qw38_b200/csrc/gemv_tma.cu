@@ -102,6 +102,8 @@ struct GtParams {
   const uint16_t* xraw;
   uint32_t xk, xvec;
   int* pack_failure;
+  // pair == 2: two reducer warps per octet take alternate groups of four tiles, each through a hand-off slot of its own
+  uint32_t reducers;
 };
 
 __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
@@ -172,9 +174,14 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
   volatile int* const abort_flag = flags;
   int* const last_flag = flags + 1;
 
-  constexpr uint32_t kFirstConsumer = kFirstReducer + NT;
+  uint32_t const kFirstConsumer = kFirstReducer + NT * p.reducers;
   uint32_t const warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint32_t const slot_mask = p.red_slots - 1, slot_shift = p.red_slots - 1;  // red_slots is 1 or 2
+  // hand-off slot of the block's it-th tile, and how often the slot was used before
+  auto hand_off = [&](uint32_t it, uint32_t& slot, uint32_t& use) {
+    if (p.reducers == 2) { slot = (it >> 2) & 1; use = (it >> 3) * 4 + (it & 3); }
+    else { slot = it & slot_mask; use = it >> slot_shift; }
+  };
   uint32_t const range = blockIdx.x / p.split_k, slice = blockIdx.x % p.split_k;
   uint32_t const sb0 = slice * cw;
   uint32_t const nact = min(cw, p.tiles_k - sb0);  // consumer warps with a real super-block
@@ -224,7 +231,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
   } else if (warp < kFirstConsumer) {
     // One reducer warp per token octet adds the consumers' 16 x 8 tiles in warp order.  Lane
     // (r = lane/4, q = lane%4) owns rows r, r+8 and tokens 2q, 2q+1 -- the MMA accumulator layout.
-    uint32_t const nt = warp - kFirstReducer;
+    uint32_t const nt = (warp - kFirstReducer) % NT, turn = (warp - kFirstReducer) / NT;
     uint32_t const r = lane >> 2, q = lane & 3;
     pdl_wait();
     pdl_launch_dependents();  // after the wait: the next launch never runs beside anything older than this one
@@ -244,9 +251,11 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
       // pair mode the even tiles are the gate's, the odd ones the up projection's, and bf16(SiLU(gate) * up) is
       // written once both are known.  Same hand-off and summation order as the plain form below.
       float g00 = 0.f, g01 = 0.f, g10 = 0.f, g11 = 0.f;
-      float px[4] = {0.f, 0.f, 0.f, 0.f};  // pair == 2: the values of the group's first tile
+      float pg[4], pu[4];  // pair == 2: gate and up values of the group's first half
       for (uint32_t it = 0; it < ntiles; ++it) {
-        uint32_t const s = it & slot_mask, use = it >> slot_shift;
+        if (p.reducers == 2 && ((it >> 2) & 1) != turn) continue;
+        uint32_t s, use;
+        hand_off(it, s, use);
         if (!mbar_wait(b_rfull + 8 * s, use & 1, abort_flag, p.status, 0x520)) break;
         float2 lo = make_float2(0.f, 0.f), hi = make_float2(0.f, 0.f);
         uint32_t src = s_red + s * red_slot + nt * 512 + lane * 16;
@@ -278,18 +287,23 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
           if (sg == 0) { g00 = v00; g01 = v01; g10 = v10; g11 = v11; continue; }
           if (p.pair == 2) {
             // The activation of the down projection, quantised here (the arithmetic of swiglu_pack_kernel,
-            // cuda/q4k_q8.cu:52-61): x = bf16(g / (1 + exp(-g)) * u), a non-finite input poisons the value.
+            // cuda/q4k_q8.cu:52-61): x = bf16(g / (1 + exp(-g)) * u), a non-finite input poisons the value.  The first
+            // half's values are kept as they are: the exponentials and divisions of a group come after its last hand-off,
+            // while the other reducer takes the next group's tiles (one reducer for all made a tile 2.8 us, not 1.5).
+            if ((local & 1u) == 0) {
+              pg[0] = g00; pg[1] = g01; pg[2] = g10; pg[3] = g11;
+              pu[0] = v00; pu[1] = v01; pu[2] = v10; pu[3] = v11;
+              continue;
+            }
             auto act = [](float gv, float uv) {
               float v = (gv / (1.f + expf(-gv))) * uv;
               if (!isfinite(gv) || !isfinite(uv)) v = __int_as_float(0x7fc00000);
               return bf16_bits_to_f32(f32_to_bf16_rne(v));
             };
             float const cx[4] = {act(g00, v00), act(g01, v01), act(g10, v10), act(g11, v11)};  // (row r | r+8) x (token 0 | 1)
-            if ((local & 1u) == 0) {
+            float px[4];
 #pragma unroll
-              for (int i = 0; i < 4; ++i) px[i] = cx[i];
-              continue;
-            }
+            for (int i = 0; i < 4; ++i) px[i] = act(pg[i], pu[i]);
             // Second tile of a 32-row group: this lane holds rows r, r+8, 16+r, 24+r of the group for two tokens; the
             // eight lanes with the same q hold the rest.
 #pragma unroll
@@ -359,8 +373,9 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
         }
       }
     } else
-    for (uint32_t it = 0; it < ntiles; ++it) {
-      uint32_t const s = it & slot_mask, use = it >> slot_shift;
+    for (uint32_t it = 0; turn == 0 && it < ntiles; ++it) {
+      uint32_t s, use;
+      hand_off(it, s, use);
       if (!mbar_wait(b_rfull + 8 * s, use & 1, abort_flag, p.status, 0x520)) break;
       float2 lo = make_float2(0.f, 0.f), hi = make_float2(0.f, 0.f);
       uint32_t src = s_red + s * red_slot + nt * 512 + lane * 16;
@@ -609,7 +624,8 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
       float4 const dd_lo = lds128f(rd_dd);        // {d, d, -dmin, -dmin} of row r
       float4 const dd_hi = lds128f(rd_dd + 8 * kTabRow);  // row r+8
       // ---- hand the tile to the reducer ----
-      uint32_t const rs = it & slot_mask, ruse = it >> slot_shift;
+      uint32_t rs, ruse;
+      hand_off(it, rs, ruse);
       if (ruse > 0 && !mbar_wait(b_rempty + 8 * rs, (ruse - 1) & 1, abort_flag, p.status, 0x540)) break;
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt) {
@@ -724,7 +740,7 @@ cudaError_t launch_cfg(const Maps& t, const GtParams& p, bool dump, uint32_t gri
   }
   cudaError_t st = allow_smem(reinterpret_cast<const void*>(kernel), int(smem));
   if (st != cudaSuccess) return st;
-  return launch_kernel(kernel, grid, (p.cw + kFirstReducer + NT) * 32, smem, stream, launch_overlap(), t.codes[0], t.meta[0],
+  return launch_kernel(kernel, grid, (p.cw + kFirstReducer + NT * p.reducers) * 32, smem, stream, launch_overlap(), t.codes[0], t.meta[0],
                        t.codes[1], t.meta[1], t.codes[2], t.meta[2], p);
 }
 
@@ -741,8 +757,8 @@ bool make_weight_maps(const WeightView& w, uint32_t cw, CUtensorMap* codes, CUte
 template <class... A>
 cudaError_t launch_by_shape(uint32_t nt, uint32_t cw, A&&... a) {
   if (nt == 1) {
-    if (cw <= 12) return launch_cfg<1, 14>(a...);
-    return launch_cfg<1, kGemvTmaMaxWarpsNarrow + 2>(a...);
+    if (cw <= 12) return launch_cfg<1, 15>(a...);
+    return launch_cfg<1, kGemvTmaMaxWarpsNarrow + 3>(a...);
   }
   if (cw <= 12) return launch_cfg<2, 15>(a...);
   return launch_cfg<2, kGemvTmaMaxWarpsWide + 3>(a...);
@@ -827,6 +843,7 @@ cudaError_t launch_gemv_tma(const WeightView& w, const Q8View& x, float* out, co
   p.row_tiles = (w.padded_n + 15) / 16; p.cw = cw; p.split_k = plan.split_k;
   p.tiles_per_range = plan.tiles_per_range; p.stages = plan.stages; p.red_slots = plan.red_slots;
   p.input_settled = plan.input_settled;
+  p.reducers = 1;
   uint32_t const grid = plan.ranges * plan.split_k, smem = smem_bytes(cw, nt, plan.stages, plan.red_slots);
   bool const dump = partials != nullptr;
   return launch_by_shape(nt, cw, t, p, dump, grid, smem, stream);
@@ -862,6 +879,7 @@ cudaError_t launch_gemv_tma_multi(const WeightView* ws, const GemvTmaOutput* out
   p.tiles_per_range = plan.tiles_per_range; p.stages = plan.stages; p.red_slots = plan.red_slots;
   p.input_settled = plan.input_settled;
   p.nseg = count; p.pair = swiglu_pair ? 1u : 0u; p.n_total = total_rows;
+  p.reducers = 1;
   if (raw) {
     p.xraw = raw->x; p.xk = raw->k; p.pack_failure = raw->failure;
     p.xvec = raw->k % 8 == 0 && reinterpret_cast<uintptr_t>(raw->x) % 16 == 0;
@@ -878,6 +896,13 @@ bool plan_gemv_tma_swiglu_q8(uint32_t m, const WeightView& gate, GemvTmaPlan* pl
   // a group of 32 rows = gate tile, up tile, gate tile, up tile: four consecutive tiles in one block
   p.tiles_per_range = (p.tiles_per_range + 3) / 4 * 4;
   p.ranges = (tiles + p.tiles_per_range - 1) / p.tiles_per_range;
+  // One octet: two reducers, a hand-off slot for each, where two ring stages still fit beside them.  (Two octets have two
+  // reducers already, and two more warps would take eight registers from every thread.)
+  if (m <= 8) {
+    uint32_t stages = 0;
+    while (stages < uint32_t(kMaxStages) && smem_bytes(p.warps, 1, stages + 1, 2) <= kSmemBudget) ++stages;
+    if (stages >= 2) { p.stages = stages; p.red_slots = 2; }
+  }
   *plan = p;
   return true;
 }
@@ -907,6 +932,7 @@ cudaError_t launch_gemv_tma_swiglu_q8(const WeightView& gate, const WeightView& 
   p.tiles_per_range = plan.tiles_per_range; p.stages = plan.stages; p.red_slots = plan.red_slots;
   p.input_settled = 0;
   p.nseg = 2; p.pair = 2; p.n_total = 2 * gate.n;
+  p.reducers = nt == 1 ? plan.red_slots : 1;
   p.q8_codes = out.codes; p.q8_scales = out.scales; p.q8_sums = out.sums; p.q8_failure = failure; p.q8_pk = out.padded_k;
   uint32_t const grid = plan.ranges, smem = smem_bytes(cw, nt, plan.stages, plan.red_slots);
   return launch_by_shape(nt, cw, t, p, false, grid, smem, stream);

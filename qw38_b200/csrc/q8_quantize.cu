@@ -114,9 +114,14 @@ __device__ __forceinline__ float block_reduce(float v, float* scratch, bool is_m
   return r;
 }
 
-// Max-scaled RMS norm, (1 + gamma) gain, bf16 rounding, then the Q8 pack of the
-// rounded row (reference: hidden_rms_kernel<3>, cuda/activation.cu:134-190).
-// One block per token; hidden % 256 == 0; dynamic shared memory = hidden * 2 bytes.
+// Max-scaled RMS norm, (1 + gamma) gain, bf16 rounding, then the Q8 pack of the rounded row (reference:
+// hidden_rms_kernel<3>, cuda/activation.cu:134-190).  One block per token; hidden % 256 == 0; dynamic shared memory =
+// hidden * 2 bytes.  Thread t owns columns t, t + 256, ... and sums them in that order.
+//
+// Bound: latency (a decode step has a handful of rows).  With Held > 0 (hidden <= 256 * Held) a thread requests its whole
+// share of the row and of the gain at once and keeps it in registers for the three passes; the loop form, which serves
+// wider rows, waits for memory in every iteration of every pass: 15 us at 5120 columns against 4 us.
+template <int Held>
 __global__ void __launch_bounds__(kThreads) hidden_rms_q8_kernel(const float* __restrict__ residual,
                                                                   const uint16_t* __restrict__ gamma,
                                                                   float eps, uint32_t hidden,
@@ -125,22 +130,53 @@ __global__ void __launch_bounds__(kThreads) hidden_rms_q8_kernel(const float* __
   extern __shared__ __align__(16) uint16_t rounded[];
   __shared__ float scratch[kThreads / 32];
   const float* x = residual + uint64_t(blockIdx.x) * hidden;
+  float held[Held > 0 ? Held : 1], gain[Held > 0 ? Held : 1];
   float scale = 0.f;
-  for (uint32_t i = threadIdx.x; i < hidden; i += kThreads) scale = fmaxf(scale, fabsf(x[i]));
+  if constexpr (Held > 0) {
+#pragma unroll
+    for (int j = 0; j < Held; ++j) {
+      uint32_t const i = threadIdx.x + j * kThreads;
+      held[j] = i < hidden ? x[i] : 0.f;
+      gain[j] = i < hidden ? bf16_bits_to_f32(gamma[i]) : 0.f;
+    }
+#pragma unroll
+    for (int j = 0; j < Held; ++j) scale = fmaxf(scale, fabsf(held[j]));
+  } else {
+#pragma unroll 8
+    for (uint32_t i = threadIdx.x; i < hidden; i += kThreads) scale = fmaxf(scale, fabsf(x[i]));
+  }
   scale = block_reduce(scale, scratch, true);
   float const safe = scale == 0.f ? 1.f : scale;
   float sumsq = 0.f;
-  for (uint32_t i = threadIdx.x; i < hidden; i += kThreads) {
-    float s = x[i] / safe;
-    sumsq += s * s;
+  if constexpr (Held > 0) {
+#pragma unroll
+    for (int j = 0; j < Held; ++j) {
+      held[j] = held[j] / safe;
+      if (threadIdx.x + j * kThreads < hidden) sumsq += held[j] * held[j];
+    }
+  } else {
+#pragma unroll 8
+    for (uint32_t i = threadIdx.x; i < hidden; i += kThreads) {
+      float s = x[i] / safe;
+      sumsq += s * s;
+    }
   }
   sumsq = block_reduce(sumsq, scratch, false);
   float const se = sqrtf(eps) / safe;
   float const inv = 1.0f / sqrtf(sumsq / float(hidden) + se * se);
-  for (uint32_t i = threadIdx.x; i < hidden; i += kThreads) {
-    float g = bf16_bits_to_f32(gamma[i]);
-    float v = (1.0f + g) * ((x[i] / safe) * inv);
-    rounded[i] = f32_to_bf16_rne(v);
+  if constexpr (Held > 0) {
+#pragma unroll
+    for (int j = 0; j < Held; ++j) {
+      uint32_t const i = threadIdx.x + j * kThreads;
+      if (i < hidden) rounded[i] = f32_to_bf16_rne((1.0f + gain[j]) * (held[j] * inv));
+    }
+  } else {
+#pragma unroll 4
+    for (uint32_t i = threadIdx.x; i < hidden; i += kThreads) {
+      float g = bf16_bits_to_f32(gamma[i]);
+      float v = (1.0f + g) * ((x[i] / safe) * inv);
+      rounded[i] = f32_to_bf16_rne(v);
+    }
   }
   __syncthreads();
   uint32_t const lane = threadIdx.x & 31, sub = lane & 3, grp = lane >> 2;
@@ -204,11 +240,13 @@ cudaError_t launch_swiglu_pack_q8(const float* gate, const float* up, Q8Out out,
 cudaError_t launch_hidden_rms_q8(const float* residual, const uint16_t* gamma, float eps,
                                  uint32_t hidden, Q8Out out, int* failure, cudaStream_t stream) {
   size_t const smem = size_t(hidden) * 2;
+  // 48 registers hold a thread's share of rows up to 6144 columns; half of that leaves room for twice the rows in flight.
+  auto kernel = hidden <= 8 * kThreads ? hidden_rms_q8_kernel<8> : (hidden <= 24 * kThreads ? hidden_rms_q8_kernel<24> : hidden_rms_q8_kernel<0>);
   if (smem > 48 * 1024) {
-    cudaError_t st = allow_smem(reinterpret_cast<const void*>(hidden_rms_q8_kernel), int(smem));
+    cudaError_t st = allow_smem(reinterpret_cast<const void*>(kernel), int(smem));
     if (st != cudaSuccess) return st;
   }
-  hidden_rms_q8_kernel<<<out.m, kThreads, smem, stream>>>(residual, gamma, eps, hidden, out.codes, out.scales, out.sums, failure);
+  kernel<<<out.m, kThreads, smem, stream>>>(residual, gamma, eps, hidden, out.codes, out.scales, out.sums, failure);
   return cudaGetLastError();
 }
 

@@ -231,8 +231,8 @@ int project_f16(const q4k_weight& w, const q4k_q8_input& x, const q4k::TcOutput&
   if (!status) return Q4K_ERR_STATUS;
   q4k::F16Plan const plan = q4k::plan_f16(x.m, w.n, w.padded_k / 256);
   q4k::StreamScratch scratch;
-  Q4K_CUDA(scratch.acquire(stream, q4k::f16_scratch_bytes(x.m, w.padded_k / 256, plan)), "scratch.acquire");
-  Q4K_CUDA(q4k::launch_mmq_f16(view(w), view(x), out, plan, scratch.p(), status, stream), "q4k_q8.mmq_f16");
+  Q4K_CUDA(scratch.acquire(stream, q4k::f16_scratch_bytes(x.m, w.padded_k / 256, plan), q4k::launch_overlap()), "scratch.acquire");
+  Q4K_CUDA(q4k::launch_mmq_f16(view(w), view(x), out, plan, scratch.p(), scratch.alternates(), status, stream), "q4k_q8.mmq_f16");
   Q4K_CUDA(scratch.release(), "scratch.release");
   return Q4K_OK;
 }
@@ -317,7 +317,9 @@ int project_impl(const q4k_weight* weight, const q4k_q8_input& x, float* output,
   if (kernel == Q4K_KERNEL_F16) {
     if (!q4k::f16_supported(view(w), view(x)) || partials)
       return fail(Q4K_ERR_INVALID_ARGUMENT, "q8.project: the fp16 kernel needs aligned operands and has no partial dots");
-    return project_f16(w, x, q4k::tc_output(output, res), stream);
+    q4k::TcOutput to = q4k::tc_output(output, res);
+    to.input_settled = (opt && (opt->flags & kFlagInputSettled)) ? 1u : 0u;
+    return project_f16(w, x, to, stream);
   }
   if (kernel == Q4K_KERNEL_TCGEN05) {
     if (!q4k::tcgen05_supported(view(w), view(x)))

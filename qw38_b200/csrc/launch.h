@@ -92,7 +92,8 @@ cudaError_t launch_mmq_tcgen05(const WeightView& w, const Q8View& x, const TcOut
                                const TcPlan& plan, void* partial_tiles, uint32_t* tickets, int* status, cudaStream_t stream);
 
 // mmq_f16.cu : tcgen05 kind::f16 on SM pairs, weights expanded into TMEM, activations as two fp16 planes.  scratch holds
-// f16_scratch_bytes (256-byte aligned) and is used until the launch ends.
+// f16_scratch_bytes (256-byte aligned) and is used until the launch ends.  alternates: the preceding launch of the stream
+// does not use this scratch, so (with launch overlap and a settled input) the planes may be written beside it.
 struct F16Plan {
   uint32_t nt;             // tokens per tile: 16, 32, 64 or 128
   uint32_t chunk;          // tokens per pass
@@ -103,8 +104,8 @@ struct F16Plan {
 bool f16_supported(const WeightView& w, const Q8View& x);
 F16Plan plan_f16(uint32_t m, uint32_t n, uint32_t tiles_k);
 uint64_t f16_scratch_bytes(uint32_t m, uint32_t tiles_k, const F16Plan& plan);
-cudaError_t launch_mmq_f16(const WeightView& w, const Q8View& x, const TcOutput& out, const F16Plan& plan, void* scratch, int* status,
-                           cudaStream_t stream);
+cudaError_t launch_mmq_f16(const WeightView& w, const Q8View& x, const TcOutput& out, const F16Plan& plan, void* scratch, bool alternates,
+                           int* status, cudaStream_t stream);
 
 // gemv_tma.cu : m <= 16.  Weights streamed by TMA into a shared-memory ring, activations held in
 // registers by warps that each own one super-block column of the block's K slice; K slices of

@@ -15,7 +15,7 @@
 //   * the products (at most 21 bits) are exact and the tensor core accumulates them in fp32; per accumulator only the 16
 //     steps of one super-block are added before it is drained and folded into fp32 registers.
 //   * min term: m is exact in fp16, a*s is split into two fp16 terms like x, and one more MMA of K = 16 (eight groups, hi
-//     and lo) per super-block adds their products into an accumulator of its own.
+//     and lo) per super-block puts the sum of their products into an accumulator of its own.
 // Error against the equation in double precision: 1.8e-7 to 2.2e-7 of the result's norm at K = 256 .. 17408 (the int8 kernel:
 // 0.7e-7 to 2.3e-7).
 //
@@ -54,7 +54,7 @@ namespace q4k {
 namespace {
 
 constexpr int kRows = 128;  // weight rows per CTA; a pair covers 256
-constexpr int kExpanders = 8, kFirstExpander = 4;  // expander warps that share a super-block; the first of them
+constexpr int kFirstExpander = 4;
 
 template <int NT> struct F16Cfg {
   // Up to 32 tokens the hi and lo planes lie side by side along N (an MMA of N = 32 costs nearly as much as one of 64);
@@ -66,20 +66,23 @@ template <int NT> struct F16Cfg {
   static constexpr int kColSplit = NT >= 128 ? 4 : (NT >= 32 ? 2 : 1);
   static constexpr int kCols = NT / kColSplit;          // tokens per epilogue warp (lane = row)
   static constexpr int kEpilogueWarps = 4 * kColSplit;
-  // Up to 64 tokens two groups of expanders take alternate super-blocks: one group needs ~1200 clk for one, a
-  // super-block of 64 tokens 1112 clk of tensor time and 790 clk of HBM time.
-  static constexpr int kGroups = NT >= 128 ? 1 : 2;
+  // Expanders: groups take alternate super-blocks; within a group four warps (one per TMEM lane quarter) times kSplit halves
+  // of K.  Few warps with long instruction streams: every warp more is another one that retries its waits.
+  static constexpr int kGroups = NT >= 128 ? 1 : 2, kSplit = NT >= 128 ? 2 : 1, kExpanders = 4 * kSplit;
   static constexpr int kFirstEpilogue = kFirstExpander + kGroups * kExpanders;
   static constexpr int kWarps = kFirstEpilogue + kEpilogueWarps, kThreads = kWarps * 32;
   // The block starts with kLaunchRegs registers per thread; control, expander and epilogue warps redistribute them.
-  static constexpr int kLaunchRegs = 65536 / kThreads / 8 * 8;
-  static constexpr int kRegsControl = 40, kRegsExpander = 56;
+  // Up to 64 tokens two warps' worth stays free: a block of planes_kernel for the next projection fits beside this one.
+  static constexpr int kBoundThreads = NT >= 128 ? kThreads : kThreads + 64;
+  static constexpr int kLaunchRegs = 65536 / ((kBoundThreads + 127) / 128 * 128) / 8 * 8;  // what ptxas gives (checked before the first launch)
+  static constexpr int kRegsControl = 40, kRegsExpander = kSplit == 2 ? 56 : 72;
   static constexpr int kRegsLeft = (kWarps * kLaunchRegs - 4 * kRegsControl - kGroups * kExpanders * kRegsExpander) / kEpilogueWarps / 8 * 8;
   static constexpr int kRegsEpilogue = kRegsLeft > 160 ? 160 : kRegsLeft;
   // TMEM: two accumulators, one min-term accumulator, weight stages.  A group of expanders always uses the same kQ stages
   // (one super-block), so that a warp sees every phase of the barriers it waits on.
   static constexpr int kQ = kStack ? 2 : 4, kACols = 128 / kQ, kAStages = kGroups * kQ;
-  static constexpr int kD2Col = 2 * kN, kACol = kD2Col + kN2;
+  static constexpr int kD2Bufs = NT <= 64 ? 2 : 1;  // with one, the min-term MMA waits for the previous super-block's epilogue
+  static constexpr int kD2Col = 2 * kN, kACol = kD2Col + kD2Bufs * kN2;
   static_assert(kACol + kAStages * kACols <= 512, "TMEM columns");
   // operand stage: plane boxes, then a*s of kTRows tokens as a K-major operand without swizzle ([hi | lo][row][16 bytes])
   static constexpr int kBRows = kStack ? NT : NT / 2;   // plane rows per box and CTA
@@ -248,9 +251,12 @@ __device__ __forceinline__ float power_of_two(int e) { return __uint_as_float(ui
 __global__ void __launch_bounds__(256) planes_kernel(const int8_t* __restrict__ codes, const float* __restrict__ scales,
                                                      const int32_t* __restrict__ sums, uint32_t m, uint32_t m_pad, uint32_t tiles_k,
                                                      __half* __restrict__ planes, __half* __restrict__ sums16, float* __restrict__ exps,
-                                                     float* __restrict__ tokens, uint32_t* __restrict__ tickets, uint32_t ticket_count) {
+                                                     float* __restrict__ tokens, uint32_t* __restrict__ tickets, uint32_t ticket_count,
+                                                     bool early) {
   __shared__ float warp_top[8];
-  pdl_wait();
+  // early: the input is older than the preceding launch and the scratch is not the one that launch reads, so the planes
+  // are written while it runs; only the grid's completion, which the matmul waits for, still follows it (block 0).
+  if (!early) pdl_wait();
   pdl_launch_dependents();
   if (blockIdx.x == 0)
     for (uint32_t i = threadIdx.x; i < ticket_count; i += 256) tickets[i] = 0u;
@@ -276,6 +282,7 @@ __global__ void __launch_bounds__(256) planes_kernel(const int8_t* __restrict__ 
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < 8; ++i) row = fmaxf(row, warp_top[i]);
+  if (early && blockIdx.x == 0) pdl_wait();
   if (!live) return;
   float top = fabsf(a);
 #pragma unroll
@@ -310,7 +317,7 @@ __global__ void __launch_bounds__(256) planes_kernel(const int8_t* __restrict__ 
 
 // ---- the matmul ------------------------------------------------------------------------------------
 template <int NT>
-__global__ void __launch_bounds__(F16Cfg<NT>::kThreads, 1)
+__global__ void __launch_bounds__(F16Cfg<NT>::kBoundThreads, 1)
 mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_constant__ CUtensorMap tm_meta,
                const __grid_constant__ CUtensorMap tm_planes, const __grid_constant__ CUtensorMap tm_sums, const F16Params p) {
   using C = F16Cfg<NT>;
@@ -352,10 +359,10 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
   if (warp == 0) {
     for (uint32_t i = lane; i < uint32_t(C::kBars); i += 32) {  // in the order of the offsets above
       uint32_t count = 1;
-      if (i >= C::kRawStages && i < oBb) count = kExpanders;                                      // raw_free
+      if (i >= C::kRawStages && i < oBb) count = C::kExpanders;                                   // raw_free
       else if (i >= oAb && i < oAb + C::kAStages) count = 2 * 4;                                  // a_full: four warps of both CTAs
       else if (i >= oDb + 2 && i < oSb) count = 2 * C::kEpilogueWarps;                            // d_free
-      else if (i >= oSb) count = i < oSb + C::kSclStages ? kExpanders / 2 + 1 : C::kEpilogueWarps;  // s_full | s_free
+      else if (i >= oSb) count = i < oSb + C::kSclStages ? 4 + 1 : C::kEpilogueWarps;  // s_full | s_free
       mbar_init(bar0 + 8 * i, count);
     }
     if (lane == 0) *abort_flag = 0;
@@ -435,7 +442,7 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
             for (int q = 0; q < C::kQ; ++q) {
               bool const last = C::kStack || pass == 1;  // the stage's last use
               if (pass == 0) ok = ok && mbar_wait_inline(a_full(a0 + q), g_.phase, abort_flag, p.status, 0x806);
-              if (last && q == C::kQ - 1 && u > u0) ok = ok && mbar_wait_inline(d_free(before.s), before.phase, abort_flag, p.status, 0x807);
+              if (C::kD2Bufs == 1 && last && q == C::kQ - 1 && u > u0) ok = ok && mbar_wait_inline(d_free(before.s), before.phase, abort_flag, p.status, 0x807);
               if (!ok) break;
               tc_fence_after();
               uint32_t const at = tmem + C::kACol + (a0 + q) * C::kACols;
@@ -448,7 +455,7 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
                 else mma_pair<true>(dt, at + i * 8, b, idesc);
               }
               if (last && q == C::kQ - 1)  // m * (a*s): sixteen K columns = eight groups, hi and lo; the mins serve both (K stride 0)
-                mma_pair_ss(tmem + C::kD2Col, umma_desc_plain(smem + C::oMins + g_.s * C::kMins, 0, 128),
+                mma_pair_ss(tmem + C::kD2Col + (C::kD2Bufs - 1) * d_.s * C::kN2, umma_desc_plain(smem + C::oMins + g_.s * C::kMins, 0, 128),
                             umma_desc_plain(stage + C::kPlanes, C::kTRows * 16, 128), idesc2);
               if (last) commit_pair(a_free(a0 + q));
             }
@@ -466,8 +473,8 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
     }
   } else if (warp < C::kFirstEpilogue) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kRegsExpander));
-    // ---- expanders: warp (quarter, half) turns its 32 rows' groups 4 half .. 4 half + 3 into fp16 in TMEM.  Lane = row.
-    uint32_t const quarter = warp & 3, half = ((warp - kFirstExpander) >> 2) & 1, group = (warp - kFirstExpander) / kExpanders;
+    // ---- expanders: a warp turns its 32 rows' share of K into fp16 in TMEM.  Lane = row.
+    uint32_t const quarter = warp & 3, part = ((warp - kFirstExpander) >> 2) % C::kSplit, group = (warp - kFirstExpander) / C::kExpanders;
     uint32_t const row = quarter * 32 + lane;
     uint32_t const a_full0 = map_to(a_full(0), 0);
     Ring<C::kRawStages> r_;
@@ -481,24 +488,24 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
       if (!mbar_wait_inline(raw_full(r), r_.phase, abort_flag, p.status, 0x808)) break;
       uint32_t const raw = smem + C::oRaw + r * C::kRaw;
       uint4 const cm = lds128(raw + 16 * 1024 + row * 16);
-      uint4 w[4];
+      constexpr int kMyGroups = 8 / C::kSplit;
+      uint4 w[kMyGroups];
 #pragma unroll
-      for (int g = 0; g < 4; ++g) w[g] = lds128(raw + row * 128 + (((half * 4 + g) ^ (row & 7)) << 4));
-      if (half == 0) {
+      for (int g = 0; g < kMyGroups; ++g) w[g] = lds128(raw + row * 128 + (((part * kMyGroups + g) ^ (row & 7)) << 4));
+      if (part == 0) {
         if (!mbar_wait_inline(s_free(sc), t_.phase ^ 1, abort_flag, p.status, 0x809)) break;
         // The tensor core truncates when it accumulates, which shortens a super-block's sum by 2^-22 on average (measured
         // on normal data, sixteen steps): the row scale takes the mean of that out.
         sts64f(smem + C::oScl + sc * C::kScl + row * 8, fp16_bits_to_f32(cm.x & 0xffffu) * (1.f + 0x1p-22f), -32.f * fp16_bits_to_f32(cm.x >> 16));
       }
-      uint32_t const scw = half == 0 ? (cm.y & 0x3f3f3f3fu) : ((cm.w & 0x0f0f0f0fu) | ((cm.y >> 2) & 0x30303030u));
-      constexpr int kMine = C::kQ / 2, kGroupsPer = 4 / kMine;  // stages of this warp, K32 groups per stage
+      ScaleMinWords const sm = decode_scale_min(cm.y, cm.z, cm.w);
+      constexpr int kMine = C::kQ / C::kSplit, kGroupsPer = 8 / C::kQ;  // stages of this warp, K32 groups per stage
 #pragma unroll
       for (int i = 0; i < kMine; ++i) {
-        uint32_t const sa = group * C::kQ + half * kMine + i;
+        uint32_t const sa = group * C::kQ + part * kMine + i;
         if (!mbar_wait_inline(a_free(sa), phase ^ 1, abort_flag, p.status, 0x80a)) { ok = false; break; }
         tc_fence_after();
-        if (half == 1 && i == kMine - 1) {
-          ScaleMinWords const sm = decode_scale_min(cm.y, cm.z, cm.w);
+        if (part == C::kSplit - 1 && i == kMine - 1) {
           uint32_t mh[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
@@ -512,7 +519,8 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
 #pragma unroll
         for (int gg = 0; gg < kGroupsPer; ++gg) {
           int const g = i * kGroupsPer + gg;
-          __half2 const S = __hsub2(u2h(__byte_perm(scw, 0x64646464u, 0x4040 | (g * 0x0101))), u2h(0x64006400u));
+          uint32_t const scw = C::kSplit == 1 ? (g < 4 ? sm.sc_lo : sm.sc_hi) : (part == 0 ? sm.sc_lo : sm.sc_hi);
+          __half2 const S = __hsub2(u2h(__byte_perm(scw, 0x64646464u, 0x4040 | ((g & 3) * 0x0101))), u2h(0x64006400u));
           // low nibbles: (1024 + q) * sc - 1024 sc; high nibbles, four bits up: (1024 + 16 q) * (sc / 16) - 64 sc
           __half2 const S16 = __hmul2(S, u2h(0x2c002c00u)), B = __hmul2(S, u2h(0xe400e400u)), B16 = __hmul2(S, u2h(0xd400d400u));
           uint32_t const ww[4] = {w[g].x, w[g].y, w[g].z, w[g].w};
@@ -533,7 +541,7 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
         if (lane == 0) arrive_cluster(a_full0 + 8 * sa);
       }
       if (lane == 0) {
-        if (half == 0) mbar_arrive(s_full(sc));
+        if (part == 0) mbar_arrive(s_full(sc));
         mbar_arrive(raw_free(r));
       }
 #pragma unroll
@@ -572,7 +580,7 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
         // Columns beyond a short tile's hold stale words: they are read and folded like the others and never stored.
         tmem_ld<W>(lane_base + d * C::kN + c0, P);
         if constexpr (C::kStack) tmem_ld<W>(lane_base + d * C::kN + cols + c0, L);
-        tmem_ld<W>(lane_base + C::kD2Col + c0, M);
+        tmem_ld<W>(lane_base + C::kD2Col + (C::kD2Bufs - 1) * d * C::kN2 + c0, M);
         tmem_wait_ld();
         if (c0 + W == C::kCols) {  // everything of this super-block is in registers
           tc_fence_before();
@@ -726,7 +734,7 @@ Carve carve(uint32_t m, uint32_t tiles_k, const F16Plan& plan) {
 }
 
 template <int NT>
-cudaError_t launch_f16(const WeightView& w, const Q8View& x, const TcOutput& o, const F16Plan& plan, uint8_t* scratch, int* status,
+cudaError_t launch_f16(const WeightView& w, const Q8View& x, const TcOutput& o, const F16Plan& plan, uint8_t* scratch, bool early, int* status,
                        cudaStream_t stream) {
   using C = F16Cfg<NT>;
   Carve const c = carve(x.m, w.tiles_k, plan);
@@ -735,7 +743,7 @@ cudaError_t launch_f16(const WeightView& w, const Q8View& x, const TcOutput& o, 
   cudaError_t st = launch_kernel(planes_kernel, grid, 256, 0, stream, launch_overlap(), x.codes, x.scales, x.sums, x.m, m_pad, w.tiles_k,
                                  reinterpret_cast<__half*>(scratch + c.planes), reinterpret_cast<__half*>(scratch + c.sums),
                                  reinterpret_cast<float*>(scratch + c.exps), reinterpret_cast<float*>(scratch + c.tokens),
-                                 reinterpret_cast<uint32_t*>(scratch), plan.unit_step == 1 ? uint32_t(kTicketBytes / 4) : 0u);
+                                 reinterpret_cast<uint32_t*>(scratch), plan.unit_step == 1 ? uint32_t(kTicketBytes / 4) : 0u, early);
   if (st != cudaSuccess) return st;
   CUtensorMap tm_codes, tm_meta, tm_planes, tm_sums;
   uint64_t const rgs = w.padded_n / 8;
@@ -772,6 +780,14 @@ cudaError_t launch_f16(const WeightView& w, const Q8View& x, const TcOutput& o, 
   p.status = status; p.n = w.n; p.m = x.m; p.m_pad = m_pad; p.tiles_k = w.tiles_k; p.tok_tiles = m_pad / NT;
   uint32_t const steps = (w.padded_n + 2 * kRows - 1) / (2 * kRows) * p.tok_tiles * w.tiles_k / plan.unit_step;
   p.run_each = steps / plan.workers; p.run_rest = steps % plan.workers; p.unit_step = plan.unit_step;
+  // setmaxnreg.inc waits for registers that the block must have been launched with: a build that allotted fewer than the
+  // split assumes may not run.
+  static cudaError_t const built = [] {
+    cudaFuncAttributes attr{};
+    cudaError_t const e = cudaFuncGetAttributes(&attr, mmq_f16_kernel<NT>);
+    return e != cudaSuccess ? e : (attr.numRegs < C::kLaunchRegs ? cudaErrorInvalidConfiguration : cudaSuccess);
+  }();
+  if (built != cudaSuccess) return built;
   if ((st = allow_smem(reinterpret_cast<const void*>(mmq_f16_kernel<NT>), C::kSmem)) != cudaSuccess) return st;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = 2 * plan.workers;
@@ -828,12 +844,13 @@ uint64_t f16_scratch_bytes(uint32_t m, uint32_t tiles_k, const F16Plan& plan) {
   return carve(m < plan.chunk ? m : plan.chunk, tiles_k, plan).total;
 }
 
-cudaError_t launch_mmq_f16(const WeightView& w, const Q8View& x, const TcOutput& out, const F16Plan& plan, void* scratch, int* status,
-                           cudaStream_t stream) {
+cudaError_t launch_mmq_f16(const WeightView& w, const Q8View& x, const TcOutput& out, const F16Plan& plan, void* scratch, bool alternates,
+                           int* status, cudaStream_t stream) {
   if (out.ndst < 1 || out.ndst > 8 || (out.out_bf16 ? out.ndst != 1 : out.out[0] == nullptr) || plan.workers < 1 ||
       plan.workers > kMaxClusters)
     return cudaErrorInvalidValue;
   uint64_t const stride = out.stride ? out.stride : w.n;
+  bool const early = alternates && launch_overlap() && out.input_settled && x.m <= plan.chunk;
   for (uint32_t t0 = 0; t0 < x.m; t0 += plan.chunk) {
     Q8View xc = x;
     uint64_t const G = x.padded_k / 32;
@@ -857,10 +874,10 @@ cudaError_t launch_mmq_f16(const WeightView& w, const Q8View& x, const TcOutput&
     uint8_t* const s = static_cast<uint8_t*>(scratch);
     cudaError_t st;
     switch (plan.nt) {
-      case 16: st = launch_f16<16>(w, xc, oc, pc, s, status, stream); break;
-      case 32: st = launch_f16<32>(w, xc, oc, pc, s, status, stream); break;
-      case 64: st = launch_f16<64>(w, xc, oc, pc, s, status, stream); break;
-      case 128: st = launch_f16<128>(w, xc, oc, pc, s, status, stream); break;
+      case 16: st = launch_f16<16>(w, xc, oc, pc, s, early, status, stream); break;
+      case 32: st = launch_f16<32>(w, xc, oc, pc, s, early, status, stream); break;
+      case 64: st = launch_f16<64>(w, xc, oc, pc, s, early, status, stream); break;
+      case 128: st = launch_f16<128>(w, xc, oc, pc, s, early, status, stream); break;
       default: return cudaErrorInvalidValue;
     }
     if (st != cudaSuccess) return st;

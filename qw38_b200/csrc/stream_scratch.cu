@@ -5,7 +5,8 @@
 //     the next synchronisation; two streams or threads never share a block.
 //   * Captured calls: one block per capture and stream, because an allocation recorded as a graph node would separate
 //     kernels that may overlap.  The graph owns the block through a user object; when the graph and its executables are
-//     gone it serves the next capture (or goes back to the pool, beyond kMaxFree idle blocks).
+//     gone it serves the next capture (or goes back to the pool, beyond kMaxFree idle blocks).  Calls that may overlap the
+//     one before them take the two halves of the block in turn.
 #include "stream_scratch.h"
 
 #include <mutex>
@@ -23,6 +24,7 @@ struct CapturedBlock {
   int device = 0;
   unsigned long long capture = 0;  // 0 = idle
   cudaStream_t stream = nullptr;
+  uint32_t turn = 0;
 };
 
 struct Pool {
@@ -70,14 +72,19 @@ void CUDART_CB retire_captured(void* data) {
   static_cast<CapturedBlock*>(data)->capture = 0;
 }
 
-cudaError_t captured_block(cudaStream_t stream, cudaGraph_t graph, unsigned long long capture, int device, uint64_t bytes, void** out) {
+cudaError_t captured_block(cudaStream_t stream, cudaGraph_t graph, unsigned long long capture, int device, uint64_t bytes, bool alternate, void** out) {
+  uint64_t const half = (bytes + 255) / 256 * 256;
+  if (alternate) bytes = 2 * half;
+  auto take = [&](CapturedBlock* b) {  // the calls of a block all alternate: its halves are half its size
+    *out = static_cast<uint8_t*>(b->p) + (alternate ? (b->turn++ & 1) * (b->bytes / 512 * 256) : 0);
+  };
   std::lock_guard<std::mutex> lock(g_mutex);
   CapturedBlock* idle = nullptr;
   size_t idle_count = 0;
   for (CapturedBlock* b : g_blocks) {
     if (b->device != device) continue;
     if (b->capture == capture && b->stream == stream && b->bytes >= bytes) {
-      *out = b->p;
+      take(b);
       return cudaSuccess;
     }
     if (b->capture == 0) {
@@ -116,13 +123,13 @@ cudaError_t captured_block(cudaStream_t stream, cudaGraph_t graph, unsigned long
     idle->capture = ~0ull;  // the object still refers to it: not reused
     return st;
   }
-  *out = idle->p;
+  take(idle);
   return cudaSuccess;
 }
 
 }  // namespace
 
-cudaError_t StreamScratch::acquire(cudaStream_t stream, uint64_t bytes) {
+cudaError_t StreamScratch::acquire(cudaStream_t stream, uint64_t bytes, bool alternate) {
   int device = 0;
   cudaError_t st = cudaGetDevice(&device);
   if (st != cudaSuccess) return st;
@@ -130,7 +137,10 @@ cudaError_t StreamScratch::acquire(cudaStream_t stream, uint64_t bytes) {
   unsigned long long capture = 0;
   cudaGraph_t graph = nullptr;
   if ((st = cudaStreamGetCaptureInfo(stream, &status, &capture, &graph)) != cudaSuccess) return st;
-  if (status == cudaStreamCaptureStatusActive) return captured_block(stream, graph, capture + 1, device, bytes, &p_);
+  if (status == cudaStreamCaptureStatusActive) {
+    alternates_ = alternate;
+    return captured_block(stream, graph, capture + 1, device, bytes, alternate, &p_);
+  }
   Pool* pool = nullptr;
   {
     std::lock_guard<std::mutex> lock(g_mutex);

@@ -9,7 +9,10 @@ namespace q4k {
 // whatever other streams, threads and graphs do.  Nothing about its contents may be assumed.
 class StreamScratch {
  public:
-  cudaError_t acquire(cudaStream_t stream, uint64_t bytes);
+  // alternate: for calls whose first kernel may run beside the call before it on the stream.  Where alternates() then says
+  // so, p() is not what that call was given.
+  cudaError_t acquire(cudaStream_t stream, uint64_t bytes, bool alternate = false);
+  bool alternates() const { return alternates_; }
   cudaError_t release();
   void* p() const { return p_; }
   ~StreamScratch() { (void)release(); }
@@ -21,6 +24,7 @@ class StreamScratch {
   void* p_ = nullptr;
   cudaStream_t stream_ = nullptr;
   bool owned_ = false;  // to be freed in stream order
+  bool alternates_ = false;
 };
 
 }  // namespace q4k

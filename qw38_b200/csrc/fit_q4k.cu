@@ -13,6 +13,11 @@
 // explicit round-to-nearest intrinsic so that no multiply-add is contracted (the reference
 // builds its host code with -ffp-contract=off, src/CMakeLists.txt:35-37).
 //
+// Bound: the FMA pipe.  A candidate costs 16 operations per weight -- four to find its level, six for the moments, six for
+// the error -- and the levels stay in registers between the two sums (96 of the 128 registers hold weights, importances
+// and levels; more blocks with fewer registers would have to find the levels twice).  5120 x 17408: 1.34 ms, 1.75 ms with
+// levels clamped by fmaxf / fminf and found again for the error.
+//
 // A block of 128 threads fits 16 consecutive super-blocks.  Their 4096 weights are loaded with
 // coalesced reads into shared memory at a row stride of 33 words, from where each thread takes
 // "its" 32 weights into registers without bank conflicts.  Output is either the logical form of the
@@ -45,47 +50,55 @@ __device__ __forceinline__ int nearest(float v) {
 }
 __device__ __forceinline__ int level(float v) { return min(15, max(0, nearest(v))); }
 
-// The same rounding kept as a float: (v + 1.5 * 2^23) - 1.5 * 2^23 is v rounded to the nearest even integer
-// whenever |v| < 2^22, and clamping that to [0, 15] gives float(level(v)) without a conversion
-// instruction.  Only used where the caller has bounded |v|.
-__device__ __forceinline__ float level_bounded(float v) {
-  return fminf(fmaxf(sub(add(v, 12582912.f), 12582912.f), 0.f), 15.f);
+// What the caller knows of grid * d: nothing, |grid * d| < 2^22, or that and grid * d < 15.5.
+enum class Range { kAny, kBounded, kBelowTop };
+
+// float(level(grid * d)).  With |grid * d| < 2^22 the product, scaled by 1/16 (exactly: grid16 = grid / 16), is clamped to
+// [0, 1] by the multiplication itself, rounded to a multiple of 1/16 by the bias 1.5 * 2^19, and brought back by one exact
+// multiply-add: four operations on the FMA pipe with the subtraction before them, where clamping with fmaxf and fminf costs
+// two more at half rate.  What is left above 15 needs the fminf, unless the caller knows better.
+template <Range R>
+__device__ __forceinline__ float level_f(float grid, float grid16, float d) {
+  if constexpr (R == Range::kAny) return float(level(mul(grid, d)));
+  float t;
+  asm("mul.rn.sat.f32 %0, %1, %2;" : "=f"(t) : "f"(grid16), "f"(d));
+  float const l = __fmaf_rn(add(t, 786432.f), 16.f, -12582912.f);
+  return R == Range::kBelowTop ? l : fminf(l, 15.f);
 }
-template <bool Bounded>
-__device__ __forceinline__ float level_f(float v) { return Bounded ? level_bounded(v) : float(level(v)); }
 
 struct GroupFit {
   float scale, the_min;  // results of the search: step and (negated) minimum
   float grid, origin;    // the levels the search settled on are level(grid * (x - origin))
 };
 
+template <Range R>
+__device__ __forceinline__ void levels(const float (&x)[32], float grid, float origin, float (&l)[32]) {
+  float const grid16 = mul(grid, 0.0625f);
+#pragma unroll
+  for (int i = 0; i < 32; ++i) l[i] = level_f<R>(grid, grid16, sub(x[i], origin));
+}
+
 struct Moments { float l, l2, xl; };
 
 // Weighted moments of the levels a candidate grid assigns (the middle loop of the search).
-template <bool Bounded>
-__device__ __forceinline__ Moments moments(const float (&x)[32], const float (&w)[32], float grid, float origin) {
+__device__ __forceinline__ Moments moments(const float (&x)[32], const float (&w)[32], const float (&l)[32]) {
   Moments s{0.f, 0.f, 0.f};
 #pragma unroll
   for (int i = 0; i < 32; ++i) {
-    float const v = x[i];
-    float const l = level_f<Bounded>(mul(grid, sub(v, origin)));
-    float const wl = mul(w[i], l);
+    float const wl = mul(w[i], l[i]);
     s.l = add(s.l, wl);
-    s.l2 = add(s.l2, mul(wl, l));
-    s.xl = add(s.xl, mul(wl, v));
+    s.l2 = add(s.l2, mul(wl, l[i]));
+    s.xl = add(s.xl, mul(wl, x[i]));
   }
   return s;
 }
 
 // Weighted squared error of step * level + base against the weights.
-template <bool Bounded>
-__device__ __forceinline__ float fit_error(const float (&x)[32], const float (&w)[32], float grid, float origin, float step, float base) {
+__device__ __forceinline__ float fit_error(const float (&x)[32], const float (&w)[32], const float (&l)[32], float step, float base) {
   float err = 0.f;
 #pragma unroll
   for (int i = 0; i < 32; ++i) {
-    float const v = x[i];
-    float const l = level_f<Bounded>(mul(grid, sub(v, origin)));
-    float const diff = sub(add(mul(step, l), base), v);
+    float const diff = sub(add(mul(step, l[i]), base), x[i]);
     err = add(err, mul(w[i], mul(diff, diff)));
   }
   return err;
@@ -118,16 +131,24 @@ __device__ GroupFit fit_group(const float (&x)[32], float average) {
   }
   float grid = quo(15.f, sub(hi, lo));
   float scale = quo(1.f, grid);
-  float best = fit_error<false>(x, w, grid, lo, scale, lo);
+  float l[32];
+  levels<Range::kAny>(x, grid, lo, l);
+  float best = fit_error(x, w, l, scale, lo);
   fit.grid = grid; fit.origin = lo;
   float floor_ = lo;  // the minimum candidates quantise against; moves when one is accepted
+#pragma unroll 1
   for (int step = 0; step <= 20; ++step) {
     // (rmin + rdelta*step + nmax) / (max - min), with the minimum as moved so far.
-    float const cand_grid = quo(add(add(-1.f, mul(0.1f, float(step))), 15.f), sub(hi, floor_));
+    float const span = sub(hi, floor_);
+    float const cand_grid = quo(add(add(-1.f, mul(0.1f, float(step))), 15.f), span);
     // Every grid * (x - origin) of this candidate is bounded by |grid| times the larger distance of
     // the extreme weights from the origin (rounding is monotonic); below 2^22 the float rounding applies.
-    bool const bounded = mul(fabsf(cand_grid), fmaxf(fabsf(sub(hi, floor_)), fabsf(sub(x_min, floor_)))) < 4194304.f;
-    Moments const s = bounded ? moments<true>(x, w, cand_grid, floor_) : moments<false>(x, w, cand_grid, floor_);
+    // With a positive span the largest of them is that of hi, 14 + step / 10 give or take two roundings.
+    bool const bounded = mul(fabsf(cand_grid), fmaxf(fabsf(span), fabsf(sub(x_min, floor_)))) < 4194304.f;
+    if (!bounded) levels<Range::kAny>(x, cand_grid, floor_, l);
+    else if (step < 15 && span > 0.f) levels<Range::kBelowTop>(x, cand_grid, floor_, l);
+    else levels<Range::kBounded>(x, cand_grid, floor_, l);
+    Moments const s = moments(x, w, l);
     float const det = sub(mul(sum_w, s.l2), mul(s.l, s.l));
     if (!(det > 0.f)) continue;
     float cand_scale = quo(sub(mul(sum_w, s.xl), mul(sum_x, s.l)), det);
@@ -136,8 +157,7 @@ __device__ GroupFit fit_group(const float (&x)[32], float average) {
       cand_min = 0.f;
       cand_scale = quo(s.xl, s.l2);
     }
-    float const err = bounded ? fit_error<true>(x, w, cand_grid, floor_, cand_scale, cand_min)
-                              : fit_error<false>(x, w, cand_grid, floor_, cand_scale, cand_min);
+    float const err = fit_error(x, w, l, cand_scale, cand_min);
     if (err < best) {
       best = err;
       scale = cand_scale;

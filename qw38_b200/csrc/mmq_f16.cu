@@ -216,11 +216,6 @@ __device__ __forceinline__ void tmem_st16(uint32_t t, const uint32_t (&r)[16]) {
                  "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
 }
 __device__ __forceinline__ float lds32f(uint32_t a) { return __uint_as_float(lds32(a)); }
-__device__ __forceinline__ float ldg_here(const float* a) {  // not to be hoisted (sixty-four of them would spill)
-  float v;
-  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(a));
-  return v;
-}
 __device__ __forceinline__ uint32_t round32(uint32_t v) { return (v + 31) / 32 * 32; }
 __device__ __forceinline__ uint32_t f16_idesc(uint32_t n) { return (1u << 4) | ((n >> 3) << 17) | (uint32_t(256 >> 4) << 24); }  // f16 -> f32, M = 256
 __device__ __forceinline__ float2 as_float2(const uint32_t* r) { return make_float2(__uint_as_float(r[0]), __uint_as_float(r[1])); }
@@ -611,6 +606,8 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
 
       // ---- end of this cluster's part of the tile
       uint32_t const tile = c.row_pair * p.tok_tiles + c.tok;
+      // lane t's share of the tokens' powers of two, requested now and handed round below
+      float const token_scale = __ldcg(p.tokens + c.tok * NT + col0 + (C::kCols < 32 ? lane & 15 : lane));
       bool write = true;
       if (max(u0, tile * KB) != tile * KB || u + 1 != (tile + 1) * KB) {
         // Partial: [cluster][first or later tile of its run][CTA][warp][token / 4][lane].
@@ -654,6 +651,9 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
           }
         }
       }
+#pragma unroll
+      for (int j = 0; j < C::kCols / 2; ++j)
+        acc[j] = __fmul2_rn(acc[j], make_float2(__shfl_sync(0xffffffffu, token_scale, 2 * j), __shfl_sync(0xffffffffu, token_scale, 2 * j + 1)));
       // A lane's values are one row of consecutive tokens: every store of a warp is 32 neighbouring rows of one token.
       uint32_t const n_row = (c.row_pair * 2 + cta) * kRows + row, tok0 = c.tok * NT + col0;
       if (write && n_row < p.n && tok0 < p.m) {
@@ -664,7 +664,7 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
           if (j0 >= live) break;
           float v[8];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) v[j] = ((j & 1) ? acc[(j0 + j) / 2].y : acc[(j0 + j) / 2].x) * ldg_here(p.tokens + tok0 + j0 + j);
+          for (int j = 0; j < 8; ++j) v[j] = (j & 1) ? acc[(j0 + j) / 2].y : acc[(j0 + j) / 2].x;
           if (p.residual) {
 #pragma unroll
             for (int j = 0; j < 8; ++j)

@@ -266,12 +266,11 @@ int project_impl(const q4k_weight* weight, const q4k_q8_input& x, float* output,
 
   uint32_t kernel = opt ? opt->kernel : Q4K_KERNEL_AUTO;
   if (kernel == Q4K_KERNEL_AUTO) {
-    // Up to sixteen tokens: the TMA-streamed kernel when the weights are 16-byte aligned (for a
-    // single token only with overlapped launches, where its early weight prefetch pays; serialised,
-    // dp4a measured a little faster there), else dp4a / cluster MMA.  Beyond: tcgen05 when TMA
-    // alignment allows.
+    // One token: dp4a (5120 x 5120 to 34816 x 5120 in 5.1 .. 17.3 us, the TMA-streamed kernel 6.5 .. 22.5; two tokens
+    // 6.1 .. 21.7 against 6.7 .. 22.4, and slower in a chain of layers).  Up to sixteen: the TMA-streamed kernel when the
+    // weights are 16-byte aligned, else dp4a / cluster MMA.  Beyond: tcgen05 when TMA alignment allows.
     bool const tma_ok = x.m <= q4k::kGemvTmaMaxTokens && q4k::gemv_tma_supported(view(w), view(x));
-    if (tma_ok && (x.m >= 2 || q4k::launch_overlap())) kernel = Q4K_KERNEL_GEMV_TMA;
+    if (tma_ok && x.m > q4k::kGemvDp4aBestTokens) kernel = Q4K_KERNEL_GEMV_TMA;
     else if (x.m <= 2 || (x.m <= q4k::kGemvDp4aMaxTokens && w.padded_n >= 32768)) kernel = Q4K_KERNEL_GEMV_DP4A;
     else if (x.m <= 16) kernel = Q4K_KERNEL_GEMV_MMA;
     else if (!partials && !(opt && opt->split_k) && q4k::f16_supported(view(w), view(x))) kernel = Q4K_KERNEL_F16;
@@ -282,7 +281,10 @@ int project_impl(const q4k_weight* weight, const q4k_q8_input& x, float* output,
                     unsigned(w.k), role, unsigned(res != nullptr), kernel == Q4K_KERNEL_GEMV_DP4A ? "integer_dp4a" : "integer_mma");
   if (kernel == Q4K_KERNEL_GEMV_DP4A) {
     if (x.m > q4k::kGemvDp4aMaxTokens) return fail(Q4K_ERR_INVALID_ARGUMENT, "q8.project: dp4a kernel takes m <= 4");
-    Q4K_CUDA(q4k::launch_gemv_dp4a(view(w), view(x), output, res, partials, stream), "q4k_q8.gemv_dp4a");
+    int* const status = q4k::kernel_status_word();
+    if (!status) return Q4K_ERR_STATUS;
+    Q4K_CUDA(q4k::launch_gemv_dp4a(view(w), view(x), output, res, partials, opt && (opt->flags & kFlagInputSettled), status, stream),
+             "q4k_q8.gemv_dp4a");
     return Q4K_OK;
   }
   if (kernel == Q4K_KERNEL_GEMV_MMA) {
@@ -719,6 +721,13 @@ int decode_fused(const q4k_decode_desc* const* descs, uint32_t count, bool swigl
   if (!raw)
     if (int st = decode_pack(*descs[0], q8, failure, stream)) return st;
   q4k::GemvTmaRaw const rows{descs[0]->input, descs[0]->weight.k, failure};
+  if (raw && !swiglu && q8.m <= q4k::kGemvDp4aBestTokens) {
+    int* const status = q4k::kernel_status_word();
+    if (!status) return Q4K_ERR_STATUS;
+    Q4K_CUDA(q4k::launch_gemv_dp4a_multi(ws, outs, count, q8.m, q8.padded_k, rows, status, stream), "decode_mmv.fused");
+    *fused = true;
+    return Q4K_OK;
+  }
   q4k::GemvTmaPlan plan = q4k::plan_gemv_tma_tiles(q8.m, uint32_t(tiles), ws[0].tiles_k, 0, 0, swiglu);
   uint64_t const partial_bytes = plan.split_k > 1 ? uint64_t(plan.split_k) * q8.m * n_total * 4 : 0;
   void* scratch = nullptr;

@@ -1,48 +1,72 @@
-// Decode GEMV for 1..4 tokens: HBM-bound stream over the split-tile Q4_K weights on dp4a.
+// GEMV for 1..4 tokens on dp4a: every warp streams its own run of weights through a private ring of bulk copies.
 //
 // Equation per output (reference: mmvq, cuda/q4k_q8.cu:63-101):
 //   out[t][row] = sum_g a[t,g] * ((d*sc_g) * dot_g - (dmin*m_g) * sum[t,g]) (+ residual)
-// with dot_g an exact int32 dot of 32 unsigned 4-bit codes and 32 int8 activations, reset for
-// every K32 group.  The kernel is issue-bound before it is bandwidth-bound, so the mapping is
-// chosen to spend few instructions per byte:
-//   * a warp iteration covers two super-blocks of one row group (2 KiB of codes); lane
-//     (h = lane/16, r = (lane/2)%8, j = lane%2) owns row r, super-block h and the four K32
-//     groups 4j..4j+3: four 16-byte code loads and one 16-byte metadata load per iteration,
-//     both six-bit words of the lane's four groups come out of one byte-parallel decode;
-//   * low nibbles (even columns) go through (w & 0x0f0f0f0f), high nibbles (odd columns)
-//     through (w & 0xf0f0f0f0) with an unsigned-by-signed dp4a, which yields 16 * dot and is
-//     shifted back once per group -- no per-word shift;
-//   * per super-block and row, d and dmin are applied once: X = sum a_g * (sc_g * dot_g),
-//     Y = sum m_g * (a_g * sum_g), acc += d * X - dmin * Y, the integer products converted
-//     to fp32 by the 1.5 * 2^23 bias trick on the integer pipe;
-//   * activations are staged once per block in shared memory as (even bytes, odd bytes) words,
-//     the two halves of a super-block 144 bytes apart so the two j lanes hit different banks.
-// A block of 8 warps takes `rgc` row groups and splits each one's K range over 8/rgc warps;
-// slice sums are added in slice order.
+// with dot_g an exact int32 dot of 32 unsigned 4-bit codes and 32 int8 activations, reset for every K32 group.
+//
+// Bound: HBM for one token, the integer pipe (sixteen dp4a per lane, token and super-block) from two on.  To get to the
+// first, few instructions are spent per byte and copies are in flight all the time:
+//   * The weights of a block (consecutive row groups of eight rows) are one list of super-blocks [8 rows][256 columns] that
+//     lie one after another in memory (1 KiB of codes, 128 B of metadata each).  The list is cut evenly over the fifteen
+//     consumer warps, wherever the cuts fall: all warps end together, whatever K and the row count are.
+//   * A warp fetches its run by cp.async.bulk, two super-blocks per stage, into a ring that nobody else touches: no barrier
+//     between warps in the main loop, and the copies start before the activations are known.
+//   * One super-block: lane (r = lane / 4, q = lane % 4) owns row r and groups 2q, 2q+1 -- three 16-byte loads for the
+//     weights, two per token and group for the activations.  Odd rows take their two groups in the other order, so that
+//     eight neighbouring lanes read eight different 16-byte bank groups.  Low nibbles (even columns) go through
+//     (w & 0x0f0f0f0f), high nibbles (odd columns) through (w & 0xf0f0f0f0) with an unsigned-by-signed dp4a, which yields
+//     16 * dot; products with the six-bit scale are converted by the 1.5 * 2^23 bias trick on the integer pipe.
+//   * Row sums are held in shared memory (one slot per warp and row group it touches) and added in warp order at the end.
+//   * Up to two tokens a block stays within half of an SM's registers and shared memory, so that with overlapped launches
+//     the next projection's copies run beside this one's end.  A control warp waits for the preceding launch and then lets
+//     the next one start, while the others already work when the caller flagged the input as settled.
+// Activations are staged once per block as (even bytes, odd bytes) words, or quantised right there from bf16 rows (Raw).
+//
 #include "common.cuh"
 #include "launch.h"
+#include "q8_pack.cuh"
+#include "tma.cuh"
 
 namespace q4k {
 namespace {
 
-constexpr int kThreads = 256;
-constexpr int kWarps = 8;
-constexpr int kActKb = 288;  // bytes of staged activations per token and super-block (128 + 16 pad + 128 + 16 pad)
+constexpr uint32_t kWarps = 15, kConsumers = kWarps * 32, kThreads = kConsumers + 32;
+constexpr uint32_t kStageUnits = 2, kStageBytes = kStageUnits * (1024 + 128);
+constexpr uint32_t kMaxStages = 4;
+constexpr uint32_t kHalfSm = 113 * 1024, kWholeSm = 227 * 1024;
+constexpr uint32_t kMaxRowGroups = 64;  // per block: bounds the slots of the row sums
 constexpr uint32_t kMagicI = 0x4B400000u;
 constexpr float kMagicF = 12582912.0f;
 
-__device__ __forceinline__ uint4 load16(const uint8_t* p, bool wide) {
-  if (wide) return __ldg(reinterpret_cast<const uint4*>(p));
-  const uint32_t* q = reinterpret_cast<const uint32_t*>(p);
-  return make_uint4(__ldg(q), __ldg(q + 1), __ldg(q + 2), __ldg(q + 3));
-}
-__device__ __forceinline__ uint4 load16_meta(const uint8_t* p, bool wide) {
-  if (wide) return __ldg(reinterpret_cast<const uint4*>(p));
-  const uint16_t* q = reinterpret_cast<const uint16_t*>(p);
-  uint32_t h[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) h[i] = __ldg(q + i);
-  return make_uint4(h[0] | (h[1] << 16), h[2] | (h[3] << 16), h[4] | (h[5] << 16), h[6] | (h[7] << 16));
+struct DpSegment {
+  const uint8_t* codes;
+  const uint8_t* meta;
+  float* out;
+  uint16_t* out_bf16;
+  const float* residual;
+  uint32_t n;
+  uint32_t rg0, u0;  // its first row group and super-block among the launch's
+};
+struct DpParams {
+  DpSegment seg[3];
+  const int8_t* codes;
+  const float* scales;
+  const int32_t* sums;
+  const uint16_t* raw;  // Raw: bf16 rows [M][k]; vec: 16-byte loads
+  uint32_t k, vec;
+  int* failure;
+  int32_t* partials;
+  int* status;
+  uint32_t nseg, rgs, tiles_k;
+  uint32_t rgs_each, rgs_rest;  // row groups per block; the first rgs_rest blocks take one more
+  uint32_t stages, parts;       // ring stages and row-sum slots of a warp
+  uint32_t wide;                // weights are 16-byte aligned: bulk copies
+  uint32_t input_settled;
+};
+
+__device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
 
 __device__ __forceinline__ int dp4a_us(uint32_t a, uint32_t b, int c) {  // unsigned bytes x signed bytes
@@ -65,177 +89,321 @@ __device__ __forceinline__ int dot32(const uint4& w, const uint4& z0, const uint
   return lo + (hi >> 4);  // hi is an exact multiple of 16
 }
 
-// Shared memory: [M][tiles_k][288] permuted codes | [M][G] a | [M][G] a*float(sum) | [8 warps][8 rows][M] slice sums
-template <int M, bool Dump>
-__global__ void __launch_bounds__(kThreads) gemv_dp4a_kernel(WeightView w, Q8View x, float* __restrict__ out,
-                                                             const float* __restrict__ residual,
-                                                             int32_t* __restrict__ partials, uint32_t rgc, bool wide) {
-  extern __shared__ __align__(16) uint8_t smem[];
-  pdl_wait();  // activations (and the residual) may come from the kernel before this one
-  pdl_launch_dependents();  // after the wait: the next launch never runs beside anything older than this one
-  uint32_t const pk = x.padded_k, G = pk / 32, tiles_k = w.tiles_k;
-  uint8_t* const zs = smem;
-  float* const as = reinterpret_cast<float*>(smem + size_t(M) * tiles_k * kActKb);
-  float* const ws = as + size_t(M) * G;
-  float* const red = ws + size_t(M) * G;
+// Segment of super-block u (of the launch).
+__device__ __forceinline__ const DpSegment& segment_of(const DpParams& p, uint32_t u) {
+  uint32_t s = 0;
+  if (p.nseg > 1 && u >= p.seg[1].u0) s = 1;
+  if (p.nseg > 2 && u >= p.seg[2].u0) s = 2;
+  return p.seg[s];
+}
 
-  uint32_t const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t const h = lane >> 4, r = (lane >> 1) & 7, j = lane & 1;
-  uint32_t const ks = kWarps / rgc;
-  uint32_t const rg = blockIdx.x * rgc + warp / ks, slice = warp % ks;
-  uint32_t const rgs = w.padded_n / 8;
-  bool const active = rg < rgs;
-  uint32_t const kb0 = (slice * tiles_k) / ks, kb1 = ((slice + 1) * tiles_k) / ks;
-
-  const uint8_t* const cp = w.codes + (uint64_t(active ? rg : 0) * tiles_k) * 1024 + r * 128 + j * 64;
-  const uint8_t* const mp = w.meta + (uint64_t(active ? rg : 0) * tiles_k) * 128 + r * 16;
-
-  // First weight loads go out before the activation staging so they overlap it.
-  uint4 wq[4], wm;
-  uint32_t kb = kb0 + h;
-  bool have = active && kb < kb1;
+// Super-blocks of the stage that starts at super-block u: they share a segment.
+__device__ __forceinline__ uint32_t stage_units(const DpParams& p, uint32_t u, uint32_t end) {
+  uint32_t left = end - u;
+  if (p.nseg > 1) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) wq[i] = make_uint4(0, 0, 0, 0);
-  wm = make_uint4(0, 0, 0, 0);
-  if (have) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) wq[i] = load16(cp + uint64_t(kb) * 1024 + i * 16, wide);
-    wm = load16_meta(mp + uint64_t(kb) * 128, wide);
+    for (int s = 1; s < 3; ++s)
+      if (s < int(p.nseg) && u < p.seg[s].u0) left = min(left, p.seg[s].u0 - u);
   }
+  return min(left, kStageUnits);
+}
 
-  // Stage activations: a 16-byte source chunk holds half a K32 group (columns 16c..16c+15).
-  {
-    uint32_t const chunks = pk / 16;
-    bool const z16 = (reinterpret_cast<uintptr_t>(x.codes) & 15) == 0;
-    for (uint32_t t = 0; t < M; ++t) {
-      const uint8_t* const src = reinterpret_cast<const uint8_t*>(x.codes) + size_t(t) * pk;
-      uint8_t* const dst = zs + size_t(t) * tiles_k * kActKb;
-      for (uint32_t c = threadIdx.x; c < chunks; c += kThreads) {
+// Shared memory: rings [warp][stage][codes | metadata], activations [token][super-block][half of a group][group][16 B],
+// {a, a * sum} [token][group], row sums [warp][part][row][token], barriers, the warps' first super-blocks and row groups,
+// abort flag.
+template <int M, bool Dump, bool Raw>
+__global__ void __launch_bounds__(kThreads, M <= 2 ? 2 : 1) gemv_dp4a_kernel(const __grid_constant__ DpParams p) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  uint32_t const tiles_k = p.tiles_k, G = tiles_k * 8;
+  uint32_t const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t const s_ring = smem_u32(smem) + warp * p.stages * kStageBytes;
+  uint32_t const s_z = smem_u32(smem) + kWarps * p.stages * kStageBytes;
+  uint32_t const s_aw = s_z + M * tiles_k * 256;
+  uint32_t const o_red = kWarps * p.stages * kStageBytes + M * tiles_k * 320;
+  float* const red = reinterpret_cast<float*>(smem + o_red);
+  uint32_t const o_bar = o_red + kWarps * p.parts * 8 * M * 4;  // a multiple of 8
+  uint32_t const bars = smem_u32(smem) + o_bar + warp * p.stages * 8;
+  uint32_t* const cuts = reinterpret_cast<uint32_t*>(smem + o_bar + kWarps * p.stages * 8);
+  uint32_t* const firsts = cuts + kWarps + 1;
+  volatile int* const abort_flag = reinterpret_cast<volatile int*>(firsts + kWarps);
+
+  uint32_t const rg_first = blockIdx.x * p.rgs_each + min(blockIdx.x, p.rgs_rest);
+  uint32_t const rg_count = p.rgs_each + (blockIdx.x < p.rgs_rest ? 1u : 0u);
+  uint32_t const units = rg_count * tiles_k;
+
+  if (warp < kWarps) {
+    uint32_t const base = rg_first * tiles_k, c0 = units * warp / kWarps;
+    uint32_t const u0 = base + c0, u1 = base + units * (warp + 1) / kWarps;
+    // lane 0 keeps the ring full: stage `ps` takes the super-blocks from `pu` on
+    uint32_t pu = u0, ps = 0;
+    auto fetch = [&] {
+      uint32_t const count = stage_units(p, pu, u1);
+      DpSegment const& s = segment_of(p, pu);
+      uint64_t const at = pu - s.u0;
+      uint32_t const dst = s_ring + ps * kStageBytes, bar = bars + ps * 8;
+      mbar_expect_tx(bar, count * 1152);
+      bulk_copy(dst, s.codes + at * 1024, count * 1024, bar);
+      bulk_copy(dst + kStageUnits * 1024, s.meta + at * 128, count * 128, bar);
+      pu += count;
+      ps = ps + 1 == p.stages ? 0 : ps + 1;
+    };
+    if (lane == 0) {
+      if (p.wide) {
+        for (uint32_t i = 0; i < p.stages; ++i) mbar_init(bars + i * 8, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        for (uint32_t i = 0; i < p.stages && pu < u1; ++i) fetch();
+      }
+      cuts[warp] = c0;
+      firsts[warp] = c0 / tiles_k;
+      if (warp == 0) { cuts[kWarps] = units; *abort_flag = 0; }
+    }
+    if (!p.input_settled || Dump) pdl_wait();
+
+    // ---- activations ----
+    if constexpr (Raw) {
+      for (uint32_t i0 = warp; i0 < M * tiles_k; i0 += kWarps * 2) {  // two super-blocks requested at a time
+        uint4 v[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t const i = i0 + h * kWarps, col = (i % tiles_k) * 256 + lane * 8;
+          const uint16_t* const src = p.raw + size_t(i / tiles_k) * p.k + col;
+          v[h] = make_uint4(0, 0, 0, 0);
+          if (i >= M * tiles_k) continue;
+          if (p.vec && col + 8 <= p.k) v[h] = *reinterpret_cast<const uint4*>(src);
+          else {
+            uint32_t e[8];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) e[c] = col + c < p.k ? src[c] : 0u;
+            v[h] = make_uint4(e[0] | e[1] << 16, e[2] | e[3] << 16, e[4] | e[5] << 16, e[6] | e[7] << 16);
+          }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t const i = i0 + h * kWarps;
+          if (i >= M * tiles_k) continue;
+          uint32_t const vw[4] = {v[h].x, v[h].y, v[h].z, v[h].w};
+          float x[8];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) { x[2 * c] = __uint_as_float(vw[c] << 16); x[2 * c + 1] = __uint_as_float(vw[c] & 0xffff0000u); }
+          Packed8 const z = quantize8(x);
+          uint32_t const g = lane >> 2, dst = s_z + i * 256 + ((lane >> 1) & 1) * 128 + g * 16 + (lane & 1) * 8;
+          asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(dst), "r"(even_bytes(z.w0, z.w1)), "r"(odd_bytes(z.w0, z.w1)) : "memory");
+          if ((lane & 3) == 0) {
+            sts64f(s_aw + (i * 8 + g) * 8, z.a, z.a * float(z.sum));
+            if (!z.valid) atomicExch(p.failure, 1);
+          }
+        }
+      }
+    } else {
+      // a 16-byte source chunk holds half a K32 group (columns 16c..16c+15)
+      bool const z16 = (reinterpret_cast<uintptr_t>(p.codes) & 15) == 0;
+      uint32_t const chunks = M * tiles_k * 16;
+#pragma unroll 4
+      for (uint32_t c = threadIdx.x; c < chunks; c += kConsumers) {
         uint4 z;
-        if (z16) z = __ldg(reinterpret_cast<const uint4*>(src + c * 16));
+        if (z16) z = __ldg(reinterpret_cast<const uint4*>(p.codes) + c);
         else {
-          const uint32_t* s32 = reinterpret_cast<const uint32_t*>(src + c * 16);
+          const uint32_t* s32 = reinterpret_cast<const uint32_t*>(p.codes) + c * 4;
           z = make_uint4(__ldg(s32), __ldg(s32 + 1), __ldg(s32 + 2), __ldg(s32 + 3));
         }
-        uint32_t const kbi = c >> 4, g = (c >> 1) & 7, half = c & 1;
-        uint32_t const off = kbi * kActKb + (g >> 2) * 144 + (g & 3) * 32 + half * 16;
-        *reinterpret_cast<uint4*>(dst + off) =
-            make_uint4(even_bytes(z.x, z.y), odd_bytes(z.x, z.y), even_bytes(z.z, z.w), odd_bytes(z.z, z.w));
+        sts128(s_z + (c >> 4) * 256 + (c & 1) * 128 + ((c >> 1) & 7) * 16, even_bytes(z.x, z.y), odd_bytes(z.x, z.y),
+               even_bytes(z.z, z.w), odd_bytes(z.z, z.w));
+      }
+#pragma unroll 2
+      for (uint32_t i = threadIdx.x; i < M * G; i += kConsumers) {
+        float const a = __ldg(p.scales + i);
+        sts64f(s_aw + i * 8, a, a * float(__ldg(p.sums + i)));
       }
     }
-    for (uint32_t i = threadIdx.x; i < M * G; i += kThreads) {
-      float const a = __ldg(x.scales + i);
-      as[i] = a;
-      ws[i] = a * float(__ldg(x.sums + i));
-    }
-  }
-  __syncthreads();
+    asm volatile("bar.sync 1, %0;" ::"n"(kConsumers) : "memory");
 
-  float acc[M];
+    // ---- the warp's run ----
+    uint32_t const r = lane >> 2, q = lane & 3;
+    uint32_t const ga = 2 * q + (r & 1), gb = ga ^ 1;  // the lane's groups in the order in which it takes them
+#if DEC
+    // groups 0..3 keep six bits in words 1 and 2 of the metadata; groups 4..7 four in word 3, the upper two in words 1 and 2
+    uint32_t const low = q & 2 ? 0x0f0f0f0fu : 0x3f3f3f3fu, up = q & 2 ? 0x30303030u : 0u, down = q & 2 ? 4u : 0u;
+    uint32_t const pick_a = 0x4440u | (ga & 3), pick_b = 0x4440u | (gb & 3), bias_a = 0x7650u | (ga & 3), bias_b = 0x7650u | (gb & 3);
+#endif
+    float acc[M];
 #pragma unroll
-  for (int t = 0; t < M; ++t) acc[t] = 0.f;
-
-  if (active) {
-    uint32_t const row = rg * 8 + r;
-    for (uint32_t base = kb0; base < kb1; base += 2) {
-      uint4 cq[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) cq[i] = wq[i];
-      uint4 const cm = wm;
-      bool const cur = have;
-      uint32_t const ckb = kb;
-      kb = base + 2 + h;
-      have = kb < kb1;
-      if (have) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) wq[i] = load16(cp + uint64_t(kb) * 1024 + i * 16, wide);
-        wm = load16_meta(mp + uint64_t(kb) * 128, wide);
+    for (int t = 0; t < M; ++t) acc[t] = 0.f;
+    uint32_t kb = u0 % tiles_k, part = 0, st = 0, phase = 0, u = u0;
+    while (u < u1) {
+      uint32_t const count = stage_units(p, u, u1), stage = s_ring + st * kStageBytes;
+      if (p.wide) {
+        bool const ready = mbar_wait(bars + st * 8, phase, abort_flag, p.status, 0x110);
+        if (!__all_sync(0xffffffffu, ready)) break;
+      } else {
+        DpSegment const& s = segment_of(p, u);
+        uint64_t const at = u - s.u0;
+        const uint32_t* const c32 = reinterpret_cast<const uint32_t*>(s.codes + at * 1024);
+        const uint16_t* const m16 = reinterpret_cast<const uint16_t*>(s.meta + at * 128);
+#pragma unroll 8
+        for (uint32_t i = lane; i < count * 256; i += 32) asm volatile("st.shared.u32 [%0], %1;" ::"r"(stage + i * 4), "r"(__ldg(c32 + i)) : "memory");
+        for (uint32_t i = lane; i < count * 64; i += 32)
+          asm volatile("st.shared.u16 [%0], %1;" ::"r"(stage + kStageUnits * 1024 + i * 2), "h"(__ldg(m16 + i)) : "memory");
+        __syncwarp();
       }
-      if (!cur) continue;  // odd tail: this half-warp has no super-block in the last iteration
-      float const d = fp16_bits_to_f32(cm.x & 0xffffu), ndmin = -fp16_bits_to_f32(cm.x >> 16);
-      ScaleMinWords const sm = decode_scale_min(cm.y, cm.z, cm.w);
-      uint32_t const scw = j ? sm.sc_hi : sm.sc_lo, mnw = j ? sm.mn_hi : sm.mn_lo;
-      int sc[4];
-      float fm[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        sc[i] = int(byte_of(scw, i));
-        fm[i] = __uint_as_float(kMagicI | byte_of(mnw, i)) - kMagicF;  // float(m_g) without the conversion pipe
-      }
-      uint32_t const gi = ckb * 8 + j * 4;
+      for (uint32_t i = 0; i < kStageUnits; ++i) {
+        if (i >= count) break;
+        uint32_t const row_codes = stage + i * 1024 + r * 128;
+        uint4 const ca = lds128(row_codes + ga * 16), cb = lds128(row_codes + gb * 16);
+        uint4 const cm = lds128(stage + kStageUnits * 1024 + i * 128 + r * 16);
+        float const d = fp16_bits_to_f32(cm.x & 0xffffu), ndmin = -fp16_bits_to_f32(cm.x >> 16);
+#if DEC
+        uint32_t const scw = ((q & 2 ? cm.w : cm.y) & low) | ((cm.y >> 2) & up), mnw = (((q & 2 ? cm.w : cm.z) >> down) & low) | ((cm.z >> 2) & up);
+        int const sca = int(__byte_perm(scw, 0, pick_a)), scb = int(__byte_perm(scw, 0, pick_b));
+        // float(m_g) without the conversion pipe
+        float const mna = __uint_as_float(__byte_perm(mnw, kMagicI, bias_a)) - kMagicF, mnb = __uint_as_float(__byte_perm(mnw, kMagicI, bias_b)) - kMagicF;
+#else
+        ScaleMinWords const sm = decode_scale_min(cm.y, cm.z, cm.w);
+        uint32_t const scw = q & 2 ? sm.sc_hi : sm.sc_lo, mnw = q & 2 ? sm.mn_hi : sm.mn_lo;
+        int const sca = int(byte_of(scw, ga & 3)), scb = int(byte_of(scw, gb & 3));
+        float const mna = __uint_as_float(kMagicI | byte_of(mnw, ga & 3)) - kMagicF;  // float(m_g) without the conversion pipe
+        float const mnb = __uint_as_float(kMagicI | byte_of(mnw, gb & 3)) - kMagicF;
+#endif
 #pragma unroll
-      for (int t = 0; t < M; ++t) {
-        const uint4* const zp = reinterpret_cast<const uint4*>(zs + (size_t(t) * tiles_k + ckb) * kActKb + j * 144);
-        float4 const a4 = *reinterpret_cast<const float4*>(as + size_t(t) * G + gi);
-        float4 const w4 = *reinterpret_cast<const float4*>(ws + size_t(t) * G + gi);
-        float const av[4] = {a4.x, a4.y, a4.z, a4.w}, wv[4] = {w4.x, w4.y, w4.z, w4.w};
-        float X = 0.f, Y = 0.f;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          int const dot = dot32(cq[i], zp[2 * i], zp[2 * i + 1]);
+        for (int t = 0; t < M; ++t) {
+          uint32_t const z = s_z + (t * tiles_k + kb) * 256, aw = s_aw + (t * tiles_k + kb) * 64;
+          int const dota = dot32(ca, lds128(z + ga * 16), lds128(z + 128 + ga * 16));
+          int const dotb = dot32(cb, lds128(z + gb * 16), lds128(z + 128 + gb * 16));
+          float2 const wa = lds64f(aw + ga * 8), wb = lds64f(aw + gb * 8);
           // sc * dot is an exact integer below 2^22; adding the bias in the multiply-add converts it
-          float const q = __uint_as_float(uint32_t(dot * sc[i]) + kMagicI) - kMagicF;
-          X = fmaf(av[i], q, X);
-          Y = fmaf(fm[i], wv[i], Y);
-          if (Dump && row < w.n) partials[(uint64_t(t) * w.n + row) * G + gi + i] = dot;
+          float const xa = __uint_as_float(uint32_t(dota * sca) + kMagicI) - kMagicF;
+          float const xb = __uint_as_float(uint32_t(dotb * scb) + kMagicI) - kMagicF;
+          acc[t] = fmaf(d, fmaf(wb.x, xb, wa.x * xa), acc[t]);
+          acc[t] = fmaf(ndmin, fmaf(mnb, wb.y, mna * wa.y), acc[t]);
+          if constexpr (Dump) {
+            uint32_t const row = (u / tiles_k) * 8 + r, n = p.seg[0].n;  // one segment
+            if (row < n) {
+              p.partials[(uint64_t(t) * n + row) * G + kb * 8 + ga] = dota;
+              p.partials[(uint64_t(t) * n + row) * G + kb * 8 + gb] = dotb;
+            }
+          }
         }
-        acc[t] = fmaf(d, X, acc[t]);
-        acc[t] = fmaf(ndmin, Y, acc[t]);
-      }
-    }
-  }
-  // Fixed-order reduction: the four lanes of a row (j, then h), then the K slices in slice order.
+        ++u;
+        if (++kb == tiles_k || u == u1) {  // the row group, or the run, ends: the row's four lanes, then the warp's slot
 #pragma unroll
-  for (int t = 0; t < M; ++t) {
-    acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], 1);
-    acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], 16);
-    if ((lane & 17u) == 0) red[(warp * 8 + r) * M + t] = acc[t];
+          for (int t = 0; t < M; ++t) {
+            acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], 1);
+            acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], 2);
+            if (q == 0) red[((warp * p.parts + part) * 8 + r) * M + t] = acc[t];
+            acc[t] = 0.f;
+          }
+          ++part;
+          kb = 0;
+        }
+      }
+      __syncwarp();  // every lane has read the stage
+      if (lane == 0 && p.wide && pu < u1) fetch();
+      if (++st == p.stages) { st = 0; phase ^= 1; }
+    }
+    if (u < u1 && p.wide) {  // gave up: no copy may land after the block is gone
+      ps = __shfl_sync(0xffffffffu, ps, 0);
+      do {
+        long long const t0 = clock64();
+        while (!mbar_try(bars + st * 8, phase) && clock64() - t0 < kWaitCycles) {}
+        if (++st == p.stages) { st = 0; phase ^= 1; }
+      } while (st != ps);
+    }
+  } else {
+    // Control warp: once everything before this launch is complete, the next launch may start beside it.
+    pdl_wait();
+    pdl_launch_dependents();
   }
   __syncthreads();
-  for (uint32_t i = threadIdx.x; i < rgc * 8 * M; i += kThreads) {
-    uint32_t const t = i % M, rr = (i / M) % 8, lrg = i / (8 * M);
-    uint32_t const row = (blockIdx.x * rgc + lrg) * 8 + rr;
-    if (row >= w.n) continue;
+  if (*abort_flag) return;
+  pdl_wait();
+  // Thread (row group, row, token) adds the parts of the warps that worked on its row group, in warp order.
+  for (uint32_t i = threadIdx.x; i < rg_count * 8 * M; i += kThreads) {
+    uint32_t const t = i % M, r = (i / M) % 8, rg = i / (8 * M);
+    DpSegment const& s = segment_of(p, (rg_first + rg) * tiles_k);
+    uint32_t const row = (rg_first + rg - s.rg0) * 8 + r;
+    if (row >= s.n) continue;
+    uint32_t const x0 = rg * tiles_k, x1 = x0 + tiles_k;
+    const float* const mine = red + r * M + t;
     float v = 0.f;
-    for (uint32_t s = 0; s < ks; ++s) v += red[((lrg * ks + s) * 8 + rr) * M + t];
-    uint64_t const o = uint64_t(t) * w.n + row;
-    out[o] = v + (residual ? residual[o] : 0.f);
+#pragma unroll
+    for (uint32_t w = 0; w < kWarps; ++w)
+      if (max(cuts[w], x0) < min(cuts[w + 1], x1)) v += mine[(w * p.parts + rg - firsts[w]) * 8 * M];
+    uint64_t const o = uint64_t(t) * s.n + row;
+    if (s.residual) v += s.residual[o];
+    if (s.out_bf16) s.out_bf16[o] = f32_to_bf16_rne(v);
+    else s.out[o] = v;
   }
 }
 
 template <int M>
-cudaError_t launch_m(const WeightView& w, const Q8View& x, float* out, const float* residual, int32_t* partials,
-                     cudaStream_t stream) {
-  uint32_t const rgs = w.padded_n / 8;
-  // Row groups per block: enough blocks to fill the machine several times over, while each
-  // warp keeps at least a few super-blocks of K.
-  uint32_t rgc = 8;
-  while (rgc > 1 && (rgs / rgc < 148 * 3 || (w.tiles_k * rgc) / kWarps > 24)) rgc >>= 1;
-  while (rgc < 8 && w.tiles_k * rgc < 2 * kWarps) rgc <<= 1;  // fewer than two super-blocks per warp
-  uint32_t const grid = (rgs + rgc - 1) / rgc;
-  size_t const G = x.padded_k / 32;
-  size_t const smem = size_t(M) * w.tiles_k * kActKb + 2 * size_t(M) * G * 4 + kWarps * 8 * M * 4;
-  bool const wide = (reinterpret_cast<uintptr_t>(w.codes) % 16 == 0) && (reinterpret_cast<uintptr_t>(w.meta) % 16 == 0);
-  auto kernel = partials ? gemv_dp4a_kernel<M, true> : gemv_dp4a_kernel<M, false>;
-  if (smem > 48 * 1024) {
-    cudaError_t st = allow_smem(reinterpret_cast<const void*>(kernel), int(smem));
-    if (st != cudaSuccess) return st;
-  }
-  return launch_kernel(kernel, grid, kThreads, smem, stream, launch_overlap(), w, x, out, residual, partials, rgc, wide);
-  return cudaGetLastError();
+cudaError_t launch_m(const DpParams& p, uint32_t grid, uint32_t smem, cudaStream_t stream) {
+  auto kernel = p.partials ? gemv_dp4a_kernel<M, true, false> : (p.raw ? gemv_dp4a_kernel<M, false, true> : gemv_dp4a_kernel<M, false, false>);
+  cudaError_t st = allow_smem(reinterpret_cast<const void*>(kernel), int(smem));
+  if (st != cudaSuccess) return st;
+  return launch_kernel(kernel, grid, kThreads, smem, stream, launch_overlap(), p);
 }
+
+// Fills the split and launches; seg, nseg, operands and outputs are set.
+cudaError_t launch_split(DpParams p, uint32_t m, uint32_t padded_k, cudaStream_t stream) {
+  p.tiles_k = padded_k / 256;
+  for (uint32_t i = 0; i < p.nseg; ++i) {
+    p.seg[i].rg0 = p.rgs;
+    p.seg[i].u0 = p.rgs * p.tiles_k;
+    p.rgs += (p.seg[i].n + 7) / 8;
+  }
+  // One block per SM, or as many rounds of them as bound a block's row groups.
+  uint32_t const sms = uint32_t(sm_count()), waves = (p.rgs + sms * kMaxRowGroups - 1) / (sms * kMaxRowGroups);
+  uint32_t const grid = p.rgs < sms * waves ? p.rgs : sms * waves;
+  p.rgs_each = p.rgs / grid;
+  p.rgs_rest = p.rgs % grid;
+  uint32_t const units = (p.rgs_each + (p.rgs_rest ? 1 : 0)) * p.tiles_k;
+  p.parts = ((units + kWarps - 1) / kWarps + p.tiles_k - 2) / p.tiles_k + 1;  // row groups that a run can touch
+  uint32_t const fixed = m * p.tiles_k * 320 + kWarps * p.parts * 8 * m * 4 + (2 * kWarps + 2) * 4, stage = kWarps * (kStageBytes + 8);
+  // Up to two tokens the next launch gets the other half of the SM, unless that would leave less than two stages.
+  uint32_t const budget = m <= 2 && fixed + 2 * stage <= kHalfSm ? kHalfSm : kWholeSm;
+  p.stages = budget > fixed ? (budget - fixed) / stage : 0;
+  if (p.stages > kMaxStages) p.stages = kMaxStages;
+  if (p.stages < 1) return cudaErrorInvalidValue;
+  uint32_t const smem = fixed + p.stages * stage;
+  switch (m) {
+    case 1: return launch_m<1>(p, grid, smem, stream);
+    case 2: return launch_m<2>(p, grid, smem, stream);
+    case 3: return launch_m<3>(p, grid, smem, stream);
+    case 4: return launch_m<4>(p, grid, smem, stream);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+bool aligned16(const WeightView& w) { return reinterpret_cast<uintptr_t>(w.codes) % 16 == 0 && reinterpret_cast<uintptr_t>(w.meta) % 16 == 0; }
 
 }  // namespace
 
-cudaError_t launch_gemv_dp4a(const WeightView& w, const Q8View& x, float* out, const float* residual,
-                             int32_t* partials, cudaStream_t stream) {
-  switch (x.m) {
-    case 1: return launch_m<1>(w, x, out, residual, partials, stream);
-    case 2: return launch_m<2>(w, x, out, residual, partials, stream);
-    case 3: return launch_m<3>(w, x, out, residual, partials, stream);
-    case 4: return launch_m<4>(w, x, out, residual, partials, stream);
-    default: return cudaErrorInvalidValue;
+cudaError_t launch_gemv_dp4a(const WeightView& w, const Q8View& x, float* out, const float* residual, int32_t* partials,
+                             bool input_settled, int* status, cudaStream_t stream) {
+  DpParams p{};
+  p.seg[0] = DpSegment{w.codes, w.meta, out, nullptr, residual, w.n, 0, 0};
+  p.nseg = 1;
+  p.codes = x.codes; p.scales = x.scales; p.sums = x.sums;
+  p.partials = partials; p.status = status;
+  p.wide = aligned16(w);
+  p.input_settled = input_settled;
+  return launch_split(p, x.m, x.padded_k, stream);
+}
+
+cudaError_t launch_gemv_dp4a_multi(const WeightView* ws, const GemvTmaOutput* outs, uint32_t count, uint32_t m, uint32_t padded_k,
+                                   const GemvTmaRaw& raw, int* status, cudaStream_t stream) {
+  if (count < 1 || count > 3) return cudaErrorInvalidValue;
+  DpParams p{};
+  p.wide = 1;
+  for (uint32_t i = 0; i < count; ++i) {
+    p.seg[i] = DpSegment{ws[i].codes, ws[i].meta, outs[i].out, outs[i].out_bf16, outs[i].residual, ws[i].n, 0, 0};
+    p.wide &= aligned16(ws[i]) ? 1u : 0u;
   }
+  p.nseg = count;
+  p.raw = raw.x; p.k = raw.k; p.failure = raw.failure;
+  p.vec = raw.k % 8 == 0 && reinterpret_cast<uintptr_t>(raw.x) % 16 == 0;
+  p.status = status;
+  return launch_split(p, m, padded_k, stream);
 }
 
 }  // namespace q4k

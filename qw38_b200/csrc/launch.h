@@ -29,9 +29,10 @@ cudaError_t launch_export_q8_1(const int8_t* codes, const float* scales, const i
                                uint64_t groups, uint8_t* records, cudaStream_t stream);
 
 // gemv_dp4a.cu : m <= 4.  partials (optional) receives the int32 K32 dots [m][n][G].
-cudaError_t launch_gemv_dp4a(const WeightView& w, const Q8View& x, float* out,
-                             const float* residual, int32_t* partials, cudaStream_t stream);
+cudaError_t launch_gemv_dp4a(const WeightView& w, const Q8View& x, float* out, const float* residual, int32_t* partials,
+                             bool input_settled, int* status, cudaStream_t stream);
 constexpr uint32_t kGemvDp4aMaxTokens = 4;
+constexpr uint32_t kGemvDp4aBestTokens = 1;  // up to which it beats gemv_tma.cu
 
 // mmq_mma.cu : any m.  split_k slices of K are reduced in slice order by the last
 // block of each tile through `scratch` (fp32 partial tiles followed by tickets).
@@ -153,6 +154,9 @@ struct GemvTmaRaw {
   uint32_t k;
   int* failure;
 };
+// The same projections (no SwiGLU pair) from bf16 rows on dp4a, in gemv_dp4a.cu: m <= 4.
+cudaError_t launch_gemv_dp4a_multi(const WeightView* ws, const GemvTmaOutput* outs, uint32_t count, uint32_t m, uint32_t padded_k,
+                                   const GemvTmaRaw& raw, int* status, cudaStream_t stream);
 cudaError_t launch_gemv_tma_multi(const WeightView* ws, const GemvTmaOutput* outs, uint32_t count, bool swiglu_pair, const Q8View& x,
                                   const GemvTmaPlan& plan, void* slices, uint32_t* tickets, int* status, cudaStream_t stream,
                                   const GemvTmaRaw* raw = nullptr);

@@ -220,11 +220,9 @@ __global__ void __launch_bounds__(kThreads, M <= 2 ? 2 : 1) gemv_dp4a_kernel(con
     // ---- the warp's run ----
     uint32_t const r = lane >> 2, q = lane & 3;
     uint32_t const ga = 2 * q + (r & 1), gb = ga ^ 1;  // the lane's groups in the order in which it takes them
-#if DEC
     // groups 0..3 keep six bits in words 1 and 2 of the metadata; groups 4..7 four in word 3, the upper two in words 1 and 2
     uint32_t const low = q & 2 ? 0x0f0f0f0fu : 0x3f3f3f3fu, up = q & 2 ? 0x30303030u : 0u, down = q & 2 ? 4u : 0u;
     uint32_t const pick_a = 0x4440u | (ga & 3), pick_b = 0x4440u | (gb & 3), bias_a = 0x7650u | (ga & 3), bias_b = 0x7650u | (gb & 3);
-#endif
     float acc[M];
 #pragma unroll
     for (int t = 0; t < M; ++t) acc[t] = 0.f;
@@ -252,18 +250,10 @@ __global__ void __launch_bounds__(kThreads, M <= 2 ? 2 : 1) gemv_dp4a_kernel(con
         uint4 const ca = lds128(row_codes + ga * 16), cb = lds128(row_codes + gb * 16);
         uint4 const cm = lds128(stage + kStageUnits * 1024 + i * 128 + r * 16);
         float const d = fp16_bits_to_f32(cm.x & 0xffffu), ndmin = -fp16_bits_to_f32(cm.x >> 16);
-#if DEC
         uint32_t const scw = ((q & 2 ? cm.w : cm.y) & low) | ((cm.y >> 2) & up), mnw = (((q & 2 ? cm.w : cm.z) >> down) & low) | ((cm.z >> 2) & up);
         int const sca = int(__byte_perm(scw, 0, pick_a)), scb = int(__byte_perm(scw, 0, pick_b));
         // float(m_g) without the conversion pipe
         float const mna = __uint_as_float(__byte_perm(mnw, kMagicI, bias_a)) - kMagicF, mnb = __uint_as_float(__byte_perm(mnw, kMagicI, bias_b)) - kMagicF;
-#else
-        ScaleMinWords const sm = decode_scale_min(cm.y, cm.z, cm.w);
-        uint32_t const scw = q & 2 ? sm.sc_hi : sm.sc_lo, mnw = q & 2 ? sm.mn_hi : sm.mn_lo;
-        int const sca = int(byte_of(scw, ga & 3)), scb = int(byte_of(scw, gb & 3));
-        float const mna = __uint_as_float(kMagicI | byte_of(mnw, ga & 3)) - kMagicF;  // float(m_g) without the conversion pipe
-        float const mnb = __uint_as_float(kMagicI | byte_of(mnw, gb & 3)) - kMagicF;
-#endif
 #pragma unroll
         for (int t = 0; t < M; ++t) {
           uint32_t const z = s_z + (t * tiles_k + kb) * 256, aw = s_aw + (t * tiles_k + kb) * 64;

@@ -12,6 +12,7 @@
 #include <cstdio>
 #include <cstring>
 #include <limits>
+#include <optional>
 #include <atomic>
 #include <mutex>
 #include <vector>
@@ -226,12 +227,13 @@ int caller_scratch(const q4k_project_options* opt, uint64_t partial_bytes, uint6
 constexpr uint32_t kFlagTrustedSpans = 1u, kFlagInputSettled = 2u;
 
 // The fp16-plane kernel with scratch of its own (stream_scratch.cu).
+constexpr uint64_t kF16SuperBlocks = 16384;  // of eight rows; below, nine to sixteen tokens stay with the TMA-streamed kernel
 int project_f16(const q4k_weight& w, const q4k_q8_input& x, const q4k::TcOutput& out, cudaStream_t stream) {
   int* const status = q4k::kernel_status_word();
   if (!status) return Q4K_ERR_STATUS;
   q4k::F16Plan const plan = q4k::plan_f16(x.m, w.n, w.padded_k / 256);
   q4k::StreamScratch scratch;
-  Q4K_CUDA(scratch.acquire(stream, q4k::f16_scratch_bytes(x.m, w.padded_k / 256, plan), q4k::launch_overlap()), "scratch.acquire");
+  Q4K_CUDA(scratch.acquire(stream, q4k::f16_scratch_bytes(x.m, w.padded_k / 256, plan), q4k_get_launch_overlap() != 0), "scratch.acquire");
   Q4K_CUDA(q4k::launch_mmq_f16(view(w), view(x), out, plan, scratch.p(), scratch.alternates(), status, stream), "q4k_q8.mmq_f16");
   Q4K_CUDA(scratch.release(), "scratch.release");
   return Q4K_OK;
@@ -270,7 +272,13 @@ int project_impl(const q4k_weight* weight, const q4k_q8_input& x, float* output,
     // 6.1 .. 21.7 against 6.7 .. 22.4, and slower in a chain of layers).  Up to sixteen: the TMA-streamed kernel when the
     // weights are 16-byte aligned, else dp4a / cluster MMA.  Beyond: tcgen05 when TMA alignment allows.
     bool const tma_ok = x.m <= q4k::kGemvTmaMaxTokens && q4k::gemv_tma_supported(view(w), view(x));
-    if (tma_ok && x.m > q4k::kGemvDp4aBestTokens) kernel = Q4K_KERNEL_GEMV_TMA;
+    // From nine tokens on the fp16 kernel spends 13.7 us on anything (its planes, its tile ends) but then gains: 16 x 34816 x
+    // 5120 34 us against 44, 17408 x 5120 22 / 28, 5120 x 17408 25 / 31, 7168 x 5120 16 / 17 (nine tokens: 16 / 15.5, and
+    // 12.6 / 13.3 with overlapped launches); 5120 x 5120 13.8 / 13.2 .. 14.6.
+    bool const whole_dots = !partials && !(opt && (opt->split_k || opt->row_groups));
+    if (x.m > 8 && x.m <= 16 && whole_dots && w.padded_n / 8 * (w.padded_k / 256) >= kF16SuperBlocks && q4k::f16_supported(view(w), view(x)))
+      kernel = Q4K_KERNEL_F16;
+    else if (tma_ok && x.m > q4k::kGemvDp4aBestTokens) kernel = Q4K_KERNEL_GEMV_TMA;
     else if (x.m <= 2 || (x.m <= q4k::kGemvDp4aMaxTokens && w.padded_n >= 32768)) kernel = Q4K_KERNEL_GEMV_DP4A;
     else if (x.m <= 16) kernel = Q4K_KERNEL_GEMV_MMA;
     else if (!partials && !(opt && opt->split_k) && q4k::f16_supported(view(w), view(x))) kernel = Q4K_KERNEL_F16;
@@ -389,9 +397,12 @@ int pack_impl(const void* input, bool fp32, uint64_t input_len, const q4k_q8_inp
 
 namespace {
 std::atomic<bool> g_launch_overlap{false};
+thread_local int t_chained = 0;
 }
 namespace q4k {
-bool launch_overlap() { return g_launch_overlap.load(std::memory_order_relaxed); }
+bool launch_overlap() { return t_chained > 0 || g_launch_overlap.load(std::memory_order_relaxed); }
+ChainedLaunches::ChainedLaunches() { ++t_chained; }
+ChainedLaunches::~ChainedLaunches() { --t_chained; }
 int set_error(int code, const char* fmt, ...) {
   va_list ap;
   va_start(ap, fmt);
@@ -720,6 +731,8 @@ int decode_fused(const q4k_decode_desc* const* descs, uint32_t count, bool swigl
   if (int st = check_distinct(regions, nreg, false)) return st;
   if (!raw)
     if (int st = decode_pack(*descs[0], q8, failure, stream)) return st;
+  std::optional<q4k::ChainedLaunches> chained;
+  if (!raw) chained.emplace();
   q4k::GemvTmaRaw const rows{descs[0]->input, descs[0]->weight.k, failure};
   if (raw && !swiglu && q8.m <= q4k::kGemvDp4aBestTokens) {
     int* const status = q4k::kernel_status_word();
@@ -806,6 +819,7 @@ int q4k_prefill_project(const q4k_decode_desc* projection, void* workspace, uint
   if (int st = carve_decode_scratch(workspace, workspace_bytes, projection->m, projection->weight.n, projection->weight.k, &s))
     return st;
   if (int st = decode_pack(*projection, s.q8, failure, stream)) return st;
+  q4k::ChainedLaunches chained;
   return decode_one(*projection, s.q8, s.rows, stream);
 }
 
@@ -825,6 +839,7 @@ int q4k_prefill_paired_swiglu(const q4k_weight* gate, const q4k_weight* up, cons
   DecodeScratch s{};
   if (int st = carve_decode_scratch(workspace, workspace_bytes, valid_tokens, gate->n, gate->k, &s)) return st;
   if (int st = decode_pack(a, s.q8, failure, stream)) return st;
+  q4k::ChainedLaunches chained;
   uint64_t const cells = uint64_t(valid_tokens) * gate->n;
   if (int st = project_impl(gate, s.q8, s.rows, cells, nullptr, 0, nullptr, stream)) return st;
   if (int st = project_impl(up, s.q8, s.rows + cells, cells, nullptr, 0, nullptr, stream)) return st;
@@ -1151,6 +1166,7 @@ int q4k_q8_mlp(const q4k_weight* gate, const q4k_weight* up, const q4k_weight* d
     ce = q4k::launch_hidden_rms_q8(residual, gamma, eps, hidden, out_view(xh), failure, stream);
   }
   if (ce != cudaSuccess) return bail(fail_cuda(ce, "q8.rms_pack"));
+  q4k::ChainedLaunches chained;
   if (fused) {
     int* status = q4k::kernel_status_word();
     if (!status) return bail(Q4K_ERR_STATUS);

@@ -189,6 +189,16 @@ cudaError_t launch_gemv_bf16w(const WeightView& w, const uint16_t* x, uint32_t m
 // (pack, dp4a, TMA gemv) are launched with programmatic stream serialization: they may start,
 // and the TMA kernel may prefetch weights, while the preceding kernel of the stream drains.
 bool launch_overlap();
+// While one lives, launch_overlap() holds on this thread whatever the switch says.  For the second and later launches of an
+// entry point that issues several on one stream: their predecessor is a kernel of this library that writes no weights, so
+// a projection may fetch its weights beside it (a GEMV behind its pack: 1.5 .. 3 us less).  The first launch of a call is
+// not covered: what runs before it is the caller's, who may just have written the weights.
+struct ChainedLaunches {
+  ChainedLaunches();
+  ~ChainedLaunches();
+  ChainedLaunches(const ChainedLaunches&) = delete;
+  ChainedLaunches& operator=(const ChainedLaunches&) = delete;
+};
 
 // cudaFuncSetAttribute(MaxDynamicSharedMemorySize), skipped where this thread has already asked for as much on the current
 // device (the runtime call costs a quarter of a microsecond on every launch).  The limit of a kernel is only ever raised,

@@ -81,6 +81,8 @@ __global__ void __launch_bounds__(kThreads) swiglu_pack_kernel(const float* __re
                                                                 int8_t* codes, float* scales,
                                                                 int32_t* sums, uint64_t chunks,
                                                                 int* failure) {
+  pdl_wait();
+  pdl_launch_dependents();
   uint32_t const lane = threadIdx.x & 31, sub = lane & 3, grp = lane >> 2;
   uint64_t const warps = uint64_t(gridDim.x) * (kThreads / 32);
   for (uint64_t task = uint64_t(blockIdx.x) * (kThreads / 32) + threadIdx.x / 32; task < chunks;
@@ -128,6 +130,8 @@ __global__ void __launch_bounds__(kThreads) hidden_rms_q8_kernel(const float* __
                                                                   int8_t* codes, float* scales,
                                                                   int32_t* sums, int* failure) {
   extern __shared__ __align__(16) uint16_t rounded[];
+  pdl_wait();
+  pdl_launch_dependents();
   __shared__ float scratch[kThreads / 32];
   const float* x = residual + uint64_t(blockIdx.x) * hidden;
   float held[Held > 0 ? Held : 1], gain[Held > 0 ? Held : 1];
@@ -233,8 +237,8 @@ cudaError_t launch_pack_q8(const void* input, bool fp32, Q8Out out, uint32_t k, 
 cudaError_t launch_swiglu_pack_q8(const float* gate, const float* up, Q8Out out, int* failure,
                                   cudaStream_t stream) {
   uint64_t const chunks = uint64_t(out.m) * (out.padded_k / 256);
-  swiglu_pack_kernel<<<grid_for(chunks), kThreads, 0, stream>>>(gate, up, out.codes, out.scales, out.sums, chunks, failure);
-  return cudaGetLastError();
+  return launch_kernel(swiglu_pack_kernel, grid_for(chunks), kThreads, 0, stream, launch_overlap(), gate, up, out.codes, out.scales, out.sums,
+                       chunks, failure);
 }
 
 cudaError_t launch_hidden_rms_q8(const float* residual, const uint16_t* gamma, float eps,
@@ -246,8 +250,8 @@ cudaError_t launch_hidden_rms_q8(const float* residual, const uint16_t* gamma, f
     cudaError_t st = allow_smem(reinterpret_cast<const void*>(kernel), int(smem));
     if (st != cudaSuccess) return st;
   }
-  kernel<<<out.m, kThreads, smem, stream>>>(residual, gamma, eps, hidden, out.codes, out.scales, out.sums, failure);
-  return cudaGetLastError();
+  return launch_kernel(kernel, out.m, kThreads, smem, stream, launch_overlap(), residual, gamma, eps, hidden, out.codes, out.scales, out.sums,
+                       failure);
 }
 
 cudaError_t launch_export_q8_1(const int8_t* codes, const float* scales, const int32_t* sums,

@@ -13,10 +13,11 @@
 // explicit round-to-nearest intrinsic so that no multiply-add is contracted (the reference
 // builds its host code with -ffp-contract=off, src/CMakeLists.txt:35-37).
 //
-// Bound: the FMA pipe.  A candidate costs 16 operations per weight -- four to find its level, six for the moments, six for
-// the error -- and the levels stay in registers between the two sums (96 of the 128 registers hold weights, importances
-// and levels; more blocks with fewer registers would have to find the levels twice).  5120 x 17408: 1.34 ms, 1.75 ms with
-// levels clamped by fmaxf / fminf and found again for the error.
+// Bound: issue slots and the FMA pipe.  A candidate costs 16 operations per weight -- four to find its level, six for the
+// moments, six for the error -- in eleven instructions, ten of the operations being packed in pairs, and the levels stay
+// in registers between the two sums (96 of the 128 registers hold weights, importances and levels; more blocks with fewer
+// registers would have to find the levels twice).  5120 x 17408: 1.26 ms (1.34 with scalar instructions only, when 86 % of
+// the issue slots were taken; 1.75 with levels clamped by fmaxf / fminf and found again for the error).
 //
 // A block of 128 threads fits 16 consecutive super-blocks.  Their 4096 weights are loaded with
 // coalesced reads into shared memory at a row stride of 33 words, from where each thread takes
@@ -53,17 +54,14 @@ __device__ __forceinline__ int level(float v) { return min(15, max(0, nearest(v)
 // What the caller knows of grid * d: nothing, |grid * d| < 2^22, or that and grid * d < 15.5.
 enum class Range { kAny, kBounded, kBelowTop };
 
-// float(level(grid * d)).  With |grid * d| < 2^22 the product, scaled by 1/16 (exactly: grid16 = grid / 16), is clamped to
+// float(level(grid * d)) with |grid * d| < 2^22: the product, scaled by 1/16 (exactly: grid16 = grid / 16), is clamped to
 // [0, 1] by the multiplication itself, rounded to a multiple of 1/16 by the bias 1.5 * 2^19, and brought back by one exact
 // multiply-add: four operations on the FMA pipe with the subtraction before them, where clamping with fmaxf and fminf costs
 // two more at half rate.  What is left above 15 needs the fminf, unless the caller knows better.
-template <Range R>
-__device__ __forceinline__ float level_f(float grid, float grid16, float d) {
-  if constexpr (R == Range::kAny) return float(level(mul(grid, d)));
+__device__ __forceinline__ float mul_sat(float a, float b) {
   float t;
-  asm("mul.rn.sat.f32 %0, %1, %2;" : "=f"(t) : "f"(grid16), "f"(d));
-  float const l = __fmaf_rn(add(t, 786432.f), 16.f, -12582912.f);
-  return R == Range::kBelowTop ? l : fminf(l, 15.f);
+  asm("mul.rn.sat.f32 %0, %1, %2;" : "=f"(t) : "f"(a), "f"(b));
+  return t;
 }
 
 struct GroupFit {
@@ -71,35 +69,49 @@ struct GroupFit {
   float grid, origin;    // the levels the search settled on are level(grid * (x - origin))
 };
 
+// Weights, importances and levels of a group are held in pairs: what is not a running sum or a saturating product takes one
+// packed instruction for two of them.  (fma(x, -1, t) rounds as t - x does.)
 template <Range R>
-__device__ __forceinline__ void levels(const float (&x)[32], float grid, float origin, float (&l)[32]) {
+__device__ __forceinline__ void levels(const float2 (&x)[16], float grid, float origin, float2 (&l)[16]) {
   float const grid16 = mul(grid, 0.0625f);
 #pragma unroll
-  for (int i = 0; i < 32; ++i) l[i] = level_f<R>(grid, grid16, sub(x[i], origin));
+  for (int i = 0; i < 16; ++i) {
+    float2 const d = __fadd2_rn(x[i], make_float2(-origin, -origin));
+    if constexpr (R == Range::kAny) {
+      l[i] = make_float2(float(level(mul(grid, d.x))), float(level(mul(grid, d.y))));
+    } else {
+      float2 const t = make_float2(mul_sat(grid16, d.x), mul_sat(grid16, d.y));
+      l[i] = __ffma2_rn(__fadd2_rn(t, make_float2(786432.f, 786432.f)), make_float2(16.f, 16.f), make_float2(-12582912.f, -12582912.f));
+      if constexpr (R == Range::kBounded) l[i] = make_float2(fminf(l[i].x, 15.f), fminf(l[i].y, 15.f));
+    }
+  }
 }
 
 struct Moments { float l, l2, xl; };
 
 // Weighted moments of the levels a candidate grid assigns (the middle loop of the search).
-__device__ __forceinline__ Moments moments(const float (&x)[32], const float (&w)[32], const float (&l)[32]) {
+__device__ __forceinline__ Moments moments(const float2 (&x)[16], const float2 (&w)[16], const float2 (&l)[16]) {
   Moments s{0.f, 0.f, 0.f};
 #pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    float const wl = mul(w[i], l[i]);
-    s.l = add(s.l, wl);
-    s.l2 = add(s.l2, mul(wl, l[i]));
-    s.xl = add(s.xl, mul(wl, x[i]));
+  for (int i = 0; i < 16; ++i) {
+    float2 const wl = __fmul2_rn(w[i], l[i]), wl2 = __fmul2_rn(wl, l[i]), wxl = __fmul2_rn(wl, x[i]);
+    s.l = add(add(s.l, wl.x), wl.y);
+    s.l2 = add(add(s.l2, wl2.x), wl2.y);
+    s.xl = add(add(s.xl, wxl.x), wxl.y);
   }
   return s;
 }
 
 // Weighted squared error of step * level + base against the weights.
-__device__ __forceinline__ float fit_error(const float (&x)[32], const float (&w)[32], const float (&l)[32], float step, float base) {
+__device__ __forceinline__ float fit_error(const float2 (&x)[16], const float2 (&w)[16], const float2 (&l)[16], float step, float base) {
   float err = 0.f;
 #pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    float const diff = sub(add(mul(step, l[i]), base), x[i]);
-    err = add(err, mul(w[i], mul(diff, diff)));
+  for (int i = 0; i < 16; ++i) {
+    // scalar products: a packed one that feeds a packed addition is contracted with it, which changes the result
+    float2 const fitted = __fadd2_rn(make_float2(mul(step, l[i].x), mul(step, l[i].y)), make_float2(base, base));
+    float2 const diff = __ffma2_rn(x[i], make_float2(-1.f, -1.f), fitted);
+    float2 const e = __fmul2_rn(w[i], __fmul2_rn(diff, diff));
+    err = add(add(err, e.x), e.y);
   }
   return err;
 }
@@ -107,20 +119,20 @@ __device__ __forceinline__ float fit_error(const float (&x)[32], const float (&w
 // The search over one group (make_qkx2_quants with n=32, nmax=15, rmin=-1, rdelta=0.1, nstep=20,
 // squared error; q4k.cpp:94-172).  x: the group's 32 weights, held in registers (every loop over them is
 // fully unrolled); the importance of a weight, average + |x|, is computed once.
-__device__ GroupFit fit_group(const float (&x)[32], float average) {
-  float w[32];
+__device__ GroupFit fit_group(const float2 (&x)[16], float average) {
+  float2 w[16];
 #pragma unroll
-  for (int i = 0; i < 32; ++i) w[i] = add(average, fabsf(x[i]));
-  float lo = x[0], hi = x[0];
-  float sum_w = w[0];
-  float sum_x = mul(sum_w, x[0]);
+  for (int i = 0; i < 16; ++i) w[i] = __fadd2_rn(make_float2(average, average), make_float2(fabsf(x[i].x), fabsf(x[i].y)));
+  float lo = x[0].x, hi = x[0].x;
+  float sum_w = w[0].x;
+  float sum_x = mul(sum_w, x[0].x);
 #pragma unroll
   for (int i = 1; i < 32; ++i) {
-    float const v = x[i];
+    float const v = i & 1 ? x[i / 2].y : x[i / 2].x, wv = i & 1 ? w[i / 2].y : w[i / 2].x;
     if (v < lo) lo = v;
     if (v > hi) hi = v;
-    sum_w = add(sum_w, w[i]);
-    sum_x = add(sum_x, mul(w[i], v));
+    sum_w = add(sum_w, wv);
+    sum_x = add(sum_x, mul(wv, v));
   }
   float const x_min = lo;  // smallest weight, before the minimum is capped at zero
   if (lo > 0.f) lo = 0.f;
@@ -131,7 +143,7 @@ __device__ GroupFit fit_group(const float (&x)[32], float average) {
   }
   float grid = quo(15.f, sub(hi, lo));
   float scale = quo(1.f, grid);
-  float l[32];
+  float2 l[16];
   levels<Range::kAny>(x, grid, lo, l);
   float best = fit_error(x, w, l, scale, lo);
   fit.grid = grid; fit.origin = lo;
@@ -202,15 +214,15 @@ __global__ void __launch_bounds__(kFitThreads) fit_q4k_kernel(const In* __restri
   uint64_t const b = block0 + (tid >> 3);
   uint32_t const g = tid & 7;
   bool const live = b < in_blocks;
-  float x[32];
+  float2 x[16];
 #pragma unroll
-  for (int i = 0; i < 32; ++i) x[i] = xs[tid * kRow + i];
+  for (int i = 0; i < 16; ++i) x[i] = make_float2(xs[tid * kRow + 2 * i], xs[tid * kRow + 2 * i + 1]);
 
   // Admission of the inputs (q4k.cpp:189-200): the first offending weight of the block decides.
   uint8_t bad = kFitOk;
 #pragma unroll
   for (int i = 31; i >= 0; --i) {
-    float const v = x[i];
+    float const v = i & 1 ? x[i / 2].y : x[i / 2].x;
     if (!finite(v)) bad = kFitNonfinite;
     else if (fabsf(v) > 1.0e10f) bad = kFitRange;
   }
@@ -224,10 +236,10 @@ __global__ void __launch_bounds__(kFitThreads) fit_q4k_kernel(const In* __restri
   GroupFit fit{0.f, 0.f, 0.f, 0.f};
   bad = kFitOk;
   if (live && !block_flaw) {
-    float lo = 0.f, hi = x[0], sum_x2 = 0.f;
+    float lo = 0.f, hi = x[0].x, sum_x2 = 0.f;
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
-      float const v = x[i];
+      float const v = i & 1 ? x[i / 2].y : x[i / 2].x;
       if (v < lo) lo = v;
       if (v > hi) hi = v;
       sum_x2 = add(sum_x2, mul(v, v));
@@ -267,7 +279,7 @@ __global__ void __launch_bounds__(kFitThreads) fit_q4k_kernel(const In* __restri
     float const offset = mul(__half2float(dmin16), float(mn6));
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
-      float const v = x[i];
+      float const v = i & 1 ? x[i / 2].y : x[i / 2].x;
       int const l = step != 0.f ? level(quo(add(v, offset), step)) : level(mul(fit.grid, sub(v, fit.origin)));
       packed[i >> 3] |= uint32_t(l) << (4 * (i & 7));
     }

@@ -1,0 +1,128 @@
+"""One to sixteen tokens: the dp4a GEMV at the edges of its split (runs of warps, row groups of blocks, rounds of blocks,
+unaligned weights), decode calls that quantise inside the projection, where the automatic choice changes kernels, the RMS
+producer's register forms, and the narrow form of the block repack."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle as orc
+from qw38_b200 import _lib as L
+from qw38_b200 import repack_blocks144, synth
+from qw38_b200.q4k_q8 import (DecodeMmvDesc, PrefillWeight, decode_workspace, hidden_rms_q8, launch_decode_mmv,
+                              launch_decode_mmv_ranges, pack_q8, q4k_q8_project)
+from tests.helpers import assert_close_contract
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def flag():
+    return torch.zeros(1, dtype=torch.int32, device=DEV)
+
+
+def kernel_status():
+    v = ctypes.c_int(-1)
+    assert L.load().q4k_kernel_status(ctypes.byref(v)) == 0
+    return v.value
+
+
+def weight(n, k, seed):
+    hc, hs = synth.split_tiles(*synth.logical_q4k(n, k, seed=seed))
+    return PrefillWeight.from_host(hc, hs, n, k), hc, hs
+
+
+def shifted(t, by):
+    """The same bytes `by` bytes off a 16-byte boundary."""
+    room = torch.empty(t.numel() + 16, dtype=torch.uint8, device=DEV)
+    room[by:by + t.numel()] = t
+    return room[by:by + t.numel()]
+
+
+# one row group and one super-block; fewer super-blocks than warps; runs within, across and of several row groups; K tails;
+# two rounds of blocks (more than 64 row groups for each of 148 SMs)
+@pytest.mark.parametrize("m,n,k", [(1, 1, 256), (1, 9, 200), (2, 8, 5120), (1, 1200, 259), (3, 2400, 1280), (4, 1190, 2304),
+                                   (1, 5120, 5120), (2, 264, 17408), (1, 75800, 256)])
+@pytest.mark.parametrize("aligned", [True, False])
+def test_dp4a_split(m, n, k, aligned):
+    w, hc, hs = weight(n, k, seed=n + k)
+    if not aligned:
+        w = PrefillWeight(shifted(w.codes, 4), shifted(w.scales, 2), n, k)
+    x = synth.activations(m, k, seed=k)
+    q = pack_q8(torch.from_numpy(x).to(DEV), flag())
+    z, a, s, _ = orc.q8_quantize(x)
+    guarded = torch.full((m * n + 2,), -7.0, dtype=torch.float32, device=DEV)
+    y = q4k_q8_project(w, q, out=guarded[1:-1].view(m, n), kernel=L.KERNEL_GEMV_DP4A)
+    assert guarded[0].item() == -7.0 and guarded[-1].item() == -7.0
+    assert_close_contract(y.cpu().numpy(), orc.project(hc, hs, n, q.padded_k, z, a, s))
+    res = torch.from_numpy(synth.activations(m, n, seed=5)).to(DEV)
+    assert torch.equal(q4k_q8_project(w, q, kernel=L.KERNEL_GEMV_DP4A, residual=res), y + res), "residual is the last fp32 add"
+    if n * k < 4 << 20:
+        p = torch.empty((m, n, q.padded_k // 32), dtype=torch.int32, device=DEV)
+        q4k_q8_project(w, q, kernel=L.KERNEL_GEMV_DP4A, partials=p)
+        assert (p.cpu().numpy() == orc.dots(hc, n, q.padded_k, z)).all()
+    assert kernel_status() == 0
+
+
+@pytest.mark.parametrize("m", [1, 2, 4, 5])
+@pytest.mark.parametrize("k", [1000, 1003, 2560])
+def test_decode_quantises_in_the_projection(m, k):
+    """Q/K/V ranges from bf16 rows: the codes a pack would give, whatever the row alignment; a bad value raises the flag."""
+    x = torch.from_numpy(synth.activations(m, k, seed=k)).to(DEV).to(torch.bfloat16)
+    z, a, s, _ = orc.q8_quantize(x.view(torch.int16).cpu().numpy().view(np.uint16), bf16_bits=True)
+    parts = [(weight(n, k, seed=n), torch.empty((m, n), dtype=t, device=DEV))
+             for n, t in ((264, torch.float32), (40, torch.bfloat16), (17, torch.bfloat16))]
+    descs = [DecodeMmvDesc(w[0], x, out, L.EPILOGUE_STORE_FP32 if out.dtype == torch.float32 else L.EPILOGUE_STORE_BF16)
+             for w, out in parts]
+    ws, f = decode_workspace(m, 264 + 40 + 17, k), flag()
+    launch_decode_mmv_ranges(descs, ws, f)
+    assert f.item() == 0
+    for (w, hc, hs), out in parts:
+        ref = orc.project(hc, hs, w.n, w.padded_k, z, a, s)
+        if out.dtype == torch.float32:
+            assert_close_contract(out.cpu().numpy(), ref)
+        else:
+            assert np.abs(out.float().cpu().numpy() - ref).max() <= np.abs(ref).max() * 2.0 ** -8
+    x[m - 1, k - 1] = float("inf")
+    launch_decode_mmv(descs[0], ws, f)
+    assert f.item() == 1 and kernel_status() == 0
+
+
+@pytest.mark.parametrize("m,n,k,kernel", [(1, 264, 512, L.KERNEL_GEMV_DP4A), (2, 264, 512, L.KERNEL_GEMV_TMA),
+                                          (8, 26216, 1280, L.KERNEL_GEMV_TMA), (9, 26208, 1280, L.KERNEL_GEMV_TMA),
+                                          (9, 26216, 1280, L.KERNEL_F16), (16, 26216, 1280, L.KERNEL_F16), (17, 264, 512, L.KERNEL_F16)])
+def test_automatic_choice(m, n, k, kernel):
+    """16384 super-blocks of eight rows lie between n = 26208 and 26216 at five super-blocks of K."""
+    w, hc, hs = weight(n, k, seed=3)
+    x = synth.activations(m, k, seed=9)
+    q = pack_q8(torch.from_numpy(x).to(DEV), flag())
+    y = q4k_q8_project(w, q)
+    assert torch.equal(y, q4k_q8_project(w, q, kernel=kernel))
+    z, a, s, _ = orc.q8_quantize(x)
+    assert_close_contract(y.cpu().numpy(), orc.project(hc, hs, n, q.padded_k, z, a, s))
+
+
+@pytest.mark.parametrize("hidden", [256, 2048, 2304, 6144, 6400])
+def test_rms_register_forms(hidden):
+    rng = np.random.default_rng(hidden)
+    x = rng.standard_normal((3, hidden)).astype(np.float32) * 2
+    gamma = torch.from_numpy(rng.standard_normal(hidden).astype(np.float32) * 0.1).to(torch.bfloat16)
+    f = flag()
+    q = hidden_rms_q8(torch.from_numpy(x).to(DEV), gamma.to(DEV), 1e-6, f)
+    bits = orc.hidden_rms_bf16(x, gamma.view(torch.int16).numpy().view(np.uint16), 1e-6)
+    z, a, _, _ = orc.q8_quantize(bits, bf16_bits=True)
+    assert f.item() == 0
+    # a bf16 rounding of the other neighbour moves a code by at most one and a scale by one part in 256
+    assert np.abs(q.codes.cpu().numpy().astype(int) - z).max() <= 1
+    assert np.abs(q.scales.cpu().numpy() / a - 1).max() <= 2.0 ** -7
+
+
+@pytest.mark.parametrize("n,k", [(1, 256), (21, 512), (64, 1280)])
+@pytest.mark.parametrize("by", [0, 4])
+def test_repack_of_unaligned_blocks(n, k, by):
+    codes, meta = synth.logical_q4k(n, k, seed=n)
+    hc, hs = synth.split_tiles(codes, meta)
+    blocks = torch.from_numpy(synth.blocks144(codes, meta).reshape(-1)).to(DEV)
+    w = repack_blocks144(shifted(blocks, by), n, k)
+    assert (w.codes.cpu().numpy() == hc.reshape(-1)).all() and (w.scales.cpu().numpy() == hs.reshape(-1)).all()

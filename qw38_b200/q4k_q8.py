@@ -76,11 +76,18 @@ class PrefillWeight:
     def padded_k(self) -> int:
         return pad_k(self.k)
 
+    # The descriptors of this module are handed to C for reading only, so the last one built is kept next to what it was
+    # built from and serves again while that is unchanged (0.6 us to compare, 1.3 to build; a decode call has up to four).
+    _built = None
+
     def c_struct(self) -> L.Weight:
-        return L.Weight(self.codes.data_ptr(), self.scales.data_ptr(), self.layout, self.quantizer, self.n,
-                        self.k, self.padded_n, self.padded_k,
-                        self.codes.numel() if self.codes_bytes is None else self.codes_bytes,
-                        self.scales.numel() if self.scales_bytes is None else self.scales_bytes)
+        key = (self.codes.data_ptr(), self.scales.data_ptr(), self.layout, self.quantizer, self.n, self.k,
+               self.codes.numel() if self.codes_bytes is None else self.codes_bytes,
+               self.scales.numel() if self.scales_bytes is None else self.scales_bytes)
+        built = self._built
+        if built is None or built[0] != key:
+            built = self._built = (key, L.Weight(*key[:6], self.padded_n, self.padded_k, *key[6:]))
+        return built[1]
 
     @staticmethod
     def from_host(codes, scales, n: int, k: int, device="cuda") -> "PrefillWeight":
@@ -111,9 +118,16 @@ class Q8Input:
     k: int
     padded_k: int
 
+    _built = None
+
     def c_struct(self) -> L.Q8:
-        return L.Q8(self.codes.data_ptr(), self.scales.data_ptr(), self.sums.data_ptr(), self.codes.numel(),
-                    self.scales.numel(), self.sums.numel(), self.m, self.k, self.padded_k)
+        codes, scales, sums = self.codes, self.scales, self.sums
+        key = (codes.data_ptr(), scales.data_ptr(), sums.data_ptr(), codes.numel(), scales.numel(), sums.numel(), self.m,
+               self.k, self.padded_k)
+        built = self._built
+        if built is None or built[0] != key:
+            built = self._built = (key, L.Q8(*key))
+        return built[1]
 
     def rows(self, r0: int, r1: int) -> "Q8Input":
         return Q8Input(self.codes[r0:r1], self.scales[r0:r1], self.sums[r0:r1], r1 - r0, self.k, self.padded_k)
@@ -253,13 +267,17 @@ class DecodeMmvDesc:
     residual: Optional[torch.Tensor] = None
     activation_policy: int = L.ACTIVATION_Q8_K32
 
+    _built = None
+
     def c_struct(self) -> L.DecodeDesc:
-        m = self.input.shape[0] if self.input.dim() == 2 else 1
-        return L.DecodeDesc(self.weight.c_struct(), self.input.data_ptr(), self.input.numel(),
-                            0 if self.output is None else self.output.data_ptr(),
-                            0 if self.output is None else self.output.numel(),
-                            0 if self.residual is None else self.residual.data_ptr(),
-                            0 if self.residual is None else self.residual.numel(), m, self.epilogue, self.activation_policy)
+        weight, x, out, res = self.weight.c_struct(), self.input, self.output, self.residual
+        key = (x.data_ptr(), x.numel(), 0 if out is None else out.data_ptr(), 0 if out is None else out.numel(),
+               0 if res is None else res.data_ptr(), 0 if res is None else res.numel(), x.shape[0] if x.dim() == 2 else 1,
+               self.epilogue, self.activation_policy)
+        built = self._built
+        if built is None or built[0] is not weight or built[1] != key:
+            built = self._built = (weight, key, L.DecodeDesc(weight, *key))
+        return built[2]
 
 
 def decode_workspace(m: int, n_total: int, k: int, device="cuda") -> torch.Tensor:

@@ -11,12 +11,8 @@ namespace {
 // sigmoid / SiLU exactly as the reference's decode epilogue states them
 // (cuda/decode_mmv.cu:78-89): the exponential is always taken of a non-positive number.
 __device__ __forceinline__ float sigmoid_fp32(float u) {
-  if (u >= 0.0f) {
-    float const e = expf(-u);
-    return 1.0f / (1.0f + e);
-  }
-  float const e = expf(u);
-  return e / (1.0f + e);
+  float const e = expf(-fabsf(u));
+  return (u >= 0.0f ? 1.0f : e) / (1.0f + e);
 }
 
 __global__ void store_bf16_kernel(const float* __restrict__ in, uint16_t* __restrict__ out, uint64_t count) {
@@ -26,13 +22,27 @@ __global__ void store_bf16_kernel(const float* __restrict__ in, uint16_t* __rest
   if (i < count) out[i] = f32_to_bf16_rne(in[i]);
 }
 
-// y = bf16(SiLU(gate) * up)  (SwigluStoreBf16, cuda/decode_mmv.cu:238-242)
+// y = bf16(SiLU(gate) * up)  (SwigluStoreBf16, cuda/decode_mmv.cu:238-242).  Bound: HBM beyond a few hundred tokens, 10
+// bytes per value; Wide (all pointers 16-byte aligned, count a multiple of eight): eight values per thread, four loads in
+// flight.
+template <bool Wide>
 __global__ void swiglu_store_bf16_kernel(const float* __restrict__ gate, const float* __restrict__ up,
                                          uint16_t* __restrict__ out, uint64_t count) {
   pdl_wait();
   pdl_launch_dependents();  // after the wait: the next launch never runs beside anything older than this one
   uint64_t const i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < count) {
+  if constexpr (Wide) {
+    if (i >= count / 8) return;
+    float4 const g0 = reinterpret_cast<const float4*>(gate)[2 * i], g1 = reinterpret_cast<const float4*>(gate)[2 * i + 1];
+    float4 const u0 = reinterpret_cast<const float4*>(up)[2 * i], u1 = reinterpret_cast<const float4*>(up)[2 * i + 1];
+    float const g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w}, u[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+    uint32_t w[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      w[j] = uint32_t(f32_to_bf16_rne(g[2 * j] * sigmoid_fp32(g[2 * j]) * u[2 * j])) |
+             uint32_t(f32_to_bf16_rne(g[2 * j + 1] * sigmoid_fp32(g[2 * j + 1]) * u[2 * j + 1])) << 16;
+    reinterpret_cast<uint4*>(out)[i] = make_uint4(w[0], w[1], w[2], w[3]);
+  } else if (i < count) {
     float const g = gate[i];
     out[i] = f32_to_bf16_rne(g * sigmoid_fp32(g) * up[i]);
   }
@@ -47,7 +57,10 @@ cudaError_t launch_store_bf16(const float* in, uint16_t* out, uint64_t count, cu
 
 cudaError_t launch_swiglu_store_bf16(const float* gate, const float* up, uint16_t* out, uint64_t count, cudaStream_t stream) {
   if (count == 0) return cudaSuccess;
-  return launch_kernel(swiglu_store_bf16_kernel, unsigned((count + 255) / 256), 256, 0, stream, launch_overlap(), gate, up, out, count);
+  bool const wide = count % 8 == 0 && ((reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(up) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+  uint64_t const threads = wide ? count / 8 : count;
+  return launch_kernel(wide ? swiglu_store_bf16_kernel<true> : swiglu_store_bf16_kernel<false>, unsigned((threads + 255) / 256), 256, 0, stream,
+                       launch_overlap(), gate, up, out, count);
 }
 
 }  // namespace q4k

@@ -103,10 +103,11 @@ struct F16Plan {
   uint32_t slot_clusters;  // clusters for whose partial tiles the scratch has room
 };
 bool f16_supported(const WeightView& w, const Q8View& x);
-F16Plan plan_f16(uint32_t m, uint32_t n, uint32_t tiles_k);
+F16Plan plan_f16(uint32_t m, uint32_t n, uint32_t tiles_k, bool pair = false);
 uint64_t f16_scratch_bytes(uint32_t m, uint32_t tiles_k, const F16Plan& plan);
+// second (plan with pair): another matrix of w's shape in the same launch, fp32 into out.out[1].
 cudaError_t launch_mmq_f16(const WeightView& w, const Q8View& x, const TcOutput& out, const F16Plan& plan, void* scratch, bool alternates,
-                           int* status, cudaStream_t stream);
+                           int* status, cudaStream_t stream, const WeightView* second = nullptr);
 
 // gemv_tma.cu : m <= 16.  Weights streamed by TMA into a shared-memory ring, activations held in
 // registers by warps that each own one super-block column of the block's K slice; K slices of

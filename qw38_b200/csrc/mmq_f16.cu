@@ -39,6 +39,9 @@
 // units; tiles cut by a run's ends go through fp32 scratch and are added in run order by whoever arrives last.  When
 // whole tiles per cluster are about as quick, runs are cut at tile boundaries instead (plan_f16).
 //
+// Two matrices of one shape over the same tokens (gate and up) go as one launch: each SM of a pair takes the rows of one of
+// them.  That is one set of planes, one prologue and one last wave instead of two.
+//
 // Warps: 0 raw weights (TMA), 1 activation planes (TMA), 2 MMA issue (leader CTA), 3 TMEM allocation and launch overlap,
 // then expanders, then epilogue.  Every wait is bounded; a wait that gives up sets the abort flag and the status word, and
 // every role leaves its loop.
@@ -118,6 +121,7 @@ struct F16Params {
   uint32_t* tickets;       // [cluster][CTA][epilogue warp]
   int* status;
   uint32_t n, m, m_pad, tiles_k, tok_tiles;
+  uint32_t pair;           // two matrices of one shape: the leader's rows are the first one's, the peer's the second one's
   // Cluster w takes units [first(w), first(w + 1)): run_each steps of unit_step units, the first run_rest clusters one more.
   uint32_t run_each, run_rest, unit_step;
 };
@@ -314,6 +318,7 @@ __global__ void __launch_bounds__(256) planes_kernel(const int8_t* __restrict__ 
 template <int NT>
 __global__ void __launch_bounds__(F16Cfg<NT>::kBoundThreads, 1)
 mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_constant__ CUtensorMap tm_meta,
+               const __grid_constant__ CUtensorMap tm_codes1, const __grid_constant__ CUtensorMap tm_meta1,
                const __grid_constant__ CUtensorMap tm_planes, const __grid_constant__ CUtensorMap tm_sums, const F16Params p) {
   using C = F16Cfg<NT>;
   extern __shared__ uint8_t smem_raw[];
@@ -344,12 +349,15 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
 
   // Raw weights are never written by an earlier launch, so they stream before any wait; the first ring of them even
   // before the block has met.
+  const CUtensorMap* const codes_map = p.pair && cta ? &tm_codes1 : &tm_codes;
+  const CUtensorMap* const meta_map = p.pair && cta ? &tm_meta1 : &tm_meta;
+  auto row_tile = [&](const Cursor& c) { return p.pair ? c.row_pair : c.row_pair * 2 + cta; };
   auto load_raw = [&](const Cursor& c, uint32_t stage) {
-    int const rg = int((c.row_pair * 2 + cta) * (kRows / 8));
+    int const rg = int(row_tile(c) * (kRows / 8));
     uint32_t const dst = smem + C::oRaw + stage * C::kRaw;
     mbar_expect_tx(raw_full(stage), C::kRaw);
-    tma_3d(dst, &tm_codes, 0, int(c.kb * 8), rg, raw_full(stage));
-    tma_3d(dst + 16 * 1024, &tm_meta, 0, int(c.kb), rg, raw_full(stage));
+    tma_3d(dst, codes_map, 0, int(c.kb * 8), rg, raw_full(stage));
+    tma_3d(dst + 16 * 1024, meta_map, 0, int(c.kb), rg, raw_full(stage));
   };
   if (warp == 0) {
     for (uint32_t i = lane; i < uint32_t(C::kBars); i += 32) {  // in the order of the offsets above
@@ -655,7 +663,7 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
       for (int j = 0; j < C::kCols / 2; ++j)
         acc[j] = __fmul2_rn(acc[j], make_float2(__shfl_sync(0xffffffffu, token_scale, 2 * j), __shfl_sync(0xffffffffu, token_scale, 2 * j + 1)));
       // A lane's values are one row of consecutive tokens: every store of a warp is 32 neighbouring rows of one token.
-      uint32_t const n_row = (c.row_pair * 2 + cta) * kRows + row, tok0 = c.tok * NT + col0;
+      uint32_t const n_row = row_tile(c) * kRows + row, tok0 = c.tok * NT + col0;
       if (write && n_row < p.n && tok0 < p.m) {
         uint32_t const live = min(p.m - tok0, uint32_t(C::kCols));
         uint64_t o = uint64_t(tok0) * p.out_stride + p.out_row0 + n_row;
@@ -675,7 +683,8 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
             for (int j = 0; j < 8; ++j)
               if (j0 + j < live) p.out_bf16[o + j * uint64_t(p.out_stride)] = f32_to_bf16_rne(v[j]);
           } else {
-            for (uint32_t g = 0; g < p.ndst; ++g) {
+            uint32_t const first = p.pair ? cta : 0u;
+            for (uint32_t g = first; g < first + p.ndst; ++g) {
 #pragma unroll
               for (int j = 0; j < 8; ++j)
                 if (j0 + j < live) p.out[g][o + j * uint64_t(p.out_stride)] = v[j];
@@ -718,6 +727,9 @@ constexpr uint64_t kTicketBytes = uint64_t(kMaxClusters) * 2 * 16 * 4;
 
 uint64_t align1k(uint64_t v) { return (v + 1023) / 1024 * 1024; }
 
+// Row tiles of a pair of CTAs: 256 rows of a matrix, or 128 of each of two.
+uint32_t row_pairs(uint32_t n, bool pair) { return pair ? (n + kRows - 1) / kRows : (n + 2 * kRows - 1) / (2 * kRows); }
+
 struct Carve {
   uint64_t slots, sums, exps, tokens, planes, total;
 };
@@ -734,7 +746,7 @@ Carve carve(uint32_t m, uint32_t tiles_k, const F16Plan& plan) {
 }
 
 template <int NT>
-cudaError_t launch_f16(const WeightView& w, const Q8View& x, const TcOutput& o, const F16Plan& plan, uint8_t* scratch, bool early, int* status,
+cudaError_t launch_f16(const WeightView& w, const WeightView* second, const Q8View& x, const TcOutput& o, const F16Plan& plan, uint8_t* scratch, bool early, int* status,
                        cudaStream_t stream) {
   using C = F16Cfg<NT>;
   Carve const c = carve(x.m, w.tiles_k, plan);
@@ -745,18 +757,17 @@ cudaError_t launch_f16(const WeightView& w, const Q8View& x, const TcOutput& o, 
                                  reinterpret_cast<float*>(scratch + c.exps), reinterpret_cast<float*>(scratch + c.tokens),
                                  reinterpret_cast<uint32_t*>(scratch), plan.unit_step == 1 ? uint32_t(kTicketBytes / 4) : 0u, early);
   if (st != cudaSuccess) return st;
-  CUtensorMap tm_codes, tm_meta, tm_planes, tm_sums;
+  CUtensorMap tm_codes[2], tm_meta[2], tm_planes, tm_sums;
   uint64_t const rgs = w.padded_n / 8;
-  {
+  WeightView const ws[2] = {w, second ? *second : w};
+  for (int i = 0; i < 2; ++i) {
     uint64_t dims[3] = {128, uint64_t(w.tiles_k) * 8, rgs}, strides[2] = {128, uint64_t(w.tiles_k) * 1024};
     uint32_t box[3] = {128, 8, 16};
-    if (!make_map(&tm_codes, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, w.codes, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B))
-      return cudaErrorInvalidValue;
-  }
-  {
-    uint64_t dims[3] = {128, w.tiles_k, rgs}, strides[2] = {128, uint64_t(w.tiles_k) * 128};
-    uint32_t box[3] = {128, 1, 16};
-    if (!make_map(&tm_meta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, w.meta, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE))
+    uint64_t mdims[3] = {128, w.tiles_k, rgs}, mstrides[2] = {128, uint64_t(w.tiles_k) * 128};
+    uint32_t mbox[3] = {128, 1, 16};
+    if (i == 1 && !second) { tm_codes[1] = tm_codes[0]; tm_meta[1] = tm_meta[0]; break; }
+    if (!make_map(&tm_codes[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, ws[i].codes, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !make_map(&tm_meta[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, ws[i].meta, mdims, mstrides, mbox, CU_TENSOR_MAP_SWIZZLE_NONE))
       return cudaErrorInvalidValue;
   }
   {
@@ -778,7 +789,9 @@ cudaError_t launch_f16(const WeightView& w, const Q8View& x, const TcOutput& o, 
   p.out_stride = o.stride ? o.stride : w.n; p.out_row0 = o.row0;
   p.exps = reinterpret_cast<const float*>(scratch + c.exps); p.tokens = reinterpret_cast<const float*>(scratch + c.tokens); p.slots = reinterpret_cast<float*>(scratch + c.slots); p.tickets = reinterpret_cast<uint32_t*>(scratch);
   p.status = status; p.n = w.n; p.m = x.m; p.m_pad = m_pad; p.tiles_k = w.tiles_k; p.tok_tiles = m_pad / NT;
-  uint32_t const steps = (w.padded_n + 2 * kRows - 1) / (2 * kRows) * p.tok_tiles * w.tiles_k / plan.unit_step;
+  p.pair = second ? 1u : 0u;
+  if (second) p.out[1] = o.out[1];
+  uint32_t const steps = row_pairs(w.padded_n, second != nullptr) * p.tok_tiles * w.tiles_k / plan.unit_step;
   p.run_each = steps / plan.workers; p.run_rest = steps % plan.workers; p.unit_step = plan.unit_step;
   // setmaxnreg.inc waits for registers that the block must have been launched with: a build that allotted fewer than the
   // split assumes may not run.
@@ -803,7 +816,7 @@ cudaError_t launch_f16(const WeightView& w, const Q8View& x, const TcOutput& o, 
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, mmq_f16_kernel<NT>, tm_codes, tm_meta, tm_planes, tm_sums, p);
+  return cudaLaunchKernelEx(&cfg, mmq_f16_kernel<NT>, tm_codes[0], tm_meta[0], tm_codes[1], tm_meta[1], tm_planes, tm_sums, p);
 }
 
 }  // namespace
@@ -813,7 +826,7 @@ bool f16_supported(const WeightView& w, const Q8View& x) {
          reinterpret_cast<uintptr_t>(x.codes) % 8 == 0;
 }
 
-F16Plan plan_f16(uint32_t m, uint32_t n, uint32_t tiles_k) {
+F16Plan plan_f16(uint32_t m, uint32_t n, uint32_t tiles_k, bool pair) {
   F16Plan p;
   // Tokens per pass: the planes of one pass (four bytes per element) stay below 64 MB, half of L2.
   uint64_t const most = (64ull << 20) / (uint64_t(tiles_k) * 1024) / 128 * 128;
@@ -822,7 +835,7 @@ F16Plan plan_f16(uint32_t m, uint32_t n, uint32_t tiles_k) {
   uint32_t const mc = p.chunk < m ? p.chunk : m;
   p.nt = mc <= 16 ? 16 : (mc <= 32 ? 32 : (mc <= 64 ? 64 : 128));
   uint32_t const clusters = uint32_t(sm_count()) / 2;
-  uint64_t const tiles = uint64_t((n + 2 * kRows - 1) / (2 * kRows)) * ((mc + p.nt - 1) / p.nt), units = tiles * tiles_k;
+  uint64_t const tiles = uint64_t(row_pairs(n, pair)) * ((mc + p.nt - 1) / p.nt), units = tiles * tiles_k;
   // Whole tiles per cluster, or equal runs of super-blocks (at least four) whose cut tiles are added through scratch?
   // In units of one super-block; the cut costs about as much as kCut of them.
   double const kCut = p.nt >= 128 ? 2.0 : (p.nt >= 64 ? 3.0 : 5.0);
@@ -845,7 +858,9 @@ uint64_t f16_scratch_bytes(uint32_t m, uint32_t tiles_k, const F16Plan& plan) {
 }
 
 cudaError_t launch_mmq_f16(const WeightView& w, const Q8View& x, const TcOutput& out, const F16Plan& plan, void* scratch, bool alternates,
-                           int* status, cudaStream_t stream) {
+                           int* status, cudaStream_t stream, const WeightView* second) {
+  if (second && (second->n != w.n || second->tiles_k != w.tiles_k || out.ndst != 1 || out.out_bf16 || out.residual || out.done || !out.out[1]))
+    return cudaErrorInvalidValue;
   if (out.ndst < 1 || out.ndst > 8 || (out.out_bf16 ? out.ndst != 1 : out.out[0] == nullptr) || plan.workers < 1 ||
       plan.workers > kMaxClusters)
     return cudaErrorInvalidValue;
@@ -857,16 +872,16 @@ cudaError_t launch_mmq_f16(const WeightView& w, const Q8View& x, const TcOutput&
     xc.m = x.m - t0 < plan.chunk ? x.m - t0 : plan.chunk;
     xc.codes += uint64_t(t0) * x.padded_k; xc.scales += t0 * G; xc.sums += t0 * G;
     TcOutput oc = out;
-    for (uint32_t g = 0; g < out.ndst; ++g) if (oc.out[g]) oc.out[g] += t0 * stride;
+    for (uint32_t g = 0; g < (second ? 2 : out.ndst); ++g) if (oc.out[g]) oc.out[g] += t0 * stride;
     if (oc.out_bf16) oc.out_bf16 += t0 * stride;
     if (oc.residual) oc.residual += t0 * stride;
     if (t0 + plan.chunk < x.m) oc.done = nullptr;  // row-sharded use: the projection counts once, with its last pass
     F16Plan pc = plan;
     if (xc.m < plan.chunk) {  // a shorter last pass: fewer token tiles of the same width
-      F16Plan const last = plan_f16(xc.m, w.n, w.tiles_k);
+      F16Plan const last = plan_f16(xc.m, w.n, w.tiles_k, second != nullptr);
       if (last.nt == plan.nt) { pc.workers = last.workers; pc.unit_step = last.unit_step; }
       else {
-        uint64_t const tiles = uint64_t((w.n + 2 * kRows - 1) / (2 * kRows)) * ((xc.m + plan.nt - 1) / plan.nt);
+        uint64_t const tiles = uint64_t(row_pairs(w.n, second != nullptr)) * ((xc.m + plan.nt - 1) / plan.nt);
         pc.unit_step = w.tiles_k;
         pc.workers = uint32_t(tiles < uint64_t(plan.workers) ? tiles : uint64_t(plan.workers));
       }
@@ -874,10 +889,10 @@ cudaError_t launch_mmq_f16(const WeightView& w, const Q8View& x, const TcOutput&
     uint8_t* const s = static_cast<uint8_t*>(scratch);
     cudaError_t st;
     switch (plan.nt) {
-      case 16: st = launch_f16<16>(w, xc, oc, pc, s, early, status, stream); break;
-      case 32: st = launch_f16<32>(w, xc, oc, pc, s, early, status, stream); break;
-      case 64: st = launch_f16<64>(w, xc, oc, pc, s, early, status, stream); break;
-      case 128: st = launch_f16<128>(w, xc, oc, pc, s, early, status, stream); break;
+      case 16: st = launch_f16<16>(w, second, xc, oc, pc, s, early, status, stream); break;
+      case 32: st = launch_f16<32>(w, second, xc, oc, pc, s, early, status, stream); break;
+      case 64: st = launch_f16<64>(w, second, xc, oc, pc, s, early, status, stream); break;
+      case 128: st = launch_f16<128>(w, second, xc, oc, pc, s, early, status, stream); break;
       default: return cudaErrorInvalidValue;
     }
     if (st != cudaSuccess) return st;

@@ -424,12 +424,13 @@ def main():
     scale = n_layers / STREAM_LAYERS
     total_bytes = stream_step_bytes() * scale
     value = total_bytes * steps / (ms * 1e-3) / 1e9
-    launches_per_step = len(tokens) * n_layers * (2 + len(SHAPES)) + (1 if fused else 0)
+    # packs and projections; beyond sixteen tokens a projection is two launches (operand planes, matmul), unless it gathers
+    launches_per_step = sum(n_layers * (2 + len(SHAPES) * (2 if m > 16 and not fused else 1)) for m in tokens) + (1 if fused else 0)
 
     # ---- the projection kernels alone, per token count (no quantiser, no cross-GPU wait inside the graph)
     peaks = json.loads((ROOT / "MEASURED_PEAKS.json").read_text()) if (ROOT / "MEASURED_PEAKS.json").exists() else {}
     hbm_peak, peak_src = (peaks["hbm_gbs"], "measured") if "hbm_gbs" in peaks else (6650.0, "fallback")
-    kernel_of = {1: "gemv_tma_kernel" if not args.no_overlap else "gemv_dp4a_kernel", 64: "mmq_tcgen05_kernel<64,64>"}
+    kernel_of = {1: "gemv_tma_kernel", 64: "mmq_tcgen05_kernel<64,64>"} if fused else {1: "gemv_dp4a_kernel<1>", 64: "mmq_f16_kernel<64>"}
     by_tokens = {}
     for m in tokens:
         gk = [capture(lambda p=p, mm=m: stream_step(p, quantise=False, only_m=mm)) for p in (0, 1)]
@@ -611,7 +612,7 @@ def single_gpu_extras(torch, lib, L, synth, dev, stream, g, failure, peaks, hbm_
         stream.synchronize()
         t = e0.elapsed_time(e1) / reps
         tops_ = 2.0 * m * n * k / (t * 1e-3) / 1e12
-        prefill[f"M{m}_N{n}_K{k}"] = {"ms": round(t, 4), "int8_TOPS": round(tops_, 1), "kernel": "mmq_tcgen05_kernel<128,128>",
+        prefill[f"M{m}_N{n}_K{k}"] = {"ms": round(t, 4), "int8_TOPS": round(tops_, 1), "kernel": "mmq_f16_kernel<128>",
                                       "frac_of_measured_int8_peak": None if not int8_peak else round(tops_ / int8_peak, 4),
                                       "frac_of_nominal_4500": round(tops_ / 4500.0, 4)}
         # comparator: the reference's other prefill route on this GPU, unpack to bf16 + library GEMM (a library path,
@@ -645,11 +646,11 @@ def single_gpu_extras(torch, lib, L, synth, dev, stream, g, failure, peaks, hbm_
     stream.synchronize()
     t = e0.elapsed_time(e1) / 10
     prefill["ragged_M1821_N34816_K5120"] = {"ms": round(t, 4), "int8_TOPS": round(2.0 * m * n * k / (t * 1e-3) / 1e12, 1),
-                                            "kernel": "mmq_tcgen05_kernel<128,128>", "requests": len(offs) - 1}
+                                            "kernel": "mmq_f16_kernel<128>", "requests": len(offs) - 1}
     del w, o, xq
     out["prefill"] = prefill
     head = prefill["M2048_N17408_K5120"]
-    out["prefill_roofline"] = {"bound": "tensor", "kernel": "mmq_tcgen05_kernel<128,128>", "workload": "config[2]: M=2048, N=17408, K=5120",
+    out["prefill_roofline"] = {"bound": "tensor", "kernel": "mmq_f16_kernel<128>", "workload": "config[2]: M=2048, N=17408, K=5120",
                                "achieved": head["int8_TOPS"], "peak": int8_peak, "unit": "TOP/s",
                                "frac": None if not int8_peak else head["int8_TOPS"] / int8_peak,
                                "peak_source": "measured" if int8_peak else "unavailable",

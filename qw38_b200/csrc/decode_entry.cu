@@ -11,8 +11,9 @@ namespace {
 // sigmoid / SiLU exactly as the reference's decode epilogue states them
 // (cuda/decode_mmv.cu:78-89): the exponential is always taken of a non-positive number.
 __device__ __forceinline__ float sigmoid_fp32(float u) {
-  float const e = expf(-fabsf(u));
-  return (u >= 0.0f ? 1.0f : e) / (1.0f + e);
+  float const e = expf(-fabsf(u)), d = 1.0f + e, n = u >= 0.0f ? 1.0f : e;
+  // below 2^-24 the divisor is 1: not sent through the division, which leaves its short form for a tiny numerator
+  return d == 1.0f ? n : n / d;
 }
 
 __global__ void store_bf16_kernel(const float* __restrict__ in, uint16_t* __restrict__ out, uint64_t count) {

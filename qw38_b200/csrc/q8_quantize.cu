@@ -12,7 +12,7 @@
 namespace q4k {
 namespace {
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 256, kBlocksPerSm = 6;
 
 // Quantise the eight values of this lane; lanes (4j..4j+3) share a group.
 __device__ __forceinline__ void pack8(const float (&x)[8], int8_t* codes, float* scales,
@@ -35,51 +35,64 @@ template <> __device__ __forceinline__ float to_f32<float>(float v) { return v; 
 // Vec: rows start 16-byte aligned and k % 8 == 0, so a lane's eight values are
 // one (bf16) or two (fp32) aligned 16-byte loads.
 template <typename T, bool Vec>
-__global__ void __launch_bounds__(kThreads) pack_kernel(const T* __restrict__ in, int8_t* codes,
-                                                         float* scales, int32_t* sums, uint32_t m,
-                                                         uint32_t k, uint32_t pk, int* failure) {
+__device__ __forceinline__ void load8(const T* src, uint32_t col0, uint32_t k, float (&x)[8]) {
+  if (Vec && col0 + 8 <= k) {
+    if constexpr (sizeof(T) == 2) {
+      uint4 v = *reinterpret_cast<const uint4*>(src + col0);
+      uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        x[2 * i] = __uint_as_float(w[i] << 16);
+        x[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+      }
+    } else {
+      float4 lo = *reinterpret_cast<const float4*>(src + col0);
+      float4 hi = *reinterpret_cast<const float4*>(src + col0 + 4);
+      x[0] = lo.x; x[1] = lo.y; x[2] = lo.z; x[3] = lo.w;
+      x[4] = hi.x; x[5] = hi.y; x[6] = hi.z; x[7] = hi.w;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = col0 + i < k ? to_f32<T>(src[col0 + i]) : 0.f;
+  }
+}
+
+// A warp takes 256 columns of a row at a time, two such tasks requested before either is quantised.
+template <typename T, bool Vec>
+__global__ void __launch_bounds__(kThreads, kBlocksPerSm) pack_kernel(const T* __restrict__ in, int8_t* __restrict__ codes,
+                                                                       float* __restrict__ scales, int32_t* __restrict__ sums, uint32_t m,
+                                                                       uint32_t k, uint32_t pk, int* failure) {
   pdl_wait();               // the input may come from the kernel before this one
   pdl_launch_dependents();  // the projection that follows may start prefetching its weights (after the wait: the
                             // next launch never runs beside anything older than this one)
   uint32_t const lane = threadIdx.x & 31, sub = lane & 3, grp = lane >> 2;
-  uint64_t const chunks_row = pk / 256;
-  uint64_t const tasks = uint64_t(m) * chunks_row;
-  uint64_t const warps = uint64_t(gridDim.x) * (kThreads / 32);
-  for (uint64_t task = uint64_t(blockIdx.x) * (kThreads / 32) + threadIdx.x / 32; task < tasks;
-       task += warps) {
-    uint32_t const row = uint32_t(task / chunks_row), chunk = uint32_t(task % chunks_row);
-    uint32_t const col0 = chunk * 256 + grp * 32 + sub * 8;
-    const T* src = in + uint64_t(row) * k;
-    float x[8];
-    if (Vec && col0 + 8 <= k) {
-      if constexpr (sizeof(T) == 2) {
-        uint4 v = *reinterpret_cast<const uint4*>(src + col0);
-        uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          x[2 * i] = __uint_as_float(w[i] << 16);
-          x[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
-        }
-      } else {
-        float4 lo = *reinterpret_cast<const float4*>(src + col0);
-        float4 hi = *reinterpret_cast<const float4*>(src + col0 + 4);
-        x[0] = lo.x; x[1] = lo.y; x[2] = lo.z; x[3] = lo.w;
-        x[4] = hi.x; x[5] = hi.y; x[6] = hi.z; x[7] = hi.w;
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) x[i] = col0 + i < k ? to_f32<T>(src[col0 + i]) : 0.f;
-    }
-    pack8(x, codes, scales, sums, uint64_t(row) * (pk / 32) + chunk * 8 + grp, sub, failure);
+  uint32_t const chunks_row = pk / 256, tasks = m * chunks_row;  // below 2^32 for every accepted shape
+  uint32_t const warps = gridDim.x * (kThreads / 32);
+  for (uint32_t task = blockIdx.x * (kThreads / 32) + threadIdx.x / 32; task < tasks; task += 2 * warps) {
+    uint32_t const other = task + warps;
+    bool const two = other < tasks;
+    float x[8], y[8];
+    load8<T, Vec>(in + uint64_t(task / chunks_row) * k, task % chunks_row * 256 + lane * 8, k, x);
+    if (two) load8<T, Vec>(in + uint64_t(other / chunks_row) * k, other % chunks_row * 256 + lane * 8, k, y);
+    pack8(x, codes, scales, sums, uint64_t(task) * 8 + grp, sub, failure);
+    if (two) pack8(y, codes, scales, sums, uint64_t(other) * 8 + grp, sub, failure);
   }
+}
+
+// g / (1 + exp(-g)), rounded as it stands.  A divisor above 2^64 is scaled (exactly: the quotient of a finite g stays a normal
+// number) and an infinite one replaced, because the division leaves its short form for both.
+__device__ __forceinline__ float silu(float g) {
+  float const d = 1.f + expf(-g);
+  bool const far = d > 0x1p64f, lost = isinf(d);
+  return g / (lost ? 1.f : (far ? d * 0x1p-64f : d)) * (lost ? 0.f : (far ? 0x1p-64f : 1.f));
 }
 
 // v = bf16_rne(silu(g) * u); non-finite g or u poisons the value
 // (reference: swiglu_pack_kernel, cuda/q4k_q8.cu:52-61).  ffn % 256 == 0.
 __global__ void __launch_bounds__(kThreads) swiglu_pack_kernel(const float* __restrict__ gate,
                                                                 const float* __restrict__ up,
-                                                                int8_t* codes, float* scales,
-                                                                int32_t* sums, uint64_t chunks,
+                                                                int8_t* __restrict__ codes, float* __restrict__ scales,
+                                                                int32_t* __restrict__ sums, uint64_t chunks,
                                                                 int* failure) {
   pdl_wait();
   pdl_launch_dependents();
@@ -95,7 +108,7 @@ __global__ void __launch_bounds__(kThreads) swiglu_pack_kernel(const float* __re
     float x[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      float v = (g[i] / (1.f + expf(-g[i]))) * u[i];
+      float v = silu(g[i]) * u[i];
       if (!isfinite(g[i]) || !isfinite(u[i])) v = __int_as_float(0x7fc00000);
       x[i] = bf16_bits_to_f32(f32_to_bf16_rne(v));
     }
@@ -211,7 +224,7 @@ __global__ void export_q8_1_kernel(const int8_t* __restrict__ codes, const float
 
 int grid_for(uint64_t tasks) {
   uint64_t blocks = (tasks + kThreads / 32 - 1) / (kThreads / 32);
-  if (blocks > 148 * 16) blocks = 148 * 16;
+  if (blocks > uint64_t(148 * kBlocksPerSm)) blocks = 148 * kBlocksPerSm;
   return int(blocks ? blocks : 1);
 }
 

@@ -126,3 +126,28 @@ def test_repack_of_unaligned_blocks(n, k, by):
     blocks = torch.from_numpy(synth.blocks144(codes, meta).reshape(-1)).to(DEV)
     w = repack_blocks144(shifted(blocks, by), n, k)
     assert (w.codes.cpu().numpy() == hc.reshape(-1)).all() and (w.scales.cpu().numpy() == hs.reshape(-1)).all()
+
+
+def quotient_rows():
+    """Every bf16 mantissa of a value against every one of its group's peak, and fp32 groups over the exponent range."""
+    mant = (1 + np.arange(128) / 128).astype(np.float32)
+    values = (mant[:, None] * (2.0 ** -np.arange(1, 11))[None, :]).reshape(-1).astype(np.float32)
+    pad = np.zeros(31 * 42 - values.size, np.float32)
+    groups = np.concatenate([values, pad]).reshape(42, 31)
+    groups = np.concatenate([np.repeat(mant[:, None, None], 42, 1), np.repeat(groups[None], 128, 0)], 2)  # peak first
+    rng = np.random.default_rng(3)
+    wide = rng.standard_normal((20000, 32)).astype(np.float32) * np.exp2(rng.integers(-120, 121, (20000, 1))).astype(np.float32)
+    wide[::7, ::3] = 0
+    wide[::11, 1::4] *= np.float32(1e-30)
+    return groups.reshape(-1, 256).astype(np.float32), wide.reshape(-1, 256)
+
+
+@pytest.mark.parametrize("which", [0, 1])
+def test_quantiser_quotients_are_the_divisions(which):
+    x = quotient_rows()[which]
+    f = flag()
+    q = pack_q8(torch.from_numpy(x).to(DEV), f)
+    z, a, s, bad = orc.q8_quantize(x)
+    assert f.item() == bad
+    assert (q.codes.cpu().numpy() == z).all() and (q.sums.cpu().numpy() == s).all()
+    assert (q.scales.cpu().numpy().view(np.uint32) == a.view(np.uint32)).all()

@@ -2,8 +2,11 @@
 // DecodeEpilogue forms of the reference (cuda/decode_mmv.hpp:45-51) applied to fp32 projection
 // rows.  StoreFp32 and ResidualAddFp32 need no kernel of their own: the projection writes the
 // destination directly (the residual is its last fp32 add, cuda/q4k_q8.cu:100).
+#include <cuda_bf16.h>
+
 #include "common.cuh"
 #include "launch.h"
+#include "q8_pack.cuh"
 
 namespace q4k {
 namespace {
@@ -11,9 +14,9 @@ namespace {
 // sigmoid / SiLU exactly as the reference's decode epilogue states them
 // (cuda/decode_mmv.cu:78-89): the exponential is always taken of a non-positive number.
 __device__ __forceinline__ float sigmoid_fp32(float u) {
+  // below 2^-24 the divisor is 1; the others are between 1 and 2, their quotient rounded as the division would be
   float const e = expf(-fabsf(u)), d = 1.0f + e, n = u >= 0.0f ? 1.0f : e;
-  // below 2^-24 the divisor is 1: not sent through the division, which leaves its short form for a tiny numerator
-  return d == 1.0f ? n : n / d;
+  return d == 1.0f ? n : rounded_quotient(n, d, __frcp_rn(d));
 }
 
 __global__ void store_bf16_kernel(const float* __restrict__ in, uint16_t* __restrict__ out, uint64_t count) {
@@ -39,9 +42,12 @@ __global__ void swiglu_store_bf16_kernel(const float* __restrict__ gate, const f
     float const g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w}, u[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
     uint32_t w[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      w[j] = uint32_t(f32_to_bf16_rne(g[2 * j] * sigmoid_fp32(g[2 * j]) * u[2 * j])) |
-             uint32_t(f32_to_bf16_rne(g[2 * j + 1] * sigmoid_fp32(g[2 * j + 1]) * u[2 * j + 1])) << 16;
+    for (int j = 0; j < 4; ++j) {
+      float const a = g[2 * j] * sigmoid_fp32(g[2 * j]) * u[2 * j], b = g[2 * j + 1] * sigmoid_fp32(g[2 * j + 1]) * u[2 * j + 1];
+      __nv_bfloat162 const v = __floats2bfloat162_rn(a, b);
+      w[j] = *reinterpret_cast<const uint32_t*>(&v);
+      if (isnan(a) || isnan(b)) w[j] = uint32_t(f32_to_bf16_rne(a)) | uint32_t(f32_to_bf16_rne(b)) << 16;  // NaNs keep their bits
+    }
     reinterpret_cast<uint4*>(out)[i] = make_uint4(w[0], w[1], w[2], w[3]);
   } else if (i < count) {
     float const g = gate[i];

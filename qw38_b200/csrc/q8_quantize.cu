@@ -5,6 +5,8 @@
 //
 // Mapping: four lanes own one K32 group, eight values per lane, so a warp covers
 // 256 consecutive columns with 16-byte loads and 8-byte stores.
+#include <cuda_bf16.h>
+
 #include "common.cuh"
 #include "launch.h"
 #include "q8_pack.cuh"
@@ -57,7 +59,7 @@ __device__ __forceinline__ void load8(const T* src, uint32_t col0, uint32_t k, f
   }
 }
 
-// A warp takes 256 columns of a row at a time, two such tasks requested before either is quantised.
+// A warp takes 256 columns of a row at a time; the next ones are requested before the present ones are quantised.
 template <typename T, bool Vec>
 __global__ void __launch_bounds__(kThreads, kBlocksPerSm) pack_kernel(const T* __restrict__ in, int8_t* __restrict__ codes,
                                                                        float* __restrict__ scales, int32_t* __restrict__ sums, uint32_t m,
@@ -68,23 +70,29 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) pack_kernel(const T* _
   uint32_t const lane = threadIdx.x & 31, sub = lane & 3, grp = lane >> 2;
   uint32_t const chunks_row = pk / 256, tasks = m * chunks_row;  // below 2^32 for every accepted shape
   uint32_t const warps = gridDim.x * (kThreads / 32);
-  for (uint32_t task = blockIdx.x * (kThreads / 32) + threadIdx.x / 32; task < tasks; task += 2 * warps) {
-    uint32_t const other = task + warps;
-    bool const two = other < tasks;
-    float x[8], y[8];
-    load8<T, Vec>(in + uint64_t(task / chunks_row) * k, task % chunks_row * 256 + lane * 8, k, x);
-    if (two) load8<T, Vec>(in + uint64_t(other / chunks_row) * k, other % chunks_row * 256 + lane * 8, k, y);
+  uint32_t task = blockIdx.x * (kThreads / 32) + threadIdx.x / 32;
+  float x[8], next[8];
+  auto load = [&](uint32_t t, float (&to)[8]) { load8<T, Vec>(in + uint64_t(t / chunks_row) * k, t % chunks_row * 256 + lane * 8, k, to); };
+  if (task < tasks) load(task, x);
+  for (; task < tasks; task += warps) {
+    bool const more = task + warps < tasks;
+    if (more) load(task + warps, next);
     pack8(x, codes, scales, sums, uint64_t(task) * 8 + grp, sub, failure);
-    if (two) pack8(y, codes, scales, sums, uint64_t(other) * 8 + grp, sub, failure);
+    if (more) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] = next[i];
+    }
   }
 }
 
-// g / (1 + exp(-g)), rounded as it stands.  A divisor above 2^64 is scaled (exactly: the quotient of a finite g stays a normal
-// number) and an infinite one replaced, because the division leaves its short form for both.
+// g / (1 + exp(-g)), rounded as the division would be.  A divisor above 2^64 is scaled (exactly: the quotient of a finite g
+// stays a normal number) and an infinite one replaced, so that no residual of the quotient underflows.  Not finite for a g
+// that is not.
 __device__ __forceinline__ float silu(float g) {
   float const d = 1.f + expf(-g);
   bool const far = d > 0x1p64f, lost = isinf(d);
-  return g / (lost ? 1.f : (far ? d * 0x1p-64f : d)) * (lost ? 0.f : (far ? 0x1p-64f : 1.f));
+  float const by = lost ? 1.f : (far ? d * 0x1p-64f : d);
+  return rounded_quotient(g, by, __frcp_rn(by)) * (lost ? 0.f : (far ? 0x1p-64f : 1.f));
 }
 
 // v = bf16_rne(silu(g) * u); non-finite g or u poisons the value
@@ -107,10 +115,11 @@ __global__ void __launch_bounds__(kThreads) swiglu_pack_kernel(const float* __re
     float u[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
     float x[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      float v = silu(g[i]) * u[i];
-      if (!isfinite(g[i]) || !isfinite(u[i])) v = __int_as_float(0x7fc00000);
-      x[i] = bf16_bits_to_f32(f32_to_bf16_rne(v));
+    for (int i = 0; i < 8; i += 2) {  // what is not finite stays so and makes the group invalid
+      __nv_bfloat162 const v = __floats2bfloat162_rn(silu(g[i]) * u[i], silu(g[i + 1]) * u[i + 1]);
+      uint32_t const w = *reinterpret_cast<const uint32_t*>(&v);
+      x[i] = __uint_as_float(w << 16);
+      x[i + 1] = __uint_as_float(w & 0xffff0000u);
     }
     pack8(x, codes, scales, sums, task * 8 + grp, sub, failure);
   }

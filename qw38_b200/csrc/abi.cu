@@ -243,14 +243,15 @@ constexpr uint32_t kFlagTrustedSpans = 1u, kFlagInputSettled = 2u;
 
 // The fp16-plane kernel with scratch of its own (stream_scratch.cu).
 constexpr uint64_t kF16SuperBlocks = 16384;  // of eight rows; below, nine to sixteen tokens stay with the TMA-streamed kernel
-int project_f16(const q4k_weight& w, const q4k_q8_input& x, const q4k::TcOutput& out, cudaStream_t stream, const q4k_weight* second = nullptr) {
+int project_f16(const q4k_weight& w, const q4k_q8_input& x, const q4k::TcOutput& out, cudaStream_t stream, const q4k_weight* second = nullptr,
+                const q4k::RawRows* raw = nullptr) {
   int* const status = q4k::kernel_status_word();
   if (!status) return Q4K_ERR_STATUS;
   q4k::F16Plan const plan = q4k::plan_f16(x.m, w.n, w.padded_k / 256, second != nullptr);
   q4k::StreamScratch scratch;
   Q4K_CUDA(scratch.acquire(stream, q4k::f16_scratch_bytes(x.m, w.padded_k / 256, plan), q4k_get_launch_overlap() != 0), "scratch.acquire");
   q4k::WeightView const other = second ? view(*second) : q4k::WeightView{};
-  Q4K_CUDA(q4k::launch_mmq_f16(view(w), view(x), out, plan, scratch.p(), scratch.alternates(), status, stream, second ? &other : nullptr),
+  Q4K_CUDA(q4k::launch_mmq_f16(view(w), view(x), out, plan, scratch.p(), scratch.alternates(), status, stream, second ? &other : nullptr, raw),
            "q4k_q8.mmq_f16");
   Q4K_CUDA(scratch.release(), "scratch.release");
   return Q4K_OK;
@@ -258,7 +259,7 @@ int project_f16(const q4k_weight& w, const q4k_q8_input& x, const q4k::TcOutput&
 
 int project_impl(const q4k_weight* weight, const q4k_q8_input& x, float* output, uint64_t output_len,
                  const float* residual, uint64_t residual_len, const q4k_project_options* opt,
-                 cudaStream_t stream, bool residual_in_place = false, char const* role = "projection") {
+                 cudaStream_t stream, bool residual_in_place = false, char const* role = "projection", const q4k::RawRows* raw = nullptr) {
   if (int st = valid_weight(weight, "weight")) return st;
   const q4k_weight& w = *weight;
   if (!valid_input(x) || x.k != w.k || output_len != uint64_t(x.m) * w.n ||
@@ -346,7 +347,7 @@ int project_impl(const q4k_weight* weight, const q4k_q8_input& x, float* output,
       return fail(Q4K_ERR_INVALID_ARGUMENT, "q8.project: the fp16 kernel needs aligned operands and has no partial dots");
     q4k::TcOutput to = q4k::tc_output(output, res);
     to.input_settled = (opt && (opt->flags & kFlagInputSettled)) ? 1u : 0u;
-    return project_f16(w, x, to, stream);
+    return project_f16(w, x, to, stream, nullptr, raw);
   }
   if (kernel == Q4K_KERNEL_TCGEN05) {
     if (!q4k::tcgen05_supported(view(w), view(x)))
@@ -398,7 +399,7 @@ int project_impl(const q4k_weight* weight, const q4k_q8_input& x, float* output,
 // A gate and an up projection of the same input.  Beyond sixteen tokens (where the automatic choice is the fp16 kernel) one
 // launch takes both: an MLP chain of 237 tokens 300 us with two launches, 291 with one.
 int project_pair(const q4k_weight* gate, const q4k_weight* up, const q4k_q8_input& x, float* g, float* u, const q4k_project_options* opt,
-                 cudaStream_t stream) {
+                 cudaStream_t stream, const q4k::RawRows* raw = nullptr) {
   uint64_t const cells = uint64_t(x.m) * gate->n;
   if (x.m <= 16 || up->n != gate->n || up->k != gate->k || !q4k::f16_supported(view(*gate), view(x)) || !q4k::f16_supported(view(*up), view(x))) {
     if (int st = project_impl(gate, x, g, cells, nullptr, 0, opt, stream, false, "gate")) return st;
@@ -418,11 +419,10 @@ int project_pair(const q4k_weight* gate, const q4k_weight* up, const q4k_q8_inpu
                     unsigned(gate->k), "gate_up", 0u, "integer_mma");
   q4k::TcOutput to = q4k::tc_output(g, nullptr);
   to.out[1] = u;
-  return project_f16(*gate, x, to, stream, up);
+  return project_f16(*gate, x, to, stream, up, raw);
 }
 
-int pack_impl(const void* input, bool fp32, uint64_t input_len, const q4k_q8_input& x, int* failure,
-              cudaStream_t stream) {
+int check_pack(const void* input, bool fp32, uint64_t input_len, const q4k_q8_input& x, int* failure) {
   if (!valid_input(x) || input_len != uint64_t(x.m) * x.k || !failure)
     return fail(Q4K_ERR_INVALID_ARGUMENT, "q8.pack: invalid geometry");
   Region regions[5] = {{input, input_len * (fp32 ? 4u : 2u), fp32 ? 4u : 2u, "input"},
@@ -430,7 +430,12 @@ int pack_impl(const void* input, bool fp32, uint64_t input_len, const q4k_q8_inp
                        {x.scales, x.scales_len * 4, 4, "output.scales"},
                        {x.sums, x.sums_len * 4, 4, "output.sums"},
                        {failure, 4, 4, "failure"}};
-  if (int st = check_distinct(regions, 5, false)) return st;
+  return check_distinct(regions, 5, false);
+}
+
+int pack_impl(const void* input, bool fp32, uint64_t input_len, const q4k_q8_input& x, int* failure,
+              cudaStream_t stream) {
+  if (int st = check_pack(input, fp32, input_len, x, failure)) return st;
   ScopedRange range("qw38:op name=q8_pack m=%u n=%u k=%u", unsigned(x.m), unsigned(x.k), 1u);
   Q4K_CUDA(q4k::launch_pack_q8(input, fp32, out_view(x), x.k, failure, stream), "q8.pack");
   return Q4K_OK;
@@ -674,10 +679,11 @@ int valid_decode_desc(const q4k_decode_desc* d, bool paired_b, const char* what,
 
 // Projection + epilogue of one descriptor whose input is already quantised.  `rows` is m*n floats of scratch.
 // fp32 rows of one descriptor under its activation policy, residual added last.
-int decode_rows(const q4k_decode_desc& d, const q4k_q8_input& q8, float* out, const float* residual, cudaStream_t stream) {
+int decode_rows(const q4k_decode_desc& d, const q4k_q8_input& q8, float* out, const float* residual, cudaStream_t stream,
+                const q4k::RawRows* raw = nullptr) {
   uint64_t const cells = uint64_t(d.m) * d.weight.n;
   if (d.activation_policy == Q4K_ACTIVATION_Q8_K32)
-    return project_impl(&d.weight, q8, out, cells, residual, residual ? cells : 0, nullptr, stream, true);
+    return project_impl(&d.weight, q8, out, cells, residual, residual ? cells : 0, nullptr, stream, true, "projection", raw);
   Region regions[3] = {{d.weight.codes, d.weight.codes_bytes, 4, "weight.codes"},
                        {d.weight.scales, d.weight.scales_bytes, 2, "weight.scales"},
                        {out, cells * 4, 4, "output"}};
@@ -688,15 +694,17 @@ int decode_rows(const q4k_decode_desc& d, const q4k_q8_input& q8, float* out, co
 }
 
 // Projection + epilogue of one descriptor whose input is already quantised.  `rows` is m*n floats of scratch.
-int decode_one(const q4k_decode_desc& d, const q4k_q8_input& q8, float* rows, cudaStream_t stream) {
+int decode_one(const q4k_decode_desc& d, const q4k_q8_input& q8, float* rows, cudaStream_t stream,
+               const q4k::RawRows* raw = nullptr) {
   uint64_t const cells = uint64_t(d.m) * d.weight.n;
   switch (d.epilogue) {
     case Q4K_EPILOGUE_STORE_FP32:
-      return decode_rows(d, q8, static_cast<float*>(d.output), nullptr, stream);
+      return decode_rows(d, q8, static_cast<float*>(d.output), nullptr, stream, raw);
     case Q4K_EPILOGUE_RESIDUAL_ADD_FP32:
-      return decode_rows(d, q8, d.output ? static_cast<float*>(d.output) : const_cast<float*>(d.residual), d.residual, stream);
+      return decode_rows(d, q8, d.output ? static_cast<float*>(d.output) : const_cast<float*>(d.residual), d.residual, stream, raw);
     case Q4K_EPILOGUE_STORE_BF16: {
-      if (int st = decode_rows(d, q8, rows, nullptr, stream)) return st;
+      if (int st = decode_rows(d, q8, rows, nullptr, stream, raw)) return st;
+      q4k::ChainedLaunches chained;
       Q4K_CUDA(q4k::launch_store_bf16(rows, static_cast<uint16_t*>(d.output), cells, stream), "decode_mmv.store_bf16");
       return Q4K_OK;
     }
@@ -776,7 +784,7 @@ int decode_fused(const q4k_decode_desc* const* descs, uint32_t count, bool swigl
     if (int st = decode_pack(*descs[0], q8, failure, stream)) return st;
   std::optional<q4k::ChainedLaunches> chained;
   if (!raw) chained.emplace();
-  q4k::GemvTmaRaw const rows{descs[0]->input, descs[0]->weight.k, failure};
+  q4k::RawRows const rows{descs[0]->input, descs[0]->weight.k, failure};
   if (raw && !swiglu && q8.m <= q4k::kGemvDp4aBestTokens) {
     int* const status = q4k::kernel_status_word();
     if (!status) return Q4K_ERR_STATUS;
@@ -852,6 +860,21 @@ int q4k_decode_mmv_paired(const q4k_decode_desc* a, const q4k_decode_desc* b, vo
   return Q4K_OK;
 }
 
+// May the fp16 kernel take the bf16 rows as they are?  Beyond sixteen tokens, unless the input lies in what a first pass
+// over some of the tokens would already overwrite (the pack form has read all of it by then).  Quantising and splitting into
+// planes in one kernel: 2048 x 17408 rows 72 us where a pack and three plane launches took 102.
+bool rows_direct(const q4k_weight& w, const q4k_weight& second, const DecodeScratch& s, const q4k_decode_desc& d) {
+  auto const from = reinterpret_cast<uintptr_t>(d.input), to = from + d.input_len * 2;
+  auto apart = [&](const void* p, uint64_t bytes) {
+    auto const b = reinterpret_cast<uintptr_t>(p);
+    return !p || to <= b || b + bytes <= from;
+  };
+  uint64_t const cells = uint64_t(d.m) * w.n;
+  return d.m > 16 && d.activation_policy == Q4K_ACTIVATION_Q8_K32 && q4k::f16_supported(view(w), view(s.q8)) &&
+         q4k::f16_supported(view(second), view(s.q8)) && apart(d.output, cells * 4) && apart(d.residual, cells * 4) &&
+         apart(s.rows, s.rows_len * 4);
+}
+
 // PrefillEngine::project / paired_swiglu (cuda/prefill.hpp:88-96) with the quantise -> MMQ dispatch: the same
 // composition as the decode entries without the 16-row limit.
 int q4k_prefill_project(const q4k_decode_desc* projection, void* workspace, uint64_t workspace_bytes, int* failure,
@@ -861,9 +884,15 @@ int q4k_prefill_project(const q4k_decode_desc* projection, void* workspace, uint
   DecodeScratch s{};
   if (int st = carve_decode_scratch(workspace, workspace_bytes, projection->m, projection->weight.n, projection->weight.k, &s))
     return st;
-  if (int st = decode_pack(*projection, s.q8, failure, stream)) return st;
+  const q4k_decode_desc& d = *projection;
+  if (rows_direct(d.weight, d.weight, s, d)) {
+    if (int st = check_pack(d.input, false, d.input_len, s.q8, failure)) return st;
+    q4k::RawRows const raw{d.input, d.weight.k, failure};
+    return decode_one(d, s.q8, s.rows, stream, &raw);
+  }
+  if (int st = decode_pack(d, s.q8, failure, stream)) return st;
   q4k::ChainedLaunches chained;
-  return decode_one(*projection, s.q8, s.rows, stream);
+  return decode_one(d, s.q8, s.rows, stream);
 }
 
 int q4k_prefill_paired_swiglu(const q4k_weight* gate, const q4k_weight* up, const uint16_t* normalized, uint16_t* swiglu,
@@ -881,10 +910,18 @@ int q4k_prefill_paired_swiglu(const q4k_weight* gate, const q4k_weight* up, cons
     return fail(Q4K_ERR_INVALID_ARGUMENT, "paired_swiglu: gate and up must have the same shape and layout");
   DecodeScratch s{};
   if (int st = carve_decode_scratch(workspace, workspace_bytes, valid_tokens, gate->n, gate->k, &s)) return st;
-  if (int st = decode_pack(a, s.q8, failure, stream)) return st;
-  q4k::ChainedLaunches chained;
   uint64_t const cells = uint64_t(valid_tokens) * gate->n;
-  if (int st = project_pair(gate, up, s.q8, s.rows, s.rows + cells, nullptr, stream)) return st;
+  bool const direct = rows_direct(*gate, *up, s, a);
+  q4k::RawRows const raw{normalized, gate->k, failure};
+  if (direct) {
+    if (int st = check_pack(normalized, false, a.input_len, s.q8, failure)) return st;
+    if (int st = project_pair(gate, up, s.q8, s.rows, s.rows + cells, nullptr, stream, &raw)) return st;
+  } else if (int st = decode_pack(a, s.q8, failure, stream)) {
+    return st;
+  }
+  q4k::ChainedLaunches chained;
+  if (!direct)
+    if (int st = project_pair(gate, up, s.q8, s.rows, s.rows + cells, nullptr, stream)) return st;
   Q4K_CUDA(q4k::launch_swiglu_store_bf16(s.rows, s.rows + cells, swiglu, cells, stream), "paired_swiglu.epilogue");
   return Q4K_OK;
 }

@@ -381,7 +381,7 @@ cudaError_t launch_gemv_dp4a(const WeightView& w, const Q8View& x, float* out, c
 }
 
 cudaError_t launch_gemv_dp4a_multi(const WeightView* ws, const GemvTmaOutput* outs, uint32_t count, uint32_t m, uint32_t padded_k,
-                                   const GemvTmaRaw& raw, int* status, cudaStream_t stream) {
+                                   const RawRows& raw, int* status, cudaStream_t stream) {
   if (count < 1 || count > 3) return cudaErrorInvalidValue;
   DpParams p{};
   p.wide = 1;

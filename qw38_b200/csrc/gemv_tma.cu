@@ -851,7 +851,7 @@ cudaError_t launch_gemv_tma(const WeightView& w, const Q8View& x, float* out, co
 
 cudaError_t launch_gemv_tma_multi(const WeightView* ws, const GemvTmaOutput* outs, uint32_t count, bool swiglu_pair, const Q8View& x,
                                   const GemvTmaPlan& plan, void* slices, uint32_t* tickets, int* status, cudaStream_t stream,
-                                  const GemvTmaRaw* raw) {
+                                  const RawRows* raw) {
   uint32_t const nt = x.m <= 8 ? 1 : 2;
   uint32_t const cw = plan.warps;
   if (count < 1 || count > 3 || (swiglu_pair && count != 2) || x.m == 0 || x.m > kGemvTmaMaxTokens || cw < 1 ||

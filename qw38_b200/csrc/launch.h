@@ -92,6 +92,14 @@ TcPlan plan_tcgen05(uint32_t m, uint32_t n, uint32_t tiles_k, uint32_t split_k_r
 cudaError_t launch_mmq_tcgen05(const WeightView& w, const Q8View& x, const TcOutput& out, int32_t* partials,
                                const TcPlan& plan, void* partial_tiles, uint32_t* tickets, int* status, cudaStream_t stream);
 
+// Activations that are still bf16 rows [m][k]: the kernel that takes them quantises them itself (its Q8View then only says m
+// and padded_k), and a non-finite group raises *failure, as the pack kernel does.
+struct RawRows {
+  const uint16_t* x;
+  uint32_t k;
+  int* failure;
+};
+
 // mmq_f16.cu : tcgen05 kind::f16 on SM pairs, weights expanded into TMEM, activations as two fp16 planes.  scratch holds
 // f16_scratch_bytes (256-byte aligned) and is used until the launch ends.  alternates: the preceding launch of the stream
 // does not use this scratch, so (with launch overlap and a settled input) the planes may be written beside it.
@@ -107,7 +115,7 @@ F16Plan plan_f16(uint32_t m, uint32_t n, uint32_t tiles_k, bool pair = false);
 uint64_t f16_scratch_bytes(uint32_t m, uint32_t tiles_k, const F16Plan& plan);
 // second (plan with pair): another matrix of w's shape in the same launch, fp32 into out.out[1].
 cudaError_t launch_mmq_f16(const WeightView& w, const Q8View& x, const TcOutput& out, const F16Plan& plan, void* scratch, bool alternates,
-                           int* status, cudaStream_t stream, const WeightView* second = nullptr);
+                           int* status, cudaStream_t stream, const WeightView* second = nullptr, const RawRows* raw = nullptr);
 
 // gemv_tma.cu : m <= 16.  Weights streamed by TMA into a shared-memory ring, activations held in
 // registers by warps that each own one super-block column of the block's K slice; K slices of
@@ -148,19 +156,12 @@ struct GemvTmaOutput {
   uint16_t* out_bf16;
   const float* residual;
 };
-// raw, if given: the activations are still bf16 rows [m][k]; every block quantises its K slice itself (x then only says m
-// and padded_k), and a non-finite group raises *failure, as the pack kernel does.
-struct GemvTmaRaw {
-  const uint16_t* x;
-  uint32_t k;
-  int* failure;
-};
 // The same projections (no SwiGLU pair) from bf16 rows on dp4a, in gemv_dp4a.cu: m <= 4.
 cudaError_t launch_gemv_dp4a_multi(const WeightView* ws, const GemvTmaOutput* outs, uint32_t count, uint32_t m, uint32_t padded_k,
-                                   const GemvTmaRaw& raw, int* status, cudaStream_t stream);
+                                   const RawRows& raw, int* status, cudaStream_t stream);
 cudaError_t launch_gemv_tma_multi(const WeightView* ws, const GemvTmaOutput* outs, uint32_t count, bool swiglu_pair, const Q8View& x,
                                   const GemvTmaPlan& plan, void* slices, uint32_t* tickets, int* status, cudaStream_t stream,
-                                  const GemvTmaRaw* raw = nullptr);
+                                  const RawRows* raw = nullptr);
 // The gate / up pair of an MLP in one launch whose reducer writes the Q8 activation of the down projection directly
 // (codes, scales, sums of bf16(silu(gate) * up), non-finite values raise `failure`): the reference's gate, up and
 // swiglu_pack launches in one.  The plan function says whether the shape qualifies (whole K in one block, rows a

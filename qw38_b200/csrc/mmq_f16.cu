@@ -48,8 +48,11 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 
+#include <optional>
+
 #include "common.cuh"
 #include "launch.h"
+#include "q8_pack.cuh"
 #include "tma.cuh"
 #include "umma.cuh"
 
@@ -84,6 +87,7 @@ template <int NT> struct F16Cfg {
   // TMEM: two accumulators, one min-term accumulator, weight stages.  A group of expanders always uses the same kQ stages
   // (one super-block), so that a warp sees every phase of the barriers it waits on.
   static constexpr int kQ = kStack ? 2 : 4, kACols = 128 / kQ, kAStages = kGroups * kQ;
+  static constexpr bool kReady = kQ == 8;
   static constexpr int kD2Bufs = NT <= 64 ? 2 : 1;  // with one, the min-term MMA waits for the previous super-block's epilogue
   static constexpr int kD2Col = 2 * kN, kACol = kD2Col + kD2Bufs * kN2;
   static_assert(kACol + kAStages * kACols <= 512, "TMEM columns");
@@ -247,42 +251,11 @@ __device__ __forceinline__ int scale_exponent(float top) {  // clamped so that 2
 }
 __device__ __forceinline__ float power_of_two(int e) { return __uint_as_float(uint32_t(127 + e) << 23); }
 
-__global__ void __launch_bounds__(256) planes_kernel(const int8_t* __restrict__ codes, const float* __restrict__ scales,
-                                                     const int32_t* __restrict__ sums, uint32_t m, uint32_t m_pad, uint32_t tiles_k,
-                                                     __half* __restrict__ planes, __half* __restrict__ sums16, float* __restrict__ exps,
-                                                     float* __restrict__ tokens, uint32_t* __restrict__ tickets, uint32_t ticket_count,
-                                                     bool early) {
-  __shared__ float warp_top[8];
-  // early: the input is older than the preceding launch and the scratch is not the one that launch reads, so the planes
-  // are written while it runs; only the grid's completion, which the matmul waits for, still follows it (block 0).
-  if (!early) pdl_wait();
-  pdl_launch_dependents();
-  if (blockIdx.x == 0)
-    for (uint32_t i = threadIdx.x; i < ticket_count; i += 256) tickets[i] = 0u;
-  uint32_t const warp = threadIdx.x >> 5, lane = threadIdx.x & 31, pk = tiles_k * 256, G = tiles_k * 8;
-  uint32_t const chunks = (tiles_k + 7) / 8, tok = blockIdx.x / chunks, kb = blockIdx.x % chunks * 8 + warp;
-  bool const real = tok < m, live = kb < tiles_k;
-  // this lane's share of the conversion is requested before the block meets
-  float a = 0.f;
-  int sum = 0;
-  uint2 z = make_uint2(0u, 0u);
-  if (real && live) {
-    z = *reinterpret_cast<const uint2*>(codes + uint64_t(tok) * pk + kb * 256 + lane * 8);
-    uint64_t const g = uint64_t(tok) * G + kb * 8 + (lane >> 2);
-    a = scales[g];
-    sum = sums[g];
-  }
-  float row = 0.f;
-  if (real)
-    for (uint32_t i = threadIdx.x; i < G; i += 256) row = fmaxf(row, fabsf(scales[uint64_t(tok) * G + i]));
-#pragma unroll
-  for (int off = 16; off; off >>= 1) row = fmaxf(row, __shfl_xor_sync(0xffffffffu, row, off));
-  if (lane == 0) warp_top[warp] = row;
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < 8; ++i) row = fmaxf(row, warp_top[i]);
-  if (early && blockIdx.x == 0) pdl_wait();
-  if (!live) return;
+// A lane's share of a super-block: eight columns whose group has scale a and sum `sum`; row = the token's largest scale.
+__device__ __forceinline__ void write_planes(float a, int sum, uint2 z, float row, uint32_t tok, uint32_t kb, uint32_t m_pad, uint32_t pk,
+                                             __half* __restrict__ planes, __half* __restrict__ sums16, float* __restrict__ exps,
+                                             float* __restrict__ tokens) {
+  uint32_t const lane = threadIdx.x & 31;
   float top = fabsf(a);
 #pragma unroll
   for (int off = 4; off < 32; off <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
@@ -311,6 +284,104 @@ __global__ void __launch_bounds__(256) planes_kernel(const int8_t* __restrict__ 
   if (lane == 0) {
     exps[uint64_t(kb) * m_pad + tok] = e == e_row || e - e_row < -126 ? (e == e_row ? 1.f : 0.f) : power_of_two(e - e_row);
     if (kb == 0) tokens[tok] = power_of_two(e_row);
+  }
+}
+// The largest scale of the block's token from each thread's.
+__device__ __forceinline__ float block_top(float row, float* warp_top) {
+#pragma unroll
+  for (int off = 16; off; off >>= 1) row = fmaxf(row, __shfl_xor_sync(0xffffffffu, row, off));
+  if ((threadIdx.x & 31) == 0) warp_top[threadIdx.x >> 5] = row;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) row = fmaxf(row, warp_top[i]);
+  return row;
+}
+
+__global__ void __launch_bounds__(256) planes_kernel(const int8_t* __restrict__ codes, const float* __restrict__ scales,
+                                                     const int32_t* __restrict__ sums, uint32_t m, uint32_t m_pad, uint32_t tiles_k,
+                                                     __half* __restrict__ planes, __half* __restrict__ sums16, float* __restrict__ exps,
+                                                     float* __restrict__ tokens, uint32_t* __restrict__ tickets, uint32_t ticket_count,
+                                                     bool early) {
+  __shared__ float warp_top[8];
+  // early: the input is older than the preceding launch and the scratch is not the one that launch reads, so the planes
+  // are written while it runs; only the grid's completion, which the matmul waits for, still follows it (block 0).
+  if (!early) pdl_wait();
+  pdl_launch_dependents();
+  if (blockIdx.x == 0)
+    for (uint32_t i = threadIdx.x; i < ticket_count; i += 256) tickets[i] = 0u;
+  uint32_t const warp = threadIdx.x >> 5, lane = threadIdx.x & 31, pk = tiles_k * 256, G = tiles_k * 8;
+  uint32_t const chunks = (tiles_k + 7) / 8, tok = blockIdx.x / chunks, kb = blockIdx.x % chunks * 8 + warp;
+  bool const real = tok < m, live = kb < tiles_k;
+  // this lane's share of the conversion is requested before the block meets
+  float a = 0.f;
+  int sum = 0;
+  uint2 z = make_uint2(0u, 0u);
+  if (real && live) {
+    z = *reinterpret_cast<const uint2*>(codes + uint64_t(tok) * pk + kb * 256 + lane * 8);
+    uint64_t const g = uint64_t(tok) * G + kb * 8 + (lane >> 2);
+    a = scales[g];
+    sum = sums[g];
+  }
+  float row = 0.f;
+  if (real)
+    for (uint32_t i = threadIdx.x; i < G; i += 256) row = fmaxf(row, fabsf(scales[uint64_t(tok) * G + i]));
+  row = block_top(row, warp_top);
+  if (early && blockIdx.x == 0) pdl_wait();
+  if (!live) return;
+  write_planes(a, sum, z, row, tok, kb, m_pad, pk, planes, sums16, exps, tokens);
+}
+
+// The same from bf16 rows [m][k]: a block quantises one token, keeps it in registers until its largest scale is known, and
+// writes the planes without the Q8 form in between.  Held: super-blocks per warp.
+template <int Held>
+__global__ void __launch_bounds__(256) rows_planes_kernel(const uint16_t* __restrict__ rows, uint32_t k, bool vec, int* failure, uint32_t m,
+                                                          uint32_t m_pad, uint32_t tiles_k, __half* __restrict__ planes,
+                                                          __half* __restrict__ sums16, float* __restrict__ exps, float* __restrict__ tokens,
+                                                          uint32_t* __restrict__ tickets, uint32_t ticket_count) {
+  __shared__ float warp_top[8];
+  pdl_wait();
+  pdl_launch_dependents();
+  if (blockIdx.x == 0)
+    for (uint32_t i = threadIdx.x; i < ticket_count; i += 256) tickets[i] = 0u;
+  uint32_t const warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tok = blockIdx.x;
+  uint4 held[Held];  // bf16 columns, then {codes, codes, scale, sum}
+#pragma unroll
+  for (int i = 0; i < Held; ++i) {
+    uint32_t const col = (warp + 8 * i) * 256 + lane * 8;
+    const uint16_t* const src = rows + uint64_t(tok) * k + col;
+    held[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (tok >= m || col >= k) continue;
+    if (vec && col + 8 <= k) held[i] = __ldg(reinterpret_cast<const uint4*>(src));
+    else {
+      uint32_t e[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) e[c] = col + c < k ? src[c] : 0u;
+      held[i] = make_uint4(e[0] | e[1] << 16, e[2] | e[3] << 16, e[4] | e[5] << 16, e[6] | e[7] << 16);
+    }
+  }
+  float row = 0.f;
+  bool valid = true;
+#pragma unroll
+  for (int i = 0; i < Held; ++i) {
+    if (warp + 8 * i >= tiles_k) break;
+    uint32_t const w[4] = {held[i].x, held[i].y, held[i].z, held[i].w};
+    float x[8];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) { x[2 * c] = __uint_as_float(w[c] << 16); x[2 * c + 1] = __uint_as_float(w[c] & 0xffff0000u); }
+    Packed8 const z = quantize8(x);
+    valid = valid && z.valid;
+    float const a = tok < m ? z.a : 0.f;
+    row = fmaxf(row, fabsf(a));
+    held[i] = make_uint4(z.w0, z.w1, __float_as_uint(a), uint32_t(z.sum));
+  }
+  if (!valid) atomicExch(failure, 1);
+  row = block_top(row, warp_top);
+#pragma unroll
+  for (int i = 0; i < Held; ++i) {
+    uint32_t const kb = warp + 8 * i;
+    if (kb >= tiles_k) break;
+    write_planes(__uint_as_float(held[i].z), int(held[i].w), make_uint2(held[i].x, held[i].y), row, tok, kb, m_pad, tiles_k * 256, planes, sums16,
+                 exps, tokens);
   }
 }
 
@@ -440,29 +511,26 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
           bool ok = mbar_wait_inline(d_free(d_.s), d_.phase ^ 1, abort_flag, p.status, 0x804) &&
                     mbar_wait_inline(b_full(b_.s), b_.phase, abort_flag, p.status, 0x805);
 #pragma unroll
-          for (int pass = 0; pass < (C::kStack ? 1 : 2); ++pass) {
-#pragma unroll
-            for (int q = 0; q < C::kQ; ++q) {
-              bool const last = C::kStack || pass == 1;  // the stage's last use
-              if (pass == 0) ok = ok && mbar_wait_inline(a_full(a0 + q), g_.phase, abort_flag, p.status, 0x806);
-              if (C::kD2Bufs == 1 && last && q == C::kQ - 1 && u > u0) ok = ok && mbar_wait_inline(d_free(before.s), before.phase, abort_flag, p.status, 0x807);
-              if (!ok) break;
-              tc_fence_after();
-              uint32_t const at = tmem + C::kACol + (a0 + q) * C::kACols;
-              constexpr int kSteps = 16 / C::kQ;
-#pragma unroll
-              for (int i = 0; i < kSteps; ++i) {
-                int const k = q * kSteps + i;
-                uint64_t const b = b0 + uint64_t((pass * C::kBBox + (k >> 2) * (C::kBRows * 128) + (k & 3) * 32) / 16);
-                if (pass == 0 && k == 0) mma_pair<false>(dt, at, b, idesc);
-                else mma_pair<true>(dt, at + i * 8, b, idesc);
-              }
-              if (last && q == C::kQ - 1)  // m * (a*s): sixteen K columns = eight groups, hi and lo; the mins serve both (K stride 0)
-                mma_pair_ss(tmem + C::kD2Col + (C::kD2Bufs - 1) * d_.s * C::kN2, umma_desc_plain(smem + C::oMins + g_.s * C::kMins, 0, 128),
-                            umma_desc_plain(stage + C::kPlanes, C::kTRows * 16, 128), idesc2);
-              if (last) commit_pair(a_free(a0 + q));
-            }
+          for (int step = 0; step < C::kQ * (C::kStack ? 1 : 2); ++step) {
+            int const pass = step / C::kQ, q = step % C::kQ;
+            bool const last = C::kStack || pass == 1;  // the stage's last use
+            if (pass == 0) ok = ok && mbar_wait_inline(a_full(a0 + q), g_.phase, abort_flag, p.status, 0x806);
+            if (C::kD2Bufs == 1 && last && q == C::kQ - 1 && u > u0) ok = ok && mbar_wait_inline(d_free(before.s), before.phase, abort_flag, p.status, 0x807);
             if (!ok) break;
+            tc_fence_after();
+            uint32_t const at = tmem + C::kACol + (a0 + q) * C::kACols;
+            constexpr int kSteps = 16 / C::kQ;
+#pragma unroll
+            for (int i = 0; i < kSteps; ++i) {
+              int const k = q * kSteps + i;
+              uint64_t const b = b0 + uint64_t((pass * C::kBBox + (k >> 2) * (C::kBRows * 128) + (k & 3) * 32) / 16);
+              if (pass == 0 && k == 0) mma_pair<false>(dt, at, b, idesc);
+              else mma_pair<true>(dt, at + i * 8, b, idesc);
+            }
+            if (last && q == C::kQ - 1)  // m * (a*s): sixteen K columns = eight groups, hi and lo; the mins serve both (K stride 0)
+              mma_pair_ss(tmem + C::kD2Col + (C::kD2Bufs - 1) * d_.s * C::kN2, umma_desc_plain(smem + C::oMins + g_.s * C::kMins, 0, 128),
+                          umma_desc_plain(stage + C::kPlanes, C::kTRows * 16, 128), idesc2);
+            if (last) commit_pair(a_free(a0 + q));
           }
           if (!ok) break;
           commit_pair(b_free(b_.s));
@@ -506,9 +574,22 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
 #pragma unroll
       for (int i = 0; i < kMine; ++i) {
         uint32_t const sa = group * C::kQ + part * kMine + i;
-        if (!mbar_wait_inline(a_free(sa), phase ^ 1, abort_flag, p.status, 0x80a)) { ok = false; break; }
-        tc_fence_after();
-        if (part == C::kSplit - 1 && i == kMine - 1) {
+        auto expand = [&](int g, uint32_t (&v)[16]) {
+          uint32_t const scw = C::kSplit == 1 ? (g < 4 ? sm.sc_lo : sm.sc_hi) : (part == 0 ? sm.sc_lo : sm.sc_hi);
+          __half2 const S = __hsub2(u2h(__byte_perm(scw, 0x64646464u, 0x4040 | ((g & 3) * 0x0101))), u2h(0x64006400u));
+          // low nibbles: (1024 + q) * sc - 1024 sc; high nibbles, four bits up: (1024 + 16 q) * (sc / 16) - 64 sc
+          __half2 const S16 = __hmul2(S, u2h(0x2c002c00u)), B = __hmul2(S, u2h(0xe400e400u)), B16 = __hmul2(S, u2h(0xd400d400u));
+          uint32_t const ww[4] = {w[g].x, w[g].y, w[g].z, w[g].w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            uint32_t const t = ww[j] >> 8;
+            v[4 * j + 0] = h2u(__hfma2(u2h(and_or(ww[j], low, magic)), S, B));
+            v[4 * j + 1] = h2u(__hfma2(u2h(and_or(ww[j], high, magic)), S16, B16));
+            v[4 * j + 2] = h2u(__hfma2(u2h(and_or(t, low, magic)), S, B));
+            v[4 * j + 3] = h2u(__hfma2(u2h(and_or(t, high, magic)), S16, B16));
+          }
+        };
+        auto mins = [&] {
           uint32_t mh[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
@@ -518,24 +599,15 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
           }
           sts128(smem + C::oMins + group * C::kMins + row * 16, mh[0], mh[1], mh[2], mh[3]);
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // read by the MMA
-        }
+        };
+        uint32_t v[16];
+        if constexpr (C::kReady) expand(i, v);  // the stage's words are ready when it is
+        if (!mbar_wait_inline(a_free(sa), phase ^ 1, abort_flag, p.status, 0x80a)) { ok = false; break; }
+        tc_fence_after();
+        if (part == C::kSplit - 1 && i == kMine - 1) mins();
 #pragma unroll
         for (int gg = 0; gg < kGroupsPer; ++gg) {
-          int const g = i * kGroupsPer + gg;
-          uint32_t const scw = C::kSplit == 1 ? (g < 4 ? sm.sc_lo : sm.sc_hi) : (part == 0 ? sm.sc_lo : sm.sc_hi);
-          __half2 const S = __hsub2(u2h(__byte_perm(scw, 0x64646464u, 0x4040 | ((g & 3) * 0x0101))), u2h(0x64006400u));
-          // low nibbles: (1024 + q) * sc - 1024 sc; high nibbles, four bits up: (1024 + 16 q) * (sc / 16) - 64 sc
-          __half2 const S16 = __hmul2(S, u2h(0x2c002c00u)), B = __hmul2(S, u2h(0xe400e400u)), B16 = __hmul2(S, u2h(0xd400d400u));
-          uint32_t const ww[4] = {w[g].x, w[g].y, w[g].z, w[g].w};
-          uint32_t v[16];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            uint32_t const t = ww[j] >> 8;
-            v[4 * j + 0] = h2u(__hfma2(u2h(and_or(ww[j], low, magic)), S, B));
-            v[4 * j + 1] = h2u(__hfma2(u2h(and_or(ww[j], high, magic)), S16, B16));
-            v[4 * j + 2] = h2u(__hfma2(u2h(and_or(t, low, magic)), S, B));
-            v[4 * j + 3] = h2u(__hfma2(u2h(and_or(t, high, magic)), S16, B16));
-          }
+          if constexpr (!C::kReady) expand(i * kGroupsPer + gg, v);
           tmem_st16(tmem + ((quarter * 32u) << 16) + C::kACol + sa * C::kACols + gg * 16, v);
         }
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -746,16 +818,28 @@ Carve carve(uint32_t m, uint32_t tiles_k, const F16Plan& plan) {
 }
 
 template <int NT>
-cudaError_t launch_f16(const WeightView& w, const WeightView* second, const Q8View& x, const TcOutput& o, const F16Plan& plan, uint8_t* scratch, bool early, int* status,
+cudaError_t launch_f16(const WeightView& w, const WeightView* second, const Q8View& x, const RawRows* raw, const TcOutput& o, const F16Plan& plan, uint8_t* scratch, bool early, int* status,
                        cudaStream_t stream) {
   using C = F16Cfg<NT>;
   Carve const c = carve(x.m, w.tiles_k, plan);
   uint32_t const m_pad = (x.m + NT - 1) / NT * NT, pk = w.tiles_k * 256;
-  uint32_t const grid = m_pad * ((w.tiles_k + 7) / 8);
-  cudaError_t st = launch_kernel(planes_kernel, grid, 256, 0, stream, launch_overlap(), x.codes, x.scales, x.sums, x.m, m_pad, w.tiles_k,
-                                 reinterpret_cast<__half*>(scratch + c.planes), reinterpret_cast<__half*>(scratch + c.sums),
-                                 reinterpret_cast<float*>(scratch + c.exps), reinterpret_cast<float*>(scratch + c.tokens),
-                                 reinterpret_cast<uint32_t*>(scratch), plan.unit_step == 1 ? uint32_t(kTicketBytes / 4) : 0u, early);
+  auto* const planes = reinterpret_cast<__half*>(scratch + c.planes);
+  auto* const sums = reinterpret_cast<__half*>(scratch + c.sums);
+  auto* const exps = reinterpret_cast<float*>(scratch + c.exps);
+  auto* const tokens = reinterpret_cast<float*>(scratch + c.tokens);
+  auto* const tickets = reinterpret_cast<uint32_t*>(scratch);
+  uint32_t const ticket_count = plan.unit_step == 1 ? uint32_t(kTicketBytes / 4) : 0u;
+  cudaError_t st;
+  if (raw) {
+    bool const vec = raw->k % 8 == 0 && reinterpret_cast<uintptr_t>(raw->x) % 16 == 0;
+    auto kernel = w.tiles_k <= 24 ? rows_planes_kernel<3> : (w.tiles_k <= 72 ? rows_planes_kernel<9> : rows_planes_kernel<16>);
+    if (w.tiles_k > 128) return cudaErrorInvalidValue;
+    st = launch_kernel(kernel, m_pad, 256, 0, stream, launch_overlap(), raw->x, raw->k, vec, raw->failure, x.m, m_pad, w.tiles_k, planes, sums,
+                       exps, tokens, tickets, ticket_count);
+  } else {
+    st = launch_kernel(planes_kernel, m_pad * ((w.tiles_k + 7) / 8), 256, 0, stream, launch_overlap(), x.codes, x.scales, x.sums, x.m, m_pad,
+                       w.tiles_k, planes, sums, exps, tokens, tickets, ticket_count, early);
+  }
   if (st != cudaSuccess) return st;
   CUtensorMap tm_codes[2], tm_meta[2], tm_planes, tm_sums;
   uint64_t const rgs = w.padded_n / 8;
@@ -858,7 +942,7 @@ uint64_t f16_scratch_bytes(uint32_t m, uint32_t tiles_k, const F16Plan& plan) {
 }
 
 cudaError_t launch_mmq_f16(const WeightView& w, const Q8View& x, const TcOutput& out, const F16Plan& plan, void* scratch, bool alternates,
-                           int* status, cudaStream_t stream, const WeightView* second) {
+                           int* status, cudaStream_t stream, const WeightView* second, const RawRows* raw) {
   if (second && (second->n != w.n || second->tiles_k != w.tiles_k || out.ndst != 1 || out.out_bf16 || out.residual || out.done || !out.out[1]))
     return cudaErrorInvalidValue;
   if (out.ndst < 1 || out.ndst > 8 || (out.out_bf16 ? out.ndst != 1 : out.out[0] == nullptr) || plan.workers < 1 ||
@@ -871,6 +955,9 @@ cudaError_t launch_mmq_f16(const WeightView& w, const Q8View& x, const TcOutput&
     uint64_t const G = x.padded_k / 32;
     xc.m = x.m - t0 < plan.chunk ? x.m - t0 : plan.chunk;
     xc.codes += uint64_t(t0) * x.padded_k; xc.scales += t0 * G; xc.sums += t0 * G;
+    RawRows rows{};
+    if (raw) { rows = *raw; rows.x += uint64_t(t0) * raw->k; }
+    const RawRows* const rc = raw ? &rows : nullptr;
     TcOutput oc = out;
     for (uint32_t g = 0; g < (second ? 2 : out.ndst); ++g) if (oc.out[g]) oc.out[g] += t0 * stride;
     if (oc.out_bf16) oc.out_bf16 += t0 * stride;
@@ -887,12 +974,14 @@ cudaError_t launch_mmq_f16(const WeightView& w, const Q8View& x, const TcOutput&
       }
     }
     uint8_t* const s = static_cast<uint8_t*>(scratch);
+    std::optional<ChainedLaunches> chained;  // a later pass follows a kernel of this one
+    if (t0) chained.emplace();
     cudaError_t st;
     switch (plan.nt) {
-      case 16: st = launch_f16<16>(w, second, xc, oc, pc, s, early, status, stream); break;
-      case 32: st = launch_f16<32>(w, second, xc, oc, pc, s, early, status, stream); break;
-      case 64: st = launch_f16<64>(w, second, xc, oc, pc, s, early, status, stream); break;
-      case 128: st = launch_f16<128>(w, second, xc, oc, pc, s, early, status, stream); break;
+      case 16: st = launch_f16<16>(w, second, xc, rc, oc, pc, s, early, status, stream); break;
+      case 32: st = launch_f16<32>(w, second, xc, rc, oc, pc, s, early, status, stream); break;
+      case 64: st = launch_f16<64>(w, second, xc, rc, oc, pc, s, early, status, stream); break;
+      case 128: st = launch_f16<128>(w, second, xc, rc, oc, pc, s, early, status, stream); break;
       default: return cudaErrorInvalidValue;
     }
     if (st != cudaSuccess) return st;

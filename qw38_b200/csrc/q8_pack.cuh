@@ -27,7 +27,7 @@ __device__ __forceinline__ float rounded_quotient(float x, float a, float r) {
 // Executed by full warps.  Scales between 2^-80 and 2^100 (one vote per warp) take the eight quotients through one
 // reciprocal, the rounding through the bias 1.5 * 2^23 (|x / a| < 127.5, so nothing needs a clamp) and the codes out of the
 // low bytes; the eight divisions of the other path are 100 instructions and leave their short form where x is tiny against
-// a or zero, as behind a SwiGLU.  Pack of 2048 x 17408 bf16 rows: 106 us before, 43 with this and two tasks in flight per warp.
+// a or zero, as behind a SwiGLU.  Pack of 2048 x 17408 bf16 rows: 106 us before, 44 with this.
 __device__ __forceinline__ Packed8 quantize8(const float (&x)[8]) {
   bool finite = true;
   float peak = 0.f;

@@ -9,7 +9,8 @@ import torch
 from oracle import oracle as orc
 from qw38_b200 import _lib as L
 from qw38_b200 import set_launch_overlap, synth
-from qw38_b200.q4k_q8 import PrefillWeight, new_q8_input, pack_q8, q4k_q8_project
+from qw38_b200.q4k_q8 import (DecodeMmvDesc, PrefillWeight, decode_workspace, new_q8_input, pack_q8, prefill_paired_swiglu,
+                              prefill_project, q4k_q8_project)
 from tests.helpers import assert_close_contract
 
 pytestmark = pytest.mark.gpu
@@ -123,3 +124,31 @@ def test_overlapped_graph_and_streams_reproduce_the_serial_result():
         for key in want:
             assert torch.equal(outs[key], want[key]), key
     assert kernel_status() == 0
+
+
+@pytest.mark.parametrize("m,n,k", [(17, 136, 200), (33, 264, 1003), (64, 264, 6400), (130, 520, 2560), (131, 264, 18688), (800, 128, 17408)])
+def test_rows_are_quantised_as_the_pack_does(m, n, k):
+    """Prefill entries hand the bf16 rows to the kernel's own quantiser: bitwise the pack and the projection, for every number
+    of super-blocks per warp, row alignments, several passes, gate and up in one launch, and a value that is not finite."""
+    (w, _, _), (w2, _, _) = weight(n, k, seed=m), weight(n, k, seed=m + 1)
+    x = torch.from_numpy(synth.activations(m, k, seed=k, scale=0.5, outlier_frac=0.01)).to(DEV).to(torch.bfloat16)
+    f, ws = flag(), decode_workspace(m, n, k)
+    q = pack_q8(x, f)
+    want = [q4k_q8_project(v, q) for v in (w, w2)]
+    out = torch.empty((m, n), device=DEV)
+    prefill_project(DecodeMmvDesc(w, x, out, L.EPILOGUE_STORE_FP32), ws, f)
+    assert torch.equal(out, want[0]) and f.item() == 0
+    # input where a first pass would write (the fp32 rows of the workspace): the pack comes first
+    at = ws.numel() // 2 * 2 - x.numel() * 2
+    inside = ws[at // 16 * 16:at // 16 * 16 + x.numel() * 2].view(torch.bfloat16).view(m, k) if at > m * k * 3 else None
+    if inside is not None:
+        inside.copy_(x)
+        prefill_project(DecodeMmvDesc(w, inside, out, L.EPILOGUE_STORE_FP32), ws, f)
+        assert torch.equal(out, want[0])
+    both = torch.empty((m, n), dtype=torch.bfloat16, device=DEV)
+    prefill_paired_swiglu(w, w2, x, both, ws, f)
+    ref = torch.nn.functional.silu(want[0].double()) * want[1].double()
+    assert (both.double() - ref).abs().max() <= ref.abs().max() * 2.0 ** -8 and f.item() == 0
+    x[m - 1, k - 1] = float("nan")
+    prefill_project(DecodeMmvDesc(w, x, out, L.EPILOGUE_STORE_FP32), ws, f)
+    assert f.item() == 1 and kernel_status() == 0

@@ -85,8 +85,11 @@ template <int NT> struct F16Cfg {
   static constexpr int kRegsLeft = (kWarps * kLaunchRegs - 4 * kRegsControl - kGroups * kExpanders * kRegsExpander) / kEpilogueWarps / 8 * 8;
   static constexpr int kRegsEpilogue = kRegsLeft > 160 ? 160 : kRegsLeft;
   // TMEM: two accumulators, one min-term accumulator, weight stages.  A group of expanders always uses the same kQ stages
-  // (one super-block), so that a warp sees every phase of the barriers it waits on.
-  static constexpr int kQ = kStack ? 2 : 4, kACols = 128 / kQ, kAStages = kGroups * kQ;
+  // (one super-block), so that a warp sees every phase of the barriers it waits on.  At 128 tokens there is room for one
+  // super-block only, and a stage is refilled between its last use and the next super-block's first: 7/16 of a super-block's
+  // time with eight stages (3/8 with four), half the work per stage, and the words are computed before the wait (kReady).
+  // 256 tokens x 17408 x 5120 78 -> 75 us, 2048 x 5120 x 17408 670 -> 630, 2048 x 17408 x 5120 (at the power limit) 585 -> 575.
+  static constexpr int kQ = kStack ? 2 : (NT >= 128 ? 8 : 4), kACols = 128 / kQ, kAStages = kGroups * kQ;
   static constexpr bool kReady = kQ == 8;
   static constexpr int kD2Bufs = NT <= 64 ? 2 : 1;  // with one, the min-term MMA waits for the previous super-block's epilogue
   static constexpr int kD2Col = 2 * kN, kACol = kD2Col + kD2Bufs * kN2;

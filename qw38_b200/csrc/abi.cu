@@ -1233,9 +1233,11 @@ int q4k_q8_mlp(const q4k_weight* gate, const q4k_weight* up, const q4k_weight* d
   probe.codes = reinterpret_cast<const int8_t*>(g);
   bool const fused = m <= q4k::kGemvTmaMaxTokens && q4k::gemv_tma_supported(view(*gate), probe) &&
                      q4k::gemv_tma_supported(view(*up), probe) && q4k::plan_gemv_tma_swiglu_q8(m, view(*gate), &fused_plan);
-  int8_t* const hcodes = fused ? reinterpret_cast<int8_t*>(g) : codes;
-  float* const hscales = fused ? reinterpret_cast<float*>(hcodes + uint64_t(m) * hidden) : scales;
-  int32_t* const hsums = fused ? reinterpret_cast<int32_t*>(hscales + uint64_t(m) * (hidden / 32)) : sums;
+  // A hidden row wider than the place meant for it goes into the output, which nothing else uses before the last launch.
+  bool const narrow = fused ? uint64_t(hidden) * 5 > uint64_t(ffn) * 32 : hidden > ffn;
+  int8_t* const hcodes = narrow ? reinterpret_cast<int8_t*>(output) : (fused ? reinterpret_cast<int8_t*>(g) : codes);
+  float* const hscales = fused || narrow ? reinterpret_cast<float*>(hcodes + uint64_t(m) * hidden) : scales;
+  int32_t* const hsums = fused || narrow ? reinterpret_cast<int32_t*>(hscales + uint64_t(m) * (hidden / 32)) : sums;
   q4k_q8_input xh{hcodes, hscales, hsums, uint64_t(m) * hidden, uint64_t(m) * (hidden / 32), uint64_t(m) * (hidden / 32), m, hidden, hidden};
   q4k_q8_input xf{codes, scales, sums, uint64_t(m) * ffn, uint64_t(m) * (ffn / 32), uint64_t(m) * (ffn / 32), m, ffn, ffn};
   q4k_project_options opt{};

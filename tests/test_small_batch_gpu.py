@@ -11,8 +11,8 @@ from oracle import oracle as orc
 from qw38_b200 import _lib as L
 from qw38_b200 import repack_blocks144, synth
 from qw38_b200.q4k_q8 import (DecodeMmvDesc, PrefillWeight, decode_workspace, hidden_rms_q8, launch_decode_mmv,
-                              launch_decode_mmv_ranges, pack_q8, q4k_q8_project)
-from tests.helpers import assert_close_contract
+                              launch_decode_mmv_ranges, pack_q8, q4k_q8_mlp, q4k_q8_project, q8_mlp_workspace_bytes)
+from tests.helpers import assert_close_contract, assert_close_reference
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -151,3 +151,18 @@ def test_quantiser_quotients_are_the_divisions(which):
     assert f.item() == bad
     assert (q.codes.cpu().numpy() == z).all() and (q.sums.cpu().numpy() == s).all()
     assert (q.scales.cpu().numpy().view(np.uint32) == a.view(np.uint32)).all()
+
+
+@pytest.mark.parametrize("m,hidden,ffn", [(4, 2048, 1024), (4, 2048, 256), (33, 2048, 1024), (130, 1024, 512)])
+def test_mlp_whose_hidden_row_is_the_wider_one(m, hidden, ffn):
+    (gate, gc, gs), (up, uc, us), (down, dc, ds) = weight(ffn, hidden, 1), weight(ffn, hidden, 2), weight(hidden, ffn, 3)
+    h = synth.activations(m, hidden, seed=m, scale=2.0)
+    gamma = torch.from_numpy(np.random.default_rng(m).standard_normal(hidden).astype(np.float32) * 0.1).to(torch.bfloat16)
+    room = torch.full((q8_mlp_workspace_bytes(m, hidden, ffn) + 64,), 77, dtype=torch.uint8, device=DEV)
+    out = torch.empty((m, hidden), device=DEV)
+    assert q4k_q8_mlp(gate, up, down, torch.from_numpy(h).to(DEV), gamma.to(DEV), 1e-6, out, m, room[:-64])
+    assert (room[-64:] == 77).all()
+    z, a, s, _ = orc.q8_quantize(orc.hidden_rms_bf16(h, gamma.view(torch.int16).numpy().view(np.uint16), 1e-6), bf16_bits=True)
+    v = orc.swiglu_bf16(orc.project(gc, gs, ffn, hidden, z, a, s), orc.project(uc, us, ffn, hidden, z, a, s))
+    z, a, s, _ = orc.q8_quantize(v, bf16_bits=True)
+    assert_close_reference(out.cpu().numpy(), orc.project(dc, ds, hidden, ffn, z, a, s, residual=h))

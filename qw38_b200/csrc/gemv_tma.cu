@@ -152,8 +152,10 @@ __device__ __forceinline__ void locate_tile(const GtParams& p, uint32_t T, uint3
 }
 
 // NT = token octets (1: m <= 8, 2: m <= 16).  MAXW bounds the block size for register allocation.  Raw: the activations
-// are bf16 rows that the consumers quantise (a kernel of its own: the extra path costs the others registers).
-template <int NT, int MAXW, bool Dump, bool Raw>
+// are bf16 rows that the consumers quantise (a kernel of its own: the extra path costs the others registers).  Quant: the gate / up
+// pair whose reducers (Quant of them per octet) write the Q8 activation of the down projection; in one kernel with the plain
+// form, its code cost that one 2 %.
+template <int NT, int MAXW, bool Dump, bool Raw, int Quant>
 __global__ void __launch_bounds__(MAXW * 32, 1)
 gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_constant__ CUtensorMap tm_meta,
                 const __grid_constant__ CUtensorMap tm_codes1, const __grid_constant__ CUtensorMap tm_meta1,
@@ -174,12 +176,13 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
   volatile int* const abort_flag = flags;
   int* const last_flag = flags + 1;
 
-  uint32_t const kFirstConsumer = kFirstReducer + NT * p.reducers;
+  constexpr int Reducers = Quant == 2 ? 2 : 1;
+  constexpr uint32_t kFirstConsumer = kFirstReducer + NT * Reducers;
   uint32_t const warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint32_t const slot_mask = p.red_slots - 1, slot_shift = p.red_slots - 1;  // red_slots is 1 or 2
   // hand-off slot of the block's it-th tile, and how often the slot was used before
   auto hand_off = [&](uint32_t it, uint32_t& slot, uint32_t& use) {
-    if (p.reducers == 2) { slot = (it >> 2) & 1; use = (it >> 3) * 4 + (it & 3); }
+    if constexpr (Reducers == 2) { slot = (it >> 2) & 1; use = (it >> 3) * 4 + (it & 3); }
     else { slot = it & slot_mask; use = it >> slot_shift; }
   };
   uint32_t const range = blockIdx.x / p.split_k, slice = blockIdx.x % p.split_k;
@@ -231,7 +234,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
   } else if (warp < kFirstConsumer) {
     // One reducer warp per token octet adds the consumers' 16 x 8 tiles in warp order.  Lane
     // (r = lane/4, q = lane%4) owns rows r, r+8 and tokens 2q, 2q+1 -- the MMA accumulator layout.
-    uint32_t const nt = (warp - kFirstReducer) % NT, turn = (warp - kFirstReducer) / NT;
+    uint32_t const nt = (warp - kFirstReducer) % NT, turn = Reducers == 1 ? 0u : (warp - kFirstReducer) / NT;
     uint32_t const r = lane >> 2, q = lane & 3;
     pdl_wait();
     pdl_launch_dependents();  // after the wait: the next launch never runs beside anything older than this one
@@ -253,7 +256,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
       float g00 = 0.f, g01 = 0.f, g10 = 0.f, g11 = 0.f;
       float pg[4], pu[4];  // pair == 2: gate and up values of the group's first half
       for (uint32_t it = 0; it < ntiles; ++it) {
-        if (p.reducers == 2 && ((it >> 2) & 1) != turn) continue;
+        if (Reducers == 2 && ((it >> 2) & 1) != turn) continue;
         uint32_t s, use;
         hand_off(it, s, use);
         if (!mbar_wait(b_rfull + 8 * s, use & 1, abort_flag, p.status, 0x520)) break;
@@ -285,7 +288,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
         size_t const a0 = size_t(tok0) * S.n + row, a1 = a0 + S.n;
         if (p.pair) {
           if (sg == 0) { g00 = v00; g01 = v01; g10 = v10; g11 = v11; continue; }
-          if (p.pair == 2) {
+          if constexpr (Quant > 0) {
             // The activation of the down projection, quantised here (the arithmetic of swiglu_pack_kernel,
             // cuda/q4k_q8.cu:52-61): x = bf16(g / (1 + exp(-g)) * u), a non-finite input poisons the value.  The first
             // half's values are kept as they are: the exponentials and divisions of a group come after its last hand-off,
@@ -734,9 +737,11 @@ struct Maps {
 
 template <int NT, int MAXW>
 cudaError_t launch_cfg(const Maps& t, const GtParams& p, bool dump, uint32_t grid, uint32_t smem, cudaStream_t stream) {
-  auto kernel = dump ? gemv_tma_kernel<NT, MAXW, true, false> : gemv_tma_kernel<NT, MAXW, false, false>;
+  auto kernel = dump ? gemv_tma_kernel<NT, MAXW, true, false, 0> : gemv_tma_kernel<NT, MAXW, false, false, 0>;
+  if (p.pair == 2) kernel = gemv_tma_kernel<NT, MAXW, false, false, 1>;
   if constexpr (NT == 1) {
-    if (p.xraw != nullptr) kernel = gemv_tma_kernel<NT, MAXW, false, true>;
+    if (p.xraw != nullptr) kernel = gemv_tma_kernel<NT, MAXW, false, true, 0>;
+    if (p.reducers == 2) kernel = gemv_tma_kernel<NT, MAXW, false, false, 2>;
   }
   cudaError_t st = allow_smem(reinterpret_cast<const void*>(kernel), int(smem));
   if (st != cudaSuccess) return st;

@@ -67,9 +67,9 @@ typedef struct q4k_q8_input {
 /* Which kernel family q4k_q8_project_ex runs; 0 lets the library choose by m
  * (the reference's switch m==1 | m>=128 | else is cuda/q4k_q8.cu:303-313). */
 #define Q4K_KERNEL_AUTO 0
-#define Q4K_KERNEL_GEMV_DP4A 1 /* m <= 4 : dp4a, one lane per K32 group */
+#define Q4K_KERNEL_GEMV_DP4A 1 /* m <= 4 : dp4a, every warp streams its own run of weights */
 #define Q4K_KERNEL_MMA 2       /* any m  : warp-level int8 mma, split-K through global scratch */
-#define Q4K_KERNEL_TCGEN05 3   /* m >= 32: tcgen05 kind::i8, TMEM accumulators */
+#define Q4K_KERNEL_TCGEN05 3   /* m >= 32: tcgen05 kind::i8, TMEM accumulators, integer partial dots */
 #define Q4K_KERNEL_GEMV_MMA 4  /* m <= 16: warp-level int8 mma, split-K inside a block cluster */
 #define Q4K_KERNEL_GEMV_TMA 5  /* m <= 16: weights streamed by TMA, activations held in registers */
 #define Q4K_KERNEL_F16 6       /* any m  : tcgen05 kind::f16 on SM pairs, activations as two fp16 planes; no partials */

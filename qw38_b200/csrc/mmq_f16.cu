@@ -27,13 +27,14 @@
 // N), because one SM alone would have to take in 60 bytes per clock of activation planes next to the weights, and L2
 // delivers about 10 TB/s to all of them.
 //
-// Measured on 17408 x 5120: 2048 tokens 0.59 ms (620 TOP/s; the int8 kernel 1.20 ms), tensor pipe 72 % active with the
-// clock at the power limit; 64 tokens x 34816 rows 49 us (95 us), of which about 10 us are launch, prologue and tile end.
+// Measured on 17408 x 5120: 2048 tokens 0.57 ms (635 TOP/s; the int8 kernel 1.20 ms) at the power limit, 1024 tokens with the
+// tensor pipe 86 % active; 64 tokens x 34816 rows 47 us (95 us), of which about 10 us are launch, prologue and tile end.
 // Bound: at prefill sizes tensor pipe and power, below 64 tokens the hand-offs between the roles (barrier to barrier a
 // super-block takes ~1.4x its tensor time).  Tried and slower: a back-off in the waits (nanosleep 16 .. 128: 1.5 - 2x), a
 // suspend hint, a four-instruction retry loop (1.5x: the retries queue up in front of the arrivals), one polling lane or
 // one polling warp per role, arrivals with cluster-scope release (a memory barrier each: 1.4x), the min term on mma.sync
-// (queues behind the tcgen05 MMAs: 1.16x).
+// (queues behind the tcgen05 MMAs: 1.16x).  Faster but less exact: lo and hi products alternating per weight stage (5 %, and
+// 3.2e-7 .. 4.1e-7 of the norm, because the lo products are then truncated at full magnitude).
 //
 // Work is a list of (row pair, token tile, super-block) units in that order.  Each cluster takes one contiguous run of
 // units; tiles cut by a run's ends go through fp32 scratch and are added in run order by whoever arrives last.  When

@@ -1226,19 +1226,27 @@ int q4k_q8_mlp(const q4k_weight* gate, const q4k_weight* up, const q4k_weight* d
   // Up to sixteen tokens with TMA-able gate / up weights whose K fits one block: the gate projection, the up
   // projection and the SwiGLU -> Q8 pack run as ONE launch (three launches for the chain instead of five).  That
   // launch reads the hidden activation while it writes the ffn activation, so the hidden activation moves out of
-  // the shared region into the (then unused) fp32 gate rows.
+  // the shared region into the (then unused) fp32 gate rows.  A hidden row wider than the place meant for it goes into the
+  // output, which nothing else uses before the last launch: its 4 * m * hidden bytes hold the pack's 1.25 * m * hidden from
+  // the first 16-byte boundary on (the output itself need only be 4-byte aligned, the kernels read codes in wider words).
+  auto hidden_pack = [&](bool beside_ffn) {
+    int8_t* c = codes;
+    float* a = scales;
+    int32_t* z = sums;
+    if (beside_ffn ? uint64_t(hidden) * 5 > uint64_t(ffn) * 32 : hidden > ffn)
+      c = reinterpret_cast<int8_t*>((reinterpret_cast<uintptr_t>(output) + 15) & ~uintptr_t(15));
+    else if (beside_ffn) c = reinterpret_cast<int8_t*>(g);
+    if (c != codes) {
+      a = reinterpret_cast<float*>(c + uint64_t(m) * hidden);
+      z = reinterpret_cast<int32_t*>(a + uint64_t(m) * (hidden / 32));
+    }
+    return q4k_q8_input{c, a, z, uint64_t(m) * hidden, uint64_t(m) * (hidden / 32), uint64_t(m) * (hidden / 32), m, hidden, hidden};
+  };
+  q4k_q8_input xh = hidden_pack(true);
   q4k::GemvTmaPlan fused_plan{};
-  q4k::Q8View probe{};
-  probe.m = m;
-  probe.codes = reinterpret_cast<const int8_t*>(g);
-  bool const fused = m <= q4k::kGemvTmaMaxTokens && q4k::gemv_tma_supported(view(*gate), probe) &&
-                     q4k::gemv_tma_supported(view(*up), probe) && q4k::plan_gemv_tma_swiglu_q8(m, view(*gate), &fused_plan);
-  // A hidden row wider than the place meant for it goes into the output, which nothing else uses before the last launch.
-  bool const narrow = fused ? uint64_t(hidden) * 5 > uint64_t(ffn) * 32 : hidden > ffn;
-  int8_t* const hcodes = narrow ? reinterpret_cast<int8_t*>(output) : (fused ? reinterpret_cast<int8_t*>(g) : codes);
-  float* const hscales = fused || narrow ? reinterpret_cast<float*>(hcodes + uint64_t(m) * hidden) : scales;
-  int32_t* const hsums = fused || narrow ? reinterpret_cast<int32_t*>(hscales + uint64_t(m) * (hidden / 32)) : sums;
-  q4k_q8_input xh{hcodes, hscales, hsums, uint64_t(m) * hidden, uint64_t(m) * (hidden / 32), uint64_t(m) * (hidden / 32), m, hidden, hidden};
+  bool const fused = m <= q4k::kGemvTmaMaxTokens && q4k::gemv_tma_supported(view(*gate), view(xh)) &&
+                     q4k::gemv_tma_supported(view(*up), view(xh)) && q4k::plan_gemv_tma_swiglu_q8(m, view(*gate), &fused_plan);
+  if (!fused) xh = hidden_pack(false);
   q4k_q8_input xf{codes, scales, sums, uint64_t(m) * ffn, uint64_t(m) * (ffn / 32), uint64_t(m) * (ffn / 32), m, ffn, ffn};
   q4k_project_options opt{};
   opt.flags = kFlagTrustedSpans;  // every span was validated above

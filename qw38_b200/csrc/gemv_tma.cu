@@ -769,11 +769,14 @@ cudaError_t launch_by_shape(uint32_t nt, uint32_t cw, A&&... a) {
   return launch_cfg<2, kGemvTmaMaxWarpsWide + 3>(a...);
 }
 
+// The consumers read codes eight at a time.
+bool codes_aligned(const Q8View& x) { return reinterpret_cast<uintptr_t>(x.codes) % 8 == 0; }
+
 }  // namespace
 
 bool gemv_tma_supported(const WeightView& w, const Q8View& x) {
   return x.m <= kGemvTmaMaxTokens && encode_fn() != nullptr && reinterpret_cast<uintptr_t>(w.codes) % 16 == 0 &&
-         reinterpret_cast<uintptr_t>(w.meta) % 16 == 0 && reinterpret_cast<uintptr_t>(x.codes) % 8 == 0;
+         reinterpret_cast<uintptr_t>(w.meta) % 16 == 0 && codes_aligned(x);
 }
 
 GemvTmaPlan plan_gemv_tma(uint32_t m, uint32_t n, uint32_t tiles_k, uint32_t split_k_request, uint32_t warps_request) {
@@ -827,7 +830,7 @@ cudaError_t launch_gemv_tma(const WeightView& w, const Q8View& x, float* out, co
   if (x.m == 0 || x.m > kGemvTmaMaxTokens || cw < 1 || cw > (nt == 1 ? kGemvTmaMaxWarpsNarrow : kGemvTmaMaxWarpsWide) ||
       plan.split_k * cw < w.tiles_k || plan.stages < 2 || plan.stages > uint32_t(kMaxStages) ||
       (plan.red_slots != 1 && plan.red_slots != 2) || smem_bytes(cw, nt, plan.stages, plan.red_slots) > kSmemBudget ||
-      (plan.split_k > 1 && (!slices || !tickets)) ||
+      (plan.split_k > 1 && (!slices || !tickets)) || !codes_aligned(x) ||
       (gather && (gather->ranks < 1 || gather->ranks > 8 || gather->rank >= gather->ranks || !gather->done || !gather->unsignalled || partials)))
     return cudaErrorInvalidValue;
   Maps t{};
@@ -862,7 +865,7 @@ cudaError_t launch_gemv_tma_multi(const WeightView* ws, const GemvTmaOutput* out
   if (count < 1 || count > 3 || (swiglu_pair && count != 2) || x.m == 0 || x.m > kGemvTmaMaxTokens || cw < 1 ||
       cw > (nt == 1 ? kGemvTmaMaxWarpsNarrow : kGemvTmaMaxWarpsWide) || plan.stages < 2 || plan.stages > uint32_t(kMaxStages) ||
       (plan.red_slots != 1 && plan.red_slots != 2) || smem_bytes(cw, nt, plan.stages, plan.red_slots) > kSmemBudget ||
-      (plan.split_k > 1 && (!slices || !tickets)) || (swiglu_pair && (plan.tiles_per_range & 1u)) || (raw && nt != 1))
+      (plan.split_k > 1 && (!slices || !tickets)) || (swiglu_pair && (plan.tiles_per_range & 1u)) || (raw ? nt != 1 : !codes_aligned(x)))
     return cudaErrorInvalidValue;
   Maps t{};
   GtParams p{};
@@ -920,7 +923,7 @@ cudaError_t launch_gemv_tma_swiglu_q8(const WeightView& gate, const WeightView& 
       cw > (nt == 1 ? kGemvTmaMaxWarpsNarrow : kGemvTmaMaxWarpsWide) || plan.stages < 2 || plan.stages > uint32_t(kMaxStages) ||
       (plan.red_slots != 1 && plan.red_slots != 2) || smem_bytes(cw, nt, plan.stages, plan.red_slots) > kSmemBudget ||
       gate.n != up.n || gate.tiles_k != up.tiles_k || gate.n % 32 != 0 || gate.n != gate.padded_n || out.m != x.m ||
-      out.padded_k != gate.n || !out.codes || !out.scales || !out.sums || !failure)
+      out.padded_k != gate.n || !out.codes || !out.scales || !out.sums || !failure || !codes_aligned(x))
     return cudaErrorInvalidValue;
   Maps t{};
   GtParams p{};

@@ -166,3 +166,21 @@ def test_mlp_whose_hidden_row_is_the_wider_one(m, hidden, ffn):
     v = orc.swiglu_bf16(orc.project(gc, gs, ffn, hidden, z, a, s), orc.project(uc, us, ffn, hidden, z, a, s))
     z, a, s, _ = orc.q8_quantize(v, bf16_bits=True)
     assert_close_reference(out.cpu().numpy(), orc.project(dc, ds, hidden, ffn, z, a, s, residual=h))
+
+
+@pytest.mark.parametrize("m,hidden,ffn", [(1, 2048, 256), (4, 2048, 256), (13, 5120, 512), (33, 2048, 1024)])
+def test_mlp_output_off_a_sixteen_byte_boundary(m, hidden, ffn):
+    """The hidden row is wider than its place in the workspace and is packed into the output, which need only be 4-byte
+    aligned: the same bits wherever it starts, and nothing written around it."""
+    ws = [weight(n, k, i)[0] for i, (n, k) in enumerate(((ffn, hidden), (ffn, hidden), (hidden, ffn)))]
+    h = torch.from_numpy(synth.activations(m, hidden, seed=m, scale=2.0)).to(DEV)
+    gamma = (torch.arange(hidden, device=DEV) % 7 * 0.03 - 0.1).to(torch.bfloat16)
+    room = torch.empty(q8_mlp_workspace_bytes(m, hidden, ffn), dtype=torch.uint8, device=DEV)
+    want = torch.empty((m, hidden), device=DEV)
+    assert want.data_ptr() % 16 == 0 and q4k_q8_mlp(*ws, h, gamma, 1e-6, want, m, room)
+    for off in (1, 2, 3):
+        guarded = torch.full((m * hidden + 8,), -7.0, device=DEV)
+        out = guarded[off:off + m * hidden].view(m, hidden)
+        assert out.data_ptr() % 16 == 4 * off and q4k_q8_mlp(*ws, h, gamma, 1e-6, out, m, room)
+        assert torch.equal(out, want) and (guarded[:off] == -7.0).all() and (guarded[off + m * hidden:] == -7.0).all()
+    assert kernel_status() == 0

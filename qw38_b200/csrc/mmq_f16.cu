@@ -178,10 +178,15 @@ __device__ __forceinline__ uint32_t map_to(uint32_t addr, uint32_t rank) {
   return r;
 }
 __device__ __forceinline__ void arrive_cluster(uint32_t cluster_addr) {
-  // Relaxed: what it announces are TMEM accesses, ordered by tcgen05.fence; a release at cluster scope costs a memory
-  // barrier of several hundred clocks per arrival.
+  // Relaxed: what it announces are TMEM accesses, ordered by tcgen05.fence (the mins besides: release_shared); a release at
+  // cluster scope costs a memory barrier of several hundred clocks per arrival.
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
+// What a relaxed arrival and a relaxed wait need around them when they stand for ordinary stores to the arriving CTA's shared
+// memory: fences at cluster scope that order shared memory alone and so wait for nothing else (not measurable; the release
+// and acquire forms of the barrier instructions took 16 to 20 % at 128 tokens, 9 % at 64).
+__device__ __forceinline__ void release_shared() { asm volatile("fence.release.sync_restrict::shared::cta.cluster;" ::: "memory"); }
+__device__ __forceinline__ void acquire_shared() { asm volatile("fence.acquire.sync_restrict::shared::cluster.cluster;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -518,7 +523,11 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
           for (int step = 0; step < C::kQ * (C::kStack ? 1 : 2); ++step) {
             int const pass = step / C::kQ, q = step % C::kQ;
             bool const last = C::kStack || pass == 1;  // the stage's last use
-            if (pass == 0) ok = ok && mbar_wait_inline(a_full(a0 + q), g_.phase, abort_flag, p.status, 0x806);
+            if (pass == 0 && q < C::kQ - 1) ok = ok && mbar_wait_inline(a_full(a0 + q), g_.phase, abort_flag, p.status, 0x806);
+            if (pass == 0 && q == C::kQ - 1) {  // the last stage comes with both CTAs' mins
+              ok = ok && mbar_wait_inline_relaxed_cluster(a_full(a0 + q), g_.phase, abort_flag, p.status, 0x806);
+              acquire_shared();
+            }
             if (C::kD2Bufs == 1 && last && q == C::kQ - 1 && u > u0) ok = ok && mbar_wait_inline(d_free(before.s), before.phase, abort_flag, p.status, 0x807);
             if (!ok) break;
             tc_fence_after();
@@ -617,7 +626,10 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) arrive_cluster(a_full0 + 8 * sa);
+        if (lane == 0) {
+          if (part == C::kSplit - 1 && i == kMine - 1) release_shared();  // the mins
+          arrive_cluster(a_full0 + 8 * sa);
+        }
       }
       if (lane == 0) {
         if (part == 0) mbar_arrive(s_full(sc));

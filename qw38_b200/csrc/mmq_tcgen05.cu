@@ -395,7 +395,7 @@ mmq_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_co
             uint32_t b0, parity;
             acc_slot<C::kAccBufs>(it, g0, b0, parity);
             uint32_t const set = b0 / C::kMmaPerCommit;
-            if (!mbar_wait_inline<256, 64>(bar_acc_empty(set), parity ^ 1, abort_flag, p.status, 5)) { ok = false; break; }
+            if (!mbar_wait_inline(bar_acc_empty(set), parity ^ 1, abort_flag, p.status, 5)) { ok = false; break; }
             tc_fence_after();
 #pragma unroll
             for (uint32_t k = 0; k < C::kMmaPerCommit; ++k) umma_i8(tmem_base + (b0 + k) * NTOK, cdesc, cdesc, idesc, 0);  // every accumulator = 2^17
@@ -441,9 +441,9 @@ mmq_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_co
           av[e] = live ? __ldg(p.xscales + idx) : 0.f;
           sv[e] = live ? __ldg(p.xsums + idx) : 0;
         }
-        if (!mbar_wait_inline<1024, 128>(bar_raw_full(r), (it / C::kRaw) & 1, abort_flag, p.status, 6)) { ok = false; break; }
-        if (!mbar_wait_inline<1024, 128>(bar_op_free(o), ((it / C::kOps) & 1) ^ 1, abort_flag, p.status, 7)) { ok = false; break; }
-        if (!mbar_wait_inline<1024, 128>(bar_s_free(sc), ((it / C::kScl) & 1) ^ 1, abort_flag, p.status, 8)) { ok = false; break; }
+        if (!mbar_wait_inline(bar_raw_full(r), (it / C::kRaw) & 1, abort_flag, p.status, 6)) { ok = false; break; }
+        if (!mbar_wait_inline(bar_op_free(o), ((it / C::kOps) & 1) ^ 1, abort_flag, p.status, 7)) { ok = false; break; }
+        if (!mbar_wait_inline(bar_s_free(sc), ((it / C::kScl) & 1) ^ 1, abort_flag, p.status, 8)) { ok = false; break; }
         uint32_t const raw = smem_s + C::oRawRing + r * C::kRawStage;
         uint32_t const ops = smem_s + C::oOps + o * C::kOpStage;
         uint32_t const scl = smem_s + C::oSclRing + sc * C::kSclStage;
@@ -567,7 +567,7 @@ mmq_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_co
       uint32_t b2, parity2;
       acc_slot<C::kAccBufs>(it2, g2, b2, parity2);
       if (wait_set) {
-        if (!mbar_wait_inline<512, 128>(bar_acc_full(b2 / C::kMmaPerCommit), parity2, abort_flag, p.status, 10)) return false;
+        if (!mbar_wait_inline(bar_acc_full(b2 / C::kMmaPerCommit), parity2, abort_flag, p.status, 10)) return false;
         tc_fence_after();
       }
       uint32_t const ta = lane_base + b2 * NTOK + 8 * UB * u;
@@ -589,7 +589,7 @@ mmq_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_co
       for (uint32_t kb = kb0; ok && kb < kb1; ++kb, ++it) {
         uint32_t const sc = it % C::kScl;
         bool const has_next = kb + 1 < kb1 || t + gridDim.x < num_tiles;
-        if (!mbar_wait_inline<512, 128>(bar_s_full(sc), (it / C::kScl) & 1, abort_flag, p.status, 9)) { ok = false; break; }
+        if (!mbar_wait_inline(bar_s_full(sc), (it / C::kScl) & 1, abort_flag, p.status, 9)) { ok = false; break; }
         uint32_t const scl = smem_s + C::oSclRing + sc * C::kSclStage;
         bool const wide = lds32(scl + C::oWide) == it + 1;
         uint32_t const ssp = scl + C::oS + (quarter * 8 + R0) * 16;  // this lane's four row scales of group g: + g * 512

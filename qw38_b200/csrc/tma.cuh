@@ -27,6 +27,12 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
                : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
 }
+__device__ __forceinline__ bool mbar_try_relaxed_cluster(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+               : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok != 0;
+}
 // One look at the barrier, never blocking.
 __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
   uint32_t ok;
@@ -61,13 +67,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 // The same wait, fully inlined: a function call inside a kernel that moves registers between warps with setmaxnreg
 // does not compile.  mbarrier.try_wait suspends the thread in hardware for a while by itself; sleeping between tries
 // (nanosleep, any back-off) only added wake-up latency to the hand-offs when it was measured, so there is none.  The
-// abort flag and the clock are looked at every eighth try.  (The template arguments are kept for the call sites.)
-template <uint32_t MaxNs = 256, uint32_t FirstNs = 32>
-__device__ __forceinline__ bool mbar_wait_inline(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
-  if (mbar_try(bar, parity)) return true;
+// abort flag and the clock are looked at every eighth try.
+template <class Try>
+__device__ __forceinline__ bool wait_inline(Try attempt, volatile int* abort_flag, int* status, int code) {
+  if (attempt()) return true;
   long long const t0 = clock64();
   for (uint32_t tries = 1;; ++tries) {
-    if (mbar_try(bar, parity)) return true;
+    if (attempt()) return true;
     if ((tries & 7u) == 0) {
       if (*abort_flag) return false;
       if (clock64() - t0 > kWaitCycles) {
@@ -77,6 +83,13 @@ __device__ __forceinline__ bool mbar_wait_inline(uint32_t bar, uint32_t parity, 
       }
     }
   }
+}
+__device__ __forceinline__ bool mbar_wait_inline(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  return wait_inline([&] { return mbar_try(bar, parity); }, abort_flag, status, code);
+}
+// For arrivals from other blocks of the cluster that stand for more than the barrier itself: an acquire fence follows.
+__device__ __forceinline__ bool mbar_wait_inline_relaxed_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  return wait_inline([&] { return mbar_try_relaxed_cluster(bar, parity); }, abort_flag, status, code);
 }
 
 // Shared-memory accesses by 32-bit shared-space address (generic pointers into the dynamic buffer cost 64-bit

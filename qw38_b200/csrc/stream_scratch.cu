@@ -6,17 +6,14 @@
 //   * Captured calls: one block per capture and stream, because an allocation recorded as a graph node would separate
 //     kernels that may overlap.  The graph owns the block through a user object; when the graph and its executables are
 //     gone it serves the next capture (or goes back to the pool, beyond kMaxFree idle blocks).  Calls that may overlap the
-//     one before them take the two halves of the block in turn.
+//     one before them take the two halves of the block in turn; the block remembers whether its last call did, because one
+//     that did not (launch overlap was off, or it failed) may lie across both halves.
 #include "stream_scratch.h"
 
 #include <mutex>
 #include <vector>
 
 namespace q4k {
-namespace {
-
-constexpr uint64_t kKeep = 192ull << 20;
-constexpr size_t kMaxFree = 4;
 
 struct CapturedBlock {
   void* p = nullptr;
@@ -25,7 +22,13 @@ struct CapturedBlock {
   unsigned long long capture = 0;  // 0 = idle
   cudaStream_t stream = nullptr;
   uint32_t turn = 0;
+  bool alternating = true;  // its last call took a half and has been launched; also before the first one
 };
+
+namespace {
+
+constexpr uint64_t kKeep = 192ull << 20;
+constexpr size_t kMaxFree = 4;
 
 struct Pool {
   cudaMemPool_t eager = nullptr, captured = nullptr;  // apart, so that blocks graphs hold do not count against what is kept
@@ -72,11 +75,15 @@ void CUDART_CB retire_captured(void* data) {
   static_cast<CapturedBlock*>(data)->capture = 0;
 }
 
-cudaError_t captured_block(cudaStream_t stream, cudaGraph_t graph, unsigned long long capture, int device, uint64_t bytes, bool alternate, void** out) {
+cudaError_t captured_block(cudaStream_t stream, cudaGraph_t graph, unsigned long long capture, int device, uint64_t bytes, bool alternate, CapturedBlock** block, void** out,
+                           bool* alternates) {
   uint64_t const half = (bytes + 255) / 256 * 256;
   if (alternate) bytes = 2 * half;
-  auto take = [&](CapturedBlock* b) {  // the calls of a block all alternate: its halves are half its size
+  auto take = [&](CapturedBlock* b) {  // halves are half the block's size, whatever the call needs
     *out = static_cast<uint8_t*>(b->p) + (alternate ? (b->turn++ & 1) * (b->bytes / 512 * 256) : 0);
+    *alternates = alternate && b->alternating;
+    b->alternating = false;  // until release()
+    *block = b;
   };
   std::lock_guard<std::mutex> lock(g_mutex);
   CapturedBlock* idle = nullptr;
@@ -119,6 +126,7 @@ cudaError_t captured_block(cudaStream_t stream, cudaGraph_t graph, unsigned long
   if ((st = cudaUserObjectCreate(&object, idle, retire_captured, 1, cudaUserObjectNoDestructorSync)) != cudaSuccess) return st;
   idle->capture = capture;
   idle->stream = stream;
+  idle->alternating = true;
   if ((st = cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove)) != cudaSuccess) {
     idle->capture = ~0ull;  // the object still refers to it: not reused
     return st;
@@ -138,8 +146,8 @@ cudaError_t StreamScratch::acquire(cudaStream_t stream, uint64_t bytes, bool alt
   cudaGraph_t graph = nullptr;
   if ((st = cudaStreamGetCaptureInfo(stream, &status, &capture, &graph)) != cudaSuccess) return st;
   if (status == cudaStreamCaptureStatusActive) {
-    alternates_ = alternate;
-    return captured_block(stream, graph, capture + 1, device, bytes, alternate, &p_);
+    alternate_ = alternate;
+    return captured_block(stream, graph, capture + 1, device, bytes, alternate, &block_, &p_, &alternates_);
   }
   Pool* pool = nullptr;
   {
@@ -156,6 +164,15 @@ cudaError_t StreamScratch::acquire(cudaStream_t stream, uint64_t bytes, bool alt
 }
 
 cudaError_t StreamScratch::release() {
+  if (block_) {
+    std::lock_guard<std::mutex> lock(g_mutex);
+    block_->alternating = alternate_;
+    block_ = nullptr;
+  }
+  return give_back();
+}
+
+cudaError_t StreamScratch::give_back() {
   if (!owned_) return cudaSuccess;
   owned_ = false;
   return cudaFreeAsync(p_, stream_);

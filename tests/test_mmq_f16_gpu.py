@@ -152,3 +152,28 @@ def test_rows_are_quantised_as_the_pack_does(m, n, k):
     x[m - 1, k - 1] = float("nan")
     prefill_project(DecodeMmvDesc(w, x, out, L.EPILOGUE_STORE_FP32), ws, f)
     assert f.item() == 1 and kernel_status() == 0
+
+
+def test_overlap_switched_inside_a_capture():
+    """Projections with settled inputs, launch overlap off and on in turn within one graph: bitwise the serial results."""
+    n, k = 5120, 2560
+    ws = [synth.device_weight(n, k, seed=60 + i) for i in range(6)]
+    q = pack_q8(torch.randn((64, k), device=DEV, generator=torch.Generator(device=DEV).manual_seed(1)), flag())
+    want = [q4k_q8_project(w, q) for w in ws]
+    outs = [torch.full((64, n), -3.0, device=DEV) for _ in ws]
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    try:
+        with torch.cuda.graph(graph, stream=stream):
+            for i, (w, out) in enumerate(zip(ws * 3, outs * 3)):
+                set_launch_overlap(i % 3 != 0)
+                q4k_q8_project(w, q, out=out, trusted=True, input_settled=True)
+    finally:
+        set_launch_overlap(False)
+    for _ in range(20):
+        for out in outs:
+            out.fill_(-3.0)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(outs, want))
+    assert kernel_status() == 0

@@ -67,7 +67,9 @@ __device__ __forceinline__ uint32_t odd_bytes(uint32_t z0, uint32_t z1) { return
 // soon as every block of this grid has called it (or exited).  Every kernel of this library calls
 // it AFTER its pdl_wait(): a successor then never runs beside anything older than its direct
 // predecessor, which is what lets a caller flag a projection's input as settled.  Both are no-ops
-// for kernels launched without the attribute.
+// for kernels launched without the attribute.  What the preceding kernel may write is read by plain loads only: __ldg, or a
+// const __restrict__ parameter that the compiler turns into it, promises data that nobody writes during this kernel, whose
+// life begins before the wait.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

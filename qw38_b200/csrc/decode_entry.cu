@@ -19,7 +19,7 @@ __device__ __forceinline__ float sigmoid_fp32(float u) {
   return d == 1.0f ? n : rounded_quotient(n, d, __frcp_rn(d));
 }
 
-__global__ void store_bf16_kernel(const float* __restrict__ in, uint16_t* __restrict__ out, uint64_t count) {
+__global__ void store_bf16_kernel(const float* in, uint16_t* __restrict__ out, uint64_t count) {
   pdl_wait();
   pdl_launch_dependents();  // after the wait: the next launch never runs beside anything older than this one
   uint64_t const i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -30,7 +30,7 @@ __global__ void store_bf16_kernel(const float* __restrict__ in, uint16_t* __rest
 // bytes per value; Wide (all pointers 16-byte aligned, count a multiple of eight): eight values per thread, four loads in
 // flight.  2048 x 17408: 53 us, 112 before (one value per thread, a division that left its short form, rounding in software).
 template <bool Wide>
-__global__ void swiglu_store_bf16_kernel(const float* __restrict__ gate, const float* __restrict__ up,
+__global__ void swiglu_store_bf16_kernel(const float* gate, const float* up,
                                          uint16_t* __restrict__ out, uint64_t count) {
   pdl_wait();
   pdl_launch_dependents();  // after the wait: the next launch never runs beside anything older than this one

@@ -19,9 +19,8 @@ namespace {
 constexpr int kThreads = 256;
 
 template <int M>
-__global__ void __launch_bounds__(kThreads) gemv_bf16w_kernel(WeightView w, const uint16_t* __restrict__ x, uint32_t k,
-                                                             uint32_t padded_k, float* __restrict__ out,
-                                                             const float* __restrict__ residual) {
+__global__ void __launch_bounds__(kThreads) gemv_bf16w_kernel(WeightView w, const uint16_t* x, uint32_t k,
+                                                             uint32_t padded_k, float* out, const float* residual) {
   extern __shared__ __align__(16) float xs[];  // [M][padded_k], zero beyond k
   pdl_wait();
   pdl_launch_dependents();  // after the wait: the next launch never runs beside anything older than this one

@@ -201,21 +201,33 @@ __global__ void __launch_bounds__(kThreads, M <= 2 ? 2 : 1) gemv_dp4a_kernel(con
       // a 16-byte source chunk holds half a K32 group (columns 16c..16c+15)
       bool const z16 = (reinterpret_cast<uintptr_t>(p.codes) & 15) == 0;
       uint32_t const chunks = M * tiles_k * 16;
-#pragma unroll 4
-      for (uint32_t c = threadIdx.x; c < chunks; c += kConsumers) {
-        uint4 z;
-        if (z16) z = __ldg(reinterpret_cast<const uint4*>(p.codes) + c);
-        else {
-          const uint32_t* s32 = reinterpret_cast<const uint32_t*>(p.codes) + c * 4;
-          z = make_uint4(__ldg(s32), __ldg(s32 + 1), __ldg(s32 + 2), __ldg(s32 + 3));
+      for (uint32_t c0 = threadIdx.x; c0 < chunks; c0 += kConsumers * 4) {  // four chunks requested at a time
+        uint4 z[4];
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          uint32_t const c = c0 + h * kConsumers;
+          if (c >= chunks) break;
+          if (z16) z[h] = reinterpret_cast<const uint4*>(p.codes)[c];
+          else {
+            const uint32_t* const s32 = reinterpret_cast<const uint32_t*>(p.codes) + c * 4;
+            z[h] = make_uint4(s32[0], s32[1], s32[2], s32[3]);
+          }
         }
-        sts128(s_z + (c >> 4) * 256 + (c & 1) * 128 + ((c >> 1) & 7) * 16, even_bytes(z.x, z.y), odd_bytes(z.x, z.y),
-               even_bytes(z.z, z.w), odd_bytes(z.z, z.w));
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          uint32_t const c = c0 + h * kConsumers;
+          if (c >= chunks) break;
+          sts128(s_z + (c >> 4) * 256 + (c & 1) * 128 + ((c >> 1) & 7) * 16, even_bytes(z[h].x, z[h].y), odd_bytes(z[h].x, z[h].y),
+                 even_bytes(z[h].z, z[h].w), odd_bytes(z[h].z, z[h].w));
+        }
       }
-#pragma unroll 2
-      for (uint32_t i = threadIdx.x; i < M * G; i += kConsumers) {
-        float const a = __ldg(p.scales + i);
-        sts64f(s_aw + i * 8, a, a * float(__ldg(p.sums + i)));
+      for (uint32_t i0 = threadIdx.x; i0 < M * G; i0 += kConsumers * 2) {
+        uint32_t const i1 = i0 + kConsumers;
+        bool const two = i1 < M * G;
+        float const a0 = p.scales[i0], a1 = two ? p.scales[i1] : 0.f;
+        int const s0 = p.sums[i0], s1 = two ? p.sums[i1] : 0;
+        sts64f(s_aw + i0 * 8, a0, a0 * float(s0));
+        if (two) sts64f(s_aw + i1 * 8, a1, a1 * float(s1));
       }
     }
     asm volatile("bar.sync 1, %0;" ::"n"(kConsumers) : "memory");

@@ -101,8 +101,8 @@ template <int Warps, int Tokens> struct Smem {
 
 // Upper: tokens 8..15 exist.  Tokens staged = 16 with Upper, else 8.
 template <bool Upper, bool Dump, bool Wide, int Warps>
-__global__ void __launch_bounds__(Warps * 32) gemv_mma_kernel(WeightView w, Q8View x, float* __restrict__ out,
-                                                              const float* __restrict__ residual,
+__global__ void __launch_bounds__(Warps * 32) gemv_mma_kernel(WeightView w, Q8View x, float* out,
+                                                              const float* residual,
                                                               int32_t* __restrict__ partials, uint32_t split_k) {
   constexpr int Tokens = Upper ? 16 : 8;
   using S = Smem<Warps, Tokens>;

@@ -306,8 +306,7 @@ __device__ __forceinline__ float block_top(float row, float* warp_top) {
   return row;
 }
 
-__global__ void __launch_bounds__(256) planes_kernel(const int8_t* __restrict__ codes, const float* __restrict__ scales,
-                                                     const int32_t* __restrict__ sums, uint32_t m, uint32_t m_pad, uint32_t tiles_k,
+__global__ void __launch_bounds__(256) planes_kernel(const int8_t* codes, const float* scales, const int32_t* sums, uint32_t m, uint32_t m_pad, uint32_t tiles_k,
                                                      __half* __restrict__ planes, __half* __restrict__ sums16, float* __restrict__ exps,
                                                      float* __restrict__ tokens, uint32_t* __restrict__ tickets, uint32_t ticket_count,
                                                      bool early) {
@@ -343,7 +342,7 @@ __global__ void __launch_bounds__(256) planes_kernel(const int8_t* __restrict__ 
 // The same from bf16 rows [m][k]: a block quantises one token, keeps it in registers until its largest scale is known, and
 // writes the planes without the Q8 form in between.  Held: super-blocks per warp.
 template <int Held>
-__global__ void __launch_bounds__(256) rows_planes_kernel(const uint16_t* __restrict__ rows, uint32_t k, bool vec, int* failure, uint32_t m,
+__global__ void __launch_bounds__(256) rows_planes_kernel(const uint16_t* rows, uint32_t k, bool vec, int* failure, uint32_t m,
                                                           uint32_t m_pad, uint32_t tiles_k, __half* __restrict__ planes,
                                                           __half* __restrict__ sums16, float* __restrict__ exps, float* __restrict__ tokens,
                                                           uint32_t* __restrict__ tickets, uint32_t ticket_count) {
@@ -360,7 +359,7 @@ __global__ void __launch_bounds__(256) rows_planes_kernel(const uint16_t* __rest
     const uint16_t* const src = rows + uint64_t(tok) * k + col;
     held[i] = make_uint4(0u, 0u, 0u, 0u);
     if (tok >= m || col >= k) continue;
-    if (vec && col + 8 <= k) held[i] = __ldg(reinterpret_cast<const uint4*>(src));
+    if (vec && col + 8 <= k) held[i] = *reinterpret_cast<const uint4*>(src);
     else {
       uint32_t e[8];
 #pragma unroll

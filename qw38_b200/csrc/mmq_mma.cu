@@ -79,8 +79,8 @@ __device__ __forceinline__ void fill_stage(uint8_t* stage, const uint8_t* codes,
 }
 
 template <int TT, bool Dump, bool Wide>
-__global__ void __launch_bounds__(kThreads) mmq_mma_kernel(WeightView w, Q8View x, float* __restrict__ out,
-                                                           const float* __restrict__ residual,
+__global__ void __launch_bounds__(kThreads) mmq_mma_kernel(WeightView w, Q8View x, float* out,
+                                                           const float* residual,
                                                            int32_t* __restrict__ partials, uint32_t split_k,
                                                            uint32_t kbs_step, float* scratch,
                                                            uint32_t* tickets) {

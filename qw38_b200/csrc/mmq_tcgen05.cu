@@ -438,8 +438,8 @@ mmq_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_co
           uint32_t const j = et + e * kET, tk = j >> 3, g = j & 7;
           bool const live = j < NTOK * 8 && tok0 + tk < p.m;
           size_t const idx = size_t(tok0 + tk) * p.G + kb * 8 + g;
-          av[e] = live ? __ldg(p.xscales + idx) : 0.f;
-          sv[e] = live ? __ldg(p.xsums + idx) : 0;
+          av[e] = live ? p.xscales[idx] : 0.f;
+          sv[e] = live ? p.xsums[idx] : 0;
         }
         if (!mbar_wait_inline(bar_raw_full(r), (it / C::kRaw) & 1, abort_flag, p.status, 6)) { ok = false; break; }
         if (!mbar_wait_inline(bar_op_free(o), ((it / C::kOps) & 1) ^ 1, abort_flag, p.status, 7)) { ok = false; break; }

@@ -61,7 +61,7 @@ __device__ __forceinline__ void load8(const T* src, uint32_t col0, uint32_t k, f
 
 // A warp takes 256 columns of a row at a time; the next ones are requested before the present ones are quantised.
 template <typename T, bool Vec>
-__global__ void __launch_bounds__(kThreads, kBlocksPerSm) pack_kernel(const T* __restrict__ in, int8_t* __restrict__ codes,
+__global__ void __launch_bounds__(kThreads, kBlocksPerSm) pack_kernel(const T* in, int8_t* __restrict__ codes,
                                                                        float* __restrict__ scales, int32_t* __restrict__ sums, uint32_t m,
                                                                        uint32_t k, uint32_t pk, int* failure) {
   pdl_wait();               // the input may come from the kernel before this one
@@ -97,8 +97,7 @@ __device__ __forceinline__ float silu(float g) {
 
 // v = bf16_rne(silu(g) * u); non-finite g or u poisons the value
 // (reference: swiglu_pack_kernel, cuda/q4k_q8.cu:52-61).  ffn % 256 == 0.
-__global__ void __launch_bounds__(kThreads) swiglu_pack_kernel(const float* __restrict__ gate,
-                                                                const float* __restrict__ up,
+__global__ void __launch_bounds__(kThreads) swiglu_pack_kernel(const float* gate, const float* up,
                                                                 int8_t* __restrict__ codes, float* __restrict__ scales,
                                                                 int32_t* __restrict__ sums, uint64_t chunks,
                                                                 int* failure) {
@@ -146,8 +145,7 @@ __device__ __forceinline__ float block_reduce(float v, float* scratch, bool is_m
 // share of the row and of the gain at once and keeps it in registers for the three passes; the loop form, which serves
 // wider rows, waits for memory in every iteration of every pass: 15 us at 5120 columns against 4 us.
 template <int Held>
-__global__ void __launch_bounds__(kThreads) hidden_rms_q8_kernel(const float* __restrict__ residual,
-                                                                  const uint16_t* __restrict__ gamma,
+__global__ void __launch_bounds__(kThreads) hidden_rms_q8_kernel(const float* residual, const uint16_t* gamma,
                                                                   float eps, uint32_t hidden,
                                                                   int8_t* codes, float* scales,
                                                                   int32_t* sums, int* failure) {

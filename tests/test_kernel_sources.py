@@ -18,3 +18,34 @@ def test_minima_are_published_across_the_cluster():
     assert writer.index("fence.proxy.async") < writer.index("release_shared();") < writer.index("arrive_cluster(a_full0")
     issuer = text[text.index("mbar_wait_inline_relaxed_cluster(a_full"):]
     assert issuer.index("acquire_shared();") < issuer.index("mma_pair_ss(")
+
+
+def kernels(text):
+    """(parameter list, body) of every __global__ function."""
+    for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__\((?:[^()]|\([^()]*\))*\)\s*)?(\w+)\s*\(", text):
+        end = text.index(")", m.end())
+        while text.count("(", m.end(), end) != text.count(")", m.end(), end):
+            end = text.index(")", end + 1)
+        start = at = text.index("{", end)
+        depth = 0
+        while True:
+            depth += {"{": 1, "}": -1}.get(text[at], 0)
+            at += 1
+            if depth == 0:
+                break
+        yield m.group(1), text[m.end():end], text[start:at]
+
+
+def test_kernels_that_start_early_read_their_operands_with_plain_loads():
+    """A kernel with griddepcontrol.wait may begin while its operands are still written: no __ldg (but of weights, which are
+    constant) and no const __restrict__ parameter, which the compiler may turn into the same load."""
+    early = 0
+    for path in sorted(CSRC.glob("*.cu")):
+        for name, params, body in kernels(code(path)):
+            if "pdl_wait()" not in body:
+                continue
+            early += 1
+            assert not re.search(r"const\s+\w+\s*\*\s*__restrict__", params), f"{path.name}: {name}"
+            loads = set(re.findall(r"__ldg\((\w[\w.]*)", body)) - {"c32", "m16"}  # dp4a: codes and metadata of the weights
+            assert not loads, f"{path.name}: {name} reads {loads}"
+    assert early >= 10

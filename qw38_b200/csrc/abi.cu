@@ -725,23 +725,23 @@ int decode_pack(const q4k_decode_desc& d, const q4k_q8_input& q8, int* failure, 
 // *fused = false when the operands do not qualify (more than 16 rows, unaligned weights, another activation policy);
 // the caller then composes separate launches.
 // Up to kDecodeRawTokens rows the launch also quantises: each block its own K slice, which at one to four tokens takes
-// less than the pack launch it saves (at eight, five warps per scheduler spend as long on it as that launch takes).
+// less than the pack launch it saves (at eight, five warps per scheduler spend as long on it as that launch takes).  Blocks then
+// read the input while others write the outputs, so a call whose input (or failure flag) shares memory with another operand
+// takes the pack launch first, at one to four tokens as at sixteen: neither is refused.
 constexpr uint32_t kDecodeRawTokens = 4;
+bool overlaps(const Region& a, const Region& b) {
+  auto const p = reinterpret_cast<uintptr_t>(a.p), q = reinterpret_cast<uintptr_t>(b.p);
+  return p < q + b.bytes && q < p + a.bytes;
+}
 int decode_fused(const q4k_decode_desc* const* descs, uint32_t count, bool swiglu, const q4k_q8_input& q8, int* failure, cudaStream_t stream,
                  bool* fused) {
   *fused = false;
-  bool const raw = q8.m <= kDecodeRawTokens;
   q4k::WeightView ws[3];
   q4k::GemvTmaOutput outs[3] = {};
   Region regions[16];
   int nreg = 0;
   // the pack of the workspace is one run of memory: codes, scales, sums
   regions[nreg++] = {q8.codes, uint64_t(reinterpret_cast<uint8_t*>(q8.sums + q8.sums_len) - reinterpret_cast<uint8_t*>(q8.codes)), 4, "workspace"};
-  if (raw) {
-    if (!failure) return fail(Q4K_ERR_INVALID_ARGUMENT, "decode_mmv: null failure flag");
-    regions[nreg++] = {descs[0]->input, descs[0]->input_len * 2, 2, "input"};
-    regions[nreg++] = {failure, 4, 4, "failure"};
-  }
   uint64_t n_total = 0, tiles = 0;
   for (uint32_t i = 0; i < count; ++i) {
     const q4k_decode_desc& d = *descs[i];
@@ -778,6 +778,13 @@ int decode_fused(const q4k_decode_desc* const* descs, uint32_t count, bool swigl
     }
     n_total += d.weight.n;
     tiles += (d.weight.padded_n + 15) / 16;
+  }
+  Region const input{descs[0]->input, descs[0]->input_len * 2, 2, "input"}, flag{failure, 4, 4, "failure"};
+  bool raw = q8.m <= kDecodeRawTokens && failure;
+  for (int i = 1; i < nreg; ++i) raw = raw && !overlaps(input, regions[i]) && !overlaps(flag, regions[i]);
+  if (raw) {
+    regions[nreg++] = input;
+    regions[nreg++] = flag;
   }
   if (int st = check_distinct(regions, nreg, false)) return st;
   if (!raw)

@@ -184,3 +184,17 @@ def test_mlp_output_off_a_sixteen_byte_boundary(m, hidden, ffn):
         assert out.data_ptr() % 16 == 4 * off and q4k_q8_mlp(*ws, h, gamma, 1e-6, out, m, room)
         assert torch.equal(out, want) and (guarded[:off] == -7.0).all() and (guarded[off + m * hidden:] == -7.0).all()
     assert kernel_status() == 0
+
+
+@pytest.mark.parametrize("m", [1, 2, 4, 5, 16])
+def test_decode_output_over_its_own_input(m):
+    """A call whose output takes the place of its input is served at every token count, as from separate buffers."""
+    n, k = 264, 512
+    (w, hc, hs), x = weight(n, k, seed=m), torch.from_numpy(synth.activations(m, k, seed=m)).to(DEV).to(torch.bfloat16)
+    z, a, s, _ = orc.q8_quantize(x.view(torch.int16).cpu().numpy().view(np.uint16), bf16_bits=True)
+    room, ws, f = torch.empty(m * n, device=DEV), decode_workspace(m, n, k), flag()
+    inside = room.view(torch.bfloat16)[:m * k].view(m, k)
+    inside.copy_(x)
+    launch_decode_mmv(DecodeMmvDesc(w, inside, room.view(m, n), L.EPILOGUE_STORE_FP32), ws, f)
+    assert_close_contract(room.view(m, n).cpu().numpy(), orc.project(hc, hs, n, k, z, a, s))
+    assert f.item() == 0 and kernel_status() == 0

@@ -16,8 +16,10 @@
 //     steps of one super-block are added before it is drained and folded into fp32 registers.
 //   * min term: m is exact in fp16, a*s is split into two fp16 terms like x, and one more MMA of K = 16 (eight groups, hi
 //     and lo) per super-block puts the sum of their products into an accumulator of its own.
-// Error against the equation in double precision: 1.8e-7 to 2.2e-7 of the result's norm at K = 256 .. 17408 (the int8 kernel:
-// 0.7e-7 to 2.3e-7).
+// Error against the equation in 64 bits, K = 512 .. 17408, of the norm of the result (largest of a token's own norm in
+// brackets): normal data, with and without outliers, 1.5e-7 .. 2.1e-7 (3.9e-7), the int8 kernel 0.7e-7 .. 1.4e-7 (1.9e-7);
+// rows with one value in all or per super-block 2.3e-7 .. 2.6e-7 (3.9e-7), the int8 kernel 0.4e-7 .. 0.9e-7 (1.2e-7): their
+// sums lose nothing to the tensor core's truncation, and the 2^-22 that compensates its mean is an error there.
 //
 // Rates that the design rests on (measured, clk per SM): tcgen05.mma with A in TMEM takes max(17, N/2) + 4 per K16 step
 // (45 at N = 16 when A comes from shared memory), the paired form the same; tcgen05.st 32x32b of 32 lanes x 16 words 17 with
@@ -578,7 +580,8 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
       if (part == 0) {
         if (!mbar_wait_inline(s_free(sc), t_.phase ^ 1, abort_flag, p.status, 0x809)) break;
         // The tensor core truncates when it accumulates, which shortens a super-block's sum by 2^-22 on average (measured
-        // on normal data, sixteen steps): the row scale takes the mean of that out.
+        // on normal data, sixteen steps): the row scale takes the mean of that out.  Sums that lose nothing (few values that
+        // are not zero) come out 2^-22 too large.
         sts64f(smem + C::oScl + sc * C::kScl + row * 8, fp16_bits_to_f32(cm.x & 0xffffu) * (1.f + 0x1p-22f), -32.f * fp16_bits_to_f32(cm.x >> 16));
       }
       ScaleMinWords const sm = decode_scale_min(cm.y, cm.z, cm.w);

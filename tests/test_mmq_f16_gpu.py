@@ -177,3 +177,40 @@ def test_overlap_switched_inside_a_capture():
         torch.cuda.synchronize()
         assert all(torch.equal(a, b) for a, b in zip(outs, want))
     assert kernel_status() == 0
+
+
+def exact(codes, meta, z, a):
+    """The equation in 64 bits from logical codes and metadata, on the device."""
+    p = meta[..., 4:].astype(np.int64)
+    sc = np.concatenate([p[..., 0:4] & 63, (p[..., 8:12] & 15) | (p[..., 0:4] >> 6 << 4)], -1)
+    mn = np.concatenate([p[..., 4:8] & 63, (p[..., 8:12] >> 4) | (p[..., 4:8] >> 6 << 4)], -1)
+    d, dmin = (np.ascontiguousarray(meta[..., i:i + 2]).view(np.float16).astype(np.float64) for i in (0, 2))
+    w = np.repeat((d * sc).reshape(len(codes), -1), 32, 1) * codes - np.repeat((dmin * mn).reshape(len(codes), -1), 32, 1)
+    x = z.astype(np.float64) * np.repeat(a.astype(np.float64), 32, 1)
+    return (torch.from_numpy(x).to(DEV) @ torch.from_numpy(w).to(DEV).T).cpu().numpy()
+
+
+# Each super-block: at most sixteen steps of the tensor core at full magnitude, each truncated by up to 2^-23 of the sum so far
+# (the mean is compensated, what is left spreads over about 2^-23), then an fp32 addition.  Sums that lose nothing come out
+# 2^-22 = 2.4e-7 too large, and the two planes carry x to 2^-23.  Measured, of a token's norm: 2.2e-7 to 3.9e-7 (the int8
+# kernel 0.5e-7 to 1.9e-7); 1e-6 is two and a half times that.
+@pytest.mark.parametrize("m,n,k", [(17, 264, 512), (64, 520, 5120), (130, 264, 17408)])
+@pytest.mark.parametrize("kind", ["dense", "outliers", "one value per super-block", "one value"])
+def test_error_against_64_bits(m, n, k, kind):
+    codes, meta = synth.logical_q4k(n, k, seed=k)
+    hc, hs = synth.split_tiles(codes, meta)
+    w = PrefillWeight.from_host(hc, hs, n, k)
+    x = synth.activations(m, k, seed=m, scale=0.5, outlier_frac=0.01 if kind == "outliers" else 0.0)
+    if kind.startswith("one"):
+        keep = np.random.default_rng(m).integers(0, 256, (m, k // 256)) + np.arange(0, k, 256)
+        mask = np.zeros_like(x)
+        np.put_along_axis(mask, keep if "per" in kind else keep[:, :1], 1.0, 1)
+        x = x * mask
+    q = pack_q8(torch.from_numpy(x).to(DEV), flag())
+    ref = exact(codes, meta, q.codes.cpu().numpy(), q.scales.cpu().numpy())
+    norm = np.sqrt((ref ** 2).sum(1))
+    for kernel in (L.KERNEL_F16, L.KERNEL_TCGEN05):
+        y = q4k_q8_project(w, q, kernel=kernel).cpu().numpy().astype(np.float64)
+        err = np.sqrt(((y - ref) ** 2).sum(1)) / norm
+        assert err.max() <= 1e-6
+    assert kernel_status() == 0

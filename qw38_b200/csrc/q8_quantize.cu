@@ -85,9 +85,9 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) pack_kernel(const T* i
   }
 }
 
-// g / (1 + exp(-g)), rounded as the division would be.  A divisor above 2^64 is scaled (exactly: the quotient of a finite g
-// stays a normal number) and an infinite one replaced, so that no residual of the quotient underflows.  Not finite for a g
-// that is not.
+// g / (1 + exp(-g)), rounded as the division would be (-0 gives +0, which changes no code).  A divisor above 2^64 is scaled
+// (exactly: the quotient of a finite g stays a normal number) and an infinite one replaced, so that no residual of the quotient
+// underflows.  Not finite for a g that is not.
 __device__ __forceinline__ float silu(float g) {
   float const d = 1.f + expf(-g);
   bool const far = d > 0x1p64f, lost = isinf(d);

@@ -342,7 +342,10 @@ __global__ void __launch_bounds__(kThreads, M <= 2 ? 2 : 1) gemv_dp4a_kernel(con
 
 template <int M>
 cudaError_t launch_m(const DpParams& p, uint32_t grid, uint32_t smem, cudaStream_t stream) {
-  auto kernel = p.partials ? gemv_dp4a_kernel<M, true, false> : (p.raw ? gemv_dp4a_kernel<M, false, true> : gemv_dp4a_kernel<M, false, false>);
+  auto kernel = p.partials ? gemv_dp4a_kernel<M, true, false> : gemv_dp4a_kernel<M, false, false>;
+  if constexpr (M <= kGemvDp4aBestTokens) {
+    if (p.raw) kernel = gemv_dp4a_kernel<M, false, true>;
+  }
   cudaError_t st = allow_smem(reinterpret_cast<const void*>(kernel), int(smem));
   if (st != cudaSuccess) return st;
   return launch_kernel(kernel, grid, kThreads, smem, stream, launch_overlap(), p);
@@ -397,7 +400,7 @@ cudaError_t launch_gemv_dp4a(const WeightView& w, const Q8View& x, float* out, c
 
 cudaError_t launch_gemv_dp4a_multi(const WeightView* ws, const GemvTmaOutput* outs, uint32_t count, uint32_t m, uint32_t padded_k,
                                    const RawRows& raw, int* status, cudaStream_t stream) {
-  if (count < 1 || count > 3) return cudaErrorInvalidValue;
+  if (count < 1 || count > 3 || m > kGemvDp4aBestTokens) return cudaErrorInvalidValue;
   DpParams p{};
   p.wide = 1;
   for (uint32_t i = 0; i < count; ++i) {

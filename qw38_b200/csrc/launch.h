@@ -156,7 +156,7 @@ struct GemvTmaOutput {
   uint16_t* out_bf16;
   const float* residual;
 };
-// The same projections (no SwiGLU pair) from bf16 rows on dp4a, in gemv_dp4a.cu: m <= 4.
+// The same projections (no SwiGLU pair) from bf16 rows on dp4a, in gemv_dp4a.cu: m <= kGemvDp4aBestTokens.
 cudaError_t launch_gemv_dp4a_multi(const WeightView* ws, const GemvTmaOutput* outs, uint32_t count, uint32_t m, uint32_t padded_k,
                                    const RawRows& raw, int* status, cudaStream_t stream);
 cudaError_t launch_gemv_tma_multi(const WeightView* ws, const GemvTmaOutput* outs, uint32_t count, bool swiglu_pair, const Q8View& x,

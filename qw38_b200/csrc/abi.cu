@@ -243,7 +243,7 @@ constexpr uint32_t kFlagTrustedSpans = 1u, kFlagInputSettled = 2u;
 
 // The fp16-plane kernel with scratch of its own (stream_scratch.cu).
 constexpr uint64_t kF16SuperBlocks = 16384;  // of eight rows; below, nine to sixteen tokens stay with the TMA-streamed kernel
-int project_f16(const q4k_weight& w, const q4k_q8_input& x, const q4k::TcOutput& out, cudaStream_t stream, const q4k_weight* second = nullptr,
+int project_f16(const q4k_weight& w, const q4k_q8_input& x, const q4k::F16Output& out, cudaStream_t stream, const q4k_weight* second = nullptr,
                 const q4k::RawRows* raw = nullptr) {
   int* const status = q4k::kernel_status_word();
   if (!status) return Q4K_ERR_STATUS;
@@ -345,8 +345,7 @@ int project_impl(const q4k_weight* weight, const q4k_q8_input& x, float* output,
   if (kernel == Q4K_KERNEL_F16) {
     if (!q4k::f16_supported(view(w), view(x)) || partials)
       return fail(Q4K_ERR_INVALID_ARGUMENT, "q8.project: the fp16 kernel needs aligned operands and has no partial dots");
-    q4k::TcOutput to = q4k::tc_output(output, res);
-    to.input_settled = (opt && (opt->flags & kFlagInputSettled)) ? 1u : 0u;
+    q4k::F16Output const to{output, nullptr, res, opt && (opt->flags & kFlagInputSettled)};
     return project_f16(w, x, to, stream, nullptr, raw);
   }
   if (kernel == Q4K_KERNEL_TCGEN05) {
@@ -417,9 +416,7 @@ int project_pair(const q4k_weight* gate, const q4k_weight* up, const q4k_q8_inpu
   }
   ScopedRange range("qw38:op name=q4k_project m=%u n=%u k=%u role=%s residual=%u compute=%s", unsigned(x.m), unsigned(2 * gate->n),
                     unsigned(gate->k), "gate_up", 0u, "integer_mma");
-  q4k::TcOutput to = q4k::tc_output(g, nullptr);
-  to.out[1] = u;
-  return project_f16(*gate, x, to, stream, up, raw);
+  return project_f16(*gate, x, q4k::F16Output{g, u, nullptr, false}, stream, up, raw);
 }
 
 int check_pack(const void* input, bool fp32, uint64_t input_len, const q4k_q8_input& x, int* failure) {

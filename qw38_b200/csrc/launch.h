@@ -65,15 +65,13 @@ struct TcPlan {
   uint32_t ntok;
   uint32_t split_k;
 };
-// Where the rows go: element (token, row) lands at token * stride + row0 + row of every fp32 destination
-// (one buffer, or each rank's copy of a gathered output, written with plain peer stores), or of the one
-// bf16 destination (round to nearest even).  residual, if set, has the destination's geometry and is
-// added last.  stride 0 = the weight's own n.
+// Where the rows go: element (token, row) lands at token * stride + row0 + row of every destination (one buffer, or
+// each rank's copy of a gathered output, written with plain peer stores).  residual, if set, has the destination's
+// geometry and is added last.  stride 0 = the weight's own n.
 // Row-sharded use (flags / done / unsignalled as in GemvTmaGather below): done != nullptr makes the launch count
 // itself as a finished projection of `rank`.
 struct TcOutput {
   float* out[8];
-  uint16_t* out_bf16;
   const float* residual;
   uint32_t ndst, stride, row0;
   uint32_t* flags[8];
@@ -110,11 +108,17 @@ struct F16Plan {
   uint32_t unit_step;      // granularity of a cluster's run of super-blocks: 1, or tiles_k = whole tiles
   uint32_t slot_clusters;  // clusters for whose partial tiles the scratch has room
 };
+struct F16Output {
+  float* out;             // [m][n]
+  float* second;          // with a second matrix: its rows
+  const float* residual;  // optional, added last (one matrix)
+  bool input_settled;     // as in TcOutput
+};
 bool f16_supported(const WeightView& w, const Q8View& x);
 F16Plan plan_f16(uint32_t m, uint32_t n, uint32_t tiles_k, bool pair = false);
 uint64_t f16_scratch_bytes(uint32_t m, uint32_t tiles_k, const F16Plan& plan);
-// second (plan with pair): another matrix of w's shape in the same launch, fp32 into out.out[1].
-cudaError_t launch_mmq_f16(const WeightView& w, const Q8View& x, const TcOutput& out, const F16Plan& plan, void* scratch, bool alternates,
+// second (plan with pair): another matrix of w's shape in the same launch.
+cudaError_t launch_mmq_f16(const WeightView& w, const Q8View& x, const F16Output& out, const F16Plan& plan, void* scratch, bool alternates,
                            int* status, cudaStream_t stream, const WeightView* second = nullptr, const RawRows* raw = nullptr);
 
 // gemv_tma.cu : m <= 16.  Weights streamed by TMA into a shared-memory ring, activations held in

@@ -119,12 +119,7 @@ template <int NT> struct F16Cfg {
 
 struct F16Params {
   const float* residual;
-  float* out[8];
-  uint16_t* out_bf16;
-  uint32_t* peer_flag[8];
-  uint32_t* done;
-  uint32_t* unsignalled;
-  uint32_t ndst, rank, out_stride, out_row0;
+  float* out[2];           // [1]: of the second matrix
   const float* exps;       // power of two of (super-block, token) relative to the token's: [kb][m_pad], 1 but for outliers
   const float* tokens;     // power of two of the token [m_pad]
   float* slots;            // partial tiles: [cluster][2][CTA][epilogue warp][value / 4][lane] float4
@@ -554,7 +549,6 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
     } else {
       pdl_wait();
       pdl_launch_dependents();
-      if (p.done != nullptr && blockIdx.x == 0 && lane == 0) announce_deliveries(p.unsignalled, p.peer_flag, p.ndst, p.rank);
     }
   } else if (warp < C::kFirstEpilogue) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kRegsExpander));
@@ -756,7 +750,8 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
       uint32_t const n_row = row_tile(c) * kRows + row, tok0 = c.tok * NT + col0;
       if (write && n_row < p.n && tok0 < p.m) {
         uint32_t const live = min(p.m - tok0, uint32_t(C::kCols));
-        uint64_t o = uint64_t(tok0) * p.out_stride + p.out_row0 + n_row;
+        float* const out = p.pair && cta ? p.out[1] : p.out[0];
+        uint64_t o = uint64_t(tok0) * p.n + n_row;
 #pragma unroll
         for (int j0 = 0; j0 < C::kCols; j0 += 8) {  // eight tokens at a time: eight residual loads in flight, few registers
           if (j0 >= live) break;
@@ -766,21 +761,12 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
           if (p.residual) {
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-              if (j0 + j < live) v[j] += p.residual[o + j * uint64_t(p.out_stride)];
+              if (j0 + j < live) v[j] += p.residual[o + j * uint64_t(p.n)];
           }
-          if (p.out_bf16) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-              if (j0 + j < live) p.out_bf16[o + j * uint64_t(p.out_stride)] = f32_to_bf16_rne(v[j]);
-          } else {
-            uint32_t const first = p.pair ? cta : 0u;
-            for (uint32_t g = first; g < first + p.ndst; ++g) {
-#pragma unroll
-              for (int j = 0; j < 8; ++j)
-                if (j0 + j < live) p.out[g][o + j * uint64_t(p.out_stride)] = v[j];
-            }
-          }
-          o += 8 * uint64_t(p.out_stride);
+          for (int j = 0; j < 8; ++j)
+            if (j0 + j < live) out[o + j * uint64_t(p.n)] = v[j];
+          o += 8 * uint64_t(p.n);
           asm volatile("" ::: "memory");
         }
       }
@@ -801,14 +787,6 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
   cluster_meet();  // neither CTA leaves while the other may still signal it or read its operands
   tc_fence_after();
   if (warp == 3) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
-  if (p.done != nullptr && threadIdx.x == 0) {
-    __threadfence();
-    uint32_t const old = atomicAdd(p.done, 1u);
-    if (old == gridDim.x - 1) {
-      *p.done = 0;
-      if (*reinterpret_cast<volatile int*>(p.status) == 0) atomicAdd(p.unsignalled, 1u);
-    }
-  }
 }
 
 // ------------------------------------------------------------------------------------------
@@ -836,7 +814,7 @@ Carve carve(uint32_t m, uint32_t tiles_k, const F16Plan& plan) {
 }
 
 template <int NT>
-cudaError_t launch_f16(const WeightView& w, const WeightView* second, const Q8View& x, const RawRows* raw, const TcOutput& o, const F16Plan& plan, uint8_t* scratch, bool early, int* status,
+cudaError_t launch_f16(const WeightView& w, const WeightView* second, const Q8View& x, const RawRows* raw, const F16Output& o, const F16Plan& plan, uint8_t* scratch, bool early, int* status,
                        cudaStream_t stream) {
   using C = F16Cfg<NT>;
   Carve const c = carve(x.m, w.tiles_k, plan);
@@ -885,14 +863,10 @@ cudaError_t launch_f16(const WeightView& w, const WeightView* second, const Q8Vi
       return cudaErrorInvalidValue;
   }
   F16Params p{};
-  p.residual = o.residual;
-  for (uint32_t g = 0; g < o.ndst; ++g) { p.out[g] = o.out[g]; p.peer_flag[g] = o.flags[g]; }
-  p.out_bf16 = o.out_bf16; p.done = o.done; p.unsignalled = o.unsignalled; p.ndst = o.ndst; p.rank = o.rank;
-  p.out_stride = o.stride ? o.stride : w.n; p.out_row0 = o.row0;
+  p.residual = o.residual; p.out[0] = o.out; p.out[1] = o.second;
   p.exps = reinterpret_cast<const float*>(scratch + c.exps); p.tokens = reinterpret_cast<const float*>(scratch + c.tokens); p.slots = reinterpret_cast<float*>(scratch + c.slots); p.tickets = reinterpret_cast<uint32_t*>(scratch);
   p.status = status; p.n = w.n; p.m = x.m; p.m_pad = m_pad; p.tiles_k = w.tiles_k; p.tok_tiles = m_pad / NT;
   p.pair = second ? 1u : 0u;
-  if (second) p.out[1] = o.out[1];
   uint32_t const steps = row_pairs(w.padded_n, second != nullptr) * p.tok_tiles * w.tiles_k / plan.unit_step;
   p.run_each = steps / plan.workers; p.run_rest = steps % plan.workers; p.unit_step = plan.unit_step;
   // setmaxnreg.inc waits for registers that the block must have been launched with: a build that allotted fewer than the
@@ -959,14 +933,10 @@ uint64_t f16_scratch_bytes(uint32_t m, uint32_t tiles_k, const F16Plan& plan) {
   return carve(m < plan.chunk ? m : plan.chunk, tiles_k, plan).total;
 }
 
-cudaError_t launch_mmq_f16(const WeightView& w, const Q8View& x, const TcOutput& out, const F16Plan& plan, void* scratch, bool alternates,
+cudaError_t launch_mmq_f16(const WeightView& w, const Q8View& x, const F16Output& out, const F16Plan& plan, void* scratch, bool alternates,
                            int* status, cudaStream_t stream, const WeightView* second, const RawRows* raw) {
-  if (second && (second->n != w.n || second->tiles_k != w.tiles_k || out.ndst != 1 || out.out_bf16 || out.residual || out.done || !out.out[1]))
-    return cudaErrorInvalidValue;
-  if (out.ndst < 1 || out.ndst > 8 || (out.out_bf16 ? out.ndst != 1 : out.out[0] == nullptr) || plan.workers < 1 ||
-      plan.workers > kMaxClusters)
-    return cudaErrorInvalidValue;
-  uint64_t const stride = out.stride ? out.stride : w.n;
+  if (second && (second->n != w.n || second->tiles_k != w.tiles_k || out.residual || !out.second)) return cudaErrorInvalidValue;
+  if (!out.out || plan.workers < 1 || plan.workers > kMaxClusters) return cudaErrorInvalidValue;
   bool const early = alternates && launch_overlap() && out.input_settled && x.m <= plan.chunk;
   for (uint32_t t0 = 0; t0 < x.m; t0 += plan.chunk) {
     Q8View xc = x;
@@ -976,11 +946,10 @@ cudaError_t launch_mmq_f16(const WeightView& w, const Q8View& x, const TcOutput&
     RawRows rows{};
     if (raw) { rows = *raw; rows.x += uint64_t(t0) * raw->k; }
     const RawRows* const rc = raw ? &rows : nullptr;
-    TcOutput oc = out;
-    for (uint32_t g = 0; g < (second ? 2 : out.ndst); ++g) if (oc.out[g]) oc.out[g] += t0 * stride;
-    if (oc.out_bf16) oc.out_bf16 += t0 * stride;
-    if (oc.residual) oc.residual += t0 * stride;
-    if (t0 + plan.chunk < x.m) oc.done = nullptr;  // row-sharded use: the projection counts once, with its last pass
+    F16Output oc = out;
+    oc.out += uint64_t(t0) * w.n;
+    if (second) oc.second += uint64_t(t0) * w.n;
+    if (oc.residual) oc.residual += uint64_t(t0) * w.n;
     F16Plan pc = plan;
     if (xc.m < plan.chunk) {  // a shorter last pass: fewer token tiles of the same width
       F16Plan const last = plan_f16(xc.m, w.n, w.tiles_k, second != nullptr);

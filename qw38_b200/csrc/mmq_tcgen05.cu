@@ -163,7 +163,6 @@ struct TcParams {
   const int32_t* xsums;    // and int32 sums
   const float* residual;   // same geometry as the destinations
   float* out[8];           // fp32 destinations: one buffer, or every rank's copy of a gathered output
-  uint16_t* out_bf16;      // when set, the single destination is bf16 (round to nearest even)
   uint32_t* peer_flag[8];  // gather only: rank g's arrival counters; [rank] counts this rank's deliveries
   uint32_t* done;          // gather only: block counter of this launch, zero on entry and on exit
   uint32_t* unsignalled;   // gather only: finished projections of this rank not yet announced to the peers
@@ -738,14 +737,10 @@ mmq_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_co
       auto store = [&](uint32_t token, uint32_t row, float v) {
         uint64_t const o = uint64_t(token) * p.out_stride + p.out_row0 + row;
         if (p.residual) v += p.residual[o];
-        if (p.out_bf16) {
-          p.out_bf16[o] = f32_to_bf16_rne(v);
-        } else {
-          p.out[0][o] = v;
+        p.out[0][o] = v;
 #pragma unroll
-          for (int g2 = 1; g2 < 8; ++g2)
-            if (g2 < int(p.ndst)) p.out[g2][o] = v;
-        }
+        for (int g2 = 1; g2 < 8; ++g2)
+          if (g2 < int(p.ndst)) p.out[g2][o] = v;
       };
       if (p.split_k == 1) {
         if (final_warp) {
@@ -858,7 +853,7 @@ cudaError_t launch_ntok(const WeightView& w, const Q8View& x, const TcOutput& o,
   for (uint32_t g = 0; g < 8; ++g) p.peer_flag[g] = g < o.ndst ? o.flags[g] : nullptr;
   p.done = o.done; p.unsignalled = o.unsignalled; p.rank = o.rank;
   for (uint32_t g = 0; g < 8; ++g) p.out[g] = g < o.ndst ? o.out[g] : nullptr;
-  p.out_bf16 = o.out_bf16; p.ndst = o.ndst; p.out_stride = o.stride ? o.stride : w.n; p.out_row0 = o.row0;
+  p.ndst = o.ndst; p.out_stride = o.stride ? o.stride : w.n; p.out_row0 = o.row0;
   p.partials = partials; p.partial_tiles = partial_tiles; p.tickets = tickets; p.status = status;
   p.input_settled = o.input_settled;
   p.n = w.n; p.m = x.m; p.tiles_k = w.tiles_k; p.split_k = split_k; p.G = uint32_t(G); p.row_tiles = row_tiles; p.tok_tiles = tok_tiles;
@@ -910,7 +905,7 @@ TcPlan plan_tcgen05(uint32_t m, uint32_t n, uint32_t tiles_k, uint32_t split_k_r
 cudaError_t launch_mmq_tcgen05(const WeightView& w, const Q8View& x, const TcOutput& out, int32_t* partials,
                                const TcPlan& plan, void* partial_tiles, uint32_t* tickets, int* status, cudaStream_t stream) {
   float* pt = static_cast<float*>(partial_tiles);
-  if (out.ndst < 1 || out.ndst > 8 || (out.out_bf16 ? out.ndst != 1 : out.out[0] == nullptr)) return cudaErrorInvalidValue;
+  if (out.ndst < 1 || out.ndst > 8 || out.out[0] == nullptr) return cudaErrorInvalidValue;
   switch (plan.ntok) {
     case 16:
       if (x.m <= 8) return launch_ntok<16, 8>(w, x, out, partials, plan.split_k, pt, tickets, status, stream);

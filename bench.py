@@ -656,37 +656,39 @@ def single_gpu_extras(torch, lib, L, synth, dev, stream, g, failure, peaks, hbm_
                                "peak_source": "measured" if int8_peak else "unavailable",
                                "ops": "2*M*N*K per launch; time by CUDA events over 10 launches"}
 
-    # ---- offline step of the same path: bf16 weights -> split-tile Q4_K on the device, and back to bf16
+    # ---- offline step of the same path: bf16 weights -> split-tile Q4_K on the device, and back to bf16.  The loops above end at
+    # the power limit: the device rests first, and each loop lasts long enough for clock samples of its own.
+    def sampled(fn, reps):
+        torch.cuda.synchronize()
+        time.sleep(1.0)
+        sampler = ClockSampler(dev.index or 0)
+        sampler.start()
+        time.sleep(0.3)
+        with torch.cuda.stream(stream):
+            for _ in range(3):
+                fn()
+            t0 = time.time()
+            e0.record(stream)
+            for _ in range(reps):
+                fn()
+            e1.record(stream)
+        stream.synchronize()
+        return e0.elapsed_time(e1) / reps, sampler.stop(t0, time.time())
+
     n, k = 5120, 17408
     wf = (torch.randn((n, k), device=dev, generator=g) * 0.02).to(torch.bfloat16)
-    with torch.cuda.stream(stream):
-        for _ in range(2):
-            quantize_q4k_weight(wf, check=False)
-        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        e0.record(stream)
-        for _ in range(5):
-            quantize_q4k_weight(wf, check=False)
-        e1.record(stream)
-    stream.synchronize()
-    t = e0.elapsed_time(e1) / 5
+    t, clk = sampled(lambda: quantize_q4k_weight(wf, check=False), 400)
     fitter = {"workload": f"fit bf16 {n}x{k} -> split-tile Q4_K", "ms": round(t, 3), "kernel": "fit_q4k_kernel",
-              "Mblocks_per_s": round(n * k / 256 / (t * 1e-3) / 1e6, 1)}
+              "Mblocks_per_s": round(n * k / 256 / (t * 1e-3) / 1e6, 1), "clocks": clk}
     pw = quantize_q4k_weight(wf, check=False)
     del wf
     deq = torch.empty((n, k), dtype=torch.bfloat16, device=dev)
     ws = pw.c_struct()
-    with torch.cuda.stream(stream):
-        for _ in range(3):
-            lib.q4k_dequantize_bf16(ctypes.byref(ws), ctypes.c_void_p(deq.data_ptr()), deq.numel(), ctypes.c_void_p(stream.cuda_stream))
-        e0.record(stream)
-        for _ in range(20):
-            lib.q4k_dequantize_bf16(ctypes.byref(ws), ctypes.c_void_p(deq.data_ptr()), deq.numel(), ctypes.c_void_p(stream.cuda_stream))
-        e1.record(stream)
-    stream.synchronize()
-    t = e0.elapsed_time(e1) / 20
+    t, clk = sampled(lambda: lib.q4k_dequantize_bf16(ctypes.byref(ws), ctypes.c_void_p(deq.data_ptr()), deq.numel(),
+                                                     ctypes.c_void_p(stream.cuda_stream)), 8000)
     nbytes = pw.nbytes() + deq.numel() * 2
     fitter["dequantize_bf16"] = {"ms": round(t, 4), "kernel": "dequantize_bf16_kernel", "GBps": round(nbytes / (t * 1e-3) / 1e9, 1),
-                                 "frac_of_hbm_peak": round(nbytes / (t * 1e-3) / 1e9 / hbm_peak, 4), "bytes": nbytes}
+                                 "frac_of_hbm_peak": round(nbytes / (t * 1e-3) / 1e9 / hbm_peak, 4), "bytes": nbytes, "clocks": clk}
     out["fitter"] = fitter
     return out
 

@@ -526,7 +526,7 @@ def main():
 
 
 def verify_against_oracle(torch, dist, world, rank, last_layer, q8, outs, shard, tokens):
-    """Sampled rows of the gathered outputs of the last layer against the CPU restatement (the checker, not the thing
+    """Sampled rows of the gathered outputs of the last layer against the CPU restatement (the oracle, not the thing
     measured): each rank computes the reference for two 8-row groups of its own shard of every matrix, the references
     are exchanged, and every rank compares ALL of them with its own copy of the gathered output."""
     from oracle import oracle as orc

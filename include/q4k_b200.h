@@ -91,9 +91,9 @@ typedef struct q4k_project_options {
 #define Q4K_FLAG_TRUSTED_SPANS 1u
 /* With launch overlap on (q4k_set_launch_overlap): the activations (codes, scales, sums) and the residual of this
  * call were NOT written by the launch directly before it on the stream -- they were complete before that launch
- * was enqueued.  The tcgen05 kernel (m > 16) then starts on SMs the preceding launch leaves idle and computes
- * while it drains, waiting for it only before its first store; without the flag it prefetches weights and waits
- * before it reads activations.  Every kernel of this library lets its successor start only once its own
+ * was enqueued.  The dp4a, TMA and int8 tcgen05 kernels then compute while it drains and wait for it only before their
+ * first store; the fp16-plane kernel, in a captured call, writes its operand planes beside it.  Without the flag they
+ * prefetch weights and wait before they read activations.  Every kernel of this library lets its successor start only once its own
  * predecessor has completed, so "not the launch directly before" is all the caller has to know. */
 #define Q4K_FLAG_INPUT_SETTLED 2u
 
@@ -109,7 +109,8 @@ uint32_t q4k_abi_version(void);
  * ResidualAddFp32 reads `residual` and writes `output`, or updates `residual` in place when `output` is NULL;
  * SwigluStoreBf16 needs the paired call, whose B side declares no output and shares A's input.
  * The reference's own Bf16 policy (weights reconstructed in fp32 and rounded to bf16, fp32 FMA with the bf16
- * activations, cuda/decode_mmv.cu:121-250) is accepted on the three decode entries as well. */
+ * activations, cuda/decode_mmv.cu:121-250) is accepted on the three decode entries as well.  Under the
+ * Q8-K32 policy an output may lie over the input; such a call quantises the input in a launch of its own first. */
 #define Q4K_EPILOGUE_STORE_BF16 1
 #define Q4K_EPILOGUE_STORE_FP32 2
 #define Q4K_EPILOGUE_RESIDUAL_ADD_FP32 3
@@ -230,9 +231,10 @@ void q4k_set_launch_overlap(int enabled);
 int q4k_get_launch_overlap(void);
 
 /* Synchronises the current device and reads the status word shared by the kernels that wait on
- * device-side barriers (tcgen05, TMA gemv, peer wait): 0 = every launch so far ran to completion;
- * nonzero = a bounded wait gave up at that site (0x5xx TMA gemv, 0x610 peer wait, 0x71x the int8
- * peak measurement, others tcgen05) and the affected block returned without writing its outputs.
+ * device-side barriers (dp4a, TMA gemv, tcgen05, peer wait): 0 = every launch so far ran to completion;
+ * nonzero = a bounded wait gave up at that site (0x110 dp4a, 0x5xx TMA gemv, 0x610 peer wait, 0x71x the int8
+ * peak measurement, 0x8xx the fp16-plane kernel, others int8 tcgen05) and the affected block returned without
+ * writing its outputs.
  * The word is a static device variable of the library (one per device, no allocation), whatever
  * scratch the launches used.  A nonzero word is cleared by the read, and the arrival counters of the
  * library-owned split-K scratch are zeroed with it (a launch that gave up may have left some behind;

@@ -242,7 +242,21 @@ int caller_scratch(const q4k_project_options* opt, uint64_t partial_bytes, uint6
 constexpr uint32_t kFlagTrustedSpans = 1u, kFlagInputSettled = 2u;
 
 // The fp16-plane kernel with scratch of its own (stream_scratch.cu).
-constexpr uint64_t kF16SuperBlocks = 16384;  // of eight rows; below, nine to sixteen tokens stay with the TMA-streamed kernel
+// Nine to sixteen tokens: from this many super-blocks of eight rows on.  The TMA-streamed kernel against this one, us, replayed
+// graph over matrices that do not fit L2, launches serialised / overlapped with settled inputs:
+//                                 nine tokens                  sixteen tokens
+//   5120 x 5120   (12800)   14.6 : 15.5 / 10.9 : 10.9    16.0 : 15.6 / 11.8 : 10.9
+//   6144 x 5120   (15360)   16.2 : 16.8 / 12.1 : 11.9    17.3 : 16.8 / 12.9 : 11.9
+//   6656 x 5120   (16640)   16.4 : 17.0 / 12.7 : 12.4    17.7 : 16.9 / 13.6 : 12.5
+//   7168 x 5120   (17920)   17.5 : 16.9 / 13.2 : 12.3    19.0 : 16.9 / 14.4 : 12.4
+//   10240 x 5120  (25600)   20.9 : 19.6 / 17.0 : 14.8    22.4 : 19.7 / 18.3 : 14.8
+//   13312 x 2560  (16640)   14.1 : 14.7 / 11.4 : 10.7    14.3 : 14.7 / 11.5 : 10.8
+//   2048 x 17408  (17408)   17.4 : 19.1 / 12.0 : 14.6    19.7 : 19.4 / 12.8 : 14.8
+//   2560 x 17408  (21760)   19.5 : 20.0 / 14.1 : 15.6    21.4 : 20.4 / 15.6 : 15.7
+// Its time hardly depends on the token count (a tile is sixteen wide), the other's does; twelve tokens lie between.  At K = 5120
+// the line is where nine serialised tokens break even, to 4 % either way.  Few rows of a long K (each of its tiles then cut over
+// many clusters) lose up to 20 % just above the line, and gain from about 2560 rows on.
+constexpr uint64_t kF16SuperBlocks = 16384;
 int project_f16(const q4k_weight& w, const q4k_q8_input& x, const q4k::F16Output& out, cudaStream_t stream, const q4k_weight* second = nullptr,
                 const q4k::RawRows* raw = nullptr) {
   int* const status = q4k::kernel_status_word();
@@ -286,13 +300,16 @@ int project_impl(const q4k_weight* weight, const q4k_q8_input& x, float* output,
 
   uint32_t kernel = opt ? opt->kernel : Q4K_KERNEL_AUTO;
   if (kernel == Q4K_KERNEL_AUTO) {
-    // One token: dp4a (5120 x 5120 to 34816 x 5120 in 5.1 .. 17.3 us, the TMA-streamed kernel 6.5 .. 22.5; two tokens
-    // 6.1 .. 21.7 against 6.7 .. 22.4, and slower in a chain of layers).  Up to sixteen: the TMA-streamed kernel when the
-    // weights are 16-byte aligned, else dp4a / cluster MMA.  Beyond: tcgen05 when TMA alignment allows.
+    // One token: dp4a.  Up to sixteen: the TMA-streamed kernel when the weights are 16-byte aligned, else dp4a / cluster MMA.
+    // Beyond: fp16 planes (int8 tcgen05 for partial dots) when TMA alignment allows.  dp4a : TMA-streamed, us, replayed graph over matrices that do not fit L2,
+    // serialised / overlapped with settled inputs:
+    //                       one token                   two tokens
+    //   5120 x 5120     7.6 :  9.0 /  5.4 :  6.1     8.4 :  9.1 /  6.1 :  6.2
+    //   7168 x 5120     8.7 : 10.1 /  6.2 :  7.6     9.9 : 10.7 /  7.0 :  7.7
+    //   34816 x 5120   22.9 : 24.3 / 17.5 : 22.5    27.7 : 24.5 / 21.8 : 22.7
+    //   5120 x 17408   14.6 : 18.1 / 11.3 : 14.9    18.2 : 17.9 / 14.5 : 15.2
+    // Two tokens in a graph of whole layers were slower on dp4a (eight layers 546 us against 477).
     bool const tma_ok = x.m <= q4k::kGemvTmaMaxTokens && q4k::gemv_tma_supported(view(w), view(x));
-    // From nine tokens on the fp16 kernel spends 13.7 us on anything (its planes, its tile ends) but then gains: 16 x 34816 x
-    // 5120 34 us against 44, 17408 x 5120 22 / 28, 5120 x 17408 25 / 31, 7168 x 5120 16 / 17 (nine tokens: 16 / 15.5, and
-    // 12.6 / 13.3 with overlapped launches); 5120 x 5120 13.8 / 13.2 .. 14.6.
     bool const whole_dots = !partials && !(opt && (opt->split_k || opt->row_groups));
     if (x.m > 8 && x.m <= 16 && whole_dots && w.padded_n / 8 * (w.padded_k / 256) >= kF16SuperBlocks && q4k::f16_supported(view(w), view(x)))
       kernel = Q4K_KERNEL_F16;

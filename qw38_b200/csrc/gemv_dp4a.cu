@@ -22,9 +22,10 @@
 //     the next one start, while the others already work when the caller flagged the input as settled.
 // Activations are staged once per block as (even bytes, odd bytes) words, or quantised right there from bf16 rows (Raw).
 //
-// One token, overlapped launches, us: 5120 x 5120 5.0 (the TMA tile kernel 6.5), 7168 x 5120 6.1 (8.0), 5120 x 17408 11.4
-// (15.3), 34816 x 5120 17.3 = 5.8 TB/s (22.4); eight layers of all four 394 (472).  Slower: sixteen-row steps whose lanes
-// share the activation loads (20.1 on the last shape), eleven to seventeen warps, thirty warps in one block per SM.
+// One token, us, matrices that do not fit L2 in a replayed graph, overlapped launches with settled inputs (the TMA tile kernel in
+// brackets): 5120 x 5120 5.4 (6.1), 7168 x 5120 6.2 (7.6), 5120 x 17408 11.3 (14.9), 34816 x 5120 17.5 = 5.7 TB/s (22.5); eight
+// layers of all four 394 (472).  Slower: sixteen-row steps whose lanes share the activation loads (20.1 on 34816 x 5120), eleven
+// to seventeen warps, thirty warps in one block per SM.
 #include "common.cuh"
 #include "launch.h"
 #include "q8_pack.cuh"

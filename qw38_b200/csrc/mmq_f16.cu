@@ -828,6 +828,9 @@ cudaError_t launch_f16(const WeightView& w, const WeightView* second, const Q8Vi
   cudaError_t st;
   if (raw) {
     bool const vec = raw->k % 8 == 0 && reinterpret_cast<uintptr_t>(raw->x) % 16 == 0;
+    // Few registers keep more rows in flight, but a row has to fit: three super-blocks per warp up to K = 6144, nine up to
+    // 18432, sixteen for the largest K.  2048 rows with a matmul of 128 rows behind them, us, for three / nine / sixteen:
+    // K = 2048 23.0 / 24.3 / 29.5, 5120 34.1 / 35.3 / 42.8, 17408 - / 133 / 146.
     auto kernel = w.tiles_k <= 24 ? rows_planes_kernel<3> : (w.tiles_k <= 72 ? rows_planes_kernel<9> : rows_planes_kernel<16>);
     if (w.tiles_k > 128) return cudaErrorInvalidValue;
     st = launch_kernel(kernel, m_pad, 256, 0, stream, launch_overlap(), raw->x, raw->k, vec, raw->failure, x.m, m_pad, w.tiles_k, planes, sums,

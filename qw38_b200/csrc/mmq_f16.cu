@@ -30,9 +30,10 @@
 // delivers about 10 TB/s to all of them.
 //
 // Measured on 17408 x 5120: 2048 tokens 0.57 ms (635 TOP/s; the int8 kernel 1.20 ms) at the power limit, 1024 tokens with the
-// tensor pipe 86 % active; 64 tokens x 34816 rows 47 us (95 us), of which about 10 us are launch, prologue and tile end.
-// Bound: at prefill sizes tensor pipe and power, below 64 tokens the hand-offs between the roles (barrier to barrier a
-// super-block takes ~1.4x its tensor time).  Tried and slower: a back-off in the waits (nanosleep 16 .. 128: 1.5 - 2x), a
+// tensor pipe 86 % active; 64 tokens x 34816 rows 42.6 us (int8 95 us), x 5120 rows 16.2 us, of which about 4 us of work.
+// Bound: at prefill sizes tensor pipe and power; at 64 tokens what L2 delivers (51 KB per SM and super-block at 35 bytes per
+// clock) and, in long runs, power; below, the instruction streams of the expanders, and in every short call the start (planes
+// kernel, first copies) and the end (partial tiles through L2).  Tried and slower: a back-off in the waits (nanosleep 16 .. 128: 1.5 - 2x), a
 // suspend hint, a four-instruction retry loop (1.5x: the retries queue up in front of the arrivals), one polling lane or
 // one polling warp per role, arrivals with cluster-scope release (a memory barrier each: 1.4x), the min term on mma.sync
 // (queues behind the tcgen05 MMAs: 1.16x).  Faster but less exact: lo and hi products alternating per weight stage (5 %, and
@@ -45,8 +46,8 @@
 // Two matrices of one shape over the same tokens (gate and up) go as one launch: each SM of a pair takes the rows of one of
 // them.  That is one set of planes, one prologue and one last wave instead of two.
 //
-// Warps: 0 raw weights (TMA), 1 activation planes (TMA), 2 MMA issue (leader CTA), 3 TMEM allocation and launch overlap,
-// then expanders, then epilogue.  Every wait is bounded; a wait that gives up sets the abort flag and the status word, and
+// Warps: 0 raw weights (TMA), 1 activation planes (TMA) and launch overlap, 2 and 3 MMA issue (leader CTA; 3 also allocates
+// TMEM), then expanders, then epilogue.  Every wait is bounded; a wait that gives up sets the abort flag and the status word, and
 // every role leaves its loop.
 #include <cuda.h>
 #include <cuda_fp16.h>
@@ -72,11 +73,11 @@ template <int NT> struct F16Cfg {
   static constexpr bool kStack = NT <= 32;
   static constexpr int kN = kStack ? 2 * NT : NT;       // MMA width = accumulator columns
   static constexpr int kN2 = NT < 32 ? 32 : NT;         // min-term accumulator columns
-  static constexpr int kColSplit = NT >= 128 ? 4 : (NT >= 32 ? 2 : 1);
+  static constexpr int kColSplit = NT >= 128 ? 4 : (NT >= 64 ? 2 : 1);
   static constexpr int kCols = NT / kColSplit;          // tokens per epilogue warp (lane = row)
   static constexpr int kEpilogueWarps = 4 * kColSplit;
-  // Expanders: groups take alternate super-blocks; within a group four warps (one per TMEM lane quarter) times kSplit halves
-  // of K.  Few warps with long instruction streams: every warp more is another one that retries its waits.
+  // Expanders: groups take super-blocks in turn; within a group four warps (one per TMEM lane quarter) times kSplit halves of K.
+  // Few warps with long instruction streams: every warp more is another one that retries its waits.
   static constexpr int kGroups = NT >= 128 ? 1 : 2, kSplit = NT >= 128 ? 2 : 1, kExpanders = 4 * kSplit;
   static constexpr int kFirstEpilogue = kFirstExpander + kGroups * kExpanders;
   static constexpr int kWarps = kFirstEpilogue + kEpilogueWarps, kThreads = kWarps * 32;
@@ -84,16 +85,16 @@ template <int NT> struct F16Cfg {
   // Up to 64 tokens two warps' worth stays free: a block of planes_kernel for the next projection fits beside this one.
   static constexpr int kBoundThreads = NT >= 128 ? kThreads : kThreads + 64;
   static constexpr int kLaunchRegs = 65536 / ((kBoundThreads + 127) / 128 * 128) / 8 * 8;  // what ptxas gives (checked before the first launch)
-  static constexpr int kRegsControl = 40, kRegsExpander = kSplit == 2 ? 56 : 72;
+  static constexpr int kRegsControl = 40, kRegsExpander = kSplit == 2 ? 56 : 64;
   static constexpr int kRegsLeft = (kWarps * kLaunchRegs - 4 * kRegsControl - kGroups * kExpanders * kRegsExpander) / kEpilogueWarps / 8 * 8;
   static constexpr int kRegsEpilogue = kRegsLeft > 160 ? 160 : kRegsLeft;
-  // TMEM: two accumulators, one min-term accumulator, weight stages.  A group of expanders always uses the same kQ stages
-  // (one super-block), so that a warp sees every phase of the barriers it waits on.  At 128 tokens there is room for one
-  // super-block only, and a stage is refilled between its last use and the next super-block's first: 7/16 of a super-block's
-  // time with eight stages (3/8 with four), half the work per stage, and the words are computed before the wait (kReady).
+  // TMEM: two accumulators, one or two for the min term, weight stages.  A group of expanders always uses the same kQ stages
+  // (one super-block), so that a warp sees every phase of the barriers it waits on.  (Four groups with half a super-block each, up
+  // to 32 tokens, were slower: the second half is then expanded between the two halves' products.)  At 128 tokens there is room
+  // for one super-block only, and a stage is refilled between its last use and the next super-block's first: 7/16 of a
+  // super-block's time with eight stages (3/8 with four), half the work per stage.
   // 256 tokens x 17408 x 5120 78 -> 75 us, 2048 x 5120 x 17408 670 -> 630, 2048 x 17408 x 5120 (at the power limit) 585 -> 575.
   static constexpr int kQ = kStack ? 2 : (NT >= 128 ? 8 : 4), kACols = 128 / kQ, kAStages = kGroups * kQ;
-  static constexpr bool kReady = kQ == 8;
   static constexpr int kD2Bufs = NT <= 64 ? 2 : 1;  // with one, the min-term MMA waits for the previous super-block's epilogue
   static constexpr int kD2Col = 2 * kN, kACol = kD2Col + kD2Bufs * kN2;
   static_assert(kACol + kAStages * kACols <= 512, "TMEM columns");
@@ -104,14 +105,16 @@ template <int NT> struct F16Cfg {
   static constexpr int kTRows = kN2 / 2;
   static constexpr int kBTx = kPlanes + kTRows * 32, kB = (kBTx + 1023) / 1024 * 1024;
   static constexpr int kRaw = 16 * 1024 + 16 * 128;
-  static constexpr int kBStages = NT >= 128 ? 2 : (NT >= 64 ? 3 : 4);  // any number: one producer, one consumer
-  static constexpr int kRawStages = NT >= 128 ? 3 : 6, kSclStages = NT >= 128 ? 3 : 4;
-  static_assert(kRawStages % kGroups == 0 && kSclStages % kGroups == 0, "a stage belongs to one group of expanders");
+  // Threads that issue MMAs, on alternate super-blocks.
+  static constexpr int kIssuers = kGroups == 2 ? 2 : 1;
+  static constexpr int kBStages = NT >= 128 ? 2 : 4, kRawStages = NT >= 128 ? 3 : (NT >= 64 ? 4 : 6), kSclStages = NT >= 128 ? 3 : 4;
+  static_assert(kRawStages % kGroups == 0 && kSclStages % kGroups == 0 && kGroups % kIssuers == 0 && kBStages % kIssuers == 0,
+                "a stage belongs to one group of expanders and one issuer: whoever waits for a phase has to see every one");
   static constexpr int kMins = kRows * 16;              // six-bit mins as fp16, one buffer per group
   static constexpr int oE = kRows * 8, kScl = oE + NT * 4;  // scale stage: {d, -32 dmin} [row] | 2^e [token]
   static constexpr int oB = 0, oRaw = oB + kBStages * kB, oMins = oRaw + kRawStages * kRaw, oScl = oMins + kGroups * kMins,
                        oCtrl = oScl + kSclStages * kScl;
-  static constexpr int kBars = 2 * kRawStages + 2 * kBStages + 2 * kAStages + 4 + 2 * kSclStages;
+  static constexpr int kBars = 2 * kRawStages + 2 * kBStages + 2 * kAStages + 4 + 2 * kSclStages + 1;
   static constexpr int kSmem = oCtrl + kBars * 8 + 32 + 1024;
   static_assert(kSmem <= 227 * 1024, "shared memory budget");
   static_assert(kRaw % 1024 == 0 && kScl % 64 == 0, "swizzled tiles need 1024-byte alignment");
@@ -184,13 +187,11 @@ __device__ __forceinline__ void arrive_cluster(uint32_t cluster_addr) {
 // and acquire forms of the barrier instructions took 16 to 20 % at 128 tokens, 9 % at 64).
 __device__ __forceinline__ void release_shared() { asm volatile("fence.release.sync_restrict::shared::cta.cluster;" ::: "memory"); }
 __device__ __forceinline__ void acquire_shared() { asm volatile("fence.acquire.sync_restrict::shared::cluster.cluster;" ::: "memory"); }
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// Execution only: no wait for the block's outstanding stores.
-__device__ __forceinline__ void cluster_meet() {
-  asm volatile("barrier.cluster.arrive.relaxed.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
-}
+// Execution only: no wait for what the block has in flight (an arrival with release semantics waited for the first copies of
+// weights from HBM, 3400 clk of every launch; the barriers' initialisation has a fence of its own).
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* map) { asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory"); }
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{ .reg .pred q; elect.sync _|q, 0xffffffff; selp.u32 %0, 1, 0, q; }" : "=r"(p));
@@ -416,6 +417,7 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
   constexpr int oSb = oDb + 4;
   auto s_full = [&](uint32_t i) { return bar0 + 8 * (oSb + i); };
   auto s_free = [&](uint32_t i) { return bar0 + 8 * (oSb + C::kSclStages + i); };
+  uint32_t const first_planes = bar0 + 8 * (oSb + 2 * C::kSclStages);
   uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(smem_g + C::oCtrl + C::kBars * 8);
   volatile int* const abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -423,8 +425,11 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
   uint32_t const u0 = first_unit(p, worker), u1 = first_unit(p, worker + 1);
   uint32_t const KB = p.tiles_k;
 
-  // Raw weights are never written by an earlier launch, so they stream before any wait; the first ring of them even
-  // before the block has met.
+  // Raw weights are never written by an earlier launch, so they stream before any wait, the first stages while the cluster meets.
+  // Copies of an SM are served in order and all SMs start at once: behind a whole ring of weights the first planes came 2.5 us
+  // after they were asked for.  So the ring's other stages follow them, unless the wait for the kernel that writes the planes is
+  // longer than the fill.
+  constexpr uint32_t kEarlyRaw = 2;
   const CUtensorMap* const codes_map = p.pair && cta ? &tm_codes1 : &tm_codes;
   const CUtensorMap* const meta_map = p.pair && cta ? &tm_meta1 : &tm_meta;
   auto row_tile = [&](const Cursor& c) { return p.pair ? c.row_pair : c.row_pair * 2 + cta; };
@@ -441,17 +446,18 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
       if (i >= C::kRawStages && i < oBb) count = C::kExpanders;                                   // raw_free
       else if (i >= oAb && i < oAb + C::kAStages) count = 2 * 4;                                  // a_full: four warps of both CTAs
       else if (i >= oDb + 2 && i < oSb) count = 2 * C::kEpilogueWarps;                            // d_free
-      else if (i >= oSb) count = i < oSb + C::kSclStages ? 4 + 1 : C::kEpilogueWarps;  // s_full | s_free
+      else if (i >= oSb && i < oSb + 2 * C::kSclStages) count = i < oSb + C::kSclStages ? 4 + 1 : C::kEpilogueWarps;  // s_full | s_free
       mbar_init(bar0 + 8 * i, count);
     }
     if (lane == 0) *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncwarp();
-    if (lane == 0) {
-      Cursor c(p, u0);
-      for (uint32_t i = 0; i < C::kRawStages && u0 + i < u1; ++i, c.next(p)) load_raw(c, i);
-    }
+  }
+  if (warp == 1 && lane == 0) {
+    prefetch_map(codes_map);
+    prefetch_map(meta_map);
+    prefetch_map(&tm_planes);
+    prefetch_map(&tm_sums);
   }
   if (warp == 3) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_slot)) : "memory");
@@ -459,19 +465,26 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
   }
   tc_fence_before();
   __syncthreads();
-  cluster_sync();  // the peer's barriers exist before anything is signalled across
+  cluster_arrive();
+  if (warp == 0 && lane == 0) {
+    Cursor c(p, u0);
+    for (uint32_t i = 0; i < kEarlyRaw && u0 + i < u1; ++i, c.next(p)) load_raw(c, i);
+  }
+  __syncwarp();
+  cluster_wait();  // the peer's barriers exist before anything is signalled across
   tc_fence_after();
   uint32_t const tmem = *tmem_slot;
 
   if (warp < kFirstExpander) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kRegsControl));
     if (warp == 0) {
-      // ---- raw weights beyond the first ring
-      if (lane == 0 && u1 - u0 > C::kRawStages) {
-        Cursor c(p, u0 + C::kRawStages);
+      // ---- raw weights beyond the first stages
+      if (lane == 0 && u1 - u0 > kEarlyRaw) {
+        for (long long const t0 = clock64(); !mbar_test(first_planes, 0) && clock64() - t0 < 2000;) {}
+        Cursor c(p, u0);
         Ring<C::kRawStages> r;
-        r.phase = 1;
-        for (uint32_t u = u0 + C::kRawStages; u < u1; ++u, c.next(p), r.next()) {
+        for (uint32_t i = 0; i < kEarlyRaw; ++i) { c.next(p); r.next(); }
+        for (uint32_t u = u0 + kEarlyRaw; u < u1; ++u, c.next(p), r.next()) {
           if (!mbar_wait_inline(raw_free(r.s), r.phase ^ 1, abort_flag, p.status, 0x801)) break;
           load_raw(c, r.s);
         }
@@ -480,6 +493,7 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
       // ---- activation planes and a*s (both CTAs' halves are counted on the leader's barrier), 2^e of the tile
       if (lane == 0) {
         pdl_wait();
+        pdl_launch_dependents();
         Cursor c(p, u0);
         Ring<C::kBStages> b;
         Ring<C::kSclStages> t;
@@ -499,16 +513,22 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
           if (!mbar_wait_inline(s_free(t.s), t.phase ^ 1, abort_flag, p.status, 0x803)) break;
           mbar_expect_tx(s_full(t.s), NT * 4);
           bulk_copy(smem + C::oScl + t.s * C::kScl + C::oE, p.exps + uint64_t(c.kb) * p.m_pad + c.tok * NT, NT * 4, s_full(t.s));
+          if (u == u0) mbar_arrive(first_planes);
         }
       }
-    } else if (warp == 2) {
-      // ---- MMA issue
-      if (cta == 0 && elect_one()) {
+    } else {
+      // ---- MMA issue: up to 64 tokens two warps take alternate super-blocks.  Of one thread's time a super-block is 33 MMAs of
+      // 20 clk, six commits of 45 and six waits of 70 to 100 even where what they wait for is there: 1500 clk at 64 tokens, where
+      // the tensor pipe needs 1150.
+      if (cta == 0 && warp - 2 < C::kIssuers && elect_one()) {
         Cursor c(p, u0);
         Ring<C::kBStages> b_;
         Ring<C::kGroups> g_;
         Ring<2> d_, before;
-        for (uint32_t u = u0; u < u1; ++u, c.next(p), b_.next(), g_.next(), before = d_, d_.next()) {
+        auto next = [&] { c.next(p); b_.next(); g_.next(); before = d_; d_.next(); };
+        auto turn = [&] { next(); if (C::kIssuers == 2) next(); };
+        if (warp == 3) next();
+        for (uint32_t u = u0 + (warp - 2); u < u1; u += C::kIssuers, turn()) {
           uint32_t const cols = tile_cols<NT>(p, c.tok);
           uint32_t const idesc = f16_idesc(cols * (C::kStack ? 2 : 1)), idesc2 = f16_idesc(round32(cols));
           uint32_t const dt = tmem + d_.s * C::kN, stage = smem + C::oB + b_.s * C::kB, a0 = g_.s * C::kQ;
@@ -518,16 +538,17 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
 #pragma unroll
           for (int step = 0; step < C::kQ * (C::kStack ? 1 : 2); ++step) {
             int const pass = step / C::kQ, q = step % C::kQ;
-            bool const last = C::kStack || pass == 1;  // the stage's last use
-            if (pass == 0 && q < C::kQ - 1) ok = ok && mbar_wait_inline(a_full(a0 + q), g_.phase, abort_flag, p.status, 0x806);
-            if (pass == 0 && q == C::kQ - 1) {  // the last stage comes with both CTAs' mins
-              ok = ok && mbar_wait_inline_relaxed_cluster(a_full(a0 + q), g_.phase, abort_flag, p.status, 0x806);
+            uint32_t const stage_q = a0 + q;
+            bool const last = C::kStack || pass == 1, end = q == C::kQ - 1;  // the stage's last use, the pass's last stage
+            if (pass == 0 && !end) ok = ok && mbar_wait_inline(a_full(stage_q), g_.phase, abort_flag, p.status, 0x806);
+            if (pass == 0 && end) {  // the last stage comes with both CTAs' mins
+              ok = ok && mbar_wait_inline_relaxed_cluster(a_full(stage_q), g_.phase, abort_flag, p.status, 0x806);
               acquire_shared();
             }
-            if (C::kD2Bufs == 1 && last && q == C::kQ - 1 && u > u0) ok = ok && mbar_wait_inline(d_free(before.s), before.phase, abort_flag, p.status, 0x807);
+            if (C::kD2Bufs == 1 && last && end && u > u0) ok = ok && mbar_wait_inline(d_free(before.s), before.phase, abort_flag, p.status, 0x807);
             if (!ok) break;
             tc_fence_after();
-            uint32_t const at = tmem + C::kACol + (a0 + q) * C::kACols;
+            uint32_t const at = tmem + C::kACol + stage_q * C::kACols;
             constexpr int kSteps = 16 / C::kQ;
 #pragma unroll
             for (int i = 0; i < kSteps; ++i) {
@@ -536,19 +557,16 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
               if (pass == 0 && k == 0) mma_pair<false>(dt, at, b, idesc);
               else mma_pair<true>(dt, at + i * 8, b, idesc);
             }
-            if (last && q == C::kQ - 1)  // m * (a*s): sixteen K columns = eight groups, hi and lo; the mins serve both (K stride 0)
+            if (last && end)  // m * (a*s): sixteen K columns = eight groups, hi and lo; the mins serve both (K stride 0)
               mma_pair_ss(tmem + C::kD2Col + (C::kD2Bufs - 1) * d_.s * C::kN2, umma_desc_plain(smem + C::oMins + g_.s * C::kMins, 0, 128),
                           umma_desc_plain(stage + C::kPlanes, C::kTRows * 16, 128), idesc2);
-            if (last) commit_pair(a_free(a0 + q));
+            if (last) commit_pair(a_free(stage_q));
           }
           if (!ok) break;
           commit_pair(b_free(b_.s));
           commit_pair(d_full(d_.s));
         }
       }
-    } else {
-      pdl_wait();
-      pdl_launch_dependents();
     }
   } else if (warp < C::kFirstEpilogue) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kRegsExpander));
@@ -558,7 +576,7 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
     uint32_t const a_full0 = map_to(a_full(0), 0);
     Ring<C::kRawStages> r_;
     Ring<C::kSclStages> t_;
-    if (group == 1) { r_.next(); t_.next(); }
+    for (uint32_t i = 0; i < group; ++i) { r_.next(); t_.next(); }
     uint32_t const low = opaque(0x000f000fu), high = opaque(0x00f000f0u), magic = opaque(0x64006400u);
     uint32_t phase = 0;
     bool ok = true;
@@ -568,9 +586,8 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
       uint32_t const raw = smem + C::oRaw + r * C::kRaw;
       uint4 const cm = lds128(raw + 16 * 1024 + row * 16);
       constexpr int kMyGroups = 8 / C::kSplit;
-      uint4 w[kMyGroups];
-#pragma unroll
-      for (int g = 0; g < kMyGroups; ++g) w[g] = lds128(raw + row * 128 + (((part * kMyGroups + g) ^ (row & 7)) << 4));
+      auto codes = [&](int g) { return lds128(raw + row * 128 + (((part * kMyGroups + g) ^ (row & 7)) << 4)); };
+      uint4 w[2] = {codes(0), codes(1)};
       if (part == 0) {
         if (!mbar_wait_inline(s_free(sc), t_.phase ^ 1, abort_flag, p.status, 0x809)) break;
         // The tensor core truncates when it accumulates, which shortens a super-block's sum by 2^-22 on average (measured
@@ -579,52 +596,57 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
         sts64f(smem + C::oScl + sc * C::kScl + row * 8, fp16_bits_to_f32(cm.x & 0xffffu) * (1.f + 0x1p-22f), -32.f * fp16_bits_to_f32(cm.x >> 16));
       }
       ScaleMinWords const sm = decode_scale_min(cm.y, cm.z, cm.w);
-      constexpr int kMine = C::kQ / C::kSplit, kGroupsPer = 8 / C::kQ;  // stages of this warp, K32 groups per stage
+      auto expand = [&](int g, uint32_t (&v)[16]) {
+        uint32_t const scw = C::kSplit == 1 ? (g < 4 ? sm.sc_lo : sm.sc_hi) : (part == 0 ? sm.sc_lo : sm.sc_hi);
+        __half2 const S = __hsub2(u2h(__byte_perm(scw, 0x64646464u, 0x4040 | ((g & 3) * 0x0101))), u2h(0x64006400u));
+        // low nibbles: (1024 + q) * sc - 1024 sc; high nibbles, four bits up: (1024 + 16 q) * (sc / 16) - 64 sc
+        __half2 const S16 = __hmul2(S, u2h(0x2c002c00u)), B = __hmul2(S, u2h(0xe400e400u)), B16 = __hmul2(S, u2h(0xd400d400u));
+        uint32_t const ww[4] = {w[g & 1].x, w[g & 1].y, w[g & 1].z, w[g & 1].w};
 #pragma unroll
-      for (int i = 0; i < kMine; ++i) {
-        uint32_t const sa = group * C::kQ + part * kMine + i;
-        auto expand = [&](int g, uint32_t (&v)[16]) {
-          uint32_t const scw = C::kSplit == 1 ? (g < 4 ? sm.sc_lo : sm.sc_hi) : (part == 0 ? sm.sc_lo : sm.sc_hi);
-          __half2 const S = __hsub2(u2h(__byte_perm(scw, 0x64646464u, 0x4040 | ((g & 3) * 0x0101))), u2h(0x64006400u));
-          // low nibbles: (1024 + q) * sc - 1024 sc; high nibbles, four bits up: (1024 + 16 q) * (sc / 16) - 64 sc
-          __half2 const S16 = __hmul2(S, u2h(0x2c002c00u)), B = __hmul2(S, u2h(0xe400e400u)), B16 = __hmul2(S, u2h(0xd400d400u));
-          uint32_t const ww[4] = {w[g].x, w[g].y, w[g].z, w[g].w};
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            uint32_t const t = ww[j] >> 8;
-            v[4 * j + 0] = h2u(__hfma2(u2h(and_or(ww[j], low, magic)), S, B));
-            v[4 * j + 1] = h2u(__hfma2(u2h(and_or(ww[j], high, magic)), S16, B16));
-            v[4 * j + 2] = h2u(__hfma2(u2h(and_or(t, low, magic)), S, B));
-            v[4 * j + 3] = h2u(__hfma2(u2h(and_or(t, high, magic)), S16, B16));
-          }
-        };
-        auto mins = [&] {
-          uint32_t mh[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            uint32_t const mw = j < 2 ? sm.mn_lo : sm.mn_hi;
-            // two bytes under the exponent of 1024, minus 1024: exact
-            mh[j] = h2u(__hsub2(u2h(__byte_perm(mw, 0x64646464u, (j & 1) ? 0x4342 : 0x4140)), u2h(0x64006400u)));
-          }
-          sts128(smem + C::oMins + group * C::kMins + row * 16, mh[0], mh[1], mh[2], mh[3]);
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // read by the MMA
-        };
-        uint32_t v[16];
-        if constexpr (C::kReady) expand(i, v);  // the stage's words are ready when it is
-        if (!mbar_wait_inline(a_free(sa), phase ^ 1, abort_flag, p.status, 0x80a)) { ok = false; break; }
-        tc_fence_after();
-        if (part == C::kSplit - 1 && i == kMine - 1) mins();
-#pragma unroll
-        for (int gg = 0; gg < kGroupsPer; ++gg) {
-          if constexpr (!C::kReady) expand(i * kGroupsPer + gg, v);
-          tmem_st16(tmem + ((quarter * 32u) << 16) + C::kACol + sa * C::kACols + gg * 16, v);
+        for (int j = 0; j < 4; ++j) {
+          uint32_t const t = ww[j] >> 8;
+          v[4 * j + 0] = h2u(__hfma2(u2h(and_or(ww[j], low, magic)), S, B));
+          v[4 * j + 1] = h2u(__hfma2(u2h(and_or(ww[j], high, magic)), S16, B16));
+          v[4 * j + 2] = h2u(__hfma2(u2h(and_or(t, low, magic)), S, B));
+          v[4 * j + 3] = h2u(__hfma2(u2h(and_or(t, high, magic)), S16, B16));
         }
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) {
-          if (part == C::kSplit - 1 && i == kMine - 1) release_shared();  // the mins
-          arrive_cluster(a_full0 + 8 * sa);
+        if (g + 2 < kMyGroups) w[g & 1] = codes(g + 2);
+      };
+      auto mins = [&] {
+        uint32_t mh[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          uint32_t const mw = j < 2 ? sm.mn_lo : sm.mn_hi;
+          // two bytes under the exponent of 1024, minus 1024: exact
+          mh[j] = h2u(__hsub2(u2h(__byte_perm(mw, 0x64646464u, (j & 1) ? 0x4342 : 0x4140)), u2h(0x64006400u)));
+        }
+        sts128(smem + C::oMins + group * C::kMins + row * 16, mh[0], mh[1], mh[2], mh[3]);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // read by the MMA
+      };
+      // The words of the next K32 group are computed while those of this one go to tensor memory.
+      constexpr int kGroupsPer = 8 / C::kQ;
+      uint32_t v[2][16];
+      expand(0, v[0]);
+#pragma unroll
+      for (int g = 0; g < kMyGroups; ++g) {
+        int const j = g / kGroupsPer;
+        uint32_t const sa = group * C::kQ + part * (kMyGroups / kGroupsPer) + j;
+        bool const first = g % kGroupsPer == 0, end = g % kGroupsPer == kGroupsPer - 1, with_mins = part == C::kSplit - 1 && g == kMyGroups - 1;
+        if (first) {
+          if (!mbar_wait_inline(a_free(sa), phase ^ 1, abort_flag, p.status, 0x80a)) { ok = false; break; }
+          tc_fence_after();
+        }
+        if (with_mins) mins();  // the last stage is free: so is the place of the mins before them
+        tmem_st16(tmem + ((quarter * 32u) << 16) + C::kACol + sa * C::kACols + (g % kGroupsPer) * 16, v[g & 1]);
+        if (g + 1 < kMyGroups) expand(g + 1, v[(g + 1) & 1]);
+        if (end) {
+          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) {
+            if (with_mins) release_shared();
+            arrive_cluster(a_full0 + 8 * sa);
+          }
         }
       }
       if (lane == 0) {
@@ -645,11 +667,23 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
     float2 acc[C::kCols / 2];
 #pragma unroll
     for (int j = 0; j < C::kCols / 2; ++j) acc[j] = make_float2(0.f, 0.f);
+    float token_scale = 0.f;
     Cursor c(p, u0);
     Ring<C::kSclStages> t_;
     Ring<2> d_;
     for (uint32_t u = u0; u < u1; ++u, c.next(p), t_.next(), d_.next()) {
       uint32_t const sc = t_.s, d = d_.s, cols = tile_cols<NT>(p, c.tok);
+      // What the end of this cluster's part of a tile needs is found while its last super-block is still being multiplied: lane
+      // t's share of the tokens' powers of two (handed round below), and the clusters that share the tile, from the one whose run
+      // holds its first unit to the one that holds its last.
+      bool const part_end = u + 1 == u1 || c.kb + 1 == KB;
+      uint32_t const tile = c.row_pair * p.tok_tiles + c.tok;
+      uint32_t w0 = worker, w1 = worker;
+      if (part_end) {
+        token_scale = __ldcg(p.tokens + c.tok * NT + col0 + (C::kCols < 32 ? lane & 15 : lane));
+        while (first_unit(p, w0) > tile * KB) --w0;
+        while (first_unit(p, w1 + 1) < (tile + 1) * KB) ++w1;
+      }
       if (!mbar_wait_inline(s_full(sc), t_.phase, abort_flag, p.status, 0x80b)) break;
       uint32_t const scl = smem + C::oScl + sc * C::kScl, et = scl + C::oE + col0 * 4;
       float2 const dm = lds64f(scl + row * 8);
@@ -694,14 +728,11 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(s_free(sc));
-      if (u + 1 < u1 && c.kb + 1 != KB) continue;
+      if (!part_end) continue;
 
       // ---- end of this cluster's part of the tile
-      uint32_t const tile = c.row_pair * p.tok_tiles + c.tok;
-      // lane t's share of the tokens' powers of two, requested now and handed round below
-      float const token_scale = __ldcg(p.tokens + c.tok * NT + col0 + (C::kCols < 32 ? lane & 15 : lane));
       bool write = true;
-      if (max(u0, tile * KB) != tile * KB || u + 1 != (tile + 1) * KB) {
+      if (w0 != w1) {
         // Partial: [cluster][first or later tile of its run][CTA][warp][token / 4][lane].
         auto slot = [&](uint32_t w) {
           uint32_t const later = first_unit(p, w) < tile * KB || first_unit(p, w) >= (tile + 1) * KB;
@@ -711,34 +742,36 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
         float4* const mine = slot(worker);
 #pragma unroll
         for (int j = 0; j < C::kCols / 4; ++j) __stcg(mine + j * 32, make_float4(acc[2 * j].x, acc[2 * j].y, acc[2 * j + 1].x, acc[2 * j + 1].y));
-        __threadfence();
         __syncwarp();
-        // Clusters that share the tile: from the one whose run holds its first unit to the one that holds its last.
-        uint32_t w0 = worker, w1 = worker;
-        while (first_unit(p, w0) > tile * KB) --w0;
-        while (first_unit(p, w1 + 1) < (tile + 1) * KB) ++w1;
         uint32_t old = 0;
         uint32_t* const ticket = p.tickets + (w0 * 2 + cta) * C::kEpilogueWarps + ep;
-        if (lane == 0) old = atomicAdd(ticket, 1u);
+        if (lane == 0) asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(ticket) : "memory");
         old = __shfl_sync(0xffffffffu, old, 0);
         write = old == w1 - w0;
         if (write) {
-          __threadfence();
 #pragma unroll
           for (int j = 0; j < C::kCols / 2; ++j) acc[j] = make_float2(0.f, 0.f);
-          for (uint32_t w = w0; w <= w1; ++w) {  // in run order, whoever arrives last
-            const float4* const src = slot(w);
+          // In run order, whoever arrives last; as many reads in flight as registers allow.
+          constexpr int kSlots = C::kCols <= 16 ? 2 : 1, kBatch = NT >= 128 ? 4 : C::kCols / 4;
+          for (uint32_t w = w0; w <= w1; w += kSlots) {
 #pragma unroll
-            for (int j0 = 0; j0 < C::kCols / 4; j0 += 4) {
-              float4 x[4];
+            for (int j0 = 0; j0 < C::kCols / 4; j0 += kBatch) {
+              float4 x[kSlots][kBatch];
 #pragma unroll
-              for (int j = 0; j < 4; ++j) x[j] = __ldcg(src + (j0 + j) * 32);
+              for (int i = 0; i < kSlots; ++i)
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                float2 &lo = acc[2 * (j0 + j)], &hi = acc[2 * (j0 + j) + 1];
-                lo = __fadd2_rn(lo, make_float2(x[j].x, x[j].y));
-                hi = __fadd2_rn(hi, make_float2(x[j].z, x[j].w));
-              }
+                for (int j = 0; j < kBatch; ++j)
+                  if (w + i <= w1) x[i][j] = __ldcg(slot(w + i) + (j0 + j) * 32);
+#pragma unroll
+              for (int i = 0; i < kSlots; ++i)
+                if (w + i <= w1) {
+#pragma unroll
+                  for (int j = 0; j < kBatch; ++j) {
+                    float2 &lo = acc[2 * (j0 + j)], &hi = acc[2 * (j0 + j) + 1];
+                    lo = __fadd2_rn(lo, make_float2(x[i][j].x, x[i][j].y));
+                    hi = __fadd2_rn(hi, make_float2(x[i][j].z, x[i][j].w));
+                  }
+                }
             }
           }
         }
@@ -784,7 +817,8 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
   if (warp >= C::kFirstEpilogue) tmem_wait_ld();
   tc_fence_before();
   __syncthreads();
-  cluster_meet();  // neither CTA leaves while the other may still signal it or read its operands
+  cluster_arrive();
+  cluster_wait();  // neither CTA leaves while the other may still signal it or read its operands
   tc_fence_after();
   if (warp == 3) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }

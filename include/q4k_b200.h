@@ -219,11 +219,11 @@ int q4k_session_take_failure(q4k_session* session, void* stream);
 
 /* Programmatic dependent launch for the decode path (no counterpart in the reference, which
  * replays its decode step as a CUDA graph of fully serialised kernels, src/runtime/language_model.cpp:324-356).
- * When enabled (process-wide, default off), q4k_pack_q8_*, and q4k_q8_project* for m <= 16 launch
- * their kernels so that they may begin while the preceding kernel of the stream is still draining:
- * blocks are placed as SMs free up, and the TMA kernel streams WEIGHT tiles into shared memory
- * before it waits for that kernel.  Activations, residual, output and scratch are touched only
- * after the preceding kernel has completed, so results are unchanged.  The caller's side of the
+ * Producers, decode and fp16 projections are always placed while the preceding kernel of the stream drains; by default
+ * they read and write nothing before it has completed (they only ask L2 for weights), as if launched without.
+ * When enabled (process-wide, default off), projections also read WEIGHTS before that: the dp4a, TMA and tcgen05
+ * kernels stream weight tiles into shared memory at once.  Activations, residual, output and scratch are still touched
+ * only after the preceding kernel has completed, so results are unchanged.  The caller's side of the
  * contract: no work still in flight earlier in the stream writes the weight operand (true for
  * decode, where weights are constant; leave it off around q4k_repack_blocks144 or uploads).
  * Works inside CUDA graph capture. */

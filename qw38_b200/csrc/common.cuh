@@ -71,6 +71,10 @@ __device__ __forceinline__ uint32_t odd_bytes(uint32_t z0, uint32_t z1) { return
 // const __restrict__ parameter that the compiler turns into it, promises data that nobody writes during this kernel, whose
 // life begins before the wait.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Asks L2 for weights that are read after the wait: nothing is read, so whoever still writes them is not disturbed.
+__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {  // multiples of 16
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Row-sharded decode: tell every rank how many more projections of this rank are complete.  Called by

@@ -59,7 +59,7 @@ __global__ void swiglu_store_bf16_kernel(const float* gate, const float* up,
 
 cudaError_t launch_store_bf16(const float* in, uint16_t* out, uint64_t count, cudaStream_t stream) {
   if (count == 0) return cudaSuccess;
-  return launch_kernel(store_bf16_kernel, unsigned((count + 255) / 256), 256, 0, stream, launch_overlap(), in, out, count);
+  return launch_kernel(store_bf16_kernel, unsigned((count + 255) / 256), 256, 0, stream, true, in, out, count);
 }
 
 cudaError_t launch_swiglu_store_bf16(const float* gate, const float* up, uint16_t* out, uint64_t count, cudaStream_t stream) {
@@ -67,7 +67,7 @@ cudaError_t launch_swiglu_store_bf16(const float* gate, const float* up, uint16_
   bool const wide = count % 8 == 0 && ((reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(up) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
   uint64_t const threads = wide ? count / 8 : count;
   return launch_kernel(wide ? swiglu_store_bf16_kernel<true> : swiglu_store_bf16_kernel<false>, unsigned((threads + 255) / 256), 256, 0, stream,
-                       launch_overlap(), gate, up, out, count);
+                       true, gate, up, out, count);
 }
 
 }  // namespace q4k

@@ -65,7 +65,8 @@ struct DpParams {
   uint32_t rgs_each, rgs_rest;  // row groups per block; the first rgs_rest blocks take one more
   uint32_t stages, parts;       // ring stages and row-sum slots of a warp
   uint32_t wide;                // weights are 16-byte aligned: bulk copies
-  uint32_t input_settled;
+  uint32_t early;               // weights may be read before the preceding launch has ended
+  uint32_t input_settled;       // so may the activations
 };
 
 __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
@@ -155,6 +156,16 @@ __global__ void __launch_bounds__(kThreads, M <= 2 ? 2 : 1) gemv_dp4a_kernel(con
       if (p.wide) {
         for (uint32_t i = 0; i < p.stages; ++i) mbar_init(bars + i * 8, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        if (!p.early) {  // the ring's first fill comes out of L2 after the wait
+          for (uint32_t i = 0, u = u0; i < p.stages && u < u1; ++i) {
+            uint32_t const count = stage_units(p, u, u1);
+            DpSegment const& s = segment_of(p, u);
+            prefetch_l2(s.codes + uint64_t(u - s.u0) * 1024, count * 1024);
+            prefetch_l2(s.meta + uint64_t(u - s.u0) * 128, count * 128);
+            u += count;
+          }
+          pdl_wait();
+        }
         for (uint32_t i = 0; i < p.stages && pu < u1; ++i) fetch();
       }
       cuts[warp] = c0;
@@ -254,9 +265,9 @@ __global__ void __launch_bounds__(kThreads, M <= 2 ? 2 : 1) gemv_dp4a_kernel(con
         const uint32_t* const c32 = reinterpret_cast<const uint32_t*>(s.codes + at * 1024);
         const uint16_t* const m16 = reinterpret_cast<const uint16_t*>(s.meta + at * 128);
 #pragma unroll 8
-        for (uint32_t i = lane; i < count * 256; i += 32) asm volatile("st.shared.u32 [%0], %1;" ::"r"(stage + i * 4), "r"(__ldg(c32 + i)) : "memory");
+        for (uint32_t i = lane; i < count * 256; i += 32) asm volatile("st.shared.u32 [%0], %1;" ::"r"(stage + i * 4), "r"(c32[i]) : "memory");
         for (uint32_t i = lane; i < count * 64; i += 32)
-          asm volatile("st.shared.u16 [%0], %1;" ::"r"(stage + kStageUnits * 1024 + i * 2), "h"(__ldg(m16 + i)) : "memory");
+          asm volatile("st.shared.u16 [%0], %1;" ::"r"(stage + kStageUnits * 1024 + i * 2), "h"(m16[i]) : "memory");
         __syncwarp();
       }
 #pragma unroll
@@ -349,12 +360,14 @@ cudaError_t launch_m(const DpParams& p, uint32_t grid, uint32_t smem, cudaStream
   }
   cudaError_t st = allow_smem(reinterpret_cast<const void*>(kernel), int(smem));
   if (st != cudaSuccess) return st;
-  return launch_kernel(kernel, grid, kThreads, smem, stream, launch_overlap(), p);
+  return launch_kernel(kernel, grid, kThreads, smem, stream, true, p);
 }
 
 // Fills the split and launches; seg, nseg, operands and outputs are set.
 cudaError_t launch_split(DpParams p, uint32_t m, uint32_t padded_k, cudaStream_t stream) {
   p.tiles_k = padded_k / 256;
+  p.early = launch_overlap();
+  p.input_settled = p.input_settled && p.early;
   for (uint32_t i = 0; i < p.nseg; ++i) {
     p.seg[i].rg0 = p.rgs;
     p.seg[i].u0 = p.rgs * p.tiles_k;

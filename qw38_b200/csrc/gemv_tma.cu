@@ -29,7 +29,7 @@
 // bf16(SiLU(gate) * up), or -- for the MLP chain -- quantises that product on the spot into the Q8 codes,
 // scales and sums of the down projection's input (two tile pairs = one group of 32 rows per token).
 //
-// Launched with programmatic stream serialization (launch.h), the producer streams weights while
+// Launched with programmatic stream serialization (launch.h), the producer streams weights, or asks L2 for them, while
 // the previous kernel of the stream is still draining; the reducers wait for that kernel first and only
 // then release the next launch; the consumers wait for it before they load activations unless the caller
 // flagged the input as settled (not the work of the launch directly before).  Row-sharded use (GemvTmaGather): the reducers store each value into every rank's copy
@@ -91,6 +91,7 @@ struct GtParams {
   GtSegment seg[3];
   uint32_t nseg, pair, n_total;  // n_total: rows of all segments = row stride of the split-K scratch
   uint32_t input_settled;        // activations were complete before the preceding launch was enqueued
+  uint32_t early;                // weights may be read before the preceding launch has ended
   // pair == 2: the gate / up pair's result is not stored as bf16 but quantised on the spot: Q8 codes, scales and sums
   // of x = bf16(silu(gate) * up), 32 consecutive rows (two 16-row tiles) per group, as swiglu_pack would produce.
   int8_t* q8_codes;
@@ -207,17 +208,15 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
   }
   __syncthreads();
 
-  // The producer streams weights at once: they are constant, whatever kernel runs before this
-  // one.  Every other role first waits for the preceding kernel of the stream, because the
-  // activations, the residual, the output and the split-K scratch may be its to write.
+  // The producer streams weights at once where the caller vouches for them (launch overlap, or a predecessor of this library
+  // that writes none); otherwise it asks L2 for the ring's first fill and waits.  Every other role first waits for the
+  // preceding kernel of the stream, because the activations, the residual, the output and the split-K scratch may be its to
+  // write.
   if (warp == kProducer) {
     if (lane == 0) {
-      uint32_t s = 0, ph = 1;  // the first pass over the ring finds every stage free
-      for (uint32_t it = 0; it < ntiles; ++it) {
-        if (it >= stages && !mbar_wait(b_empty + 8 * s, ph, abort_flag, p.status, 0x510)) break;
-        mbar_expect_tx(b_full + 8 * s, code_stage + meta_stage);
-        const CUtensorMap* mc = &tm_codes;
-        const CUtensorMap* mm = &tm_meta;
+      auto tile = [&](uint32_t it, const CUtensorMap*& mc, const CUtensorMap*& mm) {  // its maps, and its first row group
+        mc = &tm_codes;
+        mm = &tm_meta;
         uint32_t local = t0 + it;
         if (p.nseg > 1) {
           uint32_t sg;
@@ -225,7 +224,23 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
           if (sg == 1) { mc = &tm_codes1; mm = &tm_meta1; }
           if (sg == 2) { mc = &tm_codes2; mm = &tm_meta2; }
         }
-        int const rg = int(local * 2);
+        return int(local * 2);
+      };
+      if (!p.early) {
+        for (uint32_t it = 0; it < stages && it < ntiles; ++it) {
+          const CUtensorMap *mc, *mm;
+          int const rg = tile(it, mc, mm);
+          tma_3d_prefetch(mc, 0, int(sb0 * 8), rg);
+          tma_3d_prefetch(mm, 0, int(sb0), rg);
+        }
+        pdl_wait();
+      }
+      uint32_t s = 0, ph = 1;  // the first pass over the ring finds every stage free
+      for (uint32_t it = 0; it < ntiles; ++it) {
+        if (it >= stages && !mbar_wait(b_empty + 8 * s, ph, abort_flag, p.status, 0x510)) break;
+        mbar_expect_tx(b_full + 8 * s, code_stage + meta_stage);
+        const CUtensorMap *mc, *mm;
+        int const rg = tile(it, mc, mm);
         tma_3d(s_codes + s * code_stage, mc, 0, int(sb0 * 8), rg, b_full + 8 * s);
         tma_3d(s_meta + s * meta_stage, mm, 0, int(sb0), rg, b_full + 8 * s);
         if (++s == stages) { s = 0; ph ^= 1; }
@@ -745,7 +760,8 @@ cudaError_t launch_cfg(const Maps& t, const GtParams& p, bool dump, uint32_t gri
   }
   cudaError_t st = allow_smem(reinterpret_cast<const void*>(kernel), int(smem));
   if (st != cudaSuccess) return st;
-  return launch_kernel(kernel, grid, (p.cw + kFirstReducer + NT * p.reducers) * 32, smem, stream, launch_overlap(), t.codes[0], t.meta[0],
+  // Row-sharded launches keep to the switch: their counters are announced by the kernel behind them.
+  return launch_kernel(kernel, grid, (p.cw + kFirstReducer + NT * p.reducers) * 32, smem, stream, p.done == nullptr || launch_overlap(), t.codes[0], t.meta[0],
                        t.codes[1], t.meta[1], t.codes[2], t.meta[2], p);
 }
 
@@ -850,7 +866,8 @@ cudaError_t launch_gemv_tma(const WeightView& w, const Q8View& x, float* out, co
   p.n = w.n; p.m = x.m; p.padded_k = x.padded_k; p.tiles_k = w.tiles_k; p.G = x.padded_k / 32;
   p.row_tiles = (w.padded_n + 15) / 16; p.cw = cw; p.split_k = plan.split_k;
   p.tiles_per_range = plan.tiles_per_range; p.stages = plan.stages; p.red_slots = plan.red_slots;
-  p.input_settled = plan.input_settled;
+  p.early = launch_overlap();
+  p.input_settled = plan.input_settled && p.early;
   p.reducers = 1;
   uint32_t const grid = plan.ranges * plan.split_k, smem = smem_bytes(cw, nt, plan.stages, plan.red_slots);
   bool const dump = partials != nullptr;
@@ -885,7 +902,8 @@ cudaError_t launch_gemv_tma_multi(const WeightView* ws, const GemvTmaOutput* out
   p.n = ws[0].n; p.m = x.m; p.padded_k = x.padded_k; p.tiles_k = ws[0].tiles_k; p.G = x.padded_k / 32;
   p.row_tiles = total_tiles; p.cw = cw; p.split_k = plan.split_k;
   p.tiles_per_range = plan.tiles_per_range; p.stages = plan.stages; p.red_slots = plan.red_slots;
-  p.input_settled = plan.input_settled;
+  p.early = launch_overlap();
+  p.input_settled = plan.input_settled && p.early;
   p.nseg = count; p.pair = swiglu_pair ? 1u : 0u; p.n_total = total_rows;
   p.reducers = 1;
   if (raw) {
@@ -938,6 +956,7 @@ cudaError_t launch_gemv_tma_swiglu_q8(const WeightView& gate, const WeightView& 
   p.n = gate.n; p.m = x.m; p.padded_k = x.padded_k; p.tiles_k = gate.tiles_k; p.G = x.padded_k / 32;
   p.row_tiles = 2 * (gate.padded_n / 16); p.cw = cw; p.split_k = 1;
   p.tiles_per_range = plan.tiles_per_range; p.stages = plan.stages; p.red_slots = plan.red_slots;
+  p.early = launch_overlap();
   p.input_settled = 0;
   p.nseg = 2; p.pair = 2; p.n_total = 2 * gate.n;
   p.reducers = nt == 1 ? plan.red_slots : 1;

@@ -191,9 +191,9 @@ cudaError_t launch_swiglu_store_bf16(const float* gate, const float* up, uint16_
 cudaError_t launch_gemv_bf16w(const WeightView& w, const uint16_t* x, uint32_t m, uint32_t k, uint32_t padded_k, float* out,
                               const float* residual, cudaStream_t stream);
 
-// abi.cu : process-wide switch set by q4k_set_launch_overlap().  When on, the decode kernels
-// (pack, dp4a, TMA gemv) are launched with programmatic stream serialization: they may start,
-// and the TMA kernel may prefetch weights, while the preceding kernel of the stream drains.
+// abi.cu : process-wide switch set by q4k_set_launch_overlap().  Kernels are placed while the preceding kernel of the stream
+// drains (launch_kernel below) whatever it says; when it is on they may also read their weights, and settled inputs, before
+// that kernel has ended.
 bool launch_overlap();
 // While one lives, launch_overlap() holds on this thread whatever the switch says.  For the second and later launches of an
 // entry point that issues several on one stream: their predecessor is a kernel of this library that writes no weights, so
@@ -229,7 +229,9 @@ inline cudaError_t allow_smem(const void* kernel, int bytes) {
   return cudaSuccess;
 }
 
-// Launch with or without the programmatic-stream-serialization attribute.
+// Launch with or without the programmatic-stream-serialization attribute.  With it, blocks are placed and set up beside the
+// preceding kernel's end; a kernel that reads and writes nothing before its pdl_wait() (asking L2 for lines is no read) then
+// behaves as if launched without, whatever that kernel is, and starts 1 to 2 us earlier.
 template <typename... KArgs, typename... Args>
 cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                           bool overlap, Args&&... args) {

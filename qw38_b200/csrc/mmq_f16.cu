@@ -867,10 +867,10 @@ cudaError_t launch_f16(const WeightView& w, const WeightView* second, const Q8Vi
     // K = 2048 23.0 / 24.3 / 29.5, 5120 34.1 / 35.3 / 42.8, 17408 - / 133 / 146.
     auto kernel = w.tiles_k <= 24 ? rows_planes_kernel<3> : (w.tiles_k <= 72 ? rows_planes_kernel<9> : rows_planes_kernel<16>);
     if (w.tiles_k > 128) return cudaErrorInvalidValue;
-    st = launch_kernel(kernel, m_pad, 256, 0, stream, launch_overlap(), raw->x, raw->k, vec, raw->failure, x.m, m_pad, w.tiles_k, planes, sums,
+    st = launch_kernel(kernel, m_pad, 256, 0, stream, true, raw->x, raw->k, vec, raw->failure, x.m, m_pad, w.tiles_k, planes, sums,
                        exps, tokens, tickets, ticket_count);
   } else {
-    st = launch_kernel(planes_kernel, m_pad * ((w.tiles_k + 7) / 8), 256, 0, stream, launch_overlap(), x.codes, x.scales, x.sums, x.m, m_pad,
+    st = launch_kernel(planes_kernel, m_pad * ((w.tiles_k + 7) / 8), 256, 0, stream, true, x.codes, x.scales, x.sums, x.m, m_pad,
                        w.tiles_k, planes, sums, exps, tokens, tickets, ticket_count, early);
   }
   if (st != cudaSuccess) return st;
@@ -923,8 +923,8 @@ cudaError_t launch_f16(const WeightView& w, const WeightView* second, const Q8Vi
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  // Always allowed to start beside the kernel that writes the planes: that one starts (or, with launch overlap, waits
-  // until) everything before it has completed, so the weights are final by then.
+  // Its weights are read beside the kernel that writes the planes: that one lets it start after its own wait (launch overlap and
+  // settled inputs aside), so everything before has completed and the weights are final.
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;

@@ -244,12 +244,12 @@ cudaError_t launch_pack_q8(const void* input, bool fp32, Q8Out out, uint32_t k, 
   bool const vec = (k % 8 == 0) && (reinterpret_cast<uintptr_t>(input) % 16 == 0);
   if (fp32) {
     auto* in = static_cast<const float*>(input);
-    if (vec) return launch_kernel(pack_kernel<float, true>, grid, kThreads, 0, stream, launch_overlap(), in, out.codes, out.scales, out.sums, out.m, k, out.padded_k, failure);
-    else return launch_kernel(pack_kernel<float, false>, grid, kThreads, 0, stream, launch_overlap(), in, out.codes, out.scales, out.sums, out.m, k, out.padded_k, failure);
+    if (vec) return launch_kernel(pack_kernel<float, true>, grid, kThreads, 0, stream, true, in, out.codes, out.scales, out.sums, out.m, k, out.padded_k, failure);
+    else return launch_kernel(pack_kernel<float, false>, grid, kThreads, 0, stream, true, in, out.codes, out.scales, out.sums, out.m, k, out.padded_k, failure);
   } else {
     auto* in = static_cast<const uint16_t*>(input);
-    if (vec) return launch_kernel(pack_kernel<uint16_t, true>, grid, kThreads, 0, stream, launch_overlap(), in, out.codes, out.scales, out.sums, out.m, k, out.padded_k, failure);
-    else return launch_kernel(pack_kernel<uint16_t, false>, grid, kThreads, 0, stream, launch_overlap(), in, out.codes, out.scales, out.sums, out.m, k, out.padded_k, failure);
+    if (vec) return launch_kernel(pack_kernel<uint16_t, true>, grid, kThreads, 0, stream, true, in, out.codes, out.scales, out.sums, out.m, k, out.padded_k, failure);
+    else return launch_kernel(pack_kernel<uint16_t, false>, grid, kThreads, 0, stream, true, in, out.codes, out.scales, out.sums, out.m, k, out.padded_k, failure);
   }
   return cudaGetLastError();
 }
@@ -257,7 +257,7 @@ cudaError_t launch_pack_q8(const void* input, bool fp32, Q8Out out, uint32_t k, 
 cudaError_t launch_swiglu_pack_q8(const float* gate, const float* up, Q8Out out, int* failure,
                                   cudaStream_t stream) {
   uint64_t const chunks = uint64_t(out.m) * (out.padded_k / 256);
-  return launch_kernel(swiglu_pack_kernel, grid_for(chunks), kThreads, 0, stream, launch_overlap(), gate, up, out.codes, out.scales, out.sums,
+  return launch_kernel(swiglu_pack_kernel, grid_for(chunks), kThreads, 0, stream, true, gate, up, out.codes, out.scales, out.sums,
                        chunks, failure);
 }
 
@@ -270,7 +270,7 @@ cudaError_t launch_hidden_rms_q8(const float* residual, const uint16_t* gamma, f
     cudaError_t st = allow_smem(reinterpret_cast<const void*>(kernel), int(smem));
     if (st != cudaSuccess) return st;
   }
-  return launch_kernel(kernel, out.m, kThreads, smem, stream, launch_overlap(), residual, gamma, eps, hidden, out.codes, out.scales, out.sums,
+  return launch_kernel(kernel, out.m, kThreads, smem, stream, true, residual, gamma, eps, hidden, out.codes, out.scales, out.sums,
                        failure);
 }
 

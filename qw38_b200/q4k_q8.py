@@ -28,8 +28,8 @@ def _check(status: int) -> None:
 
 
 def set_launch_overlap(enabled: bool) -> None:
-    """Process-wide switch (q4k_set_launch_overlap): decode kernels may start, and stream weight tiles,
-    while the preceding kernel of the stream drains.  Only while nothing in flight writes the weights."""
+    """Process-wide switch (q4k_set_launch_overlap): projections may read their weights while the preceding kernel of the
+    stream drains.  Only while nothing in flight writes the weights."""
     L.load().q4k_set_launch_overlap(1 if enabled else 0)
 
 

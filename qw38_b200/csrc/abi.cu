@@ -414,10 +414,13 @@ int project_impl(const q4k_weight* weight, const q4k_q8_input& x, float* output,
 
 // A gate and an up projection of the same input.  Beyond sixteen tokens (where the automatic choice is the fp16 kernel) one
 // launch takes both: an MLP chain of 237 tokens 300 us with two launches, 291 with one.
+bool pair_f16(const q4k_weight* gate, const q4k_weight* up, const q4k_q8_input& x) {
+  return x.m > 16 && up->n == gate->n && up->k == gate->k && q4k::f16_supported(view(*gate), view(x)) && q4k::f16_supported(view(*up), view(x));
+}
 int project_pair(const q4k_weight* gate, const q4k_weight* up, const q4k_q8_input& x, float* g, float* u, const q4k_project_options* opt,
                  cudaStream_t stream, const q4k::RawRows* raw = nullptr) {
   uint64_t const cells = uint64_t(x.m) * gate->n;
-  if (x.m <= 16 || up->n != gate->n || up->k != gate->k || !q4k::f16_supported(view(*gate), view(x)) || !q4k::f16_supported(view(*up), view(x))) {
+  if (!pair_f16(gate, up, x)) {
     if (int st = project_impl(gate, x, g, cells, nullptr, 0, opt, stream, false, "gate")) return st;
     return project_impl(up, x, u, cells, nullptr, 0, opt, stream, false, "up");
   }
@@ -1271,13 +1274,17 @@ int q4k_q8_mlp(const q4k_weight* gate, const q4k_weight* up, const q4k_weight* d
   q4k_q8_input xf{codes, scales, sums, uint64_t(m) * ffn, uint64_t(m) * (ffn / 32), uint64_t(m) * (ffn / 32), m, ffn, ffn};
   q4k_project_options opt{};
   opt.flags = kFlagTrustedSpans;  // every span was validated above
-  cudaError_t ce;
-  {
+  // Beyond sixteen tokens the fp16 kernel makes its operand planes from the residual stream and from the gate and up rows itself.
+  bool const rms_direct = !fused && pair_f16(gate, up, xh), swiglu_direct = m > 16 && q4k::f16_supported(view(*down), view(xf));
+  q4k::RawRows const rms_rows{nullptr, hidden, failure, nullptr, nullptr, residual, gamma, eps}, swiglu_rows{nullptr, ffn, failure, g, u};
+  cudaError_t ce = cudaSuccess;
+  std::optional<q4k::ChainedLaunches> chained;
+  if (!rms_direct) {
     ScopedRange range("qw38:op name=hidden_rms_q8_pack m=%u n=%u k=%u", unsigned(m), unsigned(hidden), 1u);
     ce = q4k::launch_hidden_rms_q8(residual, gamma, eps, hidden, out_view(xh), failure, stream);
+    chained.emplace();
   }
   if (ce != cudaSuccess) return bail(fail_cuda(ce, "q8.rms_pack"));
-  q4k::ChainedLaunches chained;
   if (fused) {
     int* status = q4k::kernel_status_word();
     if (!status) return bail(Q4K_ERR_STATUS);
@@ -1288,14 +1295,16 @@ int q4k_q8_mlp(const q4k_weight* gate, const q4k_weight* up, const q4k_weight* d
     }
     if (ce != cudaSuccess) return bail(fail_cuda(ce, "q8.gate_up_swiglu_q8"));
   } else {
-  if (int st = project_pair(gate, up, xh, g, u, &opt, stream)) return bail(st);
-  {
+  if (int st = project_pair(gate, up, xh, g, u, &opt, stream, rms_direct ? &rms_rows : nullptr)) return bail(st);
+  if (!chained) chained.emplace();
+  if (!swiglu_direct) {
     ScopedRange range("qw38:op name=swiglu_q8_pack m=%u n=%u k=%u", unsigned(m), unsigned(ffn), 1u);
     ce = q4k::launch_swiglu_pack_q8(g, u, out_view(xf), failure, stream);
   }
   if (ce != cudaSuccess) return bail(fail_cuda(ce, "q8.swiglu_pack"));
   }
-  if (int st = project_impl(down, xf, output, uint64_t(m) * hidden, residual, uint64_t(m) * hidden, &opt, stream, false, "down"))
+  if (int st = project_impl(down, xf, output, uint64_t(m) * hidden, residual, uint64_t(m) * hidden, &opt, stream, false, "down",
+                            swiglu_direct ? &swiglu_rows : nullptr))
     return bail(st);
   if (pending_failure) return Q4K_OK;
   int bad = 0;

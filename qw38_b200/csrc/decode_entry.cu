@@ -6,18 +6,10 @@
 
 #include "common.cuh"
 #include "launch.h"
-#include "q8_pack.cuh"
+#include "swiglu.cuh"
 
 namespace q4k {
 namespace {
-
-// sigmoid / SiLU exactly as the reference's decode epilogue states them
-// (cuda/decode_mmv.cu:78-89): the exponential is always taken of a non-positive number.
-__device__ __forceinline__ float sigmoid_fp32(float u) {
-  // below 2^-24 the divisor is 1; the others are between 1 and 2, their quotient rounded as the division would be
-  float const e = expf(-fabsf(u)), d = 1.0f + e, n = u >= 0.0f ? 1.0f : e;
-  return d == 1.0f ? n : rounded_quotient(n, d, __frcp_rn(d));
-}
 
 __global__ void store_bf16_kernel(const float* in, uint16_t* __restrict__ out, uint64_t count) {
   pdl_wait();

@@ -91,11 +91,16 @@ cudaError_t launch_mmq_tcgen05(const WeightView& w, const Q8View& x, const TcOut
                                const TcPlan& plan, void* partial_tiles, uint32_t* tickets, int* status, cudaStream_t stream);
 
 // Activations that are still bf16 rows [m][k]: the kernel that takes them quantises them itself (its Q8View then only says m
-// and padded_k), and a non-finite group raises *failure, as the pack kernel does.
+// and padded_k), and a non-finite group raises *failure, as the pack kernel does.  The fp16 kernel also takes what such rows come
+// from (x null, k a multiple of 256): fp32 rows for bf16(silu(gate) * up), or a residual stream for its RMS norm with gain.
 struct RawRows {
   const uint16_t* x;
   uint32_t k;
   int* failure;
+  const float *gate = nullptr, *up = nullptr;
+  const float* residual = nullptr;
+  const uint16_t* gamma = nullptr;
+  float eps = 0.f;
 };
 
 // mmq_f16.cu : tcgen05 kind::f16 on SM pairs, weights expanded into TMEM, activations as two fp16 planes.  scratch holds

@@ -57,6 +57,8 @@
 #include "common.cuh"
 #include "launch.h"
 #include "q8_pack.cuh"
+#include "rms.cuh"
+#include "swiglu.cuh"
 #include "tma.cuh"
 #include "umma.cuh"
 
@@ -294,13 +296,14 @@ __device__ __forceinline__ void write_planes(float a, int sum, uint2 z, float ro
   }
 }
 // The largest scale of the block's token from each thread's.
+template <int Warps = 8>
 __device__ __forceinline__ float block_top(float row, float* warp_top) {
 #pragma unroll
   for (int off = 16; off; off >>= 1) row = fmaxf(row, __shfl_xor_sync(0xffffffffu, row, off));
   if ((threadIdx.x & 31) == 0) warp_top[threadIdx.x >> 5] = row;
   __syncthreads();
 #pragma unroll
-  for (int i = 0; i < 8; ++i) row = fmaxf(row, warp_top[i]);
+  for (int i = 0; i < Warps; ++i) row = fmaxf(row, warp_top[i]);
   return row;
 }
 
@@ -388,6 +391,93 @@ __global__ void __launch_bounds__(256) rows_planes_kernel(const uint16_t* rows, 
     if (kb >= tiles_k) break;
     write_planes(__uint_as_float(held[i].z), int(held[i].w), make_uint2(held[i].x, held[i].y), row, tok, kb, m_pad, tiles_k * 256, planes, sums16,
                  exps, tokens);
+  }
+}
+
+// The same from the rows' sources in an MLP chain, K a multiple of 256, bitwise what the Q8 producers and planes_kernel give:
+// two launches less per chain and no Q8 form in memory.  MLP chain 5120 / 17408 (us, on a rested part):
+// 64 tokens 87.0 -> 85.1, 237 tokens 222.5 -> 220.4, and 4 us less of host time.
+template <int Held, int Warps>
+__global__ void __launch_bounds__(32 * Warps) swiglu_planes_kernel(const float* gate, const float* up, int* failure, uint32_t m, uint32_t m_pad,
+                                                            uint32_t tiles_k, __half* __restrict__ planes, __half* __restrict__ sums16,
+                                                            float* __restrict__ exps, float* __restrict__ tokens,
+                                                            uint32_t* __restrict__ tickets, uint32_t ticket_count) {
+  __shared__ float warp_top[Warps];
+  pdl_wait();
+  pdl_launch_dependents();
+  if (blockIdx.x == 0)
+    for (uint32_t i = threadIdx.x; i < ticket_count; i += 32 * Warps) tickets[i] = 0u;
+  uint32_t const warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tok = blockIdx.x;
+  uint4 held[Held];  // {codes, codes, scale, sum}
+  float row = 0.f;
+  bool valid = true;
+#pragma unroll
+  for (int i = 0; i < Held; ++i) {
+    uint32_t const kb = warp + Warps * i;
+    held[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (kb >= tiles_k || tok >= m) continue;
+    uint64_t const at = (uint64_t(tok) * tiles_k + kb) * 256 + lane * 8;
+    float4 const g0 = *reinterpret_cast<const float4*>(gate + at), g1 = *reinterpret_cast<const float4*>(gate + at + 4);
+    float4 const u0 = *reinterpret_cast<const float4*>(up + at), u1 = *reinterpret_cast<const float4*>(up + at + 4);
+    float const g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w}, u[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+    float x[8];
+    swiglu8(g, u, x);
+    Packed8 const z = quantize8(x);
+    valid = valid && z.valid;
+    row = fmaxf(row, fabsf(z.a));
+    held[i] = make_uint4(z.w0, z.w1, __float_as_uint(z.a), uint32_t(z.sum));
+  }
+  if (!valid) atomicExch(failure, 1);
+  row = block_top<Warps>(row, warp_top);
+#pragma unroll
+  for (int i = 0; i < Held; ++i) {
+    uint32_t const kb = warp + Warps * i;
+    if (kb >= tiles_k) break;
+    write_planes(__uint_as_float(held[i].z), int(held[i].w), make_uint2(held[i].x, held[i].y), row, tok, kb, m_pad, tiles_k * 256, planes, sums16,
+                 exps, tokens);
+  }
+}
+
+// Held: columns per thread in the norm (rms.cuh), Blocks: super-blocks per warp.
+template <int Held, int Blocks>
+__global__ void __launch_bounds__(256) rms_planes_kernel(const float* residual, const uint16_t* gamma, float eps, int* failure, uint32_t m,
+                                                         uint32_t m_pad, uint32_t tiles_k, __half* __restrict__ planes,
+                                                         __half* __restrict__ sums16, float* __restrict__ exps, float* __restrict__ tokens,
+                                                         uint32_t* __restrict__ tickets, uint32_t ticket_count) {
+  extern __shared__ __align__(16) uint16_t rounded[];
+  __shared__ float warp_top[8];
+  pdl_wait();
+  pdl_launch_dependents();
+  if (blockIdx.x == 0)
+    for (uint32_t i = threadIdx.x; i < ticket_count; i += 256) tickets[i] = 0u;
+  uint32_t const warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tok = blockIdx.x, hidden = tiles_k * 256;
+  if (tok < m) rms_row<Held>(residual + uint64_t(tok) * hidden, gamma, eps, hidden, rounded);
+  uint4 held[Blocks];
+  float row = 0.f;
+  bool valid = true;
+#pragma unroll
+  for (int i = 0; i < Blocks; ++i) {
+    uint32_t const kb = warp + 8 * i;
+    held[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (kb >= tiles_k || tok >= m) continue;
+    uint4 const v = *reinterpret_cast<const uint4*>(rounded + kb * 256 + lane * 8);
+    uint32_t const w[4] = {v.x, v.y, v.z, v.w};
+    float x[8];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) { x[2 * c] = __uint_as_float(w[c] << 16); x[2 * c + 1] = __uint_as_float(w[c] & 0xffff0000u); }
+    Packed8 const z = quantize8(x);
+    valid = valid && z.valid;
+    row = fmaxf(row, fabsf(z.a));
+    held[i] = make_uint4(z.w0, z.w1, __float_as_uint(z.a), uint32_t(z.sum));
+  }
+  if (!valid) atomicExch(failure, 1);
+  row = block_top(row, warp_top);
+#pragma unroll
+  for (int i = 0; i < Blocks; ++i) {
+    uint32_t const kb = warp + 8 * i;
+    if (kb >= tiles_k) break;
+    write_planes(__uint_as_float(held[i].z), int(held[i].w), make_uint2(held[i].x, held[i].y), row, tok, kb, m_pad, hidden, planes, sums16, exps,
+                 tokens);
   }
 }
 
@@ -860,13 +950,25 @@ cudaError_t launch_f16(const WeightView& w, const WeightView* second, const Q8Vi
   auto* const tickets = reinterpret_cast<uint32_t*>(scratch);
   uint32_t const ticket_count = plan.unit_step == 1 ? uint32_t(kTicketBytes / 4) : 0u;
   cudaError_t st;
-  if (raw) {
+  if (w.tiles_k > 128 && raw) return cudaErrorInvalidValue;  // sixteen super-blocks per warp
+  if (raw && raw->residual) {
+    auto kernel = w.tiles_k <= 8 ? rms_planes_kernel<8, 1> : (w.tiles_k <= 24 ? rms_planes_kernel<24, 3> : rms_planes_kernel<0, 16>);
+    uint32_t const smem = pk * 2;
+    if (smem > 48 * 1024 && (st = allow_smem(reinterpret_cast<const void*>(kernel), int(smem))) != cudaSuccess) return st;
+    st = launch_kernel(kernel, m_pad, 256, smem, stream, true, raw->residual, raw->gamma, raw->eps, raw->failure, x.m, m_pad, w.tiles_k, planes,
+                       sums, exps, tokens, tickets, ticket_count);
+  } else if (raw && raw->gate) {
+    // Wide rows get more warps, so that few tokens still fill the machine: an MLP chain of 237 tokens with K = 17408
+    // 266 us with eight warps, 259 with 32.
+    auto kernel = w.tiles_k <= 24 ? swiglu_planes_kernel<3, 8> : (w.tiles_k <= 96 ? swiglu_planes_kernel<3, 32> : swiglu_planes_kernel<4, 32>);
+    st = launch_kernel(kernel, m_pad, w.tiles_k <= 24 ? 256 : 1024, 0, stream, true, raw->gate, raw->up, raw->failure, x.m, m_pad, w.tiles_k, planes, sums, exps, tokens,
+                       tickets, ticket_count);
+  } else if (raw) {
     bool const vec = raw->k % 8 == 0 && reinterpret_cast<uintptr_t>(raw->x) % 16 == 0;
     // Few registers keep more rows in flight, but a row has to fit: three super-blocks per warp up to K = 6144, nine up to
     // 18432, sixteen for the largest K.  2048 rows with a matmul of 128 rows behind them, us, for three / nine / sixteen:
     // K = 2048 23.0 / 24.3 / 29.5, 5120 34.1 / 35.3 / 42.8, 17408 - / 133 / 146.
     auto kernel = w.tiles_k <= 24 ? rows_planes_kernel<3> : (w.tiles_k <= 72 ? rows_planes_kernel<9> : rows_planes_kernel<16>);
-    if (w.tiles_k > 128) return cudaErrorInvalidValue;
     st = launch_kernel(kernel, m_pad, 256, 0, stream, true, raw->x, raw->k, vec, raw->failure, x.m, m_pad, w.tiles_k, planes, sums,
                        exps, tokens, tickets, ticket_count);
   } else {
@@ -981,7 +1083,13 @@ cudaError_t launch_mmq_f16(const WeightView& w, const Q8View& x, const F16Output
     xc.m = x.m - t0 < plan.chunk ? x.m - t0 : plan.chunk;
     xc.codes += uint64_t(t0) * x.padded_k; xc.scales += t0 * G; xc.sums += t0 * G;
     RawRows rows{};
-    if (raw) { rows = *raw; rows.x += uint64_t(t0) * raw->k; }
+    if (raw) {
+      uint64_t const at = uint64_t(t0) * raw->k;
+      rows = *raw;
+      if (rows.x) rows.x += at;
+      if (rows.gate) { rows.gate += at; rows.up += at; }
+      if (rows.residual) rows.residual += at;
+    }
     const RawRows* const rc = raw ? &rows : nullptr;
     F16Output oc = out;
     oc.out += uint64_t(t0) * w.n;

@@ -10,11 +10,13 @@
 #include "common.cuh"
 #include "launch.h"
 #include "q8_pack.cuh"
+#include "rms.cuh"
+#include "swiglu.cuh"
 
 namespace q4k {
 namespace {
 
-constexpr int kThreads = 256, kBlocksPerSm = 6;
+constexpr int kThreads = kRmsThreads, kBlocksPerSm = 6;
 
 // Quantise the eight values of this lane; lanes (4j..4j+3) share a group.
 __device__ __forceinline__ void pack8(const float (&x)[8], int8_t* codes, float* scales,
@@ -85,16 +87,6 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) pack_kernel(const T* i
   }
 }
 
-// g / (1 + exp(-g)), rounded as the division would be (-0 gives +0, which changes no code).  A divisor above 2^64 is scaled
-// (exactly: the quotient of a finite g stays a normal number) and an infinite one replaced, so that no residual of the quotient
-// underflows.  Not finite for a g that is not.
-__device__ __forceinline__ float silu(float g) {
-  float const d = 1.f + expf(-g);
-  bool const far = d > 0x1p64f, lost = isinf(d);
-  float const by = lost ? 1.f : (far ? d * 0x1p-64f : d);
-  return rounded_quotient(g, by, __frcp_rn(by)) * (lost ? 0.f : (far ? 0x1p-64f : 1.f));
-}
-
 // v = bf16_rne(silu(g) * u); non-finite g or u poisons the value
 // (reference: swiglu_pack_kernel, cuda/q4k_q8.cu:52-61).  ffn % 256 == 0.
 __global__ void __launch_bounds__(kThreads) swiglu_pack_kernel(const float* gate, const float* up,
@@ -113,37 +105,12 @@ __global__ void __launch_bounds__(kThreads) swiglu_pack_kernel(const float* gate
     float g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
     float u[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
     float x[8];
-#pragma unroll
-    for (int i = 0; i < 8; i += 2) {  // what is not finite stays so and makes the group invalid
-      __nv_bfloat162 const v = __floats2bfloat162_rn(silu(g[i]) * u[i], silu(g[i + 1]) * u[i + 1]);
-      uint32_t const w = *reinterpret_cast<const uint32_t*>(&v);
-      x[i] = __uint_as_float(w << 16);
-      x[i + 1] = __uint_as_float(w & 0xffff0000u);
-    }
+    swiglu8(g, u, x);  // what is not finite makes the group invalid
     pack8(x, codes, scales, sums, task * 8 + grp, sub, failure);
   }
 }
 
-__device__ __forceinline__ float block_reduce(float v, float* scratch, bool is_max) {
-  for (int off = 16; off; off >>= 1) {
-    float o = __shfl_xor_sync(0xffffffffu, v, off);
-    v = is_max ? fmaxf(v, o) : v + o;
-  }
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
-  __syncthreads();
-  float r = scratch[0];
-  for (int i = 1; i < kThreads / 32; ++i) r = is_max ? fmaxf(r, scratch[i]) : r + scratch[i];
-  return r;
-}
-
-// Max-scaled RMS norm, (1 + gamma) gain, bf16 rounding, then the Q8 pack of the rounded row (reference:
-// hidden_rms_kernel<3>, cuda/activation.cu:134-190).  One block per token; hidden % 256 == 0; dynamic shared memory =
-// hidden * 2 bytes.  Thread t owns columns t, t + 256, ... and sums them in that order.
-//
-// Bound: latency (a decode step has a handful of rows).  With Held > 0 (hidden <= 256 * Held) a thread requests its whole
-// share of the row and of the gain at once and keeps it in registers for the three passes; the loop form, which serves
-// wider rows, waits for memory in every iteration of every pass: 15 us at 5120 columns against 4 us.
+// RMS norm, then the Q8 pack of the rounded row.  One block per token; dynamic shared memory = hidden * 2 bytes.
 template <int Held>
 __global__ void __launch_bounds__(kThreads) hidden_rms_q8_kernel(const float* residual, const uint16_t* gamma,
                                                                   float eps, uint32_t hidden,
@@ -152,57 +119,7 @@ __global__ void __launch_bounds__(kThreads) hidden_rms_q8_kernel(const float* re
   extern __shared__ __align__(16) uint16_t rounded[];
   pdl_wait();
   pdl_launch_dependents();
-  __shared__ float scratch[kThreads / 32];
-  const float* x = residual + uint64_t(blockIdx.x) * hidden;
-  float held[Held > 0 ? Held : 1], gain[Held > 0 ? Held : 1];
-  float scale = 0.f;
-  if constexpr (Held > 0) {
-#pragma unroll
-    for (int j = 0; j < Held; ++j) {
-      uint32_t const i = threadIdx.x + j * kThreads;
-      held[j] = i < hidden ? x[i] : 0.f;
-      gain[j] = i < hidden ? bf16_bits_to_f32(gamma[i]) : 0.f;
-    }
-#pragma unroll
-    for (int j = 0; j < Held; ++j) scale = fmaxf(scale, fabsf(held[j]));
-  } else {
-#pragma unroll 8
-    for (uint32_t i = threadIdx.x; i < hidden; i += kThreads) scale = fmaxf(scale, fabsf(x[i]));
-  }
-  scale = block_reduce(scale, scratch, true);
-  float const safe = scale == 0.f ? 1.f : scale;
-  float sumsq = 0.f;
-  if constexpr (Held > 0) {
-#pragma unroll
-    for (int j = 0; j < Held; ++j) {
-      held[j] = held[j] / safe;
-      if (threadIdx.x + j * kThreads < hidden) sumsq += held[j] * held[j];
-    }
-  } else {
-#pragma unroll 8
-    for (uint32_t i = threadIdx.x; i < hidden; i += kThreads) {
-      float s = x[i] / safe;
-      sumsq += s * s;
-    }
-  }
-  sumsq = block_reduce(sumsq, scratch, false);
-  float const se = sqrtf(eps) / safe;
-  float const inv = 1.0f / sqrtf(sumsq / float(hidden) + se * se);
-  if constexpr (Held > 0) {
-#pragma unroll
-    for (int j = 0; j < Held; ++j) {
-      uint32_t const i = threadIdx.x + j * kThreads;
-      if (i < hidden) rounded[i] = f32_to_bf16_rne((1.0f + gain[j]) * (held[j] * inv));
-    }
-  } else {
-#pragma unroll 4
-    for (uint32_t i = threadIdx.x; i < hidden; i += kThreads) {
-      float g = bf16_bits_to_f32(gamma[i]);
-      float v = (1.0f + g) * ((x[i] / safe) * inv);
-      rounded[i] = f32_to_bf16_rne(v);
-    }
-  }
-  __syncthreads();
+  rms_row<Held>(residual + uint64_t(blockIdx.x) * hidden, gamma, eps, hidden, rounded);
   uint32_t const lane = threadIdx.x & 31, sub = lane & 3, grp = lane >> 2;
   for (uint32_t chunk = threadIdx.x / 32; chunk < hidden / 256; chunk += kThreads / 32) {
     uint32_t const col0 = chunk * 256 + grp * 32 + sub * 8;

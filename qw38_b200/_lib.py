@@ -5,7 +5,11 @@ and if that is impossible it raises.  There is no CPU or PyTorch fallback."""
 from __future__ import annotations
 
 import ctypes as C
+from importlib.machinery import ExtensionFileLoader
+from importlib.util import module_from_spec, spec_from_loader
 from pathlib import Path
+
+import torch
 
 from . import build as _build
 
@@ -108,6 +112,15 @@ SIGNATURES = {
 }
 
 _lib = None
+_entries = None
+
+
+def entries():
+    """The extension module through which Python callers reach the entries of a decode step (csrc/py_entries.cpp), bound to the
+    loaded library."""
+    if _entries is None:
+        load()
+    return _entries
 
 
 def library_path() -> Path:
@@ -116,7 +129,7 @@ def library_path() -> Path:
 
 def load() -> C.CDLL:
     """Load (building first if the sources are newer) and type every entry point."""
-    global _lib
+    global _lib, _entries
     if _lib is not None:
         return _lib
     import os
@@ -126,5 +139,12 @@ def load() -> C.CDLL:
     for name, (res, args) in SIGNATURES.items():
         fn = getattr(lib, name)  # AttributeError here = header and library disagree
         fn.restype, fn.argtypes = res, args
-    _lib = lib
+    loader = ExtensionFileLoader("_q4k_entries", str(_build.ENTRIES))
+    module = module_from_spec(spec_from_loader("_q4k_entries", loader))
+    loader.exec_module(module)
+    names = ("q4k_decode_mmv", "q4k_decode_mmv_ranges", "q4k_pack_q8_bf16", "q4k_pack_q8_f32", "q4k_q8_project", "q4k_q8_mlp",
+             "q4k_prefill_project", "q4k_prefill_paired_swiglu")
+    module.bind(*(C.cast(getattr(lib, name), C.c_void_p).value for name in names), torch._C._cuda_getDevice,
+                torch._C._cuda_getCurrentRawStream)
+    _lib, _entries = lib, module
     return lib

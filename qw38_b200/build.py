@@ -4,11 +4,13 @@ from __future__ import annotations
 import os
 import shutil
 import subprocess
+import sysconfig
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB = PKG / "lib" / "libq4k_b200.so"
+ENTRIES = PKG / "lib" / "_q4k_entries.so"  # Python's way into the entries of a decode step (csrc/py_entries.cpp)
 SOURCES = ["abi.cu", "q8_quantize.cu", "gemv_dp4a.cu", "gemv_mma.cu", "gemv_tma.cu", "mmq_mma.cu", "mmq_tcgen05.cu", "mmq_f16.cu", "stream_scratch.cu", "repack.cu", "no_alloc.cu", "peer.cu", "decode_entry.cu", "gemv_bf16w.cu", "fit_q4k.cu", "int8_peak.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -24,10 +26,10 @@ def nvcc() -> str:
 
 
 def needs_build() -> bool:
-    if not LIB.exists():
+    if not LIB.exists() or not ENTRIES.exists():
         return True
-    t = LIB.stat().st_mtime
-    deps = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) + \
+    t = min(LIB.stat().st_mtime, ENTRIES.stat().st_mtime)
+    deps = list(CSRC.glob("*.cpp")) + list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) + \
         [PKG.parent / "include" / "q4k_b200.h"]
     return any(d.stat().st_mtime > t for d in deps)
 
@@ -58,6 +60,10 @@ def _build_locked(verbose: bool) -> Path:
         obj = objdir / (src + ".o")
         cmd = [nvcc(), *NVCC_FLAGS, "-Xptxas", "-v" if verbose else "-warn-spills", "-c", str(CSRC / src), "-o", str(obj)]
         procs.append((src, obj, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
+    entries = ENTRIES.with_suffix(f".so.tmp{os.getpid()}")
+    cmd = ["g++", "-O2", "-std=c++17", "-Wall", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"], str(CSRC / "py_entries.cpp"), "-o",
+           str(entries)]
+    host = subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     objs = []
     for src, obj, p in procs:
         out, _ = p.communicate()
@@ -71,6 +77,10 @@ def _build_locked(verbose: bool) -> Path:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"link failed:\n{r.stdout}{r.stderr}")
+    out, _ = host.communicate()
+    if host.returncode != 0:
+        raise RuntimeError(f"g++ failed on py_entries.cpp:\n{out}")
+    os.replace(entries, ENTRIES)
     os.replace(tmp, LIB)
     return LIB
 

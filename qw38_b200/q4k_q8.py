@@ -77,7 +77,7 @@ class PrefillWeight:
         return pad_k(self.k)
 
     # The descriptors of this module are handed to C for reading only, so the last one built is kept next to what it was
-    # built from and serves again while that is unchanged (0.6 us to compare, 1.3 to build; a decode call has up to four).
+    # built from and serves again while that is unchanged (0.6 us to compare, 1.3 to build).
     _built = None
 
     def c_struct(self) -> L.Weight:
@@ -143,19 +143,15 @@ def new_q8_input(m: int, k: int, device="cuda") -> Q8Input:
 def pack_q8(x: torch.Tensor, failure: torch.Tensor, out: Optional[Q8Input] = None, stream=None) -> Q8Input:
     """pack_q8 (cuda/q4k_q8.hpp:32-34): bf16 (or fp32) rows [m, k] -> Q8.  `failure` is one
     int32 on the device that the caller cleared; a non-finite group sets it to 1."""
-    lib = L.load()
     if x.dim() != 2 or not x.is_contiguous():
         raise Q4KError(L.ERR_INVALID_ARGUMENT, "pack_q8 takes a contiguous [m, k] tensor")
     m, k = x.shape
     if out is None:
         out = new_q8_input(m, k, x.device)
-    if x.dtype == torch.bfloat16:
-        fn = lib.q4k_pack_q8_bf16
-    elif x.dtype == torch.float32:
-        fn = lib.q4k_pack_q8_f32
-    else:
+    fp32 = x.dtype == torch.float32
+    if not fp32 and x.dtype != torch.bfloat16:
         raise Q4KError(L.ERR_INVALID_ARGUMENT, "pack_q8 takes bf16 or fp32")
-    _check(fn(_ptr(x), x.numel(), out.c_struct(), _ptr(failure), _stream(stream)))
+    _check(L.entries().pack_q8(x, fp32, out, failure, stream))
     return out
 
 
@@ -165,15 +161,13 @@ def q4k_q8_project(weight: PrefillWeight, x: Q8Input, out: Optional[torch.Tensor
                    trusted: bool = False, input_settled: bool = False, stream=None) -> torch.Tensor:
     """q4k_q8_project (cuda/q4k_q8.hpp:35-37): fp32 out[token, row], token-major.
     `input_settled`: Q4K_FLAG_INPUT_SETTLED (x and residual were not written by the launch directly before)."""
-    lib = L.load()
     if out is None:
         out = torch.empty((x.m, weight.n), dtype=torch.float32, device=x.codes.device)
-    w = weight.c_struct()
     plain = kernel == L.KERNEL_AUTO and split_k == 0 and row_groups == 0 and partials is None and workspace is None and not trusted and not input_settled
     if plain:
-        _check(lib.q4k_q8_project(C.byref(w), x.c_struct(), _ptr(out), out.numel(), _ptr(residual),
-                                  0 if residual is None else residual.numel(), _stream(stream)))
+        _check(L.entries().q8_project(weight, x, out, residual, stream))
     else:
+        lib, w = L.load(), weight.c_struct()
         opt = L.ProjectOptions(kernel, split_k, row_groups, 0 if partials is None else partials.data_ptr(),
                                0 if partials is None else partials.numel(),
                                0 if workspace is None else workspace.data_ptr(),
@@ -286,8 +280,7 @@ def decode_workspace(m: int, n_total: int, k: int, device="cuda") -> torch.Tenso
 
 def launch_decode_mmv(desc: DecodeMmvDesc, workspace: torch.Tensor, failure: torch.Tensor, stream=None) -> None:
     """launch_decode_mmv (cuda/decode_mmv.hpp:207-209)."""
-    d = desc.c_struct()
-    _check(L.load().q4k_decode_mmv(C.byref(d), _ptr(workspace), workspace.numel(), _ptr(failure), _stream(stream)))
+    _check(L.entries().decode_mmv(desc, workspace, failure, stream))
 
 
 def launch_decode_mmv_paired(a: DecodeMmvDesc, b: DecodeMmvDesc, workspace: torch.Tensor, failure: torch.Tensor,
@@ -301,23 +294,18 @@ def launch_decode_mmv_paired(a: DecodeMmvDesc, b: DecodeMmvDesc, workspace: torc
 def launch_decode_mmv_ranges(ranges: Sequence[DecodeMmvDesc], workspace: torch.Tensor, failure: torch.Tensor,
                              stream=None) -> None:
     """launch_decode_mmv_ranges (cuda/decode_mmv.hpp:212-215): two or three output ranges over one input."""
-    arr = (L.DecodeDesc * len(ranges))(*[r.c_struct() for r in ranges])
-    _check(L.load().q4k_decode_mmv_ranges(arr, len(ranges), _ptr(workspace), workspace.numel(), _ptr(failure),
-                                          _stream(stream)))
+    _check(L.entries().decode_mmv_ranges(ranges, workspace, failure, stream))
 
 
 def prefill_project(projection: DecodeMmvDesc, workspace: torch.Tensor, failure: torch.Tensor, stream=None) -> None:
     """PrefillEngine::project (cuda/prefill.hpp:88-89) for a Q4_K weight: quantise -> MMQ -> PrefillEpilogue."""
-    d = projection.c_struct()
-    _check(L.load().q4k_prefill_project(C.byref(d), _ptr(workspace), workspace.numel(), _ptr(failure), _stream(stream)))
+    _check(L.entries().prefill_project(projection, workspace, failure, stream))
 
 
 def prefill_paired_swiglu(gate: PrefillWeight, up: PrefillWeight, normalized: torch.Tensor, swiglu: torch.Tensor,
                           workspace: torch.Tensor, failure: torch.Tensor, stream=None) -> None:
     """PrefillEngine::paired_swiglu (cuda/prefill.hpp:90-93): swiglu = bf16(SiLU(gate x) * (up x))."""
-    g, u = gate.c_struct(), up.c_struct()
-    _check(L.load().q4k_prefill_paired_swiglu(C.byref(g), C.byref(u), _ptr(normalized), _ptr(swiglu), normalized.shape[0],
-                                              _ptr(workspace), workspace.numel(), _ptr(failure), _stream(stream)))
+    _check(L.entries().prefill_paired_swiglu(gate, up, normalized, swiglu, normalized.shape[0], workspace, failure, stream))
 
 
 def q8_mlp_workspace_bytes(m: int, hidden: int, ffn: int) -> int:
@@ -329,17 +317,12 @@ def q4k_q8_mlp(gate: PrefillWeight, up: PrefillWeight, down: PrefillWeight, resi
                pending_failure: Optional[torch.Tensor] = None, stream=None) -> bool:
     """q4k_q8_mlp (cuda/q4k_q8.hpp:44-49).  Returns `submitted`; raises Q4KError on rejection
     or, in the synchronous form (pending_failure None), on a non-finite producer."""
-    lib = L.load()
-    submitted = C.c_int(0)
-    g, u, d = gate.c_struct(), up.c_struct(), down.c_struct()
-    st = lib.q4k_q8_mlp(C.byref(g), C.byref(u), C.byref(d), _ptr(residual), _ptr(gamma), eps, _ptr(out), m,
-                        _ptr(workspace), workspace.numel() * workspace.element_size(), _stream(stream),
-                        C.byref(submitted), _ptr(pending_failure))
+    st, submitted = L.entries().q8_mlp(gate, up, down, residual, gamma, eps, out, m, workspace, pending_failure, stream)
     if st != L.OK:
-        err = Q4KError(st, lib.q4k_last_error().decode())
-        err.submitted = bool(submitted.value)
+        err = Q4KError(st, L.load().q4k_last_error().decode())
+        err.submitted = bool(submitted)
         raise err
-    return bool(submitted.value)
+    return bool(submitted)
 
 
 def hidden_rms_q8(residual: torch.Tensor, gamma: torch.Tensor, eps: float, failure: torch.Tensor,

@@ -156,8 +156,8 @@ __global__ void __launch_bounds__(kThreads, M <= 2 ? 2 : 1) gemv_dp4a_kernel(con
       if (p.wide) {
         for (uint32_t i = 0; i < p.stages; ++i) mbar_init(bars + i * 8, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        if (!p.early) {  // the ring's first fill comes out of L2 after the wait
-          for (uint32_t i = 0, u = u0; i < p.stages && u < u1; ++i) {
+        if (!p.early) {  // the first stages come out of L2 after the wait (two: more get in the way of the kernel before)
+          for (uint32_t i = 0, u = u0; i < 2 && u < u1; ++i) {
             uint32_t const count = stage_units(p, u, u1);
             DpSegment const& s = segment_of(p, u);
             prefetch_l2(s.codes + uint64_t(u - s.u0) * 1024, count * 1024);
@@ -373,9 +373,12 @@ cudaError_t launch_split(DpParams p, uint32_t m, uint32_t padded_k, cudaStream_t
     p.seg[i].u0 = p.rgs * p.tiles_k;
     p.rgs += (p.seg[i].n + 7) / 8;
   }
-  // One block per SM, or as many rounds of them as bound a block's row groups.
-  uint32_t const sms = uint32_t(sm_count()), waves = (p.rgs + sms * kMaxRowGroups - 1) / (sms * kMaxRowGroups);
-  uint32_t const grid = p.rgs < sms * waves ? p.rgs : sms * waves;
+  // As many rounds of blocks as bound a block's row groups.  Of 148 blocks that fill half an SM each the hardware puts two on
+  // nine SMs, and these end last: 11 us after the others on 34816 x 5120 beside the next projection.  Two blocks per SM fill every
+  // half (bf16 rows, one token, us: 5120 x 5120 8.9 -> 7.2, 30000 x 7000 26.4 -> 23.7, a layer 78 -> 67).  For Q8 input there is one:
+  // a pack before or behind finds room beside it (pack and 17408 x 5120 14.5 against 15.1, four small layers 74 against 79).
+  uint32_t const slots = uint32_t(sm_count()) * (p.raw ? 2 : 1), waves = (p.rgs + slots * kMaxRowGroups - 1) / (slots * kMaxRowGroups);
+  uint32_t const grid = p.rgs < slots * waves ? p.rgs : slots * waves;
   p.rgs_each = p.rgs / grid;
   p.rgs_rest = p.rgs % grid;
   uint32_t const units = (p.rgs_each + (p.rgs_rest ? 1 : 0)) * p.tiles_k;

@@ -468,19 +468,28 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
       for (uint32_t i = lane; i < NT * 64; i += 32) sts32f(tab + kTabBytes + i * 4, 0.f);
       for (uint32_t t0 = 0; t0 < p.m; t0 += 4) {
         __syncwarp();
-        for (uint32_t j = 0; j < 4 && t0 + j < p.m; ++j) {
+        uint4 held[4];  // the four tokens' columns, requested together: one round trip per pass
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
           const uint16_t* const src = p.xraw + size_t(t0 + j) * p.xk;
           uint32_t const col = sb * 256 + lane * 8;
-          float x[8];
-          if (p.xvec && col + 8 <= p.xk) {
-            uint4 const v = *reinterpret_cast<const uint4*>(src + col);
-            uint32_t const vw[4] = {v.x, v.y, v.z, v.w};
+          held[j] = make_uint4(0u, 0u, 0u, 0u);
+          if (t0 + j >= p.m) continue;
+          if (p.xvec && col + 8 <= p.xk) held[j] = *reinterpret_cast<const uint4*>(src + col);
+          else {
+            uint32_t v[8];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) { x[2 * i] = __uint_as_float(vw[i] << 16); x[2 * i + 1] = __uint_as_float(vw[i] & 0xffff0000u); }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) x[i] = col + i < p.xk ? bf16_bits_to_f32(src[col + i]) : 0.f;
+            for (int i = 0; i < 8; ++i) v[i] = col + i < p.xk ? src[col + i] : 0u;
+            held[j] = make_uint4(v[0] | v[1] << 16, v[2] | v[3] << 16, v[4] | v[5] << 16, v[6] | v[7] << 16);
           }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (t0 + j >= p.m) break;
+          uint32_t const vw[4] = {held[j].x, held[j].y, held[j].z, held[j].w};
+          float x[8];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) { x[2 * i] = __uint_as_float(vw[i] << 16); x[2 * i + 1] = __uint_as_float(vw[i] & 0xffff0000u); }
           Packed8 const z = quantize8(x);
           asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(tab + j * 256 + lane * 8), "r"(z.w0), "r"(z.w1) : "memory");
           if ((lane & 3) == 0) {
@@ -513,31 +522,52 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
                  __uint_as_float(lds32(tab + 1024 + ((lane >> 3) * 8 + g) * 4)));
       }
     } else {
+      // All loads before the first store: the compiler keeps loads behind an earlier store, and with the table written
+      // between the groups the fill was a chain of eight round trips to L2 per token octet, before the first tile.  In one
+      // round trip (5120 / 17408 chains, L2 cold): MLP of 4 tokens 57.0 -> 53.4 us, of 13 tokens 84.5 -> 82.6, four layers
+      // of 4 tokens 242 -> 217; 12 tokens by 7168 x 5120 alone 18.7 -> 16.3.
+      float scale[2 * NT];  // token i / 8, group i % 8 of i = lane, lane + 32, ...
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-      uint32_t const tokb = nt * 8 + r, tokc = nt * 8 + 2 * q;
+      for (int j = 0; j < 2 * NT; ++j) {
+        uint32_t const tok = (lane + 32 * j) >> 3;
+        scale[j] = tok < p.m ? p.xscales[size_t(tok) * p.G + sb * 8 + (lane & 7)] : 0.f;
+      }
+      float as[NT][2];
 #pragma unroll
-      for (int g = 0; g < 8; ++g) {
-        uint2 z = make_uint2(0u, 0u);
-        if (tokb < p.m) z = *reinterpret_cast<const uint2*>(p.xcodes + size_t(tokb) * p.padded_k + sb * 256 + g * 32 + q * 8);
-        bfrag[nt][g][0] = even_bytes(z.x, z.y);
-        bfrag[nt][g][1] = odd_bytes(z.x, z.y);
-        if (r == 0) {  // lanes 0..3 fill the scale-pair table of this warp
-          float const a0 = tokc < p.m ? p.xscales[size_t(tokc) * p.G + sb * 8 + g] : 0.f;
-          float const a1 = tokc + 1 < p.m ? p.xscales[size_t(tokc + 1) * p.G + sb * 8 + g] : 0.f;
-          asm volatile("st.shared.v2.f32 [%0], {%1,%2};" ::"r"(rd_ap + (nt * 4 + g / 2) * 64 + (g % 2) * 8), "f"(a0), "f"(a1) : "memory");
+      for (int nt = 0; nt < NT; ++nt) {
+        uint32_t const tokb = nt * 8 + r;
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+          uint2 z = make_uint2(0u, 0u);
+          if (tokb < p.m) z = *reinterpret_cast<const uint2*>(p.xcodes + size_t(tokb) * p.padded_k + sb * 256 + g * 32 + q * 8);
+          bfrag[nt][g][0] = z.x;
+          bfrag[nt][g][1] = z.y;
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          as[nt][h] = 0.f;
+          if (tokb < p.m) {
+            size_t const i = size_t(tokb) * p.G + sb * 8 + q + 4 * h;
+            as[nt][h] = p.xscales[i] * float(p.xsums[i]);
+          }
         }
       }
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        float as = 0.f;
-        if (tokb < p.m) {
-          size_t const i = size_t(tokb) * p.G + sb * 8 + q + 4 * h;
-          as = p.xscales[i] * float(p.xsums[i]);
-        }
-        split(nt, h, as);
+      for (int j = 0; j < 2 * NT; ++j) {
+        uint32_t const tok = (lane + 32 * j) >> 3, g = lane & 7;
+        sts32f(tab + kTabBytes + ((tok & 7) >> 1) * 16 + ((tok >> 3) * 4 + g / 2) * 64 + (g % 2) * 8 + (tok & 1) * 4, scale[j]);
       }
-    }
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+          uint32_t const z0 = bfrag[nt][g][0], z1 = bfrag[nt][g][1];
+          bfrag[nt][g][0] = even_bytes(z0, z1);
+          bfrag[nt][g][1] = odd_bytes(z0, z1);
+        }
+        split(nt, 0, as[nt][0]);
+        split(nt, 1, as[nt][1]);
+      }
     }
     __syncwarp();
     float2 const nmagic2 = make_float2(-kMagicF, -kMagicF);

@@ -42,7 +42,7 @@
 
 #include "common.cuh"
 #include "launch.h"
-#include "q8_pack.cuh"
+#include "swiglu.cuh"
 #include "tma.cuh"
 
 namespace q4k {
@@ -136,12 +136,6 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 as_f2(uint32_t x, uint32_t y) { return make_float2(__uint_as_float(x), __uint_as_float(y)); }
 
-// sigmoid / SiLU as the reference's decode epilogue states them (cuda/decode_mmv.cu:78-89): the exponential is
-// always taken of a non-positive number.
-__device__ __forceinline__ float silu_fp32(float u) {
-  float const e = expf(u >= 0.0f ? -u : u);
-  return u * (u >= 0.0f ? 1.0f / (1.0f + e) : e / (1.0f + e));
-}
 // Which weight a global tile index of a multi-weight launch belongs to, and the tile's index inside it.
 __device__ __forceinline__ void locate_tile(const GtParams& p, uint32_t T, uint32_t& s, uint32_t& local) {
   if (p.pair) { s = T & 1u; local = T >> 1; return; }
@@ -306,70 +300,52 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
           if constexpr (Quant > 0) {
             // The activation of the down projection, quantised here (the arithmetic of swiglu_pack_kernel,
             // cuda/q4k_q8.cu:52-61): x = bf16(g / (1 + exp(-g)) * u), a non-finite input poisons the value.  The first
-            // half's values are kept as they are: the exponentials and divisions of a group come after its last hand-off,
-            // while the other reducer takes the next group's tiles (one reducer for all made a tile 2.8 us, not 1.5).
+            // half's values are kept as they are: the exponentials and quotients of a group come after its last hand-off,
+            // while the other reducer takes the next group's tiles.  Bound: the consumers run dry if this takes longer than
+            // their next tiles.  Quotients by divisions leave their short form at zeros (padded tokens) and tiny values and
+            // made it 10 to 14 thousand clocks per group; through reciprocals the MLP of 13 tokens takes 75.9 us (82.5), of
+            // 4 tokens 48.8 (53.4).
             if ((local & 1u) == 0) {
               pg[0] = g00; pg[1] = g01; pg[2] = g10; pg[3] = g11;
               pu[0] = v00; pu[1] = v01; pu[2] = v10; pu[3] = v11;
               continue;
             }
-            auto act = [](float gv, float uv) {
-              float v = (gv / (1.f + expf(-gv))) * uv;
-              if (!isfinite(gv) || !isfinite(uv)) v = __int_as_float(0x7fc00000);
-              return bf16_bits_to_f32(f32_to_bf16_rne(v));
+            auto act = [](float g0, float u0, float g1, float u1, float (&x)[2]) {  // one row, two tokens; what is not finite stays so
+              __nv_bfloat162 const v = __floats2bfloat162_rn(silu(g0) * u0, silu(g1) * u1);
+              uint32_t const w = *reinterpret_cast<const uint32_t*>(&v);
+              x[0] = __uint_as_float(w << 16);
+              x[1] = __uint_as_float(w & 0xffff0000u);
             };
-            float const cx[4] = {act(g00, v00), act(g01, v01), act(g10, v10), act(g11, v11)};  // (row r | r+8) x (token 0 | 1)
-            float px[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) px[i] = act(pg[i], pu[i]);
             // Second tile of a 32-row group: this lane holds rows r, r+8, 16+r, 24+r of the group for two tokens; the
             // eight lanes with the same q hold the rest.
+            float x[4][2];
+            act(pg[0], pu[0], pg[1], pu[1], x[0]);
+            act(pg[2], pu[2], pg[3], pu[3], x[1]);
+            act(g00, v00, g01, v01, x[2]);
+            act(g10, v10, g11, v11, x[3]);
+            Packed4x2 const z = quantize4x2(x);
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-              float const xv[4] = {px[e], px[2 + e], cx[e], cx[2 + e]};
-              bool finite = true;
-              float peak = 0.f;
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                bool const f = isfinite(xv[i]);
-                finite = finite && f;
-                peak = fmaxf(peak, f ? fabsf(xv[i]) : 0.f);
-              }
-              int fin = finite ? 1 : 0;
-#pragma unroll
-              for (int off = 4; off < 32; off <<= 1) {
-                peak = fmaxf(peak, __shfl_xor_sync(0xffffffffu, peak, off));
-                fin &= __shfl_xor_sync(0xffffffffu, fin, off);
-              }
-              float const a = peak == 0.f ? 1.f : __fdiv_rn(peak, 127.f);
-              bool const valid = fin && isfinite(a) && a > 0.f;
-              int z[4], sum = 0;
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                z[i] = valid ? max(-127, min(127, __float2int_rn(__fdiv_rn(xv[i], a)))) : 0;
-                sum += z[i];
-              }
-#pragma unroll
-              for (int off = 4; off < 32; off <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
               uint32_t const tok = tok0 + e;
               if (tok < p.m) {
                 int8_t* const c = p.q8_codes + size_t(tok) * p.q8_pk + (local - 1) * 16 + r;
-                c[0] = int8_t(z[0]); c[8] = int8_t(z[1]); c[16] = int8_t(z[2]); c[24] = int8_t(z[3]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) c[8 * i] = int8_t(z.z[i][e]);
                 if (r == 0) {
                   size_t const gi = size_t(tok) * (p.q8_pk / 32) + (local >> 1);
-                  p.q8_scales[gi] = valid ? a : __int_as_float(0x7fc00000);
-                  p.q8_sums[gi] = sum;
-                  if (!valid) atomicExch(p.q8_failure, 1);
+                  p.q8_scales[gi] = z.a[e];
+                  p.q8_sums[gi] = z.sum[e];
+                  if (!z.valid[e]) atomicExch(p.q8_failure, 1);
                 }
               }
             }
             continue;
           }
           uint16_t* const ob = p.seg[0].out_bf16;
-          if (in0 && live0) ob[a0] = f32_to_bf16_rne(silu_fp32(g00) * v00);
-          if (in0 && live1) ob[a1] = f32_to_bf16_rne(silu_fp32(g01) * v01);
-          if (in1 && live0) ob[a0 + 8] = f32_to_bf16_rne(silu_fp32(g10) * v10);
-          if (in1 && live1) ob[a1 + 8] = f32_to_bf16_rne(silu_fp32(g11) * v11);
+          if (in0 && live0) ob[a0] = f32_to_bf16_rne(g00 * sigmoid_fp32(g00) * v00);
+          if (in0 && live1) ob[a1] = f32_to_bf16_rne(g01 * sigmoid_fp32(g01) * v01);
+          if (in1 && live0) ob[a0 + 8] = f32_to_bf16_rne(g10 * sigmoid_fp32(g10) * v10);
+          if (in1 && live1) ob[a1 + 8] = f32_to_bf16_rne(g11 * sigmoid_fp32(g11) * v11);
           continue;
         }
         if (S.residual) {
@@ -722,7 +698,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
           size_t const o2 = size_t(tok) * p.n_total + p.seg[1].row_base + row;
           float u = __ldcg(p.slices + o2);
           for (uint32_t sl = 1; sl < p.split_k; ++sl) u += __ldcg(p.slices + sl * plane + o2);
-          p.seg[0].out_bf16[oo] = f32_to_bf16_rne(silu_fp32(v) * u);
+          p.seg[0].out_bf16[oo] = f32_to_bf16_rne(v * sigmoid_fp32(v) * u);
           continue;
         }
         if (S.residual) v += S.residual[oo];

@@ -84,4 +84,63 @@ __device__ __forceinline__ Packed8 quantize8(const float (&x)[8]) {
   return r;
 }
 
+struct Packed4x2 {
+  int z[4][2];  // codes of this lane's four values of either group
+  float a[2];   // scale and sum of the groups, in all eight lanes
+  int sum[2];
+  bool valid[2];
+};
+
+// The same for two groups (two tokens) held by the eight lanes with one lane & 3, four values of each per lane (x[i][e]: group e).
+// Executed by full warps.
+__device__ __forceinline__ Packed4x2 quantize4x2(const float (&x)[4][2]) {
+  constexpr uint32_t kBias = 0x4B400000u;  // 1.5 * 2^23
+  uint32_t top[2];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    top[e] = 0u;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) top[e] = max(top[e], __float_as_uint(x[i][e]) & 0x7fffffffu);
+  }
+#pragma unroll
+  for (int off = 4; off < 32; off <<= 1)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) top[e] = max(top[e], __shfl_xor_sync(0xffffffffu, top[e], off));
+  float const p0 = __uint_as_float(top[0]), p1 = __uint_as_float(top[1]);
+  Packed4x2 r;
+  bool const easy = (top[0] == 0u || (p0 >= 0x1p-73f && p0 <= 0x1p106f)) && (top[1] == 0u || (p1 >= 0x1p-73f && p1 <= 0x1p106f));
+  if (__all_sync(0xffffffffu, easy)) {
+    constexpr float kInv127 = 1.f / 127.f;
+    float2 const a2 = make_float2(top[0] == 0u ? 1.f : rounded_quotient(p0, 127.f, kInv127), top[1] == 0u ? 1.f : rounded_quotient(p1, 127.f, kInv127));
+    float2 const inv2 = make_float2(__frcp_rn(a2.x), __frcp_rn(a2.y)), bias = make_float2(12582912.f, 12582912.f);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float2 const q = __fadd2_rn(rounded_quotients(make_float2(x[i][0], x[i][1]), a2, inv2), bias);
+      r.z[i][0] = int(__float_as_uint(q.x) - kBias);
+      r.z[i][1] = int(__float_as_uint(q.y) - kBias);
+    }
+    r.a[0] = a2.x;
+    r.a[1] = a2.y;
+    r.valid[0] = r.valid[1] = true;
+  } else {
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      float const a = top[e] == 0u ? 1.f : __fdiv_rn(__uint_as_float(top[e]), 127.f);
+      r.valid[e] = top[e] < 0x7f800000u && a > 0.f;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) r.z[i][e] = r.valid[e] ? max(-127, min(127, __float2int_rn(__fdiv_rn(x[i][e], a)))) : 0;
+      r.a[e] = r.valid[e] ? a : __int_as_float(0x7fc00000);
+    }
+  }
+  // both sums are below 2^15 in magnitude: one word carries them
+  int both = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) both += r.z[i][0] + r.z[i][1] * 65536;
+#pragma unroll
+  for (int off = 4; off < 32; off <<= 1) both += __shfl_xor_sync(0xffffffffu, both, off);
+  r.sum[0] = int(int16_t(uint16_t(uint32_t(both) & 0xffffu)));
+  r.sum[1] = (both - r.sum[0]) >> 16;
+  return r;
+}
+
 }  // namespace q4k

@@ -1,0 +1,58 @@
+"""The activations inside the MLP chain.  Up to sixteen tokens the gate / up launch quantises its own product; beyond, the operand
+planes of both projections come straight from the residual stream and from the gate and up rows.  Each form against the separate
+launches, at the edges of its kernels and where the quantiser leaves its reciprocals (tiny, huge, non-finite and zero groups)."""
+import numpy as np
+import pytest
+import torch
+
+from qw38_b200 import _lib as L
+from qw38_b200 import synth
+from qw38_b200.q4k_q8 import hidden_rms_q8, q4k_q8_mlp, q4k_q8_project, q8_mlp_workspace_bytes, swiglu_pack_q8
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def chain(m, hidden, ffn, scale, poison=None):
+    gate, up, down = (synth.device_weight(ffn, hidden, seed=11), synth.device_weight(ffn, hidden, seed=12),
+                      synth.device_weight(hidden, ffn, seed=13))
+    h = torch.from_numpy(synth.activations(m, hidden, seed=m, scale=2.0)).to(DEV)
+    gamma = (torch.from_numpy(np.random.default_rng(m).standard_normal(hidden).astype(np.float32)) * scale).to(torch.bfloat16).to(DEV)
+    if poison is not None:
+        h[m - 1, hidden // 3] = poison
+    ws = torch.zeros(q8_mlp_workspace_bytes(m, hidden, ffn), dtype=torch.uint8, device=DEV)
+    out = torch.empty((m, hidden), dtype=torch.float32, device=DEV)
+    flag, other = torch.zeros(1, dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    assert q4k_q8_mlp(gate, up, down, h, gamma, 1e-6, out, m, ws, pending_failure=flag) is True
+    return gate, up, down, h, gamma, ws, out, flag, other
+
+
+@pytest.mark.parametrize("m", [2, 7, 9, 16])
+@pytest.mark.parametrize("scale", [0.0, 1e-30, 1e-12, 1e-11, 1e16, 1e17, 1e25])
+def test_reducers_quantise_as_the_separate_launch(m, scale):
+    hidden, ffn = 1024, 2048
+    gate, up, down, h, gamma, ws, out, flag, other = chain(m, hidden, ffn, scale)
+    x = hidden_rms_q8(h, gamma, 1e-6, other)
+    q = swiglu_pack_q8(q4k_q8_project(gate, x, kernel=L.KERNEL_GEMV_TMA), q4k_q8_project(up, x, kernel=L.KERNEL_GEMV_TMA), other)
+    n, g = m * ffn, m * (ffn // 32)
+    assert torch.equal(ws[:n].view(torch.int8), q.codes.view(-1))
+    scales, ref = ws[n:n + 4 * g].view(torch.float32), q.scales.view(-1)
+    assert torch.equal(torch.isnan(scales), torch.isnan(ref)) and torch.equal(scales.nan_to_num(), ref.nan_to_num())
+    assert torch.equal(ws[n + 4 * g:n + 8 * g].view(torch.int32), q.sums.view(-1))
+    assert flag.item() == other.item() == int(torch.isnan(ref).any())
+
+
+# tiles of K: up to 8, 24 and beyond (RMS); up to 24, 96 and beyond (SwiGLU).  Tokens: padded to 32, 64, 128 and one more tile.
+@pytest.mark.parametrize("m,hidden,ffn", [(17, 2048, 6144), (33, 2304, 6400), (64, 6144, 2048), (65, 6400, 24576), (130, 1024, 24832)])
+@pytest.mark.parametrize("poison", [None, float("nan")])
+def test_planes_equal_the_separate_launches(m, hidden, ffn, poison):
+    gate, up, down, h, gamma, ws, out, flag, other = chain(m, hidden, ffn, 0.1, poison)
+    x = hidden_rms_q8(h, gamma, 1e-6, other)
+    q = swiglu_pack_q8(q4k_q8_project(gate, x), q4k_q8_project(up, x), other)
+    ref = q4k_q8_project(down, q, residual=h)
+    good = slice(0, m - 1 if poison else m)  # the last token is the one with the value that is not finite
+    # Equal where the pair and a single projection cut K alike; else gate and up differ in their last bits, a bf16 tie of x may
+    # fall on its other side (2^-8 of x, at most one code), and the flips of a token add up: 2^-9 of the largest output.
+    limit = 2.0 ** -9 * ref[good].abs().amax()
+    assert (out[good] - ref[good]).abs().amax() <= limit
+    assert flag.item() == other.item() == (1 if poison else 0)

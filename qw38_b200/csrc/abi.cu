@@ -245,17 +245,17 @@ constexpr uint32_t kFlagTrustedSpans = 1u, kFlagInputSettled = 2u;
 // Nine to sixteen tokens: from this many super-blocks of eight rows on.  The TMA-streamed kernel against this one, us, replayed
 // graph over matrices that do not fit L2, launches serialised / overlapped with settled inputs:
 //                                 nine tokens                  sixteen tokens
-//   5120 x 5120   (12800)   14.6 : 15.5 / 10.9 : 10.9    16.0 : 15.6 / 11.8 : 10.9
-//   6144 x 5120   (15360)   16.2 : 16.8 / 12.1 : 11.9    17.3 : 16.8 / 12.9 : 11.9
-//   6656 x 5120   (16640)   16.4 : 17.0 / 12.7 : 12.4    17.7 : 16.9 / 13.6 : 12.5
-//   7168 x 5120   (17920)   17.5 : 16.9 / 13.2 : 12.3    19.0 : 16.9 / 14.4 : 12.4
-//   10240 x 5120  (25600)   20.9 : 19.6 / 17.0 : 14.8    22.4 : 19.7 / 18.3 : 14.8
-//   13312 x 2560  (16640)   14.1 : 14.7 / 11.4 : 10.7    14.3 : 14.7 / 11.5 : 10.8
-//   2048 x 17408  (17408)   17.4 : 19.1 / 12.0 : 14.6    19.7 : 19.4 / 12.8 : 14.8
-//   2560 x 17408  (21760)   19.5 : 20.0 / 14.1 : 15.6    21.4 : 20.4 / 15.6 : 15.7
+//   5120 x 5120   (12800)   10.5 : 12.0 /  9.0 :  9.8    12.1 : 12.4 / 10.1 : 10.0
+//   6144 x 5120   (15360)   11.9 : 13.1 / 10.3 : 10.9    13.4 : 13.2 / 11.2 : 10.9
+//   6656 x 5120   (16640)   12.2 : 13.5 / 10.7 : 11.2    13.8 : 13.6 / 11.8 : 11.2
+//   7168 x 5120   (17920)   13.1 : 13.3 / 11.4 : 11.3    14.9 : 13.2 / 12.7 : 11.4
+//   10240 x 5120  (25600)   16.1 : 15.5 / 14.5 : 13.6    18.2 : 15.6 / 16.5 : 13.7
+//   13312 x 2560  (16640)   10.1 : 12.0 /  8.7 : 10.1    11.0 : 12.0 /  9.2 : 10.2
+//   2048 x 17408  (17408)   12.9 : 15.0 / 10.1 : 12.8    15.6 : 15.3 / 11.9 : 12.9
+//   2560 x 17408  (21760)   15.0 : 16.1 / 12.9 : 13.7    17.1 : 16.2 / 14.7 : 13.7
 // Its time hardly depends on the token count (a tile is sixteen wide), the other's does; twelve tokens lie between.  At K = 5120
-// the line is where nine serialised tokens break even, to 4 % either way.  Few rows of a long K (each of its tiles then cut over
-// many clusters) lose up to 20 % just above the line, and gain from about 2560 rows on.
+// the line is where sixteen serialised tokens break even; nine do so at 18000 super-blocks.  Just above the line nine tokens
+// lose up to a tenth, and few rows of a long K (each of its tiles then cut over many clusters) or many of a short one a sixth.
 constexpr uint64_t kF16SuperBlocks = 16384;
 int project_f16(const q4k_weight& w, const q4k_q8_input& x, const q4k::F16Output& out, cudaStream_t stream, const q4k_weight* second = nullptr,
                 const q4k::RawRows* raw = nullptr) {
@@ -304,10 +304,10 @@ int project_impl(const q4k_weight* weight, const q4k_q8_input& x, float* output,
     // Beyond: fp16 planes (int8 tcgen05 for partial dots) when TMA alignment allows.  dp4a : TMA-streamed, us, replayed graph over matrices that do not fit L2,
     // serialised / overlapped with settled inputs:
     //                       one token                   two tokens
-    //   5120 x 5120     7.6 :  9.0 /  5.4 :  6.1     8.4 :  9.1 /  6.1 :  6.2
-    //   7168 x 5120     8.7 : 10.1 /  6.2 :  7.6     9.9 : 10.7 /  7.0 :  7.7
-    //   34816 x 5120   22.9 : 24.3 / 17.5 : 22.5    27.7 : 24.5 / 21.8 : 22.7
-    //   5120 x 17408   14.6 : 18.1 / 11.3 : 14.9    18.2 : 17.9 / 14.5 : 15.2
+    //   5120 x 5120     6.0 :  7.3 /  4.9 :  5.5     7.0 :  7.3 /  6.1 :  5.6
+    //   7168 x 5120     7.3 :  8.4 /  6.5 :  6.9     8.5 :  8.6 /  6.9 :  7.0
+    //   34816 x 5120   22.0 : 23.3 / 17.7 : 22.0    27.4 : 23.2 / 22.7 : 21.9
+    //   5120 x 17408   13.8 : 15.7 / 11.6 : 14.5    17.1 : 16.0 / 14.9 : 14.5
     // Two tokens in a graph of whole layers were slower on dp4a (eight layers 546 us against 477).
     bool const tma_ok = x.m <= q4k::kGemvTmaMaxTokens && q4k::gemv_tma_supported(view(w), view(x));
     bool const whole_dots = !partials && !(opt && (opt->split_k || opt->row_groups));

@@ -741,8 +741,9 @@ int decode_pack(const q4k_decode_desc& d, const q4k_q8_input& q8, int* failure, 
 // (the reference applies these epilogues inside its decode kernels too, cuda/decode_mmv.cu:182-250,619-677).
 // *fused = false when the operands do not qualify (more than 16 rows, unaligned weights, another activation policy);
 // the caller then composes separate launches.
-// Up to kDecodeRawTokens rows the launch also quantises: each block its own K slice, which at one to four tokens takes
-// less than the pack launch it saves (at eight, five warps per scheduler spend as long on it as that launch takes).  Blocks then
+// Up to kDecodeRawTokens rows the launch also quantises: each block its own K slice, which at one to three tokens takes less
+// than the pack launch it saves, at four the same on the device (5120 x 5120 9.9 us against 9.4, 5120 x 17408 19.0 : 19.5) and
+// a launch less on the host (1024 x 1024 6.0 : 8.4), at five more (7168 x 5120 12.3 : 10.7, 5120 x 17408 21.3 : 20.5).  Blocks then
 // read the input while others write the outputs, so a call whose input (or failure flag) shares memory with another operand
 // takes the pack launch first, at one to four tokens as at sixteen: neither is refused.
 constexpr uint32_t kDecodeRawTokens = 4;

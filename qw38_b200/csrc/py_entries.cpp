@@ -40,13 +40,9 @@ struct Ref {
   explicit operator bool() const { return p != nullptr; }
 };
 
-// Python integer, modulo 2^64 as ctypes takes it.  False: an exception is set.
+// Python integer or anything with __index__ (shapes read through numpy), modulo 2^64 as ctypes takes it.  False: an exception is set.
 bool as_u64(PyObject* o, uint64_t* to) {
   if (!o) return false;
-  if (!PyLong_Check(o)) {
-    PyErr_Format(PyExc_TypeError, "an integer is required, not %.100s", Py_TYPE(o)->tp_name);
-    return false;
-  }
   *to = PyLong_AsUnsignedLongLongMask(o);
   return !(*to == ~0ull && PyErr_Occurred());
 }

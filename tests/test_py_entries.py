@@ -2,6 +2,7 @@
 for plain, overridden and malformed descriptors, and errors instead of crashes for objects of another kind."""
 import ctypes as C
 
+import numpy as np
 import pytest
 import torch
 
@@ -86,3 +87,43 @@ def test_other_objects_raise(probe):
     w.n = "eight"
     with pytest.raises(TypeError):
         module.decode_mmv(d, ws, f, None)
+
+
+class Index:
+    """An integer by __index__ alone."""
+
+    def __init__(self, value):
+        self.value = value
+
+    def __index__(self):
+        return self.value
+
+
+@pytest.mark.parametrize("kind", [np.int64, np.int32, np.uint16, np.uint64, Index])
+def test_integers_of_other_types_are_taken(probe, kind):
+    """Shapes come from numpy and file headers: everything with __index__ is an integer here as in the ctypes structures."""
+    module, seen = probe
+    w = weight(40, 512)
+    want = bytes(DecodeMmvDesc(w, torch.zeros((1, 512), dtype=torch.bfloat16), None).c_struct())
+    x = torch.zeros((1, 512), dtype=torch.bfloat16)
+    d = DecodeMmvDesc(weight(40, 512), x, None)
+    d.weight.codes, d.weight.scales = w.codes, w.scales
+    d.weight.n, d.weight.k, d.weight.layout, d.weight.quantizer = kind(40), kind(512), kind(w.layout), kind(w.quantizer)
+    d.weight.codes_bytes, d.weight.scales_bytes = kind(w.codes.numel()), kind(w.scales.numel())
+    d.epilogue, d.activation_policy = kind(d.epilogue), kind(d.activation_policy)
+    ws, f = torch.zeros(512, dtype=torch.uint8), torch.zeros(1, dtype=torch.int32)
+    assert module.decode_mmv(d, ws, f, None) == 7
+    got, at = seen["one"][0], L.DecodeDesc.input.offset
+    assert got[:at] == want[:at] and got[at + 8:-2] == want[at + 8:-2]  # (all but the address of the other input)
+    # the counts that are arguments of their own, refused by the library before it looks at anything else
+    w.layout = 0
+    lib, m = L.load(), kind(3)
+    q = new_q8_input(3, 512, device="cpu")
+    q.m, q.k, q.padded_k = kind(3), kind(512), kind(512)
+    for call in (lambda: module.q8_mlp(w, w, w, f, f, 1e-6, f, m, ws, f, None)[0],
+                 lambda: module.prefill_paired_swiglu(w, w, x, x, m, ws, f, None), lambda: module.q8_project(w, q, f, None, None)):
+        assert call() == L.ERR_INVALID_ARGUMENT and lib.q4k_last_error()
+    for bad in (8.0, np.float32(8), "8", None):
+        d.weight.n = bad
+        with pytest.raises(TypeError):
+            module.decode_mmv(d, ws, f, None)

@@ -180,11 +180,12 @@ PyObject* decode_mmv_ranges(PyObject*, PyObject* const* a, Py_ssize_t n) {
   uint64_t bytes = 0;
   int* failure = nullptr;
   if (!arguments(n, 4, "decode_mmv_ranges")) return nullptr;
-  Ref const list(PySequence_Fast(a[0], "a sequence of descriptors is required"));
+  // A copy that holds its items: reading a descriptor runs Python code, during which a caller's list may change.
+  Ref const list(PySequence_Tuple(a[0]));
   if (!list) return nullptr;
-  Py_ssize_t const count = PySequence_Fast_GET_SIZE(list.p);
+  Py_ssize_t const count = PyTuple_GET_SIZE(list.p);
   for (Py_ssize_t i = 0; i < count && i < 3; ++i)  // the entry refuses any other count before it looks at them
-    if (!read_desc(PySequence_Fast_GET_ITEM(list.p, i), &d[i])) return nullptr;
+    if (!read_desc(PyTuple_GET_ITEM(list.p, i), &d[i])) return nullptr;
   if (!tensor(a[1], &workspace, &bytes) || !pointer(a[2], &failure) || !read_stream(a[3], &stream)) return nullptr;
   return PyLong_FromLong(unlocked([&] { return entries.decode_mmv_ranges(d, uint32_t(count), workspace, bytes, failure, stream); }));
 }

@@ -127,3 +127,27 @@ def test_integers_of_other_types_are_taken(probe, kind):
         d.weight.n = bad
         with pytest.raises(TypeError):
             module.decode_mmv(d, ws, f, None)
+
+
+@pytest.mark.parametrize("shrink", [list.clear, lambda ranges: ranges.__delitem__(slice(1, None))])
+def test_a_list_that_shrinks_while_it_is_read(probe, shrink):
+    """Reading a descriptor runs Python code, which may change the list of ranges: what the list held at the call counts."""
+    module, _ = probe
+    w = weight(8, 256)
+    w.layout = 0  # refused before any device work
+
+    class Shrinking(DecodeMmvDesc):
+        @property
+        def epilogue(self):
+            shrink(ranges)
+            return L.EPILOGUE_STORE_FP32
+
+        @epilogue.setter
+        def epilogue(self, value):
+            pass
+
+    x, ws, f = torch.zeros((1, 256), dtype=torch.bfloat16), torch.zeros(8, dtype=torch.uint8), torch.zeros(1, dtype=torch.int32)
+    for _ in range(200):  # (the other descriptors live in the list alone)
+        ranges = [Shrinking(w, x, torch.zeros((1, 8))), DecodeMmvDesc(w, x, torch.zeros((1, 8))), DecodeMmvDesc(w, x, torch.zeros((1, 8)))]
+        assert module.decode_mmv_ranges(ranges, ws, f, None) == L.ERR_INVALID_ARGUMENT
+        assert len(ranges) <= 1

@@ -5,6 +5,7 @@ and if that is impossible it raises.  There is no CPU or PyTorch fallback."""
 from __future__ import annotations
 
 import ctypes as C
+import os
 from importlib.machinery import ExtensionFileLoader
 from importlib.util import module_from_spec, spec_from_loader
 from pathlib import Path
@@ -12,6 +13,7 @@ from pathlib import Path
 import torch
 
 from . import build as _build
+from ._entries import CtypesEntries
 
 OK, ERR_STATUS, ERR_INVALID_ARGUMENT, ERR_OVERFLOW = 0, 1, 2, 3
 LAYOUT_SPLIT_TILES, QUANTIZER_Q4K = 0x020D, 0x0105
@@ -116,8 +118,8 @@ _entries = None
 
 
 def entries():
-    """The extension module through which Python callers reach the entries of a decode step (csrc/py_entries.cpp), bound to the
-    loaded library."""
+    """The entries of a decode step as Python callers reach them, bound to the loaded library: the extension module
+    (csrc/py_entries.cpp), or the same calls through ctypes where there is none."""
     if _entries is None:
         load()
     return _entries
@@ -127,24 +129,41 @@ def library_path() -> Path:
     return _build.LIB
 
 
+def _extension(lib: C.CDLL, path: Path):
+    """The extension at `path` bound to `lib`; None if it was built for another interpreter or against other structures."""
+    loader = ExtensionFileLoader("_q4k_entries", str(path))
+    try:
+        module = module_from_spec(spec_from_loader("_q4k_entries", loader))
+        loader.exec_module(module)
+    except ImportError:
+        return None
+    if getattr(module, "struct_sizes", None) != tuple(C.sizeof(t) for t in (Weight, Q8, DecodeDesc)):
+        return None
+    names = ("q4k_decode_mmv", "q4k_decode_mmv_ranges", "q4k_pack_q8_bf16", "q4k_pack_q8_f32", "q4k_q8_project", "q4k_q8_mlp",
+             "q4k_prefill_project", "q4k_prefill_paired_swiglu")
+    module.bind(*(C.cast(getattr(lib, name), C.c_void_p).value for name in names), torch._C._cuda_getDevice,
+                torch._C._cuda_getCurrentRawStream)
+    return module
+
+
 def load() -> C.CDLL:
-    """Load (building first if the sources are newer) and type every entry point."""
+    """Load (building first if the sources are newer) and type every entry point.
+
+    Q4K_B200_LIBRARY names an already-built library to load instead; the extension then is the one beside it, if any."""
     global _lib, _entries
     if _lib is not None:
         return _lib
-    import os
-    override = os.environ.get("Q4K_B200_LIBRARY")  # an already-built library to load instead
+    override = os.environ.get("Q4K_B200_LIBRARY")
     path = override if override else _build.build()
     lib = C.CDLL(str(path))
     for name, (res, args) in SIGNATURES.items():
         fn = getattr(lib, name)  # AttributeError here = header and library disagree
         fn.restype, fn.argtypes = res, args
-    loader = ExtensionFileLoader("_q4k_entries", str(_build.ENTRIES))
-    module = module_from_spec(spec_from_loader("_q4k_entries", loader))
-    loader.exec_module(module)
-    names = ("q4k_decode_mmv", "q4k_decode_mmv_ranges", "q4k_pack_q8_bf16", "q4k_pack_q8_f32", "q4k_q8_project", "q4k_q8_mlp",
-             "q4k_prefill_project", "q4k_prefill_paired_swiglu")
-    module.bind(*(C.cast(getattr(lib, name), C.c_void_p).value for name in names), torch._C._cuda_getDevice,
-                torch._C._cuda_getCurrentRawStream)
-    _lib, _entries = lib, module
+    if override:  # (a bare name is found by the dynamic linker, wherever that is)
+        extension = Path(os.path.abspath(override)).with_name(_build.ENTRIES.name)
+        usable = os.path.exists(override) and extension.exists()
+    else:
+        extension, usable = _build.ENTRIES, _build.entries_current()
+    _entries = (_extension(lib, extension) if usable else None) or CtypesEntries(lib, DecodeDesc)
+    _lib = lib
     return lib

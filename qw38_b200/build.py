@@ -1,4 +1,6 @@
-"""Builds libq4k_b200.so (CUDA kernels + C ABI) in-tree with nvcc for sm_100a."""
+"""Builds libq4k_b200.so (CUDA kernels + C ABI) in-tree with nvcc for sm_100a, and the extension through which Python callers reach
+its decode entries.  The library needs no Python; without Python's headers (or g++) it is built alone and those entries go through
+ctypes."""
 from __future__ import annotations
 
 import os
@@ -25,13 +27,28 @@ def nvcc() -> str:
     return exe
 
 
+HEADER = PKG.parent / "include" / "q4k_b200.h"
+
+
+def _stale(target: Path, sources) -> bool:
+    return not target.exists() or any(d.stat().st_mtime > target.stat().st_mtime for d in sources)
+
+
+def library_needs_build() -> bool:
+    return _stale(LIB, [d for suffix in ("cu", "cuh", "h") for d in CSRC.glob("*." + suffix)] + [HEADER])
+
+
+def entries_current() -> bool:
+    """The extension is there and no older than what it is built from."""
+    return not _stale(ENTRIES, [CSRC / "py_entries.cpp", HEADER])
+
+
+def entries_buildable() -> bool:
+    return shutil.which("g++") is not None and (Path(sysconfig.get_paths()["include"]) / "Python.h").exists()
+
+
 def needs_build() -> bool:
-    if not LIB.exists() or not ENTRIES.exists():
-        return True
-    t = min(LIB.stat().st_mtime, ENTRIES.stat().st_mtime)
-    deps = list(CSRC.glob("*.cpp")) + list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) + \
-        [PKG.parent / "include" / "q4k_b200.h"]
-    return any(d.stat().st_mtime > t for d in deps)
+    return library_needs_build() or (entries_buildable() and not entries_current())
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
@@ -45,14 +62,31 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     with open(LIB.parent / ".build.lock", "w") as lock:
         fcntl.flock(lock, fcntl.LOCK_EX)
         try:
-            if not force and not needs_build():
-                return LIB
-            return _build_locked(verbose)
+            extension = _start_entries() if entries_buildable() and (force or not entries_current()) else None
+            if force or library_needs_build():
+                _build_library(verbose)
+            if extension:
+                _finish_entries(*extension)
+            return LIB
         finally:
             fcntl.flock(lock, fcntl.LOCK_UN)
 
 
-def _build_locked(verbose: bool) -> Path:
+def _start_entries():
+    tmp = ENTRIES.with_suffix(f".so.tmp{os.getpid()}")
+    cmd = ["g++", "-O2", "-std=c++17", "-Wall", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"], str(CSRC / "py_entries.cpp"), "-o",
+           str(tmp)]
+    return tmp, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+
+
+def _finish_entries(tmp: Path, compiler) -> None:
+    out, _ = compiler.communicate()
+    if compiler.returncode != 0:
+        raise RuntimeError(f"g++ failed on py_entries.cpp:\n{out}")
+    os.replace(tmp, ENTRIES)
+
+
+def _build_library(verbose: bool) -> None:
     objdir = PKG / "lib" / "obj"
     objdir.mkdir(parents=True, exist_ok=True)
     procs = []
@@ -60,10 +94,6 @@ def _build_locked(verbose: bool) -> Path:
         obj = objdir / (src + ".o")
         cmd = [nvcc(), *NVCC_FLAGS, "-Xptxas", "-v" if verbose else "-warn-spills", "-c", str(CSRC / src), "-o", str(obj)]
         procs.append((src, obj, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
-    entries = ENTRIES.with_suffix(f".so.tmp{os.getpid()}")
-    cmd = ["g++", "-O2", "-std=c++17", "-Wall", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"], str(CSRC / "py_entries.cpp"), "-o",
-           str(entries)]
-    host = subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     objs = []
     for src, obj, p in procs:
         out, _ = p.communicate()
@@ -77,12 +107,7 @@ def _build_locked(verbose: bool) -> Path:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"link failed:\n{r.stdout}{r.stderr}")
-    out, _ = host.communicate()
-    if host.returncode != 0:
-        raise RuntimeError(f"g++ failed on py_entries.cpp:\n{out}")
-    os.replace(entries, ENTRIES)
     os.replace(tmp, LIB)
-    return LIB
 
 
 if __name__ == "__main__":

@@ -283,5 +283,13 @@ PyMODINIT_FUNC PyInit__q4k_entries() {
   for (auto const& e : all)
     if (!(*e.to = PyUnicode_InternFromString(e.text))) return nullptr;
   if (!(zero = PyLong_FromLong(0))) return nullptr;
-  return PyModule_Create(&module);
+  PyObject* const m = PyModule_Create(&module);
+  // What it was built against, for the loader to compare with its own structures.
+  PyObject* const sizes = m ? Py_BuildValue("(nnn)", Py_ssize_t(sizeof(q4k_weight)), Py_ssize_t(sizeof(q4k_q8_input)), Py_ssize_t(sizeof(q4k_decode_desc))) : nullptr;
+  if (!sizes || PyModule_AddObject(m, "struct_sizes", sizes) < 0) {  // (takes the reference when it succeeds)
+    Py_XDECREF(sizes);
+    Py_XDECREF(m);
+    return nullptr;
+  }
+  return m;
 }

@@ -837,6 +837,7 @@ mmq_f16_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_consta
         uint32_t* const ticket = p.tickets + (w0 * 2 + cta) * C::kEpilogueWarps + ep;
         if (lane == 0) asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(ticket) : "memory");
         old = __shfl_sync(0xffffffffu, old, 0);
+        __syncwarp();  // orders every lane's reads of the others' slots behind lane 0's acquire: the shuffle orders no memory
         write = old == w1 - w0;
         if (write) {
 #pragma unroll

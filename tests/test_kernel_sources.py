@@ -20,6 +20,15 @@ def test_minima_are_published_across_the_cluster():
     assert issuer.index("acquire_shared();") < issuer.index("mma_pair_ss(")
 
 
+def test_partial_tiles_are_read_behind_a_barrier():
+    """mmq_f16.cu: lane 0 of a warp takes the ticket of a cut tile, all lanes then read what other clusters wrote.  The barrier
+    before the ticket is cumulative with its release, the one behind it passes its acquire on; a shuffle does neither."""
+    text = code(CSRC / "mmq_f16.cu")
+    ticket = text.index("atom.acq_rel.gpu.global.add.u32")
+    assert text.rindex("__stcg(mine", 0, ticket) < text.rindex("__syncwarp();", 0, ticket)
+    assert ticket < text.index("__syncwarp();", ticket) < text.index("__ldcg(slot(", ticket)
+
+
 def kernels(text):
     """(parameter list, body) of every __global__ function."""
     for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__\((?:[^()]|\([^()]*\))*\)\s*)?(\w+)\s*\(", text):

@@ -226,7 +226,15 @@ int q4k_session_take_failure(q4k_session* session, void* stream);
  * only after the preceding kernel has completed, so results are unchanged.  The caller's side of the
  * contract: no work still in flight earlier in the stream writes the weight operand (true for
  * decode, where weights are constant; leave it off around q4k_repack_blocks144 or uploads).
- * Works inside CUDA graph capture. */
+ * Works inside CUDA graph capture.
+ *
+ * Whatever the switch says, a launch waits (griddepcontrol.wait) for the kernel directly before it in the stream, and through
+ * that kernel's own wait for everything older.  A condition on the caller's kernels follows: one that is ITSELF launched
+ * programmatically (cudaLaunchAttributeProgrammaticStreamSerialization, a programmatic edge of a graph) directly before a call
+ * of this library must execute griddepcontrol.wait (cudaGridDependencySynchronize) at some point, as every kernel of this
+ * library does.  If it ends without, it may end before what ran in front of it, and this library's kernel would not wait for
+ * that either: put a launch without the attribute, or a memset, between the two.  Kernels, copies and memsets that are issued
+ * the ordinary way need nothing. */
 void q4k_set_launch_overlap(int enabled);
 int q4k_get_launch_overlap(void);
 

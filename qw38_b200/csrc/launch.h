@@ -235,8 +235,10 @@ inline cudaError_t allow_smem(const void* kernel, int bytes) {
 }
 
 // Launch with or without the programmatic-stream-serialization attribute.  With it, blocks are placed and set up beside the
-// preceding kernel's end; a kernel that reads and writes nothing before its pdl_wait() (asking L2 for lines is no read) then
-// behaves as if launched without, whatever that kernel is, and starts 1 to 2 us earlier.
+// preceding kernel's end, 1 to 2 us earlier.  A kernel that reads and writes nothing before its pdl_wait() (asking L2 for lines
+// is no read) then behaves as if launched without, provided that the kernel directly before it was launched without the
+// attribute or waits for its own predecessor, as every kernel here does: the wait reaches one kernel back, and only through
+// that one's wait any further.  The header states this as a condition on callers' kernels (q4k_set_launch_overlap).
 template <typename... KArgs, typename... Args>
 cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                           bool overlap, Args&&... args) {

@@ -1,10 +1,15 @@
 """Launches are placed beside the end of the kernel before them without being asked to: what that kernel writes (weights,
-activations) is still read only when it has ended, eagerly, in a replayed graph and behind a join of two captured streams."""
+activations) is still read only when it has ended, eagerly, in a replayed graph and behind a join of two captured streams.  The
+same behind a caller's kernel that is launched programmatically itself, under the condition that the header states."""
+import ctypes as C
+import subprocess
+from pathlib import Path
+
 import pytest
 import torch
 
 from qw38_b200 import _lib as L
-from qw38_b200 import synth
+from qw38_b200 import build, synth
 from qw38_b200.q4k_q8 import (DecodeMmvDesc, PrefillWeight, decode_workspace, launch_decode_mmv, new_q8_input, pack_q8, prefill_project,
                               q4k_q8_project)
 
@@ -69,4 +74,51 @@ def test_weights_and_inputs_written_directly_before(m, aligned):
     for run in runs:
         for _ in range(3):
             assert all(torch.equal(a, b) for a, b in zip(results(run), want))
+    assert f.item() == 0
+
+
+@pytest.fixture(scope="module")
+def caller(tmp_path_factory):
+    """Launches a kernel that writes the rows late and lets its successor start, then a programmatic kernel that has nothing to do
+    with them."""
+    so = tmp_path_factory.mktemp("caller") / "libcaller.so"
+    source = Path(__file__).resolve().parent / "shim" / "programmatic_caller.cu"
+    r = subprocess.run([build.nvcc(), *build.NVCC_FLAGS, "-shared", str(source), "-o", str(so)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
+    lib = C.CDLL(str(so))
+    lib.caller_launch.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_void_p]
+    return lib.caller_launch
+
+
+@pytest.mark.parametrize("waits", [True, False])
+@pytest.mark.parametrize("captured", [False, True])
+def test_behind_a_callers_programmatic_kernel(caller, waits, captured):
+    """One that waits for its predecessor may stand directly before a call; one that does not has an ordinary launch behind it."""
+    m, k = 3, 2560
+    src = torch.randn((m, k), device=DEV).to(torch.bfloat16)
+    x, f, counter, other = torch.zeros_like(src), *(torch.zeros(1, dtype=torch.int32, device=DEV) for _ in range(2)), torch.ones(8, device=DEV)
+    want, q = pack_q8(src, f), new_q8_input(m, k)
+    stream = torch.cuda.Stream()
+
+    def step():
+        x.zero_()
+        assert caller(src.data_ptr(), x.data_ptr(), x.numel(), counter.data_ptr(), int(waits), torch.cuda.current_stream().cuda_stream) == 0
+        if not waits:
+            other.zero_()
+        pack_q8(x, f, out=q)
+
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        run = step
+        if captured:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=stream):
+                step()
+            run = graph.replay
+        for i in range(3):
+            q.codes.zero_()
+            run()
+            torch.cuda.synchronize()
+            assert torch.equal(q.codes, want.codes) and torch.equal(q.scales, want.scales) and torch.equal(q.sums, want.sums)
+            assert counter.item() == i + 1
     assert f.item() == 0

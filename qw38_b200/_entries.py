@@ -33,6 +33,10 @@ class CtypesEntries:
     def prefill_project(self, desc, workspace, failure, stream) -> int:
         return self._one(self._lib.q4k_prefill_project, desc, workspace, failure, stream)
 
+    def decode_mmv_paired(self, a, b, workspace, failure, stream) -> int:
+        return self._lib.q4k_decode_mmv_paired(C.byref(a.c_struct()), C.byref(b.c_struct()), _ptr(workspace), workspace.numel(), _ptr(failure),
+                                               _stream(stream))
+
     def decode_mmv_ranges(self, ranges, workspace, failure, stream) -> int:
         descs = [r.c_struct() for r in tuple(ranges)]
         return self._lib.q4k_decode_mmv_ranges((self._desc * len(descs))(*descs), len(descs), _ptr(workspace), workspace.numel(), _ptr(failure),

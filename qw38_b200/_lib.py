@@ -140,7 +140,7 @@ def _extension(lib: C.CDLL, path: Path):
     if getattr(module, "struct_sizes", None) != tuple(C.sizeof(t) for t in (Weight, Q8, DecodeDesc)):
         return None
     names = ("q4k_decode_mmv", "q4k_decode_mmv_ranges", "q4k_pack_q8_bf16", "q4k_pack_q8_f32", "q4k_q8_project", "q4k_q8_mlp",
-             "q4k_prefill_project", "q4k_prefill_paired_swiglu")
+             "q4k_prefill_project", "q4k_prefill_paired_swiglu", "q4k_decode_mmv_paired")
     module.bind(*(C.cast(getattr(lib, name), C.c_void_p).value for name in names), torch._C._cuda_getDevice,
                 torch._C._cuda_getCurrentRawStream)
     return module

@@ -27,6 +27,7 @@ struct Entries {
   decltype(&q4k_q8_mlp) q8_mlp;
   decltype(&q4k_prefill_project) prefill_project;
   decltype(&q4k_prefill_paired_swiglu) prefill_paired_swiglu;
+  decltype(&q4k_decode_mmv_paired) decode_mmv_paired;
 } entries;
 PyObject *get_device, *get_stream, *zero;
 
@@ -159,6 +160,19 @@ PyObject* one_desc(PyObject* const* a, Py_ssize_t n, const char* name, decltype(
 PyObject* decode_mmv(PyObject*, PyObject* const* a, Py_ssize_t n) { return one_desc(a, n, "decode_mmv", entries.decode_mmv); }
 PyObject* prefill_project(PyObject*, PyObject* const* a, Py_ssize_t n) { return one_desc(a, n, "prefill_project", entries.prefill_project); }
 
+// (first desc, second desc, workspace, failure, stream) -> status
+PyObject* decode_mmv_paired(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  q4k_decode_desc d[2] = {};
+  void *workspace = nullptr, *stream = nullptr;
+  uint64_t bytes = 0;
+  int* failure = nullptr;
+  if (!arguments(n, 5, "decode_mmv_paired") || !read_desc(a[0], &d[0]) || !read_desc(a[1], &d[1]) || !tensor(a[2], &workspace, &bytes) ||
+      !pointer(a[3], &failure) || !read_stream(a[4], &stream))
+    return nullptr;
+  if (!entries.decode_mmv_paired) return PyErr_Format(PyExc_RuntimeError, "decode_mmv_paired is not bound");
+  return PyLong_FromLong(unlocked([&] { return entries.decode_mmv_paired(&d[0], &d[1], workspace, bytes, failure, stream); }));
+}
+
 // (gate, up, normalized, swiglu, tokens, workspace, failure, stream) -> status
 PyObject* prefill_paired_swiglu(PyObject*, PyObject* const* a, Py_ssize_t n) {
   q4k_weight w[2] = {};
@@ -240,27 +254,31 @@ PyObject* q8_mlp(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return Py_BuildValue("ii", st, submitted);
 }
 
-// (addresses of the entries in the order above, torch's device and raw-stream lookups)
+// (addresses of the entries in the order above, torch's device and raw-stream lookups); without the last entry that one stays
+// as it is
 PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  if (!arguments(n, 10, "bind")) return nullptr;
-  uint64_t p[8];
-  for (int i = 0; i < 8; ++i)
+  if (n != 10 && !arguments(n, 11, "bind")) return nullptr;
+  uint64_t p[9];
+  p[8] = reinterpret_cast<uint64_t>(entries.decode_mmv_paired);
+  for (int i = 0; i < n - 2; ++i)
     if (!as_u64(a[i], &p[i])) return nullptr;
   entries = {reinterpret_cast<decltype(entries.decode_mmv)>(p[0]),   reinterpret_cast<decltype(entries.decode_mmv_ranges)>(p[1]),
              reinterpret_cast<decltype(entries.pack_q8_bf16)>(p[2]), reinterpret_cast<decltype(entries.pack_q8_f32)>(p[3]),
              reinterpret_cast<decltype(entries.q8_project)>(p[4]),   reinterpret_cast<decltype(entries.q8_mlp)>(p[5]),
              reinterpret_cast<decltype(entries.prefill_project)>(p[6]),
-             reinterpret_cast<decltype(entries.prefill_paired_swiglu)>(p[7])};
-  Py_INCREF(a[8]);
-  Py_INCREF(a[9]);
-  Py_XSETREF(get_device, a[8]);
-  Py_XSETREF(get_stream, a[9]);
+             reinterpret_cast<decltype(entries.prefill_paired_swiglu)>(p[7]),
+             reinterpret_cast<decltype(entries.decode_mmv_paired)>(p[8])};
+  Py_INCREF(a[n - 2]);
+  Py_INCREF(a[n - 1]);
+  Py_XSETREF(get_device, a[n - 2]);
+  Py_XSETREF(get_stream, a[n - 1]);
   Py_RETURN_NONE;
 }
 
 PyCFunction fast(PyObject* (*f)(PyObject*, PyObject* const*, Py_ssize_t)) { return reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f)); }
 PyMethodDef methods[] = {{"bind", fast(bind), METH_FASTCALL, nullptr},
                          {"decode_mmv", fast(decode_mmv), METH_FASTCALL, nullptr},
+                         {"decode_mmv_paired", fast(decode_mmv_paired), METH_FASTCALL, nullptr},
                          {"decode_mmv_ranges", fast(decode_mmv_ranges), METH_FASTCALL, nullptr},
                          {"pack_q8", fast(pack_q8), METH_FASTCALL, nullptr},
                          {"q8_project", fast(q8_project), METH_FASTCALL, nullptr},

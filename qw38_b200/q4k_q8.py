@@ -286,9 +286,7 @@ def launch_decode_mmv(desc: DecodeMmvDesc, workspace: torch.Tensor, failure: tor
 def launch_decode_mmv_paired(a: DecodeMmvDesc, b: DecodeMmvDesc, workspace: torch.Tensor, failure: torch.Tensor,
                              stream=None) -> None:
     """launch_decode_mmv_paired (cuda/decode_mmv.hpp:210-211): gate/up sharing one input; SwigluStoreBf16 lives here."""
-    da, db = a.c_struct(), b.c_struct()
-    _check(L.load().q4k_decode_mmv_paired(C.byref(da), C.byref(db), _ptr(workspace), workspace.numel(), _ptr(failure),
-                                          _stream(stream)))
+    _check(L.entries().decode_mmv_paired(a, b, workspace, failure, stream))
 
 
 def launch_decode_mmv_ranges(ranges: Sequence[DecodeMmvDesc], workspace: torch.Tensor, failure: torch.Tensor,

@@ -16,7 +16,8 @@ from qw38_b200._entries import CtypesEntries
 from qw38_b200.q4k_q8 import DecodeMmvDesc, PrefillWeight, Q8Input
 
 ROOT = Path(__file__).resolve().parents[1]
-NAMES = ("decode_mmv", "decode_mmv_ranges", "pack_q8_bf16", "pack_q8_f32", "q8_project", "q8_mlp", "prefill_project", "prefill_paired_swiglu")
+NAMES = ("decode_mmv", "decode_mmv_ranges", "pack_q8_bf16", "pack_q8_f32", "q8_project", "q8_mlp", "prefill_project", "prefill_paired_swiglu",
+         "decode_mmv_paired")
 
 
 class Stream:
@@ -49,6 +50,7 @@ def forms():
             else:
                 calls.append((name, *(plain(v) for v in got)))
             return 3
+
         return C.CFUNCTYPE(res, *args)(f)
 
     fakes = {n: recorder(n) for n in NAMES}
@@ -77,6 +79,7 @@ def test_both_forms_make_the_same_calls(forms):
     for name, args in [("decode_mmv", (d, ws, f, s)), ("decode_mmv", (e, ws, None, s)), ("prefill_project", (d, ws, f, s)),
                        ("decode_mmv_ranges", ([d, e], ws, f, s)), ("decode_mmv_ranges", ((d, e, d), ws, f, s)),
                        ("decode_mmv_ranges", ([], ws, f, s)), ("decode_mmv_ranges", ([d] * 5, ws, f, s)),
+                       ("decode_mmv_paired", (d, e, ws, f, s)), ("decode_mmv_paired", (e, d, ws, None, s)),
                        ("prefill_paired_swiglu", (w, v, x, out, 3, ws, f, s)), ("pack_q8", (x, False, q, f, s)), ("pack_q8", (res, True, q, f, s)),
                        ("q8_project", (w, q, out, None, s)), ("q8_project", (w, q, out, res, s)),
                        ("q8_mlp", (w, v, w, res, gamma, 1e-6, out, 3, wide, f, s)), ("q8_mlp", (w, v, w, res, gamma, 1e-6, out, 3, wide, None, s))]:

@@ -1,0 +1,67 @@
+"""The MLP chain beyond sixteen tokens makes its operand planes from the residual stream and from the gate and up rows: bit for bit
+what the separate launches give where a gate / up pair and a single projection cut K alike."""
+import pytest
+import torch
+
+from qw38_b200 import synth
+from qw38_b200.q4k_q8 import hidden_rms_q8, q4k_q8_mlp, q4k_q8_project, q8_mlp_workspace_bytes, swiglu_pack_q8
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def operands(m, hidden, ffn):
+    """The gain (1 + gamma) of the last 256 columns and the last 256 rows of gate and up are some 2^15 and 2^7 above the others, so
+    that the other super-blocks of both planes carry powers of two of their own."""
+    g = torch.Generator(device=DEV).manual_seed(m + hidden)
+    gate, up, down = synth.device_weight(ffn, hidden, seed=11), synth.device_weight(ffn, hidden, seed=12), synth.device_weight(hidden, ffn, seed=13)
+    h = torch.randn((m, hidden), device=DEV, generator=g) * 2
+    gamma = torch.randn(hidden, device=DEV, generator=g) * 0.01
+    gamma[-256:] *= 2.0 ** 22
+    for w in (gate, up):
+        rows = w.scales.view(torch.float16).view(ffn // 8, -1, 8, 8)[-32:, :, :, :2]
+        rows *= 2.0 ** 7
+    return gate, up, down, h, gamma.to(torch.bfloat16)
+
+
+def chain(gate, up, down, h, gamma):
+    m = h.shape[0]
+    ws = torch.zeros(q8_mlp_workspace_bytes(m, gate.k, gate.n), dtype=torch.uint8, device=DEV)
+    out, flag = torch.empty_like(h), torch.zeros(1, dtype=torch.int32, device=DEV)
+    q4k_q8_mlp(gate, up, down, h, gamma, 1e-6, out, m, ws, pending_failure=flag)
+    return out, flag.item()
+
+
+def separate(gate, up, down, h, gamma):
+    flag = torch.zeros(1, dtype=torch.int32, device=DEV)
+    x = hidden_rms_q8(h, gamma, 1e-6, flag)
+    q = swiglu_pack_q8(q4k_q8_project(gate, x), q4k_q8_project(up, x), flag)
+    return q4k_q8_project(down, q, residual=h), flag.item(), x, q
+
+
+def same(a, b):
+    return torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(a.nan_to_num().view(torch.int32), b.nan_to_num().view(torch.int32))
+
+
+def needs_148():
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the shapes take whole tiles on 148 SMs")
+
+
+# Where each projection takes whole tiles, alone and as a pair: few enough super-blocks of K that a cut costs more than it evens
+# out, or tiles in multiples of the 74 clusters (18944 rows are 74 tiles of 256, 28416 with two token tiles 222).  Forms of the
+# producers: K up to 8, 24 and beyond in super-blocks (RMS), up to 24, 96 and beyond (SwiGLU); 32, 64 and 128 tokens a tile.
+@pytest.mark.parametrize("m,hidden,ffn", [(17, 2048, 6144), (33, 1536, 6144), (64, 6144, 18944), (65, 6400, 18944), (130, 1024, 28416)])
+def test_planes_are_bitwise_those_of_the_separate_launches(m, hidden, ffn):
+    needs_148()
+    ops = operands(m, hidden, ffn)
+    out, flag = chain(*ops)
+    ref, ref_flag, x, q = separate(*ops)
+    for p in (x, q):  # the case has what it is for: super-blocks more than 2^12 below their token's largest scale
+        top = p.scales.view(m, -1, 8).amax(2)
+        assert (top < top.amax(1, keepdim=True) * 2.0 ** -13).float().mean() > 0.25
+    assert flag == ref_flag == 0 and torch.isfinite(out).all() and torch.equal(out, ref)
+    ops[3][m - 1, hidden // 3] = float("nan")
+    out, flag = chain(*ops)
+    ref, ref_flag = separate(*ops)[:2]
+    assert flag == ref_flag == 1 and same(out, ref) and torch.isnan(out[m - 1]).all() and torch.isfinite(out[:m - 1]).all()

@@ -1,5 +1,6 @@
 """The MLP chain beyond sixteen tokens makes its operand planes from the residual stream and from the gate and up rows: bit for bit
-what the separate launches give where a gate / up pair and a single projection cut K alike."""
+what the separate launches give where a gate / up pair and a single projection cut K alike, and in several passes of tokens what
+each pass gives by itself."""
 import pytest
 import torch
 
@@ -65,3 +66,26 @@ def test_planes_are_bitwise_those_of_the_separate_launches(m, hidden, ffn):
     out, flag = chain(*ops)
     ref, ref_flag = separate(*ops)[:2]
     assert flag == ref_flag == 1 and same(out, ref) and torch.isnan(out[m - 1]).all() and torch.isfinite(out[:m - 1]).all()
+
+
+# The planes of one pass stay below 64 MB: K = 17408 takes 1000 tokens as 512 and 488, in the first or in the last projection.
+@pytest.mark.parametrize("hidden,ffn", [(1024, 17408), (17408, 1024)])
+def test_several_passes_are_the_chains_of_their_tokens(hidden, ffn):
+    m, cut = 1000, 512
+    ops = operands(m, hidden, ffn)
+    ops[3][m - 3, 5] = float("inf")
+    out, flag = chain(*ops)
+    parts = [chain(*ops[:3], h.contiguous(), ops[4]) for h in (ops[3][:cut], ops[3][cut:])]
+    assert [f for _, f in parts] == [0, 1] and flag == 1
+    assert same(out, torch.cat([o for o, _ in parts]))
+    assert not torch.isfinite(out[m - 3]).any() and torch.isfinite(out[:m - 3]).all() and torch.isfinite(out[m - 2:]).all()
+
+
+def test_a_last_pass_of_one_token():
+    """2049 tokens at K = 32768: four passes of 512 and one token, which still takes a tile of 128.  Whole tiles as above: 9472 rows
+    are 37 tiles of 256, with four token tiles 148."""
+    needs_148()
+    ops = operands(2049, 32768, 9472)
+    out, flag = chain(*ops)
+    ref, ref_flag = separate(*ops)[:2]
+    assert flag == ref_flag == 0 and torch.isfinite(out).all() and torch.equal(out, ref)

@@ -304,11 +304,11 @@ int project_impl(const q4k_weight* weight, const q4k_q8_input& x, float* output,
     // Beyond: fp16 planes (int8 tcgen05 for partial dots) when TMA alignment allows.  dp4a : TMA-streamed, us, replayed graph over matrices that do not fit L2,
     // serialised / overlapped with settled inputs:
     //                       one token                   two tokens
-    //   5120 x 5120     6.0 :  7.3 /  4.9 :  5.5     7.0 :  7.3 /  6.1 :  5.6
-    //   7168 x 5120     7.3 :  8.4 /  6.5 :  6.9     8.5 :  8.6 /  6.9 :  7.0
-    //   34816 x 5120   22.0 : 23.3 / 17.7 : 22.0    27.4 : 23.2 / 22.7 : 21.9
-    //   5120 x 17408   13.8 : 15.7 / 11.6 : 14.5    17.1 : 16.0 / 14.9 : 14.5
-    // Two tokens in a graph of whole layers were slower on dp4a (eight layers 546 us against 477).
+    //   5120 x 5120     5.9 :  7.1 /  4.9 :  5.4     6.9 :  7.1 /  5.7 :  5.4
+    //   7168 x 5120     7.1 :  8.2 /  5.8 :  6.7     8.3 :  8.3 /  6.2 :  6.7
+    //   34816 x 5120   21.1 : 21.9 / 16.7 : 20.3    26.4 : 22.1 / 20.7 : 20.4
+    //   5120 x 17408   13.6 : 15.2 / 10.4 : 13.6    16.6 : 15.3 / 13.3 : 13.6
+    // Two tokens in a graph of whole layers with their packs are slower on dp4a (eight layers 544 us against 427).
     bool const tma_ok = x.m <= q4k::kGemvTmaMaxTokens && q4k::gemv_tma_supported(view(w), view(x));
     bool const whole_dots = !partials && !(opt && (opt->split_k || opt->row_groups));
     if (x.m > 8 && x.m <= 16 && whole_dots && w.padded_n / 8 * (w.padded_k / 256) >= kF16SuperBlocks && q4k::f16_supported(view(w), view(x)))

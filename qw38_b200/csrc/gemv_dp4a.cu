@@ -23,9 +23,9 @@
 // Activations are staged once per block as (even bytes, odd bytes) words, or quantised right there from bf16 rows (Raw).
 //
 // One token, us, matrices that do not fit L2 in a replayed graph, overlapped launches with settled inputs (the TMA tile kernel in
-// brackets): 5120 x 5120 5.4 (6.1), 7168 x 5120 6.2 (7.6), 5120 x 17408 11.3 (14.9), 34816 x 5120 17.5 = 5.7 TB/s (22.5); eight
-// layers of all four 394 (472).  Slower: sixteen-row steps whose lanes share the activation loads (20.1 on 34816 x 5120), eleven
-// to seventeen warps, thirty warps in one block per SM.
+// brackets): 5120 x 5120 4.9 (5.4), 7168 x 5120 5.8 (6.7), 5120 x 17408 10.4 (13.6), 34816 x 5120 16.7 = 6.0 TB/s (20.3); eight
+// layers of all four with their packs 350 to 357 (426).  Slower, when they were tried: sixteen-row steps whose lanes share the
+// activation loads (34816 x 5120 20.1 against 17.5), eleven to seventeen warps, thirty warps in one block per SM.
 #include "common.cuh"
 #include "launch.h"
 #include "q8_pack.cuh"
@@ -375,7 +375,7 @@ cudaError_t launch_split(DpParams p, uint32_t m, uint32_t padded_k, cudaStream_t
   }
   // As many rounds of blocks as bound a block's row groups.  Of 148 blocks that fill half an SM each the hardware puts two on
   // nine SMs, and these end last: 11 us after the others on 34816 x 5120 beside the next projection.  Two blocks per SM fill every
-  // half (bf16 rows, one token, us: 5120 x 5120 8.9 -> 7.2, 30000 x 7000 26.4 -> 23.7, a layer 78 -> 67).  For Q8 input there is one:
+  // half (bf16 rows, one token, us: 5120 x 5120 8.9 -> 7.2, 30000 x 7000 26.4 -> 23.7, a layer 78 -> 72).  For Q8 input there is one:
   // a pack before or behind finds room beside it (pack and 17408 x 5120 14.5 against 15.1, four small layers 74 against 79).
   uint32_t const slots = uint32_t(sm_count()) * (p.raw ? 2 : 1), waves = (p.rgs + slots * kMaxRowGroups - 1) / (slots * kMaxRowGroups);
   uint32_t const grid = p.rgs < slots * waves ? p.rgs : slots * waves;

@@ -17,7 +17,7 @@ namespace {
 // One thread turns 32 quant bytes of a block (16 low-nibble, then 16 high-nibble pairs: 32 output bytes in place) at a time, two of
 // them in flight, and every fourth thread copies the metadata, so a warp reads eight consecutive blocks of a row and writes eight
 // whole 128-byte tile rows, 32 bytes per store.  Bound: HBM, 2 x 144 bytes per block.  Measured on 17408 x 5120 (50 MB): 19.1 us (one
-// task per thread 19.6, four 20.3); repack and the decoding to bf16 behind it 58 us, 66 with 16-byte stores and one task, 229 with one byte per thread and
+// task per thread 19.6, four 20.3); repack and the decoding to bf16 behind it 58 us, 66 before, 229 with one byte per thread and
 // one block per tile row.  Blocks that are not 16-byte aligned are gathered byte by byte (Wide = false).
 template <bool Wide> __device__ __forceinline__ uint4 load_block16(const uint8_t* p) {
   if constexpr (Wide) {

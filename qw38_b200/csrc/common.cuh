@@ -60,6 +60,9 @@ __device__ __forceinline__ uint32_t byte_of(uint32_t w, uint32_t i) { return (w 
 __device__ __forceinline__ uint32_t even_bytes(uint32_t z0, uint32_t z1) { return __byte_perm(z0, z1, 0x6420); }
 __device__ __forceinline__ uint32_t odd_bytes(uint32_t z0, uint32_t z1) { return __byte_perm(z0, z1, 0x7531); }
 
+// The eleven leading bits of v, which tf32 holds.  What is left has thirteen, so three such terms add up to v exactly.
+__device__ __forceinline__ float tf32_part(float v) { return __uint_as_float(__float_as_uint(v) & 0xffffe000u); }
+
 // Programmatic dependent launch.  A kernel launched with the stream-serialization attribute may
 // start while the kernel before it in the stream is still running; it must call pdl_wait()
 // before it reads anything that kernel may have written and before it writes global memory.

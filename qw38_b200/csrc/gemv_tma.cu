@@ -51,11 +51,13 @@ namespace {
 constexpr uint32_t kMagicI = 0x4B400000u;  // bit pattern of 1.5 * 2^23
 constexpr float kMagicF = 12582912.0f;
 constexpr int kProducer = 0, kFirstReducer = 1;  // then NT reducer warps, then the consumers
-// Per consumer warp: 16 rows of 112 bytes -- 64 of scale pairs, 32 of mins, 16 of {d, d, -dmin, -dmin}; the
+// Per consumer warp: 16 rows of 112 bytes -- twice 32 of scale pairs and 16 of mins (four groups each), 16 of {d, d, -dmin, -dmin}; the
 // stride of 28 words puts the eight rows a load touches in different banks -- then NT * 256 bytes of
 // activation scale pairs.
-constexpr int kTabRow = 112, kTabMn = 64, kTabDd = 96, kTabBytes = 16 * kTabRow;
+constexpr int kTabRow = 112, kTabHalf = 48, kTabMn = 32, kTabDd = 96, kTabBytes = 16 * kTabRow;
 constexpr int kMaxStages = 8;
+constexpr uint32_t kBarEmpty = kMaxStages * 8, kBarRedFull = 2 * kBarEmpty, kBarRedEmpty = kBarRedFull + 16, kBarFlags = kBarRedEmpty + 16;
+constexpr uint32_t kBarBytes = kBarFlags + 16;
 
 // One weight of a multi-weight launch: its destination (fp32, or bf16 rounded to nearest even), its optional residual
 // ([m][n] like the destination), its rows, its 16-row tiles and its first row in the concatenated split-K scratch.
@@ -127,11 +129,6 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], uint32_t a0, uint32_t a1
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ uint32_t to_tf32(float v) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(v));
-  return r;
-}
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 as_f2(uint32_t x, uint32_t y) { return make_float2(__uint_as_float(x), __uint_as_float(y)); }
@@ -165,10 +162,12 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
   uint32_t const tab_bytes = kTabBytes + NT * 256;
   uint32_t const s_red = s_tab + cw * tab_bytes;
   uint32_t const red_slot = cw * NT * 512;
-  // barriers: full[stages] empty[stages] red_full[2] red_empty[2], then the abort and "last block" flags
-  uint32_t const b_full = s_red + p.red_slots * red_slot, b_empty = b_full + 8 * stages, b_rfull = b_empty + 8 * stages, b_rempty = b_rfull + 16;
-  int* const flags = reinterpret_cast<int*>(smem_raw + (b_rempty + 16 - smem_u32(smem_raw)));
+  // barriers: full[kMaxStages] empty[kMaxStages] red_full[2] red_empty[2], then the abort and "last block" flags, at constant
+  // distances: the roles keep one address in a register
+  uint32_t const b_full = s_red + p.red_slots * red_slot, b_empty = b_full + kBarEmpty, b_rfull = b_full + kBarRedFull, b_rempty = b_full + kBarRedEmpty;
+  int* const flags = reinterpret_cast<int*>(smem_raw + (b_full + kBarFlags - smem_u32(smem_raw)));
   volatile int* const abort_flag = flags;
+  auto wait = [&](uint32_t bar, uint32_t parity, int code) { return mbar_wait_at(bar, parity, b_full + kBarFlags, p.status, code); };
   int* const last_flag = flags + 1;
 
   constexpr int Reducers = Quant == 2 ? 2 : 1;
@@ -231,7 +230,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
       }
       uint32_t s = 0, ph = 1;  // the first pass over the ring finds every stage free
       for (uint32_t it = 0; it < ntiles; ++it) {
-        if (it >= stages && !mbar_wait(b_empty + 8 * s, ph, abort_flag, p.status, 0x510)) break;
+        if (it >= stages && !wait(b_empty + 8 * s, ph, 0x510)) break;
         mbar_expect_tx(b_full + 8 * s, code_stage + meta_stage);
         const CUtensorMap *mc, *mm;
         int const rg = tile(it, mc, mm);
@@ -268,7 +267,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
         if (Reducers == 2 && ((it >> 2) & 1) != turn) continue;
         uint32_t s, use;
         hand_off(it, s, use);
-        if (!mbar_wait(b_rfull + 8 * s, use & 1, abort_flag, p.status, 0x520)) break;
+        if (!wait(b_rfull + 8 * s, use & 1, 0x520)) break;
         float2 lo = make_float2(0.f, 0.f), hi = make_float2(0.f, 0.f);
         uint32_t src = s_red + s * red_slot + nt * 512 + lane * 16;
 #pragma unroll 4
@@ -370,7 +369,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
     for (uint32_t it = 0; turn == 0 && it < ntiles; ++it) {
       uint32_t s, use;
       hand_off(it, s, use);
-      if (!mbar_wait(b_rfull + 8 * s, use & 1, abort_flag, p.status, 0x520)) break;
+      if (!wait(b_rfull + 8 * s, use & 1, 0x520)) break;
       float2 lo = make_float2(0.f, 0.f), hi = make_float2(0.f, 0.f);
       uint32_t src = s_red + s * red_slot + nt * 512 + lane * 16;
 #pragma unroll 4
@@ -422,15 +421,10 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
     // activation scale pairs {a[2q], a[2q+1]} of (octet nt, group g) at ((nt*4 + g/2)*4 + q)*16 + (g%2)*8
     uint32_t const rd_ap = tab + kTabBytes + q * 16;
     uint32_t bfrag[NT][8][2];  // int8 activations of token nt*8 + r: even / odd columns of 8q..8q+7 in group g
-    uint32_t asplit[NT][3][2]; // tf32 terms of a*sum for token nt*8 + r, groups q and q+4
-    auto split = [&](int nt, int h, float as) {  // a * sum as three tf32 terms that add up to it exactly
-      uint32_t const hi = to_tf32(as);
-      float const r1 = as - __uint_as_float(hi);
-      uint32_t const mid = to_tf32(r1);
-      asplit[nt][0][h] = hi;
-      asplit[nt][1][h] = mid;
-      asplit[nt][2][h] = to_tf32(r1 - __uint_as_float(mid));
-    };
+    // a * sum of token nt*8 + r, groups q and q+4.  Two octets have 80 registers (23 warps), and a word spilled in the loop comes back from
+    // L2: the ring leaves L1 28 KB for what 736 threads spill.  Terms made anew per tile, one address for all barriers and fewer for the
+    // tables: MLP of 13 tokens 5120 / 17408 75.0 -> 70.3 us, four spilled words per tile for seven.
+    float as[NT][2];
     if constexpr (Raw) {
       // bf16 rows: the warp quantises the 256 columns of its super-block, a token at a time with all lanes, four tokens per
       // pass through its (still unused) decode table: codes [4][256], scales [4][8], sums [4][8].
@@ -438,8 +432,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
       for (int nt = 0; nt < NT; ++nt) {
 #pragma unroll
         for (int g = 0; g < 8; ++g) bfrag[nt][g][0] = bfrag[nt][g][1] = 0u;
-        split(nt, 0, 0.f);
-        split(nt, 1, 0.f);
+        as[nt][0] = as[nt][1] = 0.f;
       }
       for (uint32_t i = lane; i < NT * 64; i += 32) sts32f(tab + kTabBytes + i * 4, 0.f);
       for (uint32_t t0 = 0; t0 < p.m; t0 += 4) {
@@ -488,7 +481,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
               uint32_t const at = tab + 1024 + (j * 8 + q + 4 * h) * 4;
-              split(nt, h, __uint_as_float(lds32(at)) * __uint_as_float(lds32(at + 128)));
+              as[nt][h] = __uint_as_float(lds32(at)) * __uint_as_float(lds32(at + 128));
             }
           }
         }
@@ -508,7 +501,6 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
         uint32_t const tok = (lane + 32 * j) >> 3;
         scale[j] = tok < p.m ? p.xscales[size_t(tok) * p.G + sb * 8 + (lane & 7)] : 0.f;
       }
-      float as[NT][2];
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt) {
         uint32_t const tokb = nt * 8 + r;
@@ -541,8 +533,6 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
           bfrag[nt][g][0] = even_bytes(z0, z1);
           bfrag[nt][g][1] = odd_bytes(z0, z1);
         }
-        split(nt, 0, as[nt][0]);
-        split(nt, 1, as[nt][1]);
       }
     }
     __syncwarp();
@@ -553,25 +543,24 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
     // decode role of this lane: row16 = lane & 15, half h = lane >> 4 takes groups 4h..4h+3
     uint32_t const drow = lane & 15, dh = lane >> 4;
     // groups 0..3: byte & 0x3f; groups 4..7: (byte of word 3 & 0x0f) | ((byte >> 2) & 0x30)  (mins: high nibble of word 3)
-    uint32_t const dsh = dh ? 2u : 0u, dmask_a = dh ? 0x30303030u : 0x3f3f3f3fu, dmask_b = dh ? 0x0f0f0f0fu : 0u;
+    uint32_t const dsh = dh ? 2u : 0u, dmask = dh ? 0x30303030u : 0x3f3f3f3fu;
     uint32_t const dec_meta = s_meta + (drow >> 3) * cw * 128 + w * 128 + (drow & 7) * 16;
-    uint32_t const dec_sc = tab + drow * kTabRow + dh * 32, dec_mn = dec_sc - dh * 16 + kTabMn, dec_dd = tab + drow * kTabRow + kTabDd;
+    uint32_t const dec = tab + drow * kTabRow + dh * kTabHalf;
     uint32_t const rd_sc = tab + r * kTabRow, rd_mn = rd_sc + kTabMn + q * 4, rd_dd = rd_sc + kTabDd;
     // ldmatrix lane address: matrix j = lane >> 3 (bit 0: row group, bit 1: second K32 group), row i = lane & 7
     uint32_t const lj = lane >> 3, li = lane & 7;
-    uint32_t const ld_base = s_codes + (lj & 1) * cw * 1024 + w * 1024 + li * 128;
-    uint32_t const ld_x = ((lj >> 1) << 4) ^ (li << 4);
+    uint32_t const ld_base = s_codes + (lj & 1) * cw * 1024 + w * 1024 + li * 128 + (((lj >> 1) ^ li) << 4);
     uint32_t const red_dst = s_red + (w * NT * 32 + lane) * 16;
 
-    uint32_t s = 0, ph = 0, code_off = 0, meta_off = 0;
+    uint32_t bar = b_full, ph = 0, code_off = 0;  // a stage's metadata is an eighth of its codes
     for (uint32_t it = 0; it < ntiles; ++it) {
-      if (!mbar_wait(b_full + 8 * s, ph, abort_flag, p.status, 0x530)) break;
+      if (!wait(bar, ph, 0x530)) break;
       uint32_t const cbase = ld_base + code_off;
-      uint4 const mw = lds128(dec_meta + meta_off);
+      uint4 const mw = lds128(dec_meta + (code_off >> 3));
       // ---- decode the metadata of 16 rows ----
       {
-        uint32_t const sc4 = ((mw.y >> dsh) & dmask_a) | (mw.w & dmask_b);
-        uint32_t const mn4 = ((mw.z >> dsh) & dmask_a) | ((mw.w >> 4) & dmask_b);
+        uint32_t const sc4 = ((mw.y >> dsh) & dmask) | (mw.w & 0x0f0f0f0fu & ~dmask);
+        uint32_t const mn4 = ((mw.z >> dsh) & dmask) | ((mw.w >> 4) & 0x0f0f0f0fu & ~dmask);
         // byte -> float without shifts: splice the byte under the exponent of 2^23 (PRMT), then one
         // packed subtraction per pair of values; scales are stored twice, as the packed FMAs read them
         float2 const m23 = make_float2(-8388608.0f, -8388608.0f);
@@ -579,13 +568,13 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
         uint32_t const e2 = __byte_perm(sc4, 0x4b000000u, 0x7652), e3 = __byte_perm(sc4, 0x4b000000u, 0x7653);
         float2 const p0 = __fadd2_rn(as_f2(e0, e0), m23), p1 = __fadd2_rn(as_f2(e1, e1), m23);
         float2 const p2 = __fadd2_rn(as_f2(e2, e2), m23), p3 = __fadd2_rn(as_f2(e3, e3), m23);
-        sts128f(dec_sc, p0.x, p0.y, p1.x, p1.y);
-        sts128f(dec_sc + 16, p2.x, p2.y, p3.x, p3.y);
+        sts128f(dec, p0.x, p0.y, p1.x, p1.y);
+        sts128f(dec + 16, p2.x, p2.y, p3.x, p3.y);
         float2 const q0 = __fadd2_rn(as_f2(__byte_perm(mn4, 0x4b000000u, 0x7650), __byte_perm(mn4, 0x4b000000u, 0x7651)), m23);
         float2 const q1 = __fadd2_rn(as_f2(__byte_perm(mn4, 0x4b000000u, 0x7652), __byte_perm(mn4, 0x4b000000u, 0x7653)), m23);
-        sts128f(dec_mn, q0.x, q0.y, q1.x, q1.y);
+        sts128f(dec + kTabMn, q0.x, q0.y, q1.x, q1.y);
         float const d = fp16_bits_to_f32(mw.x & 0xffffu), ndmin = -fp16_bits_to_f32(mw.x >> 16);
-        sts128f(dec_dd, d, d, ndmin, ndmin);  // both halves of a row store the same words
+        if (!dh) sts128f(dec + kTabDd, d, d, ndmin, ndmin);
       }
       __syncwarp();
       float2 acc[NT][2];
@@ -599,12 +588,13 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
 #pragma unroll
       for (int gp = 0; gp < 4; ++gp) {
         uint32_t raw[4];
-        ldmatrix_x4(raw, cbase + ((uint32_t(gp) << 5) ^ ld_x));
+        ldmatrix_x4(raw, cbase ^ (uint32_t(gp) << 5));  // the tiles' rows are 128-byte aligned
         // The stage goes back to the producer as soon as its last word is in registers (the arrival has
         // release semantics, so the loads above are performed before it).
-        if (gp == 3) mbar_arrive(b_empty + 8 * s);
-        float4 const sc_lo = lds128f(rd_sc + gp * 16);         // row r:   {s_g, s_g, s_g+1, s_g+1}
-        float4 const sc_hi = lds128f(rd_sc + 8 * kTabRow + gp * 16);   // row r+8
+        if (gp == 3) mbar_arrive(bar + kBarEmpty);
+        uint32_t const at = rd_sc + (gp >> 1) * kTabHalf + (gp & 1) * 16;
+        float4 const sc_lo = lds128f(at);                // row r:   {s_g, s_g, s_g+1, s_g+1}
+        float4 const sc_hi = lds128f(at + 8 * kTabRow);  // row r+8
         float4 ap4[NT];
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) ap4[nt] = lds128f(rd_ap + (nt * 4 + gp) * 64);
@@ -638,11 +628,18 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
       }
       // ---- min term: rows x groups (6-bit integers) times groups x tokens (three tf32 terms of a*sum) ----
       {
-        uint32_t const m0 = lds32(rd_mn), m1 = lds32(rd_mn + 8 * kTabRow), m2 = lds32(rd_mn + 16), m3 = lds32(rd_mn + 8 * kTabRow + 16);
+        uint32_t const m0 = lds32(rd_mn), m1 = lds32(rd_mn + 8 * kTabRow), m2 = lds32(rd_mn + kTabHalf), m3 = lds32(rd_mn + 8 * kTabRow + kTabHalf);
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
+          uint32_t term[3][2];
 #pragma unroll
-          for (int part = 2; part >= 0; --part) mma_tf32(mins[nt], m0, m1, m2, m3, asplit[nt][part][0], asplit[nt][part][1]);
+          for (int h = 0; h < 2; ++h) {
+            asm volatile("" : "+f"(as[nt][h]));  // the terms are made anew for every tile: kept, they would cost registers
+            float const hi = tf32_part(as[nt][h]), rest = as[nt][h] - hi, mid = tf32_part(rest);
+            term[0][h] = __float_as_uint(hi); term[1][h] = __float_as_uint(mid); term[2][h] = __float_as_uint(rest - mid);
+          }
+#pragma unroll
+          for (int part = 2; part >= 0; --part) mma_tf32(mins[nt], m0, m1, m2, m3, term[part][0], term[part][1]);
         }
       }
       float4 const dd_lo = lds128f(rd_dd);        // {d, d, -dmin, -dmin} of row r
@@ -650,7 +647,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
       // ---- hand the tile to the reducer ----
       uint32_t rs, ruse;
       hand_off(it, rs, ruse);
-      if (ruse > 0 && !mbar_wait(b_rempty + 8 * rs, (ruse - 1) & 1, abort_flag, p.status, 0x540)) break;
+      if (ruse > 0 && !wait(b_rempty + 8 * rs, (ruse - 1) & 1, 0x540)) break;
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt) {
         float2 const o_lo = fma2(acc[nt][0], make_float2(dd_lo.x, dd_lo.y),
@@ -662,8 +659,8 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
       mbar_arrive(b_rfull + 8 * rs);
       __syncwarp();  // every lane has read the tables before the next tile's decode overwrites them
       code_off += code_stage;
-      meta_off += meta_stage;
-      if (++s == stages) { s = 0; ph ^= 1; code_off = 0; meta_off = 0; }
+      bar += 8;
+      if (bar == b_full + 8 * stages) { bar = b_full; ph ^= 1; code_off = 0; }
     }
   }
 
@@ -749,7 +746,7 @@ namespace {
 constexpr uint32_t kSmemBudget = 227 * 1024;
 
 uint32_t smem_bytes(uint32_t cw, uint32_t nt, uint32_t stages, uint32_t red_slots) {
-  return 1024 + stages * cw * 2304 + cw * (kTabBytes + nt * 256) + red_slots * cw * nt * 512 + (2 * stages + 4) * 8 + 16;
+  return 1024 + stages * cw * 2304 + cw * (kTabBytes + nt * 256) + red_slots * cw * nt * 512 + kBarBytes;
 }
 
 struct Maps {

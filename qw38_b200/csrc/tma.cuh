@@ -64,6 +64,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   if (mbar_try(bar, parity)) return true;
   return mbar_wait_slow(bar, parity, abort_flag, status, code);
 }
+// The same with the abort flag given by its shared-space address (one register where a pointer takes two).
+static __device__ __noinline__ bool mbar_wait_slow_at(uint32_t bar, uint32_t parity, uint32_t abort_at, int* status, int code) {
+  return mbar_wait_spin(bar, parity, reinterpret_cast<volatile int*>(__cvta_shared_to_generic(abort_at)), status, code);
+}
+__device__ __forceinline__ bool mbar_wait_at(uint32_t bar, uint32_t parity, uint32_t abort_at, int* status, int code) {
+  if (mbar_try(bar, parity)) return true;
+  return mbar_wait_slow_at(bar, parity, abort_at, status, code);
+}
 // The same wait, fully inlined: a function call inside a kernel that moves registers between warps with setmaxnreg
 // does not compile.  mbarrier.try_wait suspends the thread in hardware for a while by itself; sleeping between tries
 // (nanosleep, any back-off) only added wake-up latency to the hand-offs when it was measured, so there is none.  The

@@ -241,22 +241,24 @@ int caller_scratch(const q4k_project_options* opt, uint64_t partial_bytes, uint6
 
 constexpr uint32_t kFlagTrustedSpans = 1u, kFlagInputSettled = 2u;
 
-// The fp16-plane kernel with scratch of its own (stream_scratch.cu).
-// Nine to sixteen tokens: from this many super-blocks of eight rows on.  The TMA-streamed kernel against this one, us, replayed
-// graph over matrices that do not fit L2, launches serialised / overlapped with settled inputs:
+// Nine to sixteen tokens: the kind::i8 kernel from this many super-blocks of eight rows on, the TMA-streamed one below.  The latter against
+// the former, us, replayed graph over matrices that do not fit L2, launches serialised / overlapped with settled inputs:
 //                                 nine tokens                  sixteen tokens
-//   5120 x 5120   (12800)   10.5 : 12.0 /  9.0 :  9.8    12.1 : 12.4 / 10.1 : 10.0
-//   6144 x 5120   (15360)   11.9 : 13.1 / 10.3 : 10.9    13.4 : 13.2 / 11.2 : 10.9
-//   6656 x 5120   (16640)   12.2 : 13.5 / 10.7 : 11.2    13.8 : 13.6 / 11.8 : 11.2
-//   7168 x 5120   (17920)   13.1 : 13.3 / 11.4 : 11.3    14.9 : 13.2 / 12.7 : 11.4
-//   10240 x 5120  (25600)   16.1 : 15.5 / 14.5 : 13.6    18.2 : 15.6 / 16.5 : 13.7
-//   13312 x 2560  (16640)   10.1 : 12.0 /  8.7 : 10.1    11.0 : 12.0 /  9.2 : 10.2
-//   2048 x 17408  (17408)   12.9 : 15.0 / 10.1 : 12.8    15.6 : 15.3 / 11.9 : 12.9
-//   2560 x 17408  (21760)   15.0 : 16.1 / 12.9 : 13.7    17.1 : 16.2 / 14.7 : 13.7
-// Its time hardly depends on the token count (a tile is sixteen wide), the other's does; twelve tokens lie between.  At K = 5120
-// the line is where sixteen serialised tokens break even; nine do so at 18000 super-blocks.  Just above the line nine tokens
-// lose up to a tenth, and few rows of a long K (each of its tiles then cut over many clusters) or many of a short one a sixth.
-constexpr uint64_t kF16SuperBlocks = 16384;
+//   1024 x 1024   (512)      2.3 :  4.6 /  2.0 :  3.6     2.5 :  4.7 /  2.0 :  3.7
+//   2560 x 5120   (6400)     8.0 :  7.8 /  6.4 :  7.0     8.9 :  8.0 /  6.8 :  7.2
+//   5120 x 5120   (12800)   10.5 : 10.1 /  9.0 :  9.3    12.5 : 10.3 / 10.1 :  9.6
+//   7168 x 5120   (17920)   13.0 : 11.4 / 11.4 : 10.5    15.4 : 11.9 / 12.7 : 10.8
+//   10240 x 5120  (25600)   16.1 : 15.4 / 14.4 : 14.0    18.5 : 15.7 / 16.8 : 14.4
+//   13312 x 2560  (16640)   10.1 : 10.3 /  8.7 :  9.0    11.1 : 10.6 /  9.3 :  9.2
+//   2048 x 17408  (17408)   13.3 : 14.0 / 10.2 : 12.2    15.8 : 14.2 / 11.7 : 12.4
+//   17408 x 5120  (43520)   20.9 : 16.6 / 20.1 : 16.0    22.2 : 17.0 / 21.5 : 16.4
+// Its time hardly depends on the token count.  The line lies where nine tokens break even at K = 5120.  Both take the same operands
+// but for the alignment of the activations, and a plan or partial dots are the TMA-streamed kernel's.
+constexpr uint64_t kI8SuperBlocks = 12288;
+bool mmv_i8_better(const q4k::WeightView& w, const q4k::Q8View& x) {
+  return x.m > 8 && uint64_t(w.padded_n / 8) * w.tiles_k >= kI8SuperBlocks && q4k::mmv_i8_supported(w, x);
+}
+// The fp16-plane kernel with scratch of its own (stream_scratch.cu).
 int project_f16(const q4k_weight& w, const q4k_q8_input& x, const q4k::F16Output& out, cudaStream_t stream, const q4k_weight* second = nullptr,
                 const q4k::RawRows* raw = nullptr) {
   int* const status = q4k::kernel_status_word();
@@ -310,18 +312,28 @@ int project_impl(const q4k_weight* weight, const q4k_q8_input& x, float* output,
     //   5120 x 17408   13.6 : 15.2 / 10.4 : 13.6    16.6 : 15.3 / 13.3 : 13.6
     // Two tokens in a graph of whole layers with their packs are slower on dp4a (eight layers 544 us against 427).
     bool const tma_ok = x.m <= q4k::kGemvTmaMaxTokens && q4k::gemv_tma_supported(view(w), view(x));
-    bool const whole_dots = !partials && !(opt && (opt->split_k || opt->row_groups));
-    if (x.m > 8 && x.m <= 16 && whole_dots && w.padded_n / 8 * (w.padded_k / 256) >= kF16SuperBlocks && q4k::f16_supported(view(w), view(x)))
-      kernel = Q4K_KERNEL_F16;
-    else if (tma_ok && x.m > q4k::kGemvDp4aBestTokens) kernel = Q4K_KERNEL_GEMV_TMA;
+    if (tma_ok && x.m > q4k::kGemvDp4aBestTokens) kernel = Q4K_KERNEL_GEMV_TMA;
     else if (x.m <= 2 || (x.m <= q4k::kGemvDp4aMaxTokens && w.padded_n >= 32768)) kernel = Q4K_KERNEL_GEMV_DP4A;
     else if (x.m <= 16) kernel = Q4K_KERNEL_GEMV_MMA;
     else if (!partials && !(opt && opt->split_k) && q4k::f16_supported(view(w), view(x))) kernel = Q4K_KERNEL_F16;
     else kernel = q4k::tcgen05_supported(view(w), view(x)) ? Q4K_KERNEL_TCGEN05 : Q4K_KERNEL_MMA;
   }
   const float* res = residual_len ? residual : nullptr;
+  q4k::WeightView const wv = view(w);
+  // Nine to sixteen tokens of a large matrix, and what asks for the fp16 kernel below its token counts: tcgen05 kind::i8.
+  bool const whole_dots = !partials && !(opt && (opt->split_k || opt->row_groups));
+  bool const i8 = whole_dots && ((kernel == Q4K_KERNEL_GEMV_TMA && mmv_i8_better(wv, view(x))) ||
+                                 (kernel == Q4K_KERNEL_F16 && q4k::mmv_i8_supported(wv, view(x))));
   ScopedRange range("qw38:op name=q4k_project m=%u n=%u k=%u role=%s residual=%u compute=%s", unsigned(x.m), unsigned(w.n),
                     unsigned(w.k), role, unsigned(res != nullptr), kernel == Q4K_KERNEL_GEMV_DP4A ? "integer_dp4a" : "integer_mma");
+  if (i8) {
+    int* const status = q4k::kernel_status_word();
+    if (!status) return Q4K_ERR_STATUS;
+    q4k::GemvTmaOutput const to{output, nullptr, res};
+    Q4K_CUDA(q4k::launch_mmv_i8(&wv, &to, 1, view(x), q4k::plan_mmv_i8((w.padded_n + 127) / 128, wv.tiles_k), opt && (opt->flags & kFlagInputSettled), status, stream),
+             "q4k_q8.mmv_i8");
+    return Q4K_OK;
+  }
   if (kernel == Q4K_KERNEL_GEMV_DP4A) {
     if (x.m > q4k::kGemvDp4aMaxTokens) return fail(Q4K_ERR_INVALID_ARGUMENT, "q8.project: dp4a kernel takes m <= 4");
     int* const status = q4k::kernel_status_word();
@@ -417,10 +429,15 @@ int project_impl(const q4k_weight* weight, const q4k_q8_input& x, float* output,
 bool pair_f16(const q4k_weight* gate, const q4k_weight* up, const q4k_q8_input& x) {
   return x.m > 16 && up->n == gate->n && up->k == gate->k && q4k::f16_supported(view(*gate), view(x)) && q4k::f16_supported(view(*up), view(x));
 }
+// The same for nine to sixteen tokens and the kind::i8 kernel, with the K slices that either matrix would get by itself.
+bool pair_i8(const q4k_weight* gate, const q4k_weight* up, const q4k_q8_input& x) {
+  return up->n == gate->n && up->k == gate->k && mmv_i8_better(view(*gate), view(x)) && q4k::mmv_i8_supported(view(*up), view(x));
+}
 int project_pair(const q4k_weight* gate, const q4k_weight* up, const q4k_q8_input& x, float* g, float* u, const q4k_project_options* opt,
                  cudaStream_t stream, const q4k::RawRows* raw = nullptr) {
   uint64_t const cells = uint64_t(x.m) * gate->n;
-  if (!pair_f16(gate, up, x)) {
+  bool const i8 = pair_i8(gate, up, x);
+  if (!i8 && !pair_f16(gate, up, x)) {
     if (int st = project_impl(gate, x, g, cells, nullptr, 0, opt, stream, false, "gate")) return st;
     return project_impl(up, x, u, cells, nullptr, 0, opt, stream, false, "up");
   }
@@ -436,6 +453,16 @@ int project_pair(const q4k_weight* gate, const q4k_weight* up, const q4k_q8_inpu
   }
   ScopedRange range("qw38:op name=q4k_project m=%u n=%u k=%u role=%s residual=%u compute=%s", unsigned(x.m), unsigned(2 * gate->n),
                     unsigned(gate->k), "gate_up", 0u, "integer_mma");
+  if (i8) {
+    int* const status = q4k::kernel_status_word();
+    if (!status) return Q4K_ERR_STATUS;
+    q4k::WeightView const views[2] = {view(*gate), view(*up)};
+    q4k::GemvTmaOutput const to[2] = {{g, nullptr, nullptr}, {u, nullptr, nullptr}};
+    Q4K_CUDA(q4k::launch_mmv_i8(views, to, 2, view(x), q4k::plan_mmv_i8((gate->padded_n + 127) / 128, views[0].tiles_k), opt && (opt->flags & kFlagInputSettled),
+                                status, stream),
+             "q4k_q8.mmv_i8");
+    return Q4K_OK;
+  }
   return project_f16(*gate, x, q4k::F16Output{g, u, nullptr, false}, stream, up, raw);
 }
 
@@ -760,7 +787,7 @@ int decode_fused(const q4k_decode_desc* const* descs, uint32_t count, bool swigl
   int nreg = 0;
   // the pack of the workspace is one run of memory: codes, scales, sums
   regions[nreg++] = {q8.codes, uint64_t(reinterpret_cast<uint8_t*>(q8.sums + q8.sums_len) - reinterpret_cast<uint8_t*>(q8.codes)), 4, "workspace"};
-  uint64_t n_total = 0, tiles = 0;
+  uint64_t n_total = 0, tiles = 0, tiles128 = 0, super_blocks = 0;
   for (uint32_t i = 0; i < count; ++i) {
     const q4k_decode_desc& d = *descs[i];
     if (d.activation_policy != Q4K_ACTIVATION_Q8_K32 || d.m > q4k::kGemvTmaMaxTokens || d.weight.k != descs[0]->weight.k) return Q4K_OK;
@@ -796,6 +823,8 @@ int decode_fused(const q4k_decode_desc* const* descs, uint32_t count, bool swigl
     }
     n_total += d.weight.n;
     tiles += (d.weight.padded_n + 15) / 16;
+    tiles128 += (d.weight.padded_n + 127) / 128;
+    super_blocks += uint64_t(d.weight.padded_n / 8) * ws[i].tiles_k;
   }
   Region const input{descs[0]->input, descs[0]->input_len * 2, 2, "input"}, flag{failure, 4, 4, "failure"};
   bool raw = q8.m <= kDecodeRawTokens && failure;
@@ -814,6 +843,15 @@ int decode_fused(const q4k_decode_desc* const* descs, uint32_t count, bool swigl
     int* const status = q4k::kernel_status_word();
     if (!status) return Q4K_ERR_STATUS;
     Q4K_CUDA(q4k::launch_gemv_dp4a_multi(ws, outs, count, q8.m, q8.padded_k, rows, status, stream), "decode_mmv.fused");
+    *fused = true;
+    return Q4K_OK;
+  }
+  bool i8 = !swiglu && !raw && q8.m > 8 && super_blocks >= kI8SuperBlocks;
+  for (uint32_t i = 0; i < count; ++i) i8 = i8 && q4k::mmv_i8_supported(ws[i], view(q8));
+  if (i8) {
+    int* const status = q4k::kernel_status_word();
+    if (!status) return Q4K_ERR_STATUS;
+    Q4K_CUDA(q4k::launch_mmv_i8(ws, outs, count, view(q8), q4k::plan_mmv_i8(uint32_t(tiles128), ws[0].tiles_k), false, status, stream), "decode_mmv.fused");
     *fused = true;
     return Q4K_OK;
   }
@@ -1269,9 +1307,10 @@ int q4k_q8_mlp(const q4k_weight* gate, const q4k_weight* up, const q4k_weight* d
   };
   q4k_q8_input xh = hidden_pack(true);
   q4k::GemvTmaPlan fused_plan{};
-  bool const fused = m <= q4k::kGemvTmaMaxTokens && q4k::gemv_tma_supported(view(*gate), view(xh)) &&
+  q4k_q8_input const beside = hidden_pack(false);
+  bool const fused = !pair_i8(gate, up, beside) && m <= q4k::kGemvTmaMaxTokens && q4k::gemv_tma_supported(view(*gate), view(xh)) &&
                      q4k::gemv_tma_supported(view(*up), view(xh)) && q4k::plan_gemv_tma_swiglu_q8(m, view(*gate), &fused_plan);
-  if (!fused) xh = hidden_pack(false);
+  if (!fused) xh = beside;
   q4k_q8_input xf{codes, scales, sums, uint64_t(m) * ffn, uint64_t(m) * (ffn / 32), uint64_t(m) * (ffn / 32), m, ffn, ffn};
   q4k_project_options opt{};
   opt.flags = kFlagTrustedSpans;  // every span was validated above

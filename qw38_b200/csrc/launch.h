@@ -107,7 +107,7 @@ struct RawRows {
 // f16_scratch_bytes (256-byte aligned) and is used until the launch ends.  alternates: the preceding launch of the stream
 // does not use this scratch, so (with launch overlap and a settled input) the planes may be written beside it.
 struct F16Plan {
-  uint32_t nt;             // tokens per tile: 16, 32, 64 or 128
+  uint32_t nt;             // tokens per tile: 32, 64 or 128
   uint32_t chunk;          // tokens per pass
   uint32_t workers;        // clusters of two SMs
   uint32_t unit_step;      // granularity of a cluster's run of super-blocks: 1, or tiles_k = whole tiles
@@ -181,6 +181,16 @@ cudaError_t launch_gemv_tma_swiglu_q8(const WeightView& gate, const WeightView& 
 cudaError_t launch_gemv_tma(const WeightView& w, const Q8View& x, float* out, const float* residual, int32_t* partials,
                             const GemvTmaPlan& plan, void* slices, uint32_t* tickets, int* status, cudaStream_t stream,
                             const GemvTmaGather* gather = nullptr);
+
+// mmv_i8.cu : tcgen05 kind::i8 with the weights in tensor memory, m <= 16.  The projections of up to three weights that share x
+// (GemvTmaOutput as above) in one launch; splits: K slices of a 128-row tile, the blocks of a cluster, from plan_mmv_i8 over the
+// tiles of the weights.  Results of a tile depend on K and splits alone, so the launch of a pair cut as one of its matrices is
+// bitwise the two launches.
+constexpr uint32_t kMmvI8MaxTokens = 16;
+bool mmv_i8_supported(const WeightView& w, const Q8View& x);
+uint32_t plan_mmv_i8(uint32_t tiles, uint32_t tiles_k);
+cudaError_t launch_mmv_i8(const WeightView* ws, const GemvTmaOutput* outs, uint32_t count, const Q8View& x, uint32_t splits,
+                          bool input_settled, int* status, cudaStream_t stream);
 
 // peer.cu : announces this rank's finished projections to every rank, then waits (bounded) until every
 // rank's counter in this rank's own flag array has reached this rank's own; a wait that gives up

@@ -1,0 +1,531 @@
+// Q4_K x Q8 for up to sixteen tokens on tcgen05 kind::i8: weights as bytes in tensor memory, one accumulator per K32 group,
+// drained once per super-block.
+//
+//   out[t][n] = sum_kb ( d[n,kb] * sum_g a[t,g] * (sc[n,g] * dot[n,t,g]) - dmin[n,kb] * sum_g mn[n,g] * (a*s)[t,g] )
+//
+// With sixteen columns an accumulator is so small that all eight groups of a super-block have one of their own (128 TMEM columns, two
+// sets of them): a hand-off between the tensor core and the warps that scale is due once per super-block, not per group, and a
+// weight costs a mask (and a shift) to expand instead of a conversion.  Per 128 rows x 256 columns about 2200 warp instructions,
+// where the warp-level MMAs of gemv_tma.cu take 3460 at two token octets and the fp16 planes' expanders alone 1800.
+//   * Expanders (lane = row): nibbles -> bytes -> TMEM (A operand).  Byte order inside eight columns: even ones, then odd ones.
+//   * Activation warps put the codes into that order (B operand in shared memory), with a and the terms of a * s beside.  What they
+//     read comes by TMA three super-blocks ahead: behind the weights' copies a load from L2 takes 1500 clk.
+//   * A constant MMA presets an accumulator to 2^17 and the data MMA adds the dot (|dot| <= 60960): a positive integer v below
+//     2^18, whose bits are the subnormal v * 2^-149.  One FMA with sc * 2^121 and -sc * 2^-11 makes it sc * dot * 2^-28,
+//     exactly and without a conversion; the next folds a * 2^28.  A token with a scale of 2^90 or more in this super-block keeps
+//     a as it is and gets its 2^28 afterwards.
+//   * Min term: mn (six bits) times the three tf32 terms that add up to a * s exactly, three kind::tf32 MMAs.
+// Dots are exact integers and never cross a group; scales stay fp32.  Error against the equation in 64 bits as the other int8 kernels.
+//
+// A block has an SM to itself and takes 128-row tiles: whole ones in turn, or one K slice of one.  The K slices of a tile are the blocks of
+// a cluster; their rows are added in slice order through distributed shared memory: no scratch in global memory, no tickets, so calls
+// on several streams share nothing.
+//
+// Sixteen tokens, us, replayed graph over matrices that do not fit L2, launches serialised / overlapped with settled inputs (TMA-streamed
+// kernel, fp16 planes before): 5120 x 5120 10.3 / 9.6 (12.5 / 10.1, 12.3 / 9.8), 7168 x 5120 11.9 / 10.8 (15.4 / 12.7, 13.4 / 11.4),
+// 17408 x 5120 17.0 / 16.4 (22.2 / 21.5, 19.6 / 17.9), 34816 x 5120 30.4 / 29.1 (36.0 / 34.4, 31.5 / 29.8), 5120 x 17408 19.5 / 19.1
+// (28.7 / 25.1, 21.8 / 20.0).  Bound: 950 clk per super-block, where HBM needs 800: a warp gets an instruction out every ten clocks (five
+// warps per scheduler, each behind a barrier or a TMEM access much of the time).  Tried and slower: two blocks per SM with one set of
+// accumulators each (1420 clk), one group of epilogue warps (1250), sixteen epilogue warps of eight tokens (1100), factors of the rows
+// from a table in shared memory, registers handed round by setmaxnreg (no change), one polling lane per warp (+8 %), back-off in the
+// waits (no change).
+//
+// Warps: 0 raw weights (TMA), 1 MMA issue, 2 and 3 activations, then two groups of four expanders and two of four epilogue warps; what comes
+// in twos takes super-blocks in turn.  Every wait is bounded; a wait that gives up sets the abort flag and the status word, and every
+// role leaves its loop.
+#include <cuda.h>
+
+#include "common.cuh"
+#include "launch.h"
+#include "tma.cuh"
+#include "umma.cuh"
+
+namespace q4k {
+namespace {
+
+constexpr uint32_t kRows = 128, kTok = 16;  // tile rows; MMA width
+constexpr uint32_t kFirstExpander = 4, kFirstEpilogue = 12, kThreads = (kFirstEpilogue + 8) * 32;
+constexpr uint32_t kRawStages = 8, kRaw = 16 * 1024 + 2 * 1024;
+constexpr uint32_t kQ8Stages = 6, kQ8 = 4096 + 2 * 512;  // codes [half][token][128 B, swizzled], scales and sums [token][8]
+// Activation stage: codes [16-byte chunk of K][token octet][8][16 B], three terms of a * s [term][half of the groups][token octet][8][16 B],
+// a' [group][token], 2^0 or 2^28 [token].
+constexpr uint32_t kStages = 4, kZ = 4096, kTerm = 512, oTerms = kZ, oA = oTerms + 3 * kTerm, oE = oA + 512, kB = oE + 128;
+constexpr uint32_t kSclStages = 4, kScl = kRows * 16;  // {six-bit scales, d | dmin} of a row
+constexpr uint32_t kPart = kTok * kRows * 4;           // rows of a tile, of one group of epilogue warps
+constexpr uint32_t oRaw = 0, oQ8 = oRaw + kRawStages * kRaw, oB = oQ8 + kQ8Stages * kQ8, oScl = oB + kStages * kB, oParts = oScl + kSclStages * kScl,
+                   oConst = oParts + 2 * kPart, oBar = oConst + kTok * 32;
+constexpr uint32_t bRawFull = 0, bRawFree = bRawFull + 8 * kRawStages, bFull = bRawFree + 8 * kRawStages, bFree = bFull + 8 * kStages,
+                   bSclFull = bFree + 8 * kStages, bSclFree = bSclFull + 8 * kSclStages, bAFull = bSclFree + 8 * kSclStages, bDone = bAFull + 16,
+                   bDFree = bDone + 16, bQ8 = bDFree + 16, bPartFull = bQ8 + 8 * kQ8Stages, bPartFree = bPartFull + 8, kBars = bPartFree + 8;
+constexpr uint32_t kSmem = oBar + kBars + 16 + 1024;
+static_assert(kSmem <= 227 * 1024, "shared memory");
+static_assert(kB % 128 == 0 && oConst % 128 == 0, "operands without swizzle are read in units of 16 bytes");
+// TMEM columns, two sets: accumulators of the eight groups and of the min term; weights (eight columns per group) and mins.  A constant operand.
+constexpr uint32_t cM = 8 * kTok, kD = cM + kTok, cA = 2 * kD, cMins = 64, kA = cMins + 8, cConst = cA + 2 * kA, kCols = 512;
+static_assert(cConst + 8 <= kCols, "TMEM columns");
+
+struct I8Segment {
+  float* out;
+  uint16_t* out_bf16;
+  const float* residual;
+  uint32_t n, tile0;  // rows; first tile among the launch's
+};
+struct I8Params {
+  I8Segment seg[3];
+  int* status;
+  uint32_t nseg, m, padded_k, tiles_k, splits, tiles;
+  uint32_t early;          // weights may be read before the preceding launch has ended
+  uint32_t input_settled;  // so may the activations
+};
+
+// D = A * B (+ D); A in tensor memory, B in shared memory.
+template <bool Acc> __device__ __forceinline__ void mma_i8(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc) {
+  asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p; }"
+               ::"r"(d), "r"(a), "l"(b), "r"(idesc), "n"(Acc ? 1 : 0) : "memory");
+}
+template <bool Acc> __device__ __forceinline__ void mma_tf32(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc) {
+  asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p; }"
+               ::"r"(d), "r"(a), "l"(b), "r"(idesc), "n"(Acc ? 1 : 0) : "memory");
+}
+constexpr uint32_t kIdescI8 = (2u << 4) | (1u << 7) | (1u << 10) | ((kTok >> 3) << 17) | ((kRows >> 4) << 24);    // s8 x s8 -> s32
+constexpr uint32_t kIdescTf32 = (1u << 4) | (2u << 7) | (2u << 10) | ((kTok >> 3) << 17) | ((kRows >> 4) << 24);  // tf32 x tf32 -> f32
+__device__ __forceinline__ void tmem_st8(uint32_t t, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+               ::"r"(t), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
+// Are the phases of all three barriers over?
+__device__ __forceinline__ bool mbar_try3(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1, uint32_t bar2, uint32_t parity2) {
+  uint32_t ok;
+  asm volatile("{ .reg .pred p, q, r;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n mbarrier.test_wait.parity.shared::cta.b64 q, [%3], %4;\n"
+               " mbarrier.test_wait.parity.shared::cta.b64 r, [%5], %6;\n and.pred p, p, q;\n and.pred p, p, r;\n selp.u32 %0, 1, 0, p; }"
+               : "=r"(ok) : "r"(bar0), "r"(parity0), "r"(bar1), "r"(parity1), "r"(bar2), "r"(parity2) : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ float peer_f32(uint32_t addr, uint32_t rank) {
+  float v;
+  asm volatile("{ .reg .b32 a; mapa.shared::cluster.u32 a, %1, %2; ld.shared::cluster.f32 %0, [a]; }" : "=f"(v) : "r"(addr), "r"(rank) : "memory");
+  return v;
+}
+__device__ __forceinline__ void store(const I8Segment& s, uint64_t o, float v) {
+  if (s.residual) v += s.residual[o];
+  if (s.out_bf16) s.out_bf16[o] = f32_to_bf16_rne(v);
+  else s.out[o] = v;
+}
+// Byte i of w as a float.
+__device__ __forceinline__ float byte_float(uint32_t w, int i) { return __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7650 | i)) - 8388608.0f; }
+
+// Octets: of tokens that are read back and scaled.
+template <int Octets>
+__global__ void __launch_bounds__(kThreads, 1)
+mmv_i8_kernel(const __grid_constant__ CUtensorMap tm_codes0, const __grid_constant__ CUtensorMap tm_meta0,
+              const __grid_constant__ CUtensorMap tm_codes1, const __grid_constant__ CUtensorMap tm_meta1,
+              const __grid_constant__ CUtensorMap tm_codes2, const __grid_constant__ CUtensorMap tm_meta2, const __grid_constant__ CUtensorMap tm_x,
+              const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_s, const __grid_constant__ I8Params p) {
+  constexpr int NTOK = 8 * Octets;  // tokens of an epilogue warp
+  extern __shared__ uint8_t smem_raw[];
+  uint32_t const smem = (smem_u32(smem_raw) + 1023u) & ~1023u, bars = smem + oBar;
+  volatile int* const abort_flag = reinterpret_cast<volatile int*>(smem_raw + (smem - smem_u32(smem_raw)) + oBar + kBars);
+  uint32_t const tmem_slot = bars + kBars + 4;
+  uint32_t const warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint32_t const rank = p.splits > 1 ? cluster_rank() : 0u;
+  // A block's tiles; with K slices it has one.  Super-blocks are counted through all of them.
+  uint32_t const first = blockIdx.x / p.splits, step = gridDim.x / p.splits, tiles = (p.tiles - first + step - 1) / step;
+  auto segment = [&](uint32_t tile) { return p.nseg > 2 && tile >= p.seg[2].tile0 ? 2u : (p.nseg > 1 && tile >= p.seg[1].tile0 ? 1u : 0u); };
+  uint32_t const kb0 = p.tiles_k * rank / p.splits, units = p.tiles_k * (rank + 1) / p.splits - kb0, N = tiles * units;
+  auto wait = [&](uint32_t bar, uint32_t parity, int code) { return mbar_wait_inline(bar, parity, abort_flag, p.status, code); };
+  // A barrier that is ready answers after a hundred clocks and more, so the three of one place are asked in one breath.
+  auto wait3 = [&](uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1, uint32_t bar2, uint32_t parity2, int code) {
+    return mbar_try3(bar0, parity0, bar1, parity1, bar2, parity2) ||
+           (wait(bar0, parity0, code) && wait(bar1, parity1, code) && wait(bar2, parity2, code));
+  };
+
+  if (warp == 0 && lane == 0) {
+    for (uint32_t i = 0; i < kBars / 8; ++i) {
+      uint32_t const at = 8 * i;
+      uint32_t count = 1;
+      if ((at >= bRawFree && at < bFull) || (at >= bSclFull && at < bSclFree) || (at >= bAFull && at < bDone)) count = 4;  // expander warps
+      if ((at >= bSclFree && at < bAFull) || (at >= bDFree && at < bQ8) || at >= bPartFull) count = 4;                       // epilogue warps
+      if (at >= bFree && at < bSclFull) count = 1 + 4;                                                                       // products, epilogue warps
+      mbar_init(bars + at, count);
+    }
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "n"(kCols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (warp == 2) {  // constant operand: 64 * 64 * 32 columns = 2^17
+    sts128(smem + oConst + lane * 16, 0x40404040u, 0x40404040u, 0x40404040u, 0x40404040u);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  uint32_t const tmem = lds32(tmem_slot);
+
+  if (warp == 0) {
+    // ---- raw weights: streamed at once where the caller vouches for them, else L2 is asked for the first stages
+    if (lane == 0) {
+      uint32_t s = 0, ph = 1;
+      for (uint32_t i = 0; i < tiles; ++i) {
+        uint32_t const tile = first + i * step, sg = segment(tile);
+        const CUtensorMap* const mc = sg == 0 ? &tm_codes0 : (sg == 1 ? &tm_codes1 : &tm_codes2);
+        const CUtensorMap* const mm = sg == 0 ? &tm_meta0 : (sg == 1 ? &tm_meta1 : &tm_meta2);
+        int const rg = int((tile - p.seg[sg].tile0) * (kRows / 8));
+        if (i == 0 && !p.early) {
+          for (uint32_t u = 0; u < kRawStages && u < units; ++u) {
+            tma_3d_prefetch(mc, 0, int((kb0 + u) * 8), rg);
+            tma_3d_prefetch(mm, 0, int(kb0 + u), rg);
+          }
+          pdl_wait();
+        }
+        bool ok = true;
+        for (uint32_t u = 0; u < units; ++u) {
+          uint32_t const full = bars + bRawFull + 8 * s, dst = smem + oRaw + s * kRaw;
+          ok = wait(bars + bRawFree + 8 * s, ph, 0x901);
+          if (!ok) break;
+          mbar_expect_tx(full, kRaw);
+          tma_3d(dst, mc, 0, int((kb0 + u) * 8), rg, full);
+          tma_3d(dst + 16 * 1024, mm, 0, int(kb0 + u), rg, full);
+          if (++s == kRawStages) { s = 0; ph ^= 1; }
+        }
+        if (!ok) break;
+      }
+    }
+  } else if (warp == 1) {
+    // ---- MMA issue
+    if (elect_one()) {
+      uint64_t const one = umma_desc_plain(smem + oConst, 256, 128);
+      for (uint32_t u = 0; u < N; ++u) {
+        uint32_t const s = u % kStages, e = u & 1, ph = (u >> 1) & 1, b = smem + oB + s * kB, d = tmem + e * kD, a = tmem + cA + e * kA;
+        if (!wait3(bars + bFull + 8 * s, (u / kStages) & 1, bars + bAFull + 8 * e, ph, bars + bDFree + 8 * e, ph ^ 1, 0x902)) break;
+        tc_fence_after();
+#pragma unroll
+        for (uint32_t g = 0; g < 8; ++g) {
+          mma_i8<false>(d + g * kTok, tmem + cConst, one, kIdescI8);  // same kind and shape: runs before the next one
+          mma_i8<true>(d + g * kTok, a + g * 8, umma_desc_plain(b + g * 512, 256, 128), kIdescI8);
+        }
+        // small terms first
+        mma_tf32<false>(d + cM, a + cMins, umma_desc_plain(b + oTerms + 2 * kTerm, 256, 128), kIdescTf32);
+        mma_tf32<true>(d + cM, a + cMins, umma_desc_plain(b + oTerms + kTerm, 256, 128), kIdescTf32);
+        mma_tf32<true>(d + cM, a + cMins, umma_desc_plain(b + oTerms, 256, 128), kIdescTf32);
+        umma_commit(bars + bDone + 8 * e);
+        umma_commit(bars + bFree + 8 * s);
+      }
+    }
+  } else if (warp < 4) {
+    // ---- activations.  Lane = (chunk of K, token) for the codes, (token, half of the groups) for the rest.
+    if (!p.input_settled) pdl_wait();
+    uint32_t const w = warp - 2, zt = lane & 15, zc = lane >> 4, at = lane >> 1, ah = lane & 1;
+    auto fetch = [&](uint32_t u) {  // super-block u into the warp's ring of three
+      uint32_t const q = (u >> 1) % 3 * 2 + w, dst = smem + oQ8 + q * kQ8, bar = bars + bQ8 + 8 * q, kb = kb0 + u % units;
+      mbar_expect_tx(bar, kQ8);
+      tma_3d(dst, &tm_x, 0, 0, int(kb * 2), bar);
+      tma_2d(dst + 4096, &tm_a, int(kb * 8), 0, bar);
+      tma_2d(dst + 4096 + 512, &tm_s, int(kb * 8), 0, bar);
+    };
+    if (lane == 0)
+      for (uint32_t u = w; u < 6 && u < N; u += 2) fetch(u);
+    for (uint32_t u = w; u < N; u += 2) {
+      uint32_t const s = u % kStages, ph = (u / kStages & 1) ^ 1, b = smem + oB + s * kB, q = (u >> 1) % 3 * 2 + w, from = smem + oQ8 + q * kQ8;
+      if (!wait(bars + bQ8 + 8 * q, (u / 6) & 1, 0x904)) break;
+      uint4 z[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) z[i] = lds128(from + (i >> 2) * 2048 + zt * 128 + (((2 * i + zc) ^ zt) & 7) * 16);
+      float4 const av = lds128f(from + 4096 + lane * 16);
+      uint4 const sv = lds128(from + 4096 + 512 + lane * 16);
+      float const a[4] = {av.x, av.y, av.z, av.w};
+      int const sum[4] = {int(sv.x), int(sv.y), int(sv.z), int(sv.w)};
+      __syncwarp();
+      if (lane == 0 && u + 6 < N) fetch(u + 6);
+      if (!wait(bars + bFree + 8 * s, ph, 0x905)) break;
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        sts128(b + (2 * i + zc) * 256 + zt * 16, even_bytes(z[i].x, z[i].y), odd_bytes(z[i].x, z[i].y), even_bytes(z[i].z, z[i].w),
+               odd_bytes(z[i].z, z[i].w));
+      float hi[4], mid[4], lo[4];
+      bool big = false;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float const as = a[j] * float(sum[j]);
+        hi[j] = tf32_part(as);
+        mid[j] = tf32_part(as - hi[j]);
+        lo[j] = as - hi[j] - mid[j];
+        big = big || fabsf(a[j]) >= 0x1p90f;
+      }
+      uint32_t const row = b + oTerms + ah * 256 + at * 16;
+      sts128f(row, hi[0], hi[1], hi[2], hi[3]);
+      sts128f(row + kTerm, mid[0], mid[1], mid[2], mid[3]);
+      sts128f(row + 2 * kTerm, lo[0], lo[1], lo[2], lo[3]);
+      big = __shfl_xor_sync(0xffffffffu, int(big), 1) || big;  // of the token's eight groups
+#pragma unroll
+      for (int j = 0; j < 4; ++j) sts32f(b + oA + (ah * 4 + j) * 64 + at * 4, big ? a[j] : a[j] * 0x1p28f);
+      if (ah == 0) sts32f(b + oE + at * 4, big ? 0x1p28f : 1.f);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bars + bFull + 8 * s);
+    }
+  } else if (warp < kFirstEpilogue) {
+    // ---- expanders: two groups of four warps take every other super-block
+    uint32_t const quarter = warp & 3, row = quarter * 32 + lane, base = tmem + ((quarter * 32u) << 16);
+    {
+      uint32_t const c[8] = {0x40404040u, 0x40404040u, 0x40404040u, 0x40404040u, 0x40404040u, 0x40404040u, 0x40404040u, 0x40404040u};
+      tmem_st8(base + cConst, c);
+    }
+    uint32_t const e = (warp - kFirstExpander) >> 2, a = base + cA + e * kA;
+    for (uint32_t u = e; u < N; u += 2) {
+      uint32_t const ph = (u >> 1) & 1, r = u % kRawStages, rph = (u / kRawStages) & 1, raw = smem + oRaw + r * kRaw;
+      uint32_t const sc = u % kSclStages, sph = (u / kSclStages) & 1;
+      // the weights, the place of the scales, and the products that read this operand before
+      if (!wait3(bars + bRawFull + 8 * r, rph, bars + bSclFree + 8 * sc, sph ^ 1, bars + bDone + 8 * e, ph ^ 1, 0x906)) break;
+      tc_fence_after();
+      uint4 const cm = lds128(raw + 16 * 1024 + row * 16);
+      uint4 w[8];
+#pragma unroll
+      for (int g = 0; g < 8; ++g) w[g] = lds128(raw + row * 128 + ((uint32_t(g) ^ (row & 7)) << 4));
+      ScaleMinWords const sm = decode_scale_min(cm.y, cm.z, cm.w);
+      sts128(smem + oScl + sc * kScl + row * 16, sm.sc_lo, sm.sc_hi, cm.x, 0u);
+      uint32_t mn[8];
+#pragma unroll
+      for (int g = 0; g < 8; ++g) mn[g] = __float_as_uint(byte_float(g < 4 ? sm.mn_lo : sm.mn_hi, g & 3));
+      tmem_st8(a + cMins, mn);
+#pragma unroll
+      for (int g = 0; g < 8; g += 2) {
+        uint32_t v[16];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          uint32_t const ww[4] = {w[g + i].x, w[g + i].y, w[g + i].z, w[g + i].w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            v[i * 8 + 2 * j] = ww[j] & 0x0f0f0f0fu;
+            v[i * 8 + 2 * j + 1] = (ww[j] >> 4) & 0x0f0f0f0fu;
+          }
+        }
+        tmem_st16(a + g * 8, v);
+      }
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(bars + bSclFull + 8 * sc);
+        mbar_arrive(bars + bRawFree + 8 * r);
+      }
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bars + bAFull + 8 * e);
+    }
+  } else {
+    // ---- epilogue: lane = row, all tokens; two groups of four warps take every other super-block
+    pdl_wait();
+    if (warp == kFirstEpilogue) pdl_launch_dependents();
+    uint32_t const quarter = warp & 3, row = quarter * 32 + lane, e = (warp - kFirstEpilogue) >> 2, base = tmem + ((quarter * 32u) << 16);
+    bool ok = true;
+    uint32_t u = e;
+    for (uint32_t i = 0; ok && i < tiles; ++i) {
+      uint32_t const tile = first + i * step, sg = segment(tile), n_row = (tile - p.seg[sg].tile0) * kRows + row;
+      I8Segment const& S = p.seg[sg];
+      float2 total[NTOK / 2];
+#pragma unroll
+      for (int j = 0; j < NTOK / 2; ++j) total[j] = make_float2(0.f, 0.f);
+      for (; u < (i + 1) * units; u += 2) {
+        uint32_t const s = u % kStages, ph = (u >> 1) & 1, b = smem + oB + s * kB, d0 = base + e * kD, ss = u % kSclStages;
+        ok = wait3(bars + bFull + 8 * s, (u / kStages) & 1, bars + bSclFull + 8 * ss, (u / kSclStages) & 1, bars + bDone + 8 * e, ph, 0x909);
+        if (!ok) break;
+        tc_fence_after();
+        uint4 const sc = lds128(smem + oScl + ss * kScl + row * 16);
+        bool const plain = __all_sync(0xffffffffu, __uint_as_float(lds32(b + oE + (lane % NTOK) * 4)) == 1.f);
+        float2 acc[NTOK / 2];
+#pragma unroll
+        for (int j = 0; j < NTOK / 2; ++j) acc[j] = make_float2(0.f, 0.f);
+        uint32_t M[NTOK];
+        // A batch of groups at a time, the next requested before this one is scaled.
+        constexpr int kBatch = 2 / Octets;
+        uint32_t words[2][kBatch][NTOK];
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) tmem_ld<NTOK>(d0 + i * kTok, words[0][i]);
+#pragma unroll
+        for (int g0 = 0; g0 < 8; g0 += kBatch) {
+          tmem_wait_ld();
+          auto& D = words[(g0 / kBatch) & 1];
+          if (g0 + kBatch < 8) {
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i) tmem_ld<NTOK>(d0 + (g0 + kBatch + i) * kTok, words[(g0 / kBatch + 1) & 1][i]);
+            if (g0 + 2 * kBatch == 8) tmem_ld<NTOK>(d0 + cM, M);
+          } else {  // everything of this super-block is in registers
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bars + bDFree + 8 * e);
+          }
+#pragma unroll
+          for (int i = 0; i < kBatch; ++i) {
+            int const g = g0 + i;
+            float const f = byte_float(g < 4 ? sc.x : sc.y, g & 3), big = f * 0x1p121f, bias = f * -0x1p-11f;
+            float4 a[NTOK / 4];
+#pragma unroll
+            for (int j = 0; j < NTOK / 4; ++j) a[j] = lds128f(b + oA + g * 64 + j * 16);
+#pragma unroll
+            for (int j = 0; j < NTOK / 2; ++j) {
+              float2 const t = __ffma2_rn(make_float2(__uint_as_float(D[i][2 * j]), __uint_as_float(D[i][2 * j + 1])), make_float2(big, big), make_float2(bias, bias));
+              float2 const aj = (j & 1) ? make_float2(a[j / 2].z, a[j / 2].w) : make_float2(a[j / 2].x, a[j / 2].y);
+              acc[j] = __ffma2_rn(t, aj, acc[j]);
+            }
+          }
+        }
+        if (!plain) {
+#pragma unroll
+          for (int j = 0; j < NTOK / 2; ++j) {
+            acc[j].x *= __uint_as_float(lds32(b + oE + j * 8));
+            acc[j].y *= __uint_as_float(lds32(b + oE + j * 8 + 4));
+          }
+        }
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(bars + bFree + 8 * s);
+          mbar_arrive(bars + bSclFree + 8 * ss);
+        }
+        float const d = fp16_bits_to_f32(sc.z & 0xffffu), ndmin = -fp16_bits_to_f32(sc.z >> 16);
+#pragma unroll
+        for (int j = 0; j < NTOK / 2; ++j)
+          total[j] = __fadd2_rn(total[j], __ffma2_rn(acc[j], make_float2(d, d),
+                                                     __fmul2_rn(make_float2(__uint_as_float(M[2 * j]), __uint_as_float(M[2 * j + 1])), make_float2(ndmin, ndmin))));
+      }
+      if (!ok) break;
+      // The two groups' rows meet.  Of a block's last tile (with K slices its only one) both lie in shared memory in the end, where all
+      // threads of the cluster finish them; of an earlier one the first group takes the second one's.
+      uint32_t const part = smem + oParts + e * kPart + row * 4;
+      bool const last = i + 1 == tiles;
+      if (e == 1 || last) {
+        if (e == 1) ok = wait(bars + bPartFree, (i & 1) ^ 1, 0x90a);
+        if (!ok) break;
+#pragma unroll
+        for (int t = 0; t < NTOK; ++t) sts32f(part + t * kRows * 4, (t & 1) ? total[t / 2].y : total[t / 2].x);
+        __syncwarp();
+        if (lane == 0 && !last) mbar_arrive(bars + bPartFull);
+      } else {
+        ok = wait(bars + bPartFull, i & 1, 0x90b);
+        if (!ok) break;
+#pragma unroll
+        for (int t = 0; t < NTOK; ++t) {
+          float& v = (t & 1) ? total[t / 2].y : total[t / 2].x;
+          v += __uint_as_float(lds32(part + kPart + t * kRows * 4));
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bars + bPartFree);
+        if (n_row < S.n) {
+#pragma unroll
+          for (int t = 0; t < NTOK; ++t)
+            if (t < int(p.m)) store(S, uint64_t(t) * S.n + n_row, (t & 1) ? total[t / 2].y : total[t / 2].x);
+        }
+      }
+    }
+  }
+
+  // ---- teardown
+  __syncwarp();
+  if (*abort_flag) {  // copies still in flight land before shared memory is used again or goes away
+    long long const t0 = clock64();
+    while (clock64() - t0 < 4000000LL) {}
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kCols) : "memory");
+  if (p.splits > 1) {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+  pdl_wait();
+  {
+    uint32_t const tile = first + (tiles - 1) * step, row = threadIdx.x & (kRows - 1);
+    I8Segment const& S = p.seg[segment(tile)];
+    uint32_t const n_row = (tile - S.tile0) * kRows + row;
+    // Slice r of the cluster finishes tokens r, r + splits, ...; the groups of 128 threads take them in turn.
+    for (uint32_t t = rank + p.splits * (threadIdx.x / kRows); t < p.m && n_row < S.n; t += p.splits * (kThreads / kRows)) {
+      uint32_t const at = smem + oParts + (t * kRows + row) * 4;
+      float v = 0.f;
+      if (p.splits == 1) v = __uint_as_float(lds32(at)) + __uint_as_float(lds32(at + kPart));
+      else
+        for (uint32_t q = 0; q < p.splits; ++q) v += peer_f32(at, q) + peer_f32(at + kPart, q);
+      store(S, uint64_t(t) * S.n + n_row, v);
+    }
+  }
+  if (p.splits > 1) {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // nobody leaves while another reads its rows
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+}
+
+}  // namespace
+
+bool mmv_i8_supported(const WeightView& w, const Q8View& x) {
+  return x.m <= kMmvI8MaxTokens && encode_fn() != nullptr && reinterpret_cast<uintptr_t>(w.codes) % 16 == 0 && reinterpret_cast<uintptr_t>(w.meta) % 16 == 0 &&
+         reinterpret_cast<uintptr_t>(x.codes) % 16 == 0 && reinterpret_cast<uintptr_t>(x.scales) % 16 == 0 &&
+         reinterpret_cast<uintptr_t>(x.sums) % 16 == 0;
+}
+
+uint32_t plan_mmv_i8(uint32_t tiles, uint32_t tiles_k) {
+  uint32_t const sms = uint32_t(sm_count());
+  uint32_t best = 1, least = (tiles + sms - 1) / sms * tiles_k;
+  for (uint32_t c = 2; c <= 4 && c <= tiles_k && tiles * c <= sms; ++c) {
+    uint32_t const units = (tiles_k + c - 1) / c;
+    if (units < least) { least = units; best = c; }
+  }
+  return best;
+}
+
+cudaError_t launch_mmv_i8(const WeightView* ws, const GemvTmaOutput* outs, uint32_t count, const Q8View& x, uint32_t splits,
+                          bool input_settled, int* status, cudaStream_t stream) {
+  if (count < 1 || count > 3 || x.m == 0 || x.m > kMmvI8MaxTokens || splits < 1 || splits > 8) return cudaErrorInvalidValue;
+  CUtensorMap codes[3], meta[3];
+  I8Params p{};
+  uint32_t tiles = 0;
+  for (uint32_t i = 0; i < count; ++i) {
+    const WeightView& w = ws[i];
+    if (w.tiles_k != ws[0].tiles_k || splits > w.tiles_k || !mmv_i8_supported(w, x) || (!outs[i].out && !outs[i].out_bf16)) return cudaErrorInvalidValue;
+    uint64_t const rgs = w.padded_n / 8;
+    uint64_t dims[3] = {128, uint64_t(w.tiles_k) * 8, rgs}, strides[2] = {128, uint64_t(w.tiles_k) * 1024};
+    uint32_t box[3] = {128, 8, kRows / 8};
+    uint64_t mdims[3] = {128, w.tiles_k, rgs}, mstrides[2] = {128, uint64_t(w.tiles_k) * 128};
+    uint32_t mbox[3] = {128, 1, kRows / 8};
+    if (!make_map(&codes[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, w.codes, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !make_map(&meta[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, w.meta, mdims, mstrides, mbox, CU_TENSOR_MAP_SWIZZLE_NONE))
+      return cudaErrorInvalidValue;
+    p.seg[i] = I8Segment{outs[i].out, outs[i].out_bf16, outs[i].residual, w.n, tiles};
+    tiles += (w.padded_n + kRows - 1) / kRows;
+  }
+  for (uint32_t i = count; i < 3; ++i) { codes[i] = codes[0]; meta[i] = meta[0]; }
+  p.status = status;
+  p.nseg = count; p.m = x.m; p.padded_k = x.padded_k; p.tiles_k = ws[0].tiles_k; p.splits = splits; p.tiles = tiles;
+  CUtensorMap xm[3];
+  {
+    uint64_t dims[3] = {128, x.m, x.padded_k / 128}, strides[2] = {x.padded_k, 128};
+    uint32_t box[3] = {128, kTok, 2};
+    uint64_t gdims[2] = {x.padded_k / 32, x.m}, gstrides[1] = {uint64_t(x.padded_k) / 8};
+    uint32_t gbox[2] = {8, kTok};
+    if (!make_map(&xm[0], CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, x.codes, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !make_map(&xm[1], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, x.scales, gdims, gstrides, gbox, CU_TENSOR_MAP_SWIZZLE_NONE) ||
+        !make_map(&xm[2], CU_TENSOR_MAP_DATA_TYPE_INT32, 2, x.sums, gdims, gstrides, gbox, CU_TENSOR_MAP_SWIZZLE_NONE))
+      return cudaErrorInvalidValue;
+  }
+  p.early = launch_overlap();
+  p.input_settled = input_settled && p.early;
+  uint32_t const octets = x.m <= 8 ? 1 : 2;
+  auto kernel = octets == 1 ? mmv_i8_kernel<1> : mmv_i8_kernel<2>;
+  cudaError_t st = allow_smem(reinterpret_cast<const void*>(kernel), int(kSmem));
+  if (st != cudaSuccess) return st;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = splits > 1 || tiles < uint32_t(sm_count()) ? tiles * splits : uint32_t(sm_count());
+  cfg.blockDim = kThreads;
+  cfg.dynamicSmemBytes = kSmem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = splits; attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = splits > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, codes[0], meta[0], codes[1], meta[1], codes[2], meta[2], xm[0], xm[1], xm[2], p);
+}
+
+}  // namespace q4k

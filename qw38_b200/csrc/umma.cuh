@@ -41,6 +41,7 @@ __device__ __forceinline__ void tmem_dealloc_all(uint32_t base) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(base) : "memory");
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
@@ -61,5 +62,20 @@ template <int N> __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_
   if constexpr (N == 8) tmem_ld8(taddr, r);
   else tmem_ld16(taddr, r);
 }
+
+// 32x32b store: lane i of the warp writes 16 consecutive columns of its TMEM lane.
+__device__ __forceinline__ void tmem_st16(uint32_t t, const uint32_t (&r)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+               ::"r"(t), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+                 "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+// One lane of a converged warp.  The compiler then knows that the operands of what it issues are uniform: behind a comparison of the
+// lane index a tcgen05.mma comes with a loop over lanes, 61 clk instead of 9 (N = 16).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{ .reg .pred q; elect.sync _|q, 0xffffffff; selp.u32 %0, 1, 0, q; }" : "=r"(p));
+  return p != 0;
+}
+__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
 
 }  // namespace q4k

@@ -1,0 +1,93 @@
+"""The kind::i8 kernel for up to sixteen tokens (nine to sixteen of a large matrix by itself, any number through KERNEL_F16): edges of its
+tiles, K slices and super-block turns, several tiles per block, activation scales far apart, and the entries that take it."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle as orc
+from qw38_b200 import _lib as L
+from qw38_b200 import synth
+from qw38_b200.q4k_q8 import DecodeMmvDesc, PrefillWeight, decode_workspace, launch_decode_mmv_ranges, pack_q8, q4k_q8_project
+from tests.helpers import assert_close_contract
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def flag():
+    return torch.zeros(1, dtype=torch.int32, device=DEV)
+
+
+def kernel_status():
+    v = ctypes.c_int(-1)
+    assert L.load().q4k_kernel_status(ctypes.byref(v)) == 0
+    return v.value
+
+
+def weight(n, k, seed):
+    hc, hs = synth.split_tiles(*synth.logical_q4k(n, k, seed=seed))
+    return PrefillWeight.from_host(hc, hs, n, k), hc, hs
+
+
+# One to four K slices of one to eleven super-blocks (a slice of one has nothing for the second group of warps), rows at both sides of a
+# tile, 149 and 297 tiles (two and three of a block, an odd and an even number of super-blocks each), both token octets.
+@pytest.mark.parametrize("m,n,k", [(1, 1, 256), (8, 128, 512), (9, 129, 768), (16, 127, 1024), (13, 5000, 1280), (10, 9600, 2816), (5, 136, 10752),
+                                   (16, 19000, 768), (8, 19008, 512), (11, 37900, 256)])
+def test_tiles_and_slices_match_the_oracle(m, n, k):
+    w, hc, hs = weight(n, k, seed=m + n)
+    x = synth.activations(m, k, seed=k, scale=0.5, outlier_frac=0.01)
+    q = pack_q8(torch.from_numpy(x).to(DEV), flag())
+    z, a, s, _ = orc.q8_quantize(x)
+    guarded = torch.full((m * n + 2,), -7.0, dtype=torch.float32, device=DEV)
+    y = q4k_q8_project(w, q, out=guarded[1:-1].view(m, n), kernel=L.KERNEL_F16)
+    assert guarded[0].item() == -7.0 and guarded[-1].item() == -7.0
+    assert_close_contract(y.cpu().numpy(), orc.project(hc, hs, n, q.padded_k, z, a, s))
+    # Against the kernel of warp-level MMAs: exact dots in both, so that only the order of the super-blocks' sums differs, fp32 sums of K / 256
+    # terms of a row's size.
+    t = q4k_q8_project(w, q, kernel=L.KERNEL_GEMV_TMA, row_groups=min(20, q.padded_k // 256))
+    assert (y - t).norm() <= 2.0 ** -24 * (k // 256 + 1) * t.norm()
+    res = torch.from_numpy(synth.activations(m, n, seed=5)).to(DEV)
+    assert torch.equal(q4k_q8_project(w, q, kernel=L.KERNEL_F16, residual=res), y + res), "residual is the last fp32 add"
+    assert kernel_status() == 0
+
+
+@pytest.mark.parametrize("m", [8, 16])
+def test_scales_far_apart(m):
+    """A token at 1e30, one with a single group there, one at 1e-30 and one that is not a number: each as it is among ordinary ones."""
+    n, k = 264, 1280
+    w, _, _ = weight(n, k, seed=4)
+    x = synth.activations(m, k, seed=11)
+    x[0] *= 1e30
+    x[1, 300:310] = 1e30
+    x[2] *= 1e-30
+    x[3, 5] = np.nan
+    q = pack_q8(torch.from_numpy(x).to(DEV), flag())
+    y, t = (q4k_q8_project(w, q, kernel=kern, row_groups=groups) for kern, groups in ((L.KERNEL_F16, 0), (L.KERNEL_GEMV_TMA, 5)))
+    assert torch.isnan(y[3]).all() and torch.isnan(t[3]).all()
+    keep = [i for i in range(m) if i != 3]
+    y, t = y[keep].double(), t[keep].double()
+    assert torch.isfinite(y).all() and ((y - t).norm(dim=1) <= 2.0 ** -21 * t.norm(dim=1)).all()
+    assert kernel_status() == 0
+
+
+@pytest.mark.parametrize("m", [9, 16])
+def test_ranges_share_a_launch(m):
+    """Three ranges whose tiles end inside a tile: fp32, bf16 and residual rows, each what its own projection gives."""
+    k, ns = 2560, (9608, 520, 136)
+    ws = [weight(n, k, seed=n)[0] for n in ns]
+    x = torch.from_numpy(synth.activations(m, k, seed=2)).to(DEV).to(torch.bfloat16)
+    res = torch.from_numpy(synth.activations(m, ns[2], seed=5)).to(DEV)
+    outs = [torch.empty((m, ns[0]), device=DEV), torch.empty((m, ns[1]), dtype=torch.bfloat16, device=DEV), torch.empty((m, ns[2]), device=DEV)]
+    descs = [DecodeMmvDesc(ws[0], x, outs[0], L.EPILOGUE_STORE_FP32), DecodeMmvDesc(ws[1], x, outs[1], L.EPILOGUE_STORE_BF16),
+             DecodeMmvDesc(ws[2], x, outs[2], L.EPILOGUE_RESIDUAL_ADD_FP32, res)]
+    f = flag()
+    launch_decode_mmv_ranges(descs, decode_workspace(m, sum(ns), k), f)
+    q = pack_q8(x, f)
+    want = [q4k_q8_project(w, q, kernel=L.KERNEL_GEMV_TMA, row_groups=10) for w in ws]
+    want[2] = want[2] + res
+    for y, t in zip(outs, want):
+        unit = 2.0 ** -8 if y.dtype == torch.bfloat16 else 2.0 ** -20
+        assert ((y.double() - t.double()).abs() <= unit * t.abs() + 2.0 ** -20 * t.abs().amax()).all()
+    assert f.item() == 0 and kernel_status() == 0

@@ -373,11 +373,19 @@ cudaError_t launch_split(DpParams p, uint32_t m, uint32_t padded_k, cudaStream_t
     p.seg[i].u0 = p.rgs * p.tiles_k;
     p.rgs += (p.seg[i].n + 7) / 8;
   }
-  // As many rounds of blocks as bound a block's row groups.  Of 148 blocks that fill half an SM each the hardware puts two on
-  // nine SMs, and these end last: 11 us after the others on 34816 x 5120 beside the next projection.  Two blocks per SM fill every
-  // half (bf16 rows, one token, us: 5120 x 5120 8.9 -> 7.2, 30000 x 7000 26.4 -> 23.7, a layer 78 -> 72).  For Q8 input there is one:
-  // a pack before or behind finds room beside it (pack and 17408 x 5120 14.5 against 15.1, four small layers 74 against 79).
-  uint32_t const slots = uint32_t(sm_count()) * (p.raw ? 2 : 1), waves = (p.rgs + slots * kMaxRowGroups - 1) / (slots * kMaxRowGroups);
+  // One token: blocks that fill half an SM each are put on 139 to 145 of the 148 SMs, two on some, and those end last.  Where the input may
+  // come from the launch before, no block of this kernel computes beside another launch's, so a block asks for more than half of an SM's shared memory
+  // and gets the SM to itself: pack and 17408 x 5120 in a replayed graph 18.0 -> 12.0 us, 5120 x 5120 8.9 -> 7.0, MLP 5120 / 17408 49.1 ->
+  // 41.9 (51.3 -> 44.4 eager), layer 4096 / 12288 44.8 -> 40.9.  With settled inputs the next launch's blocks work beside this one's end and
+  // that is worth more (eight layers 397 us, 439 with every other launch spread).
+  // bf16 rows, which every block quantises for itself: from 320 super-blocks per SM on two blocks share an SM, whose thirty warps then hide
+  // more of the copies than the second quantiser costs (us, two blocks : one): 3000 x 3000 (30) 4.0 : 3.7, 5120 x 5120 (86) 6.1 : 5.8,
+  // 10240 x 5120 (173) 8.5 : 7.9, 17408 x 5120 (294) 11.1 : 11.0, 24000 x 5120 (405) 14.1 : 14.4, 34816 x 5120 (588) 19.0 : 19.7.
+  // As many rounds of blocks as bound a block's row groups.
+  constexpr uint64_t kSharedUnits = 320;
+  uint32_t const sms = uint32_t(sm_count());
+  bool const shared = p.raw && (m > 1 || uint64_t(p.rgs) * p.tiles_k >= kSharedUnits * sms), spread = m == 1 && !p.input_settled && !shared;
+  uint32_t const slots = sms * (shared ? 2 : 1), waves = (p.rgs + slots * kMaxRowGroups - 1) / (slots * kMaxRowGroups);
   uint32_t const grid = p.rgs < slots * waves ? p.rgs : slots * waves;
   p.rgs_each = p.rgs / grid;
   p.rgs_rest = p.rgs % grid;
@@ -389,7 +397,8 @@ cudaError_t launch_split(DpParams p, uint32_t m, uint32_t padded_k, cudaStream_t
   p.stages = budget > fixed ? (budget - fixed) / stage : 0;
   if (p.stages > kMaxStages) p.stages = kMaxStages;
   if (p.stages < 1) return cudaErrorInvalidValue;
-  uint32_t const smem = fixed + p.stages * stage;
+  uint32_t smem = fixed + p.stages * stage;
+  if (spread && smem <= kHalfSm) smem = kHalfSm + 1024;
   switch (m) {
     case 1: return launch_m<1>(p, grid, smem, stream);
     case 2: return launch_m<2>(p, grid, smem, stream);

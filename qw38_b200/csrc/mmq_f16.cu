@@ -286,14 +286,15 @@ __device__ __forceinline__ void write_planes(float a, int sum, uint2 z, float ro
   }
 }
 // The largest scale of the block's token from each thread's.
-template <int Warps = 8>
 __device__ __forceinline__ float block_top(float row, float* warp_top) {
 #pragma unroll
   for (int off = 16; off; off >>= 1) row = fmaxf(row, __shfl_xor_sync(0xffffffffu, row, off));
-  if ((threadIdx.x & 31) == 0) warp_top[threadIdx.x >> 5] = row;
+  uint32_t const lane = threadIdx.x & 31;
+  if (lane == 0) warp_top[threadIdx.x >> 5] = row;
   __syncthreads();
+  row = lane < blockDim.x / 32 ? warp_top[lane] : 0.f;
 #pragma unroll
-  for (int i = 0; i < Warps; ++i) row = fmaxf(row, warp_top[i]);
+  for (int off = 16; off; off >>= 1) row = fmaxf(row, __shfl_xor_sync(0xffffffffu, row, off));
   return row;
 }
 
@@ -387,74 +388,80 @@ __global__ void __launch_bounds__(256) rows_planes_kernel(const uint16_t* rows, 
 // The same from the rows' sources in an MLP chain, K a multiple of 256, bitwise what the Q8 producers and planes_kernel give:
 // two launches less per chain and no Q8 form in memory.  MLP chain 5120 / 17408 (us, on a rested part):
 // 64 tokens 87.0 -> 85.1, 237 tokens 222.5 -> 220.4, and 4 us less of host time.
-template <int Held, int Warps>
-__global__ void __launch_bounds__(32 * Warps) swiglu_planes_kernel(const float* gate, const float* up, int* failure, uint32_t m, uint32_t m_pad,
-                                                            uint32_t tiles_k, __half* __restrict__ planes, __half* __restrict__ sums16,
-                                                            float* __restrict__ exps, float* __restrict__ tokens,
+//
+// SwiGLU: a cluster per token and a super-block per warp, so that the loads of one block run beside the stores of another and a few
+// tokens of a long row still spread over the machine.  The blocks give each other their largest scales through distributed shared
+// memory.  Bound: issue (690 instructions per warp, 0.64 per clock and scheduler), 20 us for 237 tokens of 17408.  One block of 1024
+// threads per token, and the norm with 24 columns per thread: MLP chain of 237 tokens 258.7 us, now 256.1 (under power).
+constexpr uint32_t kSwigluCluster = 8;  // most blocks per token
+__global__ void __launch_bounds__(512) swiglu_planes_kernel(const float* gate, const float* up, int* failure, uint32_t m, uint32_t m_pad,
+                                                            uint32_t tiles_k, uint32_t blocks, __half* __restrict__ planes,
+                                                            __half* __restrict__ sums16, float* __restrict__ exps, float* __restrict__ tokens,
                                                             uint32_t* __restrict__ tickets, uint32_t ticket_count) {
-  __shared__ float warp_top[Warps];
+  __shared__ float warp_top[32], block_tops[kSwigluCluster];
+  cluster_arrive();  // met below: every block of the cluster is there before one writes into another
   pdl_wait();
   pdl_launch_dependents();
   if (blockIdx.x == 0)
-    for (uint32_t i = threadIdx.x; i < ticket_count; i += 32 * Warps) tickets[i] = 0u;
-  uint32_t const warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tok = blockIdx.x;
-  uint4 held[Held];  // {codes, codes, scale, sum}
-  float row = 0.f;
-  bool valid = true;
-#pragma unroll
-  for (int i = 0; i < Held; ++i) {
-    uint32_t const kb = warp + Warps * i;
-    held[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (kb >= tiles_k || tok >= m) continue;
+    for (uint32_t i = threadIdx.x; i < ticket_count; i += blockDim.x) tickets[i] = 0u;
+  uint32_t const lane = threadIdx.x & 31, tok = blockIdx.x / blocks, rank = blockIdx.x % blocks;
+  uint32_t const kb = rank * (blockDim.x / 32) + (threadIdx.x >> 5);
+  bool const live = kb < tiles_k;
+  Packed8 z{0u, 0u, 0.f, 0, true};
+  if (live && tok < m) {
     uint64_t const at = (uint64_t(tok) * tiles_k + kb) * 256 + lane * 8;
     float4 const g0 = *reinterpret_cast<const float4*>(gate + at), g1 = *reinterpret_cast<const float4*>(gate + at + 4);
     float4 const u0 = *reinterpret_cast<const float4*>(up + at), u1 = *reinterpret_cast<const float4*>(up + at + 4);
     float const g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w}, u[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
     float x[8];
     swiglu8(g, u, x);
-    Packed8 const z = quantize8(x);
-    valid = valid && z.valid;
-    row = fmaxf(row, fabsf(z.a));
-    held[i] = make_uint4(z.w0, z.w1, __float_as_uint(z.a), uint32_t(z.sum));
+    z = quantize8(x);
+    if (!z.valid) atomicExch(failure, 1);
   }
-  if (!valid) atomicExch(failure, 1);
-  row = block_top<Warps>(row, warp_top);
-#pragma unroll
-  for (int i = 0; i < Held; ++i) {
-    uint32_t const kb = warp + Warps * i;
-    if (kb >= tiles_k) break;
-    write_planes(__uint_as_float(held[i].z), int(held[i].w), make_uint2(held[i].x, held[i].y), row, tok, kb, m_pad, tiles_k * 256, planes, sums16,
-                 exps, tokens);
-  }
+  float row = block_top(fabsf(z.a), warp_top);
+  cluster_wait();
+  if (threadIdx.x < blocks)
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(map_to(smem_u32(block_tops + rank), threadIdx.x)), "f"(row) : "memory");
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  for (uint32_t i = 0; i < blocks; ++i) row = fmaxf(row, block_tops[i]);
+  if (live) write_planes(z.a, z.sum, make_uint2(z.w0, z.w1), row, tok, kb, m_pad, tiles_k * 256, planes, sums16, exps, tokens);
 }
 
-// Held: columns per thread in the norm (rms.cuh), Blocks: super-blocks per warp.
-template <int Held, int Blocks>
-__global__ void __launch_bounds__(256) rms_planes_kernel(const float* residual, const uint16_t* gamma, float eps, int* failure, uint32_t m,
-                                                         uint32_t m_pad, uint32_t tiles_k, __half* __restrict__ planes,
-                                                         __half* __restrict__ sums16, float* __restrict__ exps, float* __restrict__ tokens,
-                                                         uint32_t* __restrict__ tickets, uint32_t ticket_count) {
-  extern __shared__ __align__(16) uint16_t rounded[];
-  __shared__ float warp_top[8];
+// Held: eight columns per thread from the norm to the planes (rms.cuh); wider rows go through shared memory, sixteen super-blocks per warp.
+template <bool Held>
+__global__ void __launch_bounds__(Held ? kRmsHeldColumns / 8 : kRmsThreads)
+    rms_planes_kernel(const float* residual, const uint16_t* gamma, float eps, bool vec, int* failure, uint32_t m, uint32_t m_pad,
+                      uint32_t tiles_k, __half* __restrict__ planes, __half* __restrict__ sums16, float* __restrict__ exps,
+                      float* __restrict__ tokens, uint32_t* __restrict__ tickets, uint32_t ticket_count) {
+  extern __shared__ __align__(16) uint8_t staged[];
+  __shared__ float warp_top[32];
   pdl_wait();
   pdl_launch_dependents();
   if (blockIdx.x == 0)
-    for (uint32_t i = threadIdx.x; i < ticket_count; i += 256) tickets[i] = 0u;
-  uint32_t const warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tok = blockIdx.x, hidden = tiles_k * 256;
-  if (tok < m) rms_row<Held>(residual + uint64_t(tok) * hidden, gamma, eps, hidden, rounded);
-  uint4 held[Blocks];
+    for (uint32_t i = threadIdx.x; i < ticket_count; i += blockDim.x) tickets[i] = 0u;
+  constexpr int kBlocks = Held ? 1 : 16;
+  uint32_t const warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x / 32, tok = blockIdx.x, hidden = tiles_k * 256;
+  const float* const mine = residual + uint64_t(tok) * hidden;
+  uint16_t* const rounded = reinterpret_cast<uint16_t*>(staged);
+  float x[8];
+  if (tok < m) {
+    if constexpr (Held) rms_row_held(mine, gamma, eps, hidden, vec, reinterpret_cast<float*>(staged), x);
+    else rms_row(mine, gamma, eps, hidden, rounded);
+  }
+  uint4 held[kBlocks];
   float row = 0.f;
   bool valid = true;
 #pragma unroll
-  for (int i = 0; i < Blocks; ++i) {
-    uint32_t const kb = warp + 8 * i;
+  for (int i = 0; i < kBlocks; ++i) {
+    uint32_t const kb = warp + warps * i;
     held[i] = make_uint4(0u, 0u, 0u, 0u);
     if (kb >= tiles_k || tok >= m) continue;
-    uint4 const v = *reinterpret_cast<const uint4*>(rounded + kb * 256 + lane * 8);
-    uint32_t const w[4] = {v.x, v.y, v.z, v.w};
-    float x[8];
+    if constexpr (!Held) {
+      uint4 const v = *reinterpret_cast<const uint4*>(rounded + kb * 256 + lane * 8);
+      uint32_t const w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-    for (int c = 0; c < 4; ++c) { x[2 * c] = __uint_as_float(w[c] << 16); x[2 * c + 1] = __uint_as_float(w[c] & 0xffff0000u); }
+      for (int c = 0; c < 4; ++c) { x[2 * c] = __uint_as_float(w[c] << 16); x[2 * c + 1] = __uint_as_float(w[c] & 0xffff0000u); }
+    }
     Packed8 const z = quantize8(x);
     valid = valid && z.valid;
     row = fmaxf(row, fabsf(z.a));
@@ -463,8 +470,8 @@ __global__ void __launch_bounds__(256) rms_planes_kernel(const float* residual, 
   if (!valid) atomicExch(failure, 1);
   row = block_top(row, warp_top);
 #pragma unroll
-  for (int i = 0; i < Blocks; ++i) {
-    uint32_t const kb = warp + 8 * i;
+  for (int i = 0; i < kBlocks; ++i) {
+    uint32_t const kb = warp + warps * i;
     if (kb >= tiles_k) break;
     write_planes(__uint_as_float(held[i].z), int(held[i].w), make_uint2(held[i].x, held[i].y), row, tok, kb, m_pad, hidden, planes, sums16, exps,
                  tokens);
@@ -933,17 +940,29 @@ cudaError_t launch_f16(const WeightView& w, const WeightView* second, const Q8Vi
   cudaError_t st;
   if (w.tiles_k > 128 && raw) return cudaErrorInvalidValue;  // sixteen super-blocks per warp
   if (raw && raw->residual) {
-    auto kernel = w.tiles_k <= 8 ? rms_planes_kernel<8, 1> : (w.tiles_k <= 24 ? rms_planes_kernel<24, 3> : rms_planes_kernel<0, 16>);
-    uint32_t const smem = pk * 2;
+    bool const held = pk <= kRmsHeldColumns;
+    auto kernel = held ? rms_planes_kernel<true> : rms_planes_kernel<false>;
+    uint32_t const smem = pk * (held ? 4 : 2);
     if (smem > 48 * 1024 && (st = allow_smem(reinterpret_cast<const void*>(kernel), int(smem))) != cudaSuccess) return st;
-    st = launch_kernel(kernel, m_pad, 256, smem, stream, true, raw->residual, raw->gamma, raw->eps, raw->failure, x.m, m_pad, w.tiles_k, planes,
-                       sums, exps, tokens, tickets, ticket_count);
+    st = launch_kernel(kernel, m_pad, held ? rms_held_threads(pk) : kRmsThreads, smem, stream, true, raw->residual, raw->gamma, raw->eps,
+                       rms_vector_rows(raw->residual, raw->gamma), raw->failure, x.m, m_pad, w.tiles_k, planes, sums, exps, tokens, tickets,
+                       ticket_count);
   } else if (raw && raw->gate) {
-    // Wide rows get more warps, so that few tokens still fill the machine: an MLP chain of 237 tokens with K = 17408
-    // 266 us with eight warps, 259 with 32.
-    auto kernel = w.tiles_k <= 24 ? swiglu_planes_kernel<3, 8> : (w.tiles_k <= 96 ? swiglu_planes_kernel<3, 32> : swiglu_planes_kernel<4, 32>);
-    st = launch_kernel(kernel, m_pad, w.tiles_k <= 24 ? 256 : 1024, 0, stream, true, raw->gate, raw->up, raw->failure, x.m, m_pad, w.tiles_k, planes, sums, exps, tokens,
-                       tickets, ticket_count);
+    // A super-block per warp (at most 128: sixteen warps).
+    uint32_t const blocks = w.tiles_k < 8 * kSwigluCluster ? (w.tiles_k + 7) / 8 : kSwigluCluster;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = m_pad * blocks;
+    cfg.blockDim = (w.tiles_k + blocks - 1) / blocks * 32;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = blocks; attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    st = cudaLaunchKernelEx(&cfg, swiglu_planes_kernel, raw->gate, raw->up, raw->failure, x.m, m_pad, w.tiles_k, blocks, planes, sums, exps,
+                            tokens, tickets, ticket_count);
   } else if (raw) {
     bool const vec = raw->k % 8 == 0 && reinterpret_cast<uintptr_t>(raw->x) % 16 == 0;
     // Few registers keep more rows in flight, but a row has to fit: three super-blocks per warp up to K = 6144, nine up to

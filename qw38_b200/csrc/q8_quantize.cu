@@ -110,23 +110,32 @@ __global__ void __launch_bounds__(kThreads) swiglu_pack_kernel(const float* gate
   }
 }
 
-// RMS norm, then the Q8 pack of the rounded row.  One block per token; dynamic shared memory = hidden * 2 bytes.
-template <int Held>
-__global__ void __launch_bounds__(kThreads) hidden_rms_q8_kernel(const float* residual, const uint16_t* gamma,
-                                                                  float eps, uint32_t hidden,
-                                                                  int8_t* codes, float* scales,
-                                                                  int32_t* sums, int* failure) {
-  extern __shared__ __align__(16) uint16_t rounded[];
+// RMS norm, then the Q8 pack of the rounded row.  One block per token; dynamic shared memory = the scaled row as floats (Held), or the
+// rounded one.
+template <bool Held>
+__global__ void __launch_bounds__(Held ? kRmsHeldColumns / 8 : kThreads) hidden_rms_q8_kernel(const float* residual, const uint16_t* gamma,
+                                                                                             float eps, uint32_t hidden, bool vec,
+                                                                                             int8_t* codes, float* scales,
+                                                                                             int32_t* sums, int* failure) {
+  extern __shared__ __align__(16) uint8_t row[];
   pdl_wait();
   pdl_launch_dependents();
-  rms_row<Held>(residual + uint64_t(blockIdx.x) * hidden, gamma, eps, hidden, rounded);
+  const float* const x = residual + uint64_t(blockIdx.x) * hidden;
   uint32_t const lane = threadIdx.x & 31, sub = lane & 3, grp = lane >> 2;
-  for (uint32_t chunk = threadIdx.x / 32; chunk < hidden / 256; chunk += kThreads / 32) {
-    uint32_t const col0 = chunk * 256 + grp * 32 + sub * 8;
-    float v[8];
+  uint64_t const group0 = uint64_t(blockIdx.x) * (hidden / 32) + grp;
+  float v[8];
+  if constexpr (Held) {
+    rms_row_held(x, gamma, eps, hidden, vec, reinterpret_cast<float*>(row), v);
+    if (threadIdx.x * 8 < hidden) pack8(v, codes, scales, sums, group0 + threadIdx.x / 32 * 8, sub, failure);
+  } else {
+    uint16_t* const rounded = reinterpret_cast<uint16_t*>(row);
+    rms_row(x, gamma, eps, hidden, rounded);
+    for (uint32_t chunk = threadIdx.x / 32; chunk < hidden / 256; chunk += kThreads / 32) {
+      uint32_t const col0 = chunk * 256 + grp * 32 + sub * 8;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = bf16_bits_to_f32(rounded[col0 + i]);
-    pack8(v, codes, scales, sums, uint64_t(blockIdx.x) * (hidden / 32) + chunk * 8 + grp, sub, failure);
+      for (int i = 0; i < 8; ++i) v[i] = bf16_bits_to_f32(rounded[col0 + i]);
+      pack8(v, codes, scales, sums, group0 + chunk * 8, sub, failure);
+    }
   }
 }
 
@@ -180,15 +189,15 @@ cudaError_t launch_swiglu_pack_q8(const float* gate, const float* up, Q8Out out,
 
 cudaError_t launch_hidden_rms_q8(const float* residual, const uint16_t* gamma, float eps,
                                  uint32_t hidden, Q8Out out, int* failure, cudaStream_t stream) {
-  size_t const smem = size_t(hidden) * 2;
-  // 48 registers hold a thread's share of rows up to 6144 columns; half of that leaves room for twice the rows in flight.
-  auto kernel = hidden <= 8 * kThreads ? hidden_rms_q8_kernel<8> : (hidden <= 24 * kThreads ? hidden_rms_q8_kernel<24> : hidden_rms_q8_kernel<0>);
+  bool const held = hidden <= kRmsHeldColumns;
+  size_t const smem = size_t(hidden) * (held ? 4 : 2);
+  auto kernel = held ? hidden_rms_q8_kernel<true> : hidden_rms_q8_kernel<false>;
   if (smem > 48 * 1024) {
     cudaError_t st = allow_smem(reinterpret_cast<const void*>(kernel), int(smem));
     if (st != cudaSuccess) return st;
   }
-  return launch_kernel(kernel, out.m, kThreads, smem, stream, true, residual, gamma, eps, hidden, out.codes, out.scales, out.sums,
-                       failure);
+  return launch_kernel(kernel, out.m, held ? rms_held_threads(hidden) : kThreads, smem, stream, true, residual, gamma, eps, hidden,
+                       rms_vector_rows(residual, gamma), out.codes, out.scales, out.sums, failure);
 }
 
 cudaError_t launch_export_q8_1(const int8_t* codes, const float* scales, const int32_t* sums,

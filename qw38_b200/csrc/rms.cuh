@@ -21,62 +21,102 @@ __device__ __forceinline__ float block_reduce(float v, float* scratch, bool is_m
   return r;
 }
 
-// (1 + gamma) * x / rms(x) rounded to bf16 into shared memory; hidden % 256 == 0.  Thread t owns columns t, t + 256, ... and sums
-// them in that order.
+// (1 + gamma) * x / rms(x) rounded to bf16; hidden % 256 == 0.  The squares of columns t, t + 256, ... are summed in that order for
+// t = 0 .. 255, then over t: both forms give the same bits.
 //
-// Bound: latency (a decode step has a handful of rows).  With Held > 0 (hidden <= 256 * Held) a thread requests its whole
-// share of the row and of the gain at once and keeps it in registers for the three passes; the loop form, which serves
-// wider rows, waits for memory in every iteration of every pass: 15 us at 5120 columns against 4 us.
-template <int Held>
+// Bound: latency (a decode step has a handful of rows).  Up to kRmsHeldColumns a thread holds eight consecutive columns from the load to
+// the pack (a block of hidden / 8 threads, 256 at least): one load of row and gain, two block reductions, and only the scaled row goes
+// through shared memory, where the first 256 threads find the columns whose squares they sum.  Against 256 threads with 24 columns each
+// (three passes over registers and the pack out of shared memory in three rounds), MLP chains 5120 / 17408,
+// us: one token 45.0 -> 42.0, four 48.8 -> 46.1, thirteen 58.3 -> 56.5.
+constexpr uint32_t kRmsHeldColumns = 8192;
+__host__ __device__ constexpr uint32_t rms_held_threads(uint32_t hidden) { return hidden / 8 > kRmsThreads ? hidden / 8 : kRmsThreads; }
+
+inline bool rms_vector_rows(const float* residual, const uint16_t* gamma) {
+  return (reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(gamma)) % 16 == 0;  // rows are multiples of 1024 bytes
+}
+
+// Thread t's columns 8t .. 8t + 7 as bf16 values in v (zeros beyond the row); scaled: shared memory, hidden floats.  vec: row and gain are
+// 16-byte aligned.
+__device__ __forceinline__ void rms_row_held(const float* x, const uint16_t* gamma, float eps, uint32_t hidden, bool vec, float* scaled,
+                                             float (&v)[8]) {
+  __shared__ uint32_t tops[32];
+  __shared__ float4 sums[2];
+  uint32_t const t = threadIdx.x, lane = t & 31, warp = t >> 5, col = t * 8;
+  bool const live = col < hidden;  // whole warps
+  uint32_t gain[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = 0.f;
+  if (live) {
+    if (vec) {
+      float4 const lo = *reinterpret_cast<const float4*>(x + col), hi = *reinterpret_cast<const float4*>(x + col + 4);
+      uint4 const g = *reinterpret_cast<const uint4*>(gamma + col);
+      v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w; v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
+      gain[0] = g.x; gain[1] = g.y; gain[2] = g.z; gain[3] = g.w;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = x[col + i];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) gain[i] = uint32_t(gamma[col + 2 * i]) | uint32_t(gamma[col + 2 * i + 1]) << 16;
+    }
+  }
+  float top = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) top = fmaxf(top, fabsf(v[i]));  // never a NaN, so its bits compare as it does
+  uint32_t const warp_top = __reduce_max_sync(0xffffffffu, __float_as_uint(top));
+  if (lane == 0) tops[warp] = warp_top;
+  __syncthreads();
+  float const scale = __uint_as_float(__reduce_max_sync(0xffffffffu, lane < blockDim.x / 32 ? tops[lane] : 0u));
+  float const safe = scale == 0.f ? 1.f : scale;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = v[i] / safe;
+  if (live) {
+    *reinterpret_cast<float4*>(scaled + col) = make_float4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<float4*>(scaled + col + 4) = make_float4(v[4], v[5], v[6], v[7]);
+  }
+  __syncthreads();
+  if (t < kRmsThreads) {
+    float sumsq = 0.f;
+#pragma unroll 4
+    for (uint32_t i = t; i < hidden; i += kRmsThreads) sumsq += scaled[i] * scaled[i];
+#pragma unroll
+    for (int off = 16; off; off >>= 1) sumsq += __shfl_xor_sync(0xffffffffu, sumsq, off);
+    if (lane == 0) reinterpret_cast<float*>(sums)[warp] = sumsq;
+  }
+  float const se = sqrtf(eps) / safe;
+  __syncthreads();
+  float4 const s0 = sums[0], s1 = sums[1];
+  float const sumsq = s0.x + s0.y + s0.z + s0.w + s1.x + s1.y + s1.z + s1.w;
+  float const inv = 1.0f / sqrtf(sumsq / float(hidden) + se * se);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    float const g = __uint_as_float(i & 1 ? gain[i / 2] & 0xffff0000u : gain[i / 2] << 16);
+    v[i] = bf16_bits_to_f32(f32_to_bf16_rne((1.0f + g) * (v[i] * inv)));
+  }
+}
+
+// Wider rows, into shared memory: 256 threads in passes over memory.
 __device__ __forceinline__ void rms_row(const float* x, const uint16_t* gamma, float eps, uint32_t hidden, uint16_t* rounded) {
   __shared__ float scratch[kRmsThreads / 32];
-  float held[Held > 0 ? Held : 1], gain[Held > 0 ? Held : 1];
   float scale = 0.f;
-  if constexpr (Held > 0) {
-#pragma unroll
-    for (int j = 0; j < Held; ++j) {
-      uint32_t const i = threadIdx.x + j * kRmsThreads;
-      held[j] = i < hidden ? x[i] : 0.f;
-      gain[j] = i < hidden ? bf16_bits_to_f32(gamma[i]) : 0.f;
-    }
-#pragma unroll
-    for (int j = 0; j < Held; ++j) scale = fmaxf(scale, fabsf(held[j]));
-  } else {
 #pragma unroll 8
-    for (uint32_t i = threadIdx.x; i < hidden; i += kRmsThreads) scale = fmaxf(scale, fabsf(x[i]));
-  }
+  for (uint32_t i = threadIdx.x; i < hidden; i += kRmsThreads) scale = fmaxf(scale, fabsf(x[i]));
   scale = block_reduce(scale, scratch, true);
   float const safe = scale == 0.f ? 1.f : scale;
   float sumsq = 0.f;
-  if constexpr (Held > 0) {
-#pragma unroll
-    for (int j = 0; j < Held; ++j) {
-      held[j] = held[j] / safe;
-      if (threadIdx.x + j * kRmsThreads < hidden) sumsq += held[j] * held[j];
-    }
-  } else {
 #pragma unroll 8
-    for (uint32_t i = threadIdx.x; i < hidden; i += kRmsThreads) {
-      float s = x[i] / safe;
-      sumsq += s * s;
-    }
+  for (uint32_t i = threadIdx.x; i < hidden; i += kRmsThreads) {
+    float s = x[i] / safe;
+    sumsq += s * s;
   }
   sumsq = block_reduce(sumsq, scratch, false);
   float const se = sqrtf(eps) / safe;
   float const inv = 1.0f / sqrtf(sumsq / float(hidden) + se * se);
-  if constexpr (Held > 0) {
-#pragma unroll
-    for (int j = 0; j < Held; ++j) {
-      uint32_t const i = threadIdx.x + j * kRmsThreads;
-      if (i < hidden) rounded[i] = f32_to_bf16_rne((1.0f + gain[j]) * (held[j] * inv));
-    }
-  } else {
 #pragma unroll 4
-    for (uint32_t i = threadIdx.x; i < hidden; i += kRmsThreads) {
-      float g = bf16_bits_to_f32(gamma[i]);
-      float v = (1.0f + g) * ((x[i] / safe) * inv);
-      rounded[i] = f32_to_bf16_rne(v);
-    }
+  for (uint32_t i = threadIdx.x; i < hidden; i += kRmsThreads) {
+    float g = bf16_bits_to_f32(gamma[i]);
+    float v = (1.0f + g) * ((x[i] / safe) * inv);
+    rounded[i] = f32_to_bf16_rne(v);
   }
   __syncthreads();
 }

@@ -224,7 +224,7 @@ struct ChainedLaunches {
 // cudaFuncSetAttribute(MaxDynamicSharedMemorySize), skipped where this thread has already asked for as much on the current
 // device (the runtime call costs a quarter of a microsecond on every launch).  The limit of a kernel is only ever raised,
 // so that what one thread remembers stays true whatever the others ask for.
-inline cudaError_t allow_smem(const void* kernel, int bytes) {
+inline cudaError_t allow_smem(const void* kernel, int bytes, bool whole = false) {
   struct Seen { const void* kernel; int device, bytes; };
   static thread_local Seen seen[64];
   static std::mutex mutex;
@@ -238,6 +238,7 @@ inline cudaError_t allow_smem(const void* kernel, int bytes) {
   int& limit = limits[{kernel, device}];
   if (limit < bytes) {
     if ((st = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)) != cudaSuccess) return st;
+    if (whole && (st = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared)) != cudaSuccess) return st;
     limit = bytes;
   }
   slot = Seen{kernel, device, limit};

@@ -24,7 +24,7 @@
 //
 // One token, us, matrices that do not fit L2 in a replayed graph, overlapped launches with settled inputs (the TMA tile kernel in
 // brackets): 5120 x 5120 4.9 (5.4), 7168 x 5120 5.8 (6.7), 5120 x 17408 10.4 (13.6), 34816 x 5120 16.7 = 6.0 TB/s (20.3); eight
-// layers of all four with their packs 350 to 357 (426).  Slower, when they were tried: sixteen-row steps whose lanes share the
+// layers of all four with their packs 313 (426).  Slower, when they were tried: sixteen-row steps whose lanes share the
 // activation loads (34816 x 5120 20.1 against 17.5), eleven to seventeen warps, thirty warps in one block per SM.
 #include "common.cuh"
 #include "launch.h"
@@ -152,11 +152,15 @@ __global__ void __launch_bounds__(kThreads, M <= 2 ? 2 : 1) gemv_dp4a_kernel(con
       pu += count;
       ps = ps + 1 == p.stages ? 0 : ps + 1;
     };
+    auto fill_ring = [&] {
+      if (lane == 0 && p.wide)
+        for (uint32_t i = 0; i < p.stages && pu < u1; ++i) fetch();
+    };
     if (lane == 0) {
       if (p.wide) {
         for (uint32_t i = 0; i < p.stages; ++i) mbar_init(bars + i * 8, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        if (!p.early) {  // the first stages come out of L2 after the wait (two: more get in the way of the kernel before)
+        if (!p.early)  // the first stages come out of L2 after the wait (two: more get in the way of the kernel before)
           for (uint32_t i = 0, u = u0; i < 2 && u < u1; ++i) {
             uint32_t const count = stage_units(p, u, u1);
             DpSegment const& s = segment_of(p, u);
@@ -164,20 +168,22 @@ __global__ void __launch_bounds__(kThreads, M <= 2 ? 2 : 1) gemv_dp4a_kernel(con
             prefetch_l2(s.meta + uint64_t(u - s.u0) * 128, count * 128);
             u += count;
           }
-          pdl_wait();
-        }
-        for (uint32_t i = 0; i < p.stages && pu < u1; ++i) fetch();
       }
       cuts[warp] = c0;
       firsts[warp] = c0 / tiles_k;
       if (warp == 0) { cuts[kWarps] = units; *abort_flag = 0; }
     }
+    // What an SM asks for comes in order, and behind a ring of weights the activations took 3 us.  So they are asked for first, unless they
+    // are waited for while the weights may come.  us, graphs: pack and 5120 x 5120 8.1 -> 7.2, and 17408 x 5120 13.6 -> 12.8; bf16 rows by 5120 x
+    // 5120 7.0 -> 6.3, by 17408 x 5120 13.2 -> 12.4; eight layers 335 -> 326.
+    bool const weights_first = p.early && !p.input_settled;
+    if (weights_first) fill_ring();
     if (!p.input_settled || Dump) pdl_wait();
 
     // ---- activations ----
     if constexpr (Raw) {
-      for (uint32_t i0 = warp; i0 < M * tiles_k; i0 += kWarps * 2) {  // two super-blocks requested at a time
-        uint4 v[2];
+      uint4 v[2];  // two super-blocks requested at a time
+      auto load = [&](uint32_t i0) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           uint32_t const i = i0 + h * kWarps, col = (i % tiles_k) * 256 + lane * 8;
@@ -192,6 +198,11 @@ __global__ void __launch_bounds__(kThreads, M <= 2 ? 2 : 1) gemv_dp4a_kernel(con
             v[h] = make_uint4(e[0] | e[1] << 16, e[2] | e[3] << 16, e[4] | e[5] << 16, e[6] | e[7] << 16);
           }
         }
+      };
+      load(warp);
+      if (!weights_first) fill_ring();
+      for (uint32_t i0 = warp; i0 < M * tiles_k; i0 += kWarps * 2) {
+        if (i0 != warp) load(i0);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           uint32_t const i = i0 + h * kWarps;
@@ -213,8 +224,10 @@ __global__ void __launch_bounds__(kThreads, M <= 2 ? 2 : 1) gemv_dp4a_kernel(con
       // a 16-byte source chunk holds half a K32 group (columns 16c..16c+15)
       bool const z16 = (reinterpret_cast<uintptr_t>(p.codes) & 15) == 0;
       uint32_t const chunks = M * tiles_k * 16;
-      for (uint32_t c0 = threadIdx.x; c0 < chunks; c0 += kConsumers * 4) {  // four chunks requested at a time
-        uint4 z[4];
+      uint4 z[4];  // four chunks and two groups' scales and sums requested at a time
+      float a[2];
+      int sum[2];
+      auto load_codes = [&](uint32_t c0) {
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
           uint32_t const c = c0 + h * kConsumers;
@@ -225,6 +238,21 @@ __global__ void __launch_bounds__(kThreads, M <= 2 ? 2 : 1) gemv_dp4a_kernel(con
             z[h] = make_uint4(s32[0], s32[1], s32[2], s32[3]);
           }
         }
+      };
+      auto load_scales = [&](uint32_t i0) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t const i = i0 + h * kConsumers;
+          if (i >= M * G) break;
+          a[h] = p.scales[i];
+          sum[h] = p.sums[i];
+        }
+      };
+      load_codes(threadIdx.x);
+      load_scales(threadIdx.x);
+      if (!weights_first) fill_ring();
+      for (uint32_t c0 = threadIdx.x; c0 < chunks; c0 += kConsumers * 4) {
+        if (c0 != threadIdx.x) load_codes(c0);
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
           uint32_t const c = c0 + h * kConsumers;
@@ -234,12 +262,13 @@ __global__ void __launch_bounds__(kThreads, M <= 2 ? 2 : 1) gemv_dp4a_kernel(con
         }
       }
       for (uint32_t i0 = threadIdx.x; i0 < M * G; i0 += kConsumers * 2) {
-        uint32_t const i1 = i0 + kConsumers;
-        bool const two = i1 < M * G;
-        float const a0 = p.scales[i0], a1 = two ? p.scales[i1] : 0.f;
-        int const s0 = p.sums[i0], s1 = two ? p.sums[i1] : 0;
-        sts64f(s_aw + i0 * 8, a0, a0 * float(s0));
-        if (two) sts64f(s_aw + i1 * 8, a1, a1 * float(s1));
+        if (i0 != threadIdx.x) load_scales(i0);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t const i = i0 + h * kConsumers;
+          if (i >= M * G) break;
+          sts64f(s_aw + i * 8, a[h], a[h] * float(sum[h]));
+        }
       }
     }
     asm volatile("bar.sync 1, %0;" ::"n"(kConsumers) : "memory");

@@ -78,6 +78,10 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {  // multiples of 16
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
+// The same for the 128-byte line at p: rows, residuals and gains that are read once, right after the wait, and often lie in memory.
+// us, before and after: bf16 rows of one token by 5120 x 5120 with a residual 6.30 -> 5.85 (3000 x 3000 4.16 -> 3.84), fp32 pack and 17408 x 5120
+// 13.4 -> 13.0; a stream whose rows are in L2 anyway 310 -> 311.
+__device__ __forceinline__ void prefetch_line(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Row-sharded decode: tell every rank how many more projections of this rank are complete.  Called by

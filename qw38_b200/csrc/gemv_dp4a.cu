@@ -355,7 +355,15 @@ __global__ void __launch_bounds__(kThreads, M <= 2 ? 2 : 1) gemv_dp4a_kernel(con
       } while (st != ps);
     }
   } else {
-    // Control warp: once everything before this launch is complete, the next launch may start beside it.
+    // Control warp: once everything before this launch is complete, the next launch may start beside it.  Meanwhile it asks L2 for the
+    // residual of the block's rows and for its share of the bf16 rows.
+    for (uint32_t i = lane; i < rg_count * M; i += 32) {
+      uint32_t const rg = i / M;
+      DpSegment const& s = segment_of(p, (rg_first + rg) * tiles_k);
+      if (s.residual) prefetch_line(s.residual + uint64_t(i % M) * s.n + (rg_first + rg - s.rg0) * 8);
+    }
+    if constexpr (Raw)
+      for (uint64_t i = (uint64_t(blockIdx.x) + uint64_t(lane) * gridDim.x) * 64; i < uint64_t(M) * p.k; i += uint64_t(gridDim.x) * 32 * 64) prefetch_line(p.raw + i);
     pdl_wait();
     pdl_launch_dependents();
   }

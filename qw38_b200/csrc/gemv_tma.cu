@@ -244,6 +244,15 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
     // (r = lane/4, q = lane%4) owns rows r, r+8 and tokens 2q, 2q+1 -- the MMA accumulator layout.
     uint32_t const nt = (warp - kFirstReducer) % NT, turn = Reducers == 1 ? 0u : (warp - kFirstReducer) / NT;
     uint32_t const r = lane >> 2, q = lane & 3;
+    if (slice == 0 && warp == kFirstReducer && !p.pair && p.done == nullptr)  // the residual's lines
+      for (uint32_t i = lane; i < ntiles * p.m; i += 32) {
+        uint32_t const tok = i / ntiles;
+        uint32_t sg = 0, local = t0 + i % ntiles;
+        if (p.nseg != 0) locate_tile(p, local, sg, local);
+        const float* const rows = p.nseg != 0 ? p.seg[sg].residual : p.residual;
+        uint32_t const n = p.nseg != 0 ? p.seg[sg].n : p.n;
+        if (rows && local * 16 < n) prefetch_line(rows + size_t(tok) * n + local * 16);
+      }
     pdl_wait();
     pdl_launch_dependents();  // after the wait: the next launch never runs beside anything older than this one
     if (p.done != nullptr && blockIdx.x == 0 && warp == kFirstReducer && lane == 0) announce_deliveries(p.unsignalled, p.peer_flag, p.ndst, p.rank);
@@ -415,6 +424,11 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
   } else if (warp - kFirstConsumer < nact) {
     uint32_t const w = warp - kFirstConsumer, sb = sb0 + w;
     uint32_t const r = lane >> 2, q = lane & 3;
+    if constexpr (Raw) {  // four lines per token
+      uint32_t const col = sb * 256 + (lane & 3) * 64;
+      for (uint32_t tok = lane >> 2; tok < p.m; tok += 8)
+        if (col < p.xk) prefetch_line(p.xraw + size_t(tok) * p.xk + col);
+    }
     if (!p.input_settled || p.partials != nullptr) pdl_wait();  // activations; the reducer waits before anything is stored
     // ---- K-stationary operands ----
     uint32_t const tab = s_tab + w * tab_bytes;
@@ -675,6 +689,19 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
       if (old == p.split_k - 1) p.tickets[range] = 0;
     }
     __syncthreads();
+    // In slice order, four slices requested at a time: one after another each is a round trip to L2 (down projection of an MLP: 2 us).
+    auto slice_sum = [&](size_t o, size_t plane) {
+      float v = 0.f;
+      for (uint32_t sl = 0; sl < p.split_k; sl += 4) {
+        float x[4];
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) x[j] = sl + j < p.split_k ? __ldcg(p.slices + (sl + j) * plane + o) : 0.f;
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j)
+          if (sl + j < p.split_k) v = sl + j ? v + x[j] : x[j];
+      }
+      return v;
+    };
     if (*last_flag && p.nseg != 0) {
       __threadfence();
       // One thread per (token, row of a tile); in pair mode per row of a gate tile, which also reads the up tile.
@@ -688,17 +715,15 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
         uint32_t const row = local * 16 + r16;
         if (row >= S.n) continue;
         size_t const o = size_t(tok) * p.n_total + S.row_base + row;
-        float v = __ldcg(p.slices + o);
-        for (uint32_t sl = 1; sl < p.split_k; ++sl) v += __ldcg(p.slices + sl * plane + o);
         size_t const oo = size_t(tok) * S.n + row;
         if (p.pair) {
-          size_t const o2 = size_t(tok) * p.n_total + p.seg[1].row_base + row;
-          float u = __ldcg(p.slices + o2);
-          for (uint32_t sl = 1; sl < p.split_k; ++sl) u += __ldcg(p.slices + sl * plane + o2);
+          float const v = slice_sum(o, plane), u = slice_sum(size_t(tok) * p.n_total + p.seg[1].row_base + row, plane);
           p.seg[0].out_bf16[oo] = f32_to_bf16_rne(v * sigmoid_fp32(v) * u);
           continue;
         }
-        if (S.residual) v += S.residual[oo];
+        float const rest = S.residual ? S.residual[oo] : 0.f;
+        float v = slice_sum(o, plane);
+        if (S.residual) v += rest;
         if (S.out_bf16) S.out_bf16[oo] = f32_to_bf16_rne(v);
         else S.out[oo] = v;
       }
@@ -709,10 +734,10 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tm_codes, const __grid_const
       for (uint32_t i = threadIdx.x; i < rows * p.m; i += blockDim.x) {
         uint32_t const tok = i / rows, row = row0 + i % rows;
         size_t const o = size_t(tok) * p.n + row;
-        float v = __ldcg(p.slices + o);
-        for (uint32_t sl = 1; sl < p.split_k; ++sl) v += __ldcg(p.slices + size_t(sl) * p.m * p.n + o);
         size_t const oo = size_t(tok) * p.out_stride + p.out_row0 + row;
-        if (p.residual) v += p.residual[oo];
+        float const rest = p.residual ? p.residual[oo] : 0.f;
+        float v = slice_sum(o, size_t(p.m) * p.n);
+        if (p.residual) v += rest;
         p.out[0][oo] = v;
 #pragma unroll
         for (int g = 1; g < 8; ++g)

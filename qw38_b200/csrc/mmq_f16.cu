@@ -435,6 +435,7 @@ __global__ void __launch_bounds__(Held ? kRmsHeldColumns / 8 : kRmsThreads)
                       float* __restrict__ tokens, uint32_t* __restrict__ tickets, uint32_t ticket_count) {
   extern __shared__ __align__(16) uint8_t staged[];
   __shared__ float warp_top[32];
+  if (blockIdx.x < m) rms_prefetch(residual + uint64_t(blockIdx.x) * tiles_k * 256, gamma, tiles_k * 256);
   pdl_wait();
   pdl_launch_dependents();
   if (blockIdx.x == 0)

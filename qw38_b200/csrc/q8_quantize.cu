@@ -66,13 +66,17 @@ template <typename T, bool Vec>
 __global__ void __launch_bounds__(kThreads, kBlocksPerSm) pack_kernel(const T* in, int8_t* __restrict__ codes,
                                                                        float* __restrict__ scales, int32_t* __restrict__ sums, uint32_t m,
                                                                        uint32_t k, uint32_t pk, int* failure) {
-  pdl_wait();               // the input may come from the kernel before this one
-  pdl_launch_dependents();  // the projection that follows may start prefetching its weights (after the wait: the
-                            // next launch never runs beside anything older than this one)
   uint32_t const lane = threadIdx.x & 31, sub = lane & 3, grp = lane >> 2;
   uint32_t const chunks_row = pk / 256, tasks = m * chunks_row;  // below 2^32 for every accepted shape
   uint32_t const warps = gridDim.x * (kThreads / 32);
   uint32_t task = blockIdx.x * (kThreads / 32) + threadIdx.x / 32;
+  if (task < tasks && lane * 8 % (128 / sizeof(T)) == 0) {
+    uint32_t const col = task % chunks_row * 256 + lane * 8;
+    if (col < k) prefetch_line(in + uint64_t(task / chunks_row) * k + col);
+  }
+  pdl_wait();               // the input may come from the kernel before this one
+  pdl_launch_dependents();  // the projection that follows may start prefetching its weights (after the wait: the
+                            // next launch never runs beside anything older than this one)
   float x[8], next[8];
   auto load = [&](uint32_t t, float (&to)[8]) { load8<T, Vec>(in + uint64_t(t / chunks_row) * k, t % chunks_row * 256 + lane * 8, k, to); };
   if (task < tasks) load(task, x);
@@ -118,9 +122,10 @@ __global__ void __launch_bounds__(Held ? kRmsHeldColumns / 8 : kThreads) hidden_
                                                                                              int8_t* codes, float* scales,
                                                                                              int32_t* sums, int* failure) {
   extern __shared__ __align__(16) uint8_t row[];
+  const float* const x = residual + uint64_t(blockIdx.x) * hidden;
+  rms_prefetch(x, gamma, hidden);
   pdl_wait();
   pdl_launch_dependents();
-  const float* const x = residual + uint64_t(blockIdx.x) * hidden;
   uint32_t const lane = threadIdx.x & 31, sub = lane & 3, grp = lane >> 2;
   uint64_t const group0 = uint64_t(blockIdx.x) * (hidden / 32) + grp;
   float v[8];

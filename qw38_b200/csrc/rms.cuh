@@ -36,6 +36,13 @@ inline bool rms_vector_rows(const float* residual, const uint16_t* gamma) {
   return (reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(gamma)) % 16 == 0;  // rows are multiples of 1024 bytes
 }
 
+// Asks L2 for a thread's share; before the wait for what writes the row.
+__device__ __forceinline__ void rms_prefetch(const float* x, const uint16_t* gamma, uint32_t hidden) {
+  uint32_t const col = threadIdx.x * 8;
+  if (col < hidden && threadIdx.x % 4 == 0) prefetch_line(x + col);
+  if (col < hidden && threadIdx.x % 8 == 0) prefetch_line(gamma + col);
+}
+
 // Thread t's columns 8t .. 8t + 7 as bf16 values in v (zeros beyond the row); scaled: shared memory, hidden floats.  vec: row and gain are
 // 16-byte aligned.
 __device__ __forceinline__ void rms_row_held(const float* x, const uint16_t* gamma, float eps, uint32_t hidden, bool vec, float* scaled,

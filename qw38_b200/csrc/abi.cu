@@ -258,6 +258,10 @@ constexpr uint64_t kI8SuperBlocks = 12288;
 bool mmv_i8_better(const q4k::WeightView& w, const q4k::Q8View& x) {
   return x.m > 8 && uint64_t(w.padded_n / 8) * w.tiles_k >= kI8SuperBlocks && q4k::mmv_i8_supported(w, x);
 }
+// One token's gate / up pair on dp4a, from this many super-blocks of one of them on.  MLP chains, us, TMA-streamed pair : dp4a pair: 5120 / 17408
+// 41.1 : 37.4, 2560 / 3584 13.1 : 11.4, 768 / 11008 14.9 : 11.4, 4096 / 1024 (2048 super-blocks) 13.1 : 12.2, 1024 / 4096 (2048) 10.6 : 10.0,
+// 1024 / 2048 (1024) 10.5 : 10.5, where the host sets the pace.
+constexpr uint64_t kDp4aPairSuperBlocks = 2048;
 // The fp16-plane kernel with scratch of its own (stream_scratch.cu).
 int project_f16(const q4k_weight& w, const q4k_q8_input& x, const q4k::F16Output& out, cudaStream_t stream, const q4k_weight* second = nullptr,
                 const q4k::RawRows* raw = nullptr) {
@@ -1311,6 +1315,7 @@ int q4k_q8_mlp(const q4k_weight* gate, const q4k_weight* up, const q4k_weight* d
   bool const fused = !pair_i8(gate, up, beside) && m <= q4k::kGemvTmaMaxTokens && q4k::gemv_tma_supported(view(*gate), view(xh)) &&
                      q4k::gemv_tma_supported(view(*up), view(xh)) && q4k::plan_gemv_tma_swiglu_q8(m, view(*gate), &fused_plan);
   if (!fused) xh = beside;
+  bool const dp4a = fused && uint64_t(ffn / 8) * (hidden / 256) >= kDp4aPairSuperBlocks && q4k::gemv_dp4a_swiglu_q8_supported(view(*gate), view(*up), m);
   q4k_q8_input xf{codes, scales, sums, uint64_t(m) * ffn, uint64_t(m) * (ffn / 32), uint64_t(m) * (ffn / 32), m, ffn, ffn};
   q4k_project_options opt{};
   opt.flags = kFlagTrustedSpans;  // every span was validated above
@@ -1331,7 +1336,8 @@ int q4k_q8_mlp(const q4k_weight* gate, const q4k_weight* up, const q4k_weight* d
     {
       ScopedRange range("qw38:op name=q4k_project m=%u n=%u k=%u role=%s residual=%u compute=%s", unsigned(m), unsigned(2 * ffn),
                         unsigned(hidden), "gate_up_swiglu_q8", 0u, "q8");
-      ce = q4k::launch_gemv_tma_swiglu_q8(view(*gate), view(*up), view(xh), out_view(xf), failure, fused_plan, status, stream);
+      ce = dp4a ? q4k::launch_gemv_dp4a_swiglu_q8(view(*gate), view(*up), view(xh), out_view(xf), failure, status, stream)
+                : q4k::launch_gemv_tma_swiglu_q8(view(*gate), view(*up), view(xh), out_view(xf), failure, fused_plan, status, stream);
     }
     if (ce != cudaSuccess) return bail(fail_cuda(ce, "q8.gate_up_swiglu_q8"));
   } else {

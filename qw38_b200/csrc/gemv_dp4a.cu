@@ -29,6 +29,7 @@
 #include "common.cuh"
 #include "launch.h"
 #include "q8_pack.cuh"
+#include "swiglu.cuh"
 #include "tma.cuh"
 
 namespace q4k {
@@ -67,6 +68,9 @@ struct DpParams {
   uint32_t wide;                // weights are 16-byte aligned: bulk copies
   uint32_t early;               // weights may be read before the preceding launch has ended
   uint32_t input_settled;       // so may the activations
+  int8_t* q8_codes;             // Quant: the activation of the down projection
+  float* q8_scales;
+  int32_t* q8_sums;
 };
 
 __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
@@ -116,7 +120,10 @@ __device__ __forceinline__ uint32_t stage_units(const DpParams& p, uint32_t u, u
 // Shared memory: rings [warp][stage][codes | metadata], activations [token][super-block][half of a group][group][16 B],
 // {a, a * sum} [token][group], row sums [warp][part][row][token], barriers, the warps' first super-blocks and row groups,
 // abort flag.
-template <int M, bool Dump, bool Raw>
+// Quant: a gate / up pair, seg[0] and seg[1].  A block takes groups of 32 rows, four row groups of gate and four of up in turn, cut at even
+// super-blocks (a stage then never spans both), and quantises bf16(silu(gate) * up) when its rows are complete (four groups of 32
+// at most for a mean of 3.7 at 17408 rows).
+template <int M, bool Dump, bool Raw, bool Quant>
 __global__ void __launch_bounds__(kThreads, M <= 2 ? 2 : 1) gemv_dp4a_kernel(const __grid_constant__ DpParams p) {
   extern __shared__ __align__(128) uint8_t smem[];
   uint32_t const tiles_k = p.tiles_k, G = tiles_k * 8;
@@ -132,23 +139,35 @@ __global__ void __launch_bounds__(kThreads, M <= 2 ? 2 : 1) gemv_dp4a_kernel(con
   uint32_t* const firsts = cuts + kWarps + 1;
   volatile int* const abort_flag = reinterpret_cast<volatile int*>(firsts + kWarps);
 
-  uint32_t const rg_first = blockIdx.x * p.rgs_each + min(blockIdx.x, p.rgs_rest);
-  uint32_t const rg_count = p.rgs_each + (blockIdx.x < p.rgs_rest ? 1u : 0u);
+  uint32_t const rg_first = blockIdx.x * p.rgs_each + min(blockIdx.x, p.rgs_rest);  // Quant: first group
+  uint32_t const rg_count = (p.rgs_each + (blockIdx.x < p.rgs_rest ? 1u : 0u)) * (Quant ? 8u : 1u);
   uint32_t const units = rg_count * tiles_k;
 
   if (warp < kWarps) {
-    uint32_t const base = rg_first * tiles_k, c0 = units * warp / kWarps;
-    uint32_t const u0 = base + c0, u1 = base + units * (warp + 1) / kWarps;
+    constexpr uint32_t kCut = Quant ? ~1u : ~0u;
+    uint32_t const base = Quant ? 0u : rg_first * tiles_k, c0 = units * warp / kWarps & kCut;
+    uint32_t const u0 = base + c0, u1 = base + (units * (warp + 1) / kWarps & kCut);
+    // Super-blocks of the stage that starts at u, and where they lie.
+    auto count_at = [&](uint32_t u) { return Quant ? kStageUnits : stage_units(p, u, u1); };
+    auto place = [&](uint32_t u, const DpSegment*& s) -> uint64_t {
+      if constexpr (Quant) {
+        uint32_t const run = 4 * tiles_k, c = u / run;
+        s = &p.seg[c & 1u];
+        return uint64_t(rg_first + (c >> 1)) * run + (u - c * run);
+      }
+      s = &segment_of(p, u);
+      return u - s->u0;
+    };
     // lane 0 keeps the ring full: stage `ps` takes the super-blocks from `pu` on
     uint32_t pu = u0, ps = 0;
     auto fetch = [&] {
-      uint32_t const count = stage_units(p, pu, u1);
-      DpSegment const& s = segment_of(p, pu);
-      uint64_t const at = pu - s.u0;
+      uint32_t const count = count_at(pu);
+      const DpSegment* s;
+      uint64_t const at = place(pu, s);
       uint32_t const dst = s_ring + ps * kStageBytes, bar = bars + ps * 8;
       mbar_expect_tx(bar, count * 1152);
-      bulk_copy(dst, s.codes + at * 1024, count * 1024, bar);
-      bulk_copy(dst + kStageUnits * 1024, s.meta + at * 128, count * 128, bar);
+      bulk_copy(dst, s->codes + at * 1024, count * 1024, bar);
+      bulk_copy(dst + kStageUnits * 1024, s->meta + at * 128, count * 128, bar);
       pu += count;
       ps = ps + 1 == p.stages ? 0 : ps + 1;
     };
@@ -162,10 +181,11 @@ __global__ void __launch_bounds__(kThreads, M <= 2 ? 2 : 1) gemv_dp4a_kernel(con
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         if (!p.early)  // the first stages come out of L2 after the wait (two: more get in the way of the kernel before)
           for (uint32_t i = 0, u = u0; i < 2 && u < u1; ++i) {
-            uint32_t const count = stage_units(p, u, u1);
-            DpSegment const& s = segment_of(p, u);
-            prefetch_l2(s.codes + uint64_t(u - s.u0) * 1024, count * 1024);
-            prefetch_l2(s.meta + uint64_t(u - s.u0) * 128, count * 128);
+            uint32_t const count = count_at(u);
+            const DpSegment* s;
+            uint64_t const at = place(u, s);
+            prefetch_l2(s->codes + at * 1024, count * 1024);
+            prefetch_l2(s->meta + at * 128, count * 128);
             u += count;
           }
       }
@@ -284,11 +304,11 @@ __global__ void __launch_bounds__(kThreads, M <= 2 ? 2 : 1) gemv_dp4a_kernel(con
     for (int t = 0; t < M; ++t) acc[t] = 0.f;
     uint32_t kb = u0 % tiles_k, part = 0, st = 0, phase = 0, u = u0;
     while (u < u1) {
-      uint32_t const count = stage_units(p, u, u1), stage = s_ring + st * kStageBytes;
+      uint32_t const count = count_at(u), stage = s_ring + st * kStageBytes;
       if (p.wide) {
         bool const ready = mbar_wait(bars + st * 8, phase, abort_flag, p.status, 0x110);
         if (!__all_sync(0xffffffffu, ready)) break;
-      } else {
+      } else if constexpr (!Quant) {
         DpSegment const& s = segment_of(p, u);
         uint64_t const at = u - s.u0;
         const uint32_t* const c32 = reinterpret_cast<const uint32_t*>(s.codes + at * 1024);
@@ -357,7 +377,7 @@ __global__ void __launch_bounds__(kThreads, M <= 2 ? 2 : 1) gemv_dp4a_kernel(con
   } else {
     // Control warp: once everything before this launch is complete, the next launch may start beside it.  Meanwhile it asks L2 for the
     // residual of the block's rows and for its share of the bf16 rows.
-    for (uint32_t i = lane; i < rg_count * M; i += 32) {
+    for (uint32_t i = lane; !Quant && i < rg_count * M; i += 32) {
       uint32_t const rg = i / M;
       DpSegment const& s = segment_of(p, (rg_first + rg) * tiles_k);
       if (s.residual) prefetch_line(s.residual + uint64_t(i % M) * s.n + (rg_first + rg - s.rg0) * 8);
@@ -371,10 +391,11 @@ __global__ void __launch_bounds__(kThreads, M <= 2 ? 2 : 1) gemv_dp4a_kernel(con
   if (*abort_flag) return;
   pdl_wait();
   // Thread (row group, row, token) adds the parts of the warps that worked on its row group, in warp order.
+  float* const rows = reinterpret_cast<float*>(smem);  // Quant: over the rings, whose copies have all been read
   for (uint32_t i = threadIdx.x; i < rg_count * 8 * M; i += kThreads) {
     uint32_t const t = i % M, r = (i / M) % 8, rg = i / (8 * M);
-    DpSegment const& s = segment_of(p, (rg_first + rg) * tiles_k);
-    uint32_t const row = (rg_first + rg - s.rg0) * 8 + r;
+    DpSegment const& s = Quant ? p.seg[0] : segment_of(p, (rg_first + rg) * tiles_k);
+    uint32_t const row = Quant ? 0u : (rg_first + rg - s.rg0) * 8 + r;
     if (row >= s.n) continue;
     uint32_t const x0 = rg * tiles_k, x1 = x0 + tiles_k;
     const float* const mine = red + r * M + t;
@@ -382,18 +403,45 @@ __global__ void __launch_bounds__(kThreads, M <= 2 ? 2 : 1) gemv_dp4a_kernel(con
 #pragma unroll
     for (uint32_t w = 0; w < kWarps; ++w)
       if (max(cuts[w], x0) < min(cuts[w + 1], x1)) v += mine[(w * p.parts + rg - firsts[w]) * 8 * M];
+    if constexpr (Quant) {
+      rows[i] = v;
+      continue;
+    }
     uint64_t const o = uint64_t(t) * s.n + row;
     if (s.residual) v += s.residual[o];
     if (s.out_bf16) s.out_bf16[o] = f32_to_bf16_rne(v);
     else s.out[o] = v;
   }
+  if constexpr (Quant) {  // four lanes per group of 32 rows, a row group each
+    __syncthreads();
+    uint32_t const sub = lane & 3, groups = rg_count / 8;
+    for (uint32_t g0 = warp * 8; g0 < groups; g0 += kThreads / 4) {
+      uint32_t const g = min(g0 + (lane >> 2), groups - 1);
+      const float* const src = rows + (g * 8 + sub) * 8;
+      float a[8], b[8], x[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) { a[i] = src[i]; b[i] = src[32 + i]; }
+      swiglu8(a, b, x);
+      Packed8 const z = quantize8(x);
+      if (g0 + (lane >> 2) >= groups) continue;
+      uint32_t* const dst = reinterpret_cast<uint32_t*>(p.q8_codes + (rg_first + g) * 32 + sub * 8);
+      dst[0] = z.w0;
+      dst[1] = z.w1;
+      if (sub == 0) {
+        p.q8_scales[rg_first + g] = z.a;
+        p.q8_sums[rg_first + g] = z.sum;
+        if (!z.valid) atomicExch(p.failure, 1);
+      }
+    }
+  }
 }
 
 template <int M>
 cudaError_t launch_m(const DpParams& p, uint32_t grid, uint32_t smem, cudaStream_t stream) {
-  auto kernel = p.partials ? gemv_dp4a_kernel<M, true, false> : gemv_dp4a_kernel<M, false, false>;
+  auto kernel = p.partials ? gemv_dp4a_kernel<M, true, false, false> : gemv_dp4a_kernel<M, false, false, false>;
   if constexpr (M <= kGemvDp4aBestTokens) {
-    if (p.raw) kernel = gemv_dp4a_kernel<M, false, true>;
+    if (p.raw) kernel = gemv_dp4a_kernel<M, false, true, false>;
+    if (p.q8_codes) kernel = gemv_dp4a_kernel<M, false, false, true>;
   }
   cudaError_t st = allow_smem(reinterpret_cast<const void*>(kernel), int(smem), true);
   if (st != cudaSuccess) return st;
@@ -410,6 +458,8 @@ cudaError_t launch_split(DpParams p, uint32_t m, uint32_t padded_k, cudaStream_t
     p.seg[i].u0 = p.rgs * p.tiles_k;
     p.rgs += (p.seg[i].n + 7) / 8;
   }
+  uint32_t const each = p.q8_codes ? 8 : 1;  // a pair goes by groups of 32 rows of either
+  p.rgs /= each;
   // One token: blocks that fill half an SM each are put on 139 to 145 of the 148 SMs, two on some, and those end last.  Where the input may
   // come from the launch before, no block of this kernel computes beside another launch's, so a block asks for more than half of an SM's shared memory
   // and gets the SM to itself: pack and 17408 x 5120 in a replayed graph 18.0 -> 12.0 us, 5120 x 5120 8.9 -> 7.0, MLP 5120 / 17408 49.1 ->
@@ -422,12 +472,12 @@ cudaError_t launch_split(DpParams p, uint32_t m, uint32_t padded_k, cudaStream_t
   constexpr uint64_t kSharedUnits = 320;
   uint32_t const sms = uint32_t(sm_count());
   bool const shared = p.raw && (m > 1 || uint64_t(p.rgs) * p.tiles_k >= kSharedUnits * sms), spread = m == 1 && !p.input_settled && !shared;
-  uint32_t const slots = sms * (shared ? 2 : 1), waves = (p.rgs + slots * kMaxRowGroups - 1) / (slots * kMaxRowGroups);
+  uint32_t const slots = sms * (shared ? 2 : 1), waves = (p.rgs * each + slots * kMaxRowGroups - 1) / (slots * kMaxRowGroups);
   uint32_t const grid = p.rgs < slots * waves ? p.rgs : slots * waves;
   p.rgs_each = p.rgs / grid;
   p.rgs_rest = p.rgs % grid;
-  uint32_t const units = (p.rgs_each + (p.rgs_rest ? 1 : 0)) * p.tiles_k;
-  p.parts = ((units + kWarps - 1) / kWarps + p.tiles_k - 2) / p.tiles_k + 1;  // row groups that a run can touch
+  uint32_t const units = (p.rgs_each + (p.rgs_rest ? 1 : 0)) * each * p.tiles_k;
+  p.parts = ((units + kWarps - 1) / kWarps + each / 8 + p.tiles_k - 2) / p.tiles_k + 1;  // row groups that a run can touch
   uint32_t const fixed = m * p.tiles_k * 320 + kWarps * p.parts * 8 * m * 4 + (2 * kWarps + 2) * 4, stage = kWarps * (kStageBytes + 8);
   // Up to two tokens the next launch gets the other half of the SM, unless that would leave less than two stages.  With settled inputs every
   // other launch of a thread asks for a little more than half and the ones between for a little less: neither two of the former fit an SM
@@ -481,6 +531,23 @@ cudaError_t launch_gemv_dp4a_multi(const WeightView* ws, const GemvTmaOutput* ou
   p.vec = raw.k % 8 == 0 && reinterpret_cast<uintptr_t>(raw.x) % 16 == 0;
   p.status = status;
   return launch_split(p, m, padded_k, stream);
+}
+
+bool gemv_dp4a_swiglu_q8_supported(const WeightView& gate, const WeightView& up, uint32_t m) {
+  return m == 1 && gate.n == up.n && gate.n % 32 == 0 && gate.tiles_k == up.tiles_k && aligned16(gate) && aligned16(up);
+}
+
+cudaError_t launch_gemv_dp4a_swiglu_q8(const WeightView& gate, const WeightView& up, const Q8View& x, Q8Out out, int* failure, int* status,
+                                       cudaStream_t stream) {
+  if (!gemv_dp4a_swiglu_q8_supported(gate, up, x.m)) return cudaErrorInvalidValue;
+  DpParams p{};
+  const WeightView* const ws[2] = {&gate, &up};
+  for (int i = 0; i < 2; ++i) p.seg[i] = DpSegment{ws[i]->codes, ws[i]->meta, nullptr, nullptr, nullptr, ws[i]->n, 0, 0};
+  p.nseg = 2;
+  p.codes = x.codes; p.scales = x.scales; p.sums = x.sums;
+  p.q8_codes = out.codes; p.q8_scales = out.scales; p.q8_sums = out.sums;
+  p.failure = failure; p.status = status; p.wide = 1;
+  return launch_split(p, 1, x.padded_k, stream);
 }
 
 }  // namespace q4k

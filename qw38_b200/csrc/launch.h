@@ -168,6 +168,10 @@ struct GemvTmaOutput {
 // The same projections (no SwiGLU pair) from bf16 rows on dp4a, in gemv_dp4a.cu: m <= kGemvDp4aBestTokens.
 cudaError_t launch_gemv_dp4a_multi(const WeightView* ws, const GemvTmaOutput* outs, uint32_t count, uint32_t m, uint32_t padded_k,
                                    const RawRows& raw, int* status, cudaStream_t stream);
+// The gate / up pair of an MLP for one token, whose Q8 activation for the down projection it writes (as launch_gemv_tma_swiglu_q8 below).
+bool gemv_dp4a_swiglu_q8_supported(const WeightView& gate, const WeightView& up, uint32_t m);
+cudaError_t launch_gemv_dp4a_swiglu_q8(const WeightView& gate, const WeightView& up, const Q8View& x, Q8Out out, int* failure, int* status,
+                                       cudaStream_t stream);
 cudaError_t launch_gemv_tma_multi(const WeightView* ws, const GemvTmaOutput* outs, uint32_t count, bool swiglu_pair, const Q8View& x,
                                   const GemvTmaPlan& plan, void* slices, uint32_t* tickets, int* status, cudaStream_t stream,
                                   const RawRows* raw = nullptr);
